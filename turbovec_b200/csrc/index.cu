@@ -724,7 +724,6 @@ struct MaskSpec {
     bool any() const { return bool_host || words_host || words_device || slots_host || ids_host || prepared; }
 };
 
-int candidate_capacity(size_t k) { return k <= 512 ? 4096 : 8192; }
 constexpr size_t kPageK = 4096;            // most results one selection pass keeps per query; larger k runs in pages
 
 // Takes a search context from the handle's pool for the duration of a call.
@@ -754,7 +753,7 @@ struct SearchScratch {
     uint32_t *wfrag;
     uint8_t *luts;
     uint64_t *cand, *thr, *topk, *lo;      // lo: lowest admissible key per query (paged top-k), or nullptr
-    uint32_t *cnt;
+    uint32_t *cnt, *done;                  // done follows cnt: both are cleared together
     size_t w_rows, dim_pad, lut_pitch;
     int cap;
     bool allow_tc;
@@ -965,7 +964,7 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
     const size_t n_blocks = (n + kBlock - 1) / kBlock;
     const int mt_total = int((nq + 15) / 16);
     CandidateBuffers cb{};
-    cb.cand = S.cand; cb.cnt = S.cnt; cb.thr = S.thr; cb.topk = S.topk; cb.lo = S.lo;
+    cb.cand = S.cand; cb.cnt = S.cnt; cb.done = S.done; cb.thr = S.thr; cb.topk = S.topk; cb.lo = S.lo;
     cb.overflow = d_overflow; cb.error = d_error; cb.cap = S.cap; cb.k = int(kk);
 
     ScanParams sp = base_scan_params(h, mode);
@@ -979,7 +978,7 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
         if (rc != TV_OK) return rc;
     }
 
-    TV_CUDA(cudaMemsetAsync(S.cnt, 0, nq * 4, st));
+    TV_CUDA(cudaMemsetAsync(S.cnt, 0, 2 * nq * 4, st));
     TV_CUDA(cudaMemsetAsync(S.thr, 0xff, nq * 8, st));
     TV_CUDA(cudaMemsetAsync(S.topk, 0xff, nq * kk * 8, st));
     // Chunk 0 holds at most `cap` vectors, so every one of them may pass.  Later chunks grow so that the
@@ -1001,9 +1000,9 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
         }
         const size_t end = std::min(n_blocks, begin + len);
         sp.pos_begin = uint32_t(begin); sp.pos_end = uint32_t(end);
-        // first chunk on the tensor-memory path without a filter (the host then knows how many vectors
-        // the chunk holds): every key is written in place, nothing is counted
-        const bool dense = plan.use_tc && stage == 0 && !careful && m.words == nullptr && S.lo == nullptr;
+        // first chunk: nothing is dismissed, so every key is written in place and nothing is counted.  The sorting
+        // selection of large k takes the number of keys from the host, which does not know it under a filter.
+        const bool dense = stage == 0 && !careful && S.lo == nullptr && (int(kk) <= kSelectMaxK || (plan.use_tc && m.words == nullptr));
         sp.dense = dense ? 1 : 0;
         ++stage;
         if (plan.use_tc) {
@@ -1050,7 +1049,7 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
                 h->launches++;
             }
         }
-        TV_CUDA(launch_select(cb, int(nq), dense ? int((end - sp.pos_begin) * kBlock) : 0, st));
+        TV_CUDA(launch_select(cb, int(nq), dense ? uint32_t(end) : 0u, m.n_live, st));
         h->launches++;
         begin = end;
     }
@@ -1127,7 +1126,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     // r - 1 (keys are unique: they carry the slot), one full scan each.  Exact for any k <= len, slow by design.
     const size_t pages = (kk + kPageK - 1) / kPageK;
     const size_t k_page = pages == 1 ? kk : kPageK;
-    const int cap = candidate_capacity(k_page);
+    const int cap = candidate_capacity(k_page, nq, n);
     const size_t nq_pad = (nq + 15) / 16 * 16;
     const int mt_total = int(nq_pad / 16);
     const size_t dim_pad = (dim + 127) / 128 * 128;
@@ -1152,7 +1151,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         TV_CUDA(c.d_luts.reserve(w_rows * lut_pitch));           // padded to whole query groups and whole K slabs for the tensor path
     }
     TV_CUDA(c.d_cand.reserve(nq * size_t(cap)));
-    TV_CUDA(c.d_cnt.reserve(nq));
+    TV_CUDA(c.d_cnt.reserve(2 * nq));                            // candidate counts, then the selection's part counters
     TV_CUDA(c.d_thr.reserve(nq));
     TV_CUDA(c.d_topk.reserve(nq * k_page));
     if (pages > 1) {
@@ -1167,7 +1166,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     SearchScratch S{};
     S.q_rot = c.d_qrot.ptr; S.qscale = c.d_qscale.ptr; S.qbias = c.d_qbias.ptr; S.weights = c.d_weights.ptr;
     S.wfrag = c.d_wfrag.ptr; S.luts = c.d_luts.ptr; S.cand = c.d_cand.ptr; S.thr = c.d_thr.ptr; S.topk = c.d_topk.ptr;
-    S.cnt = c.d_cnt.ptr; S.lo = nullptr; S.w_rows = w_rows; S.dim_pad = dim_pad; S.lut_pitch = lut_pitch; S.cap = cap; S.allow_tc = pages == 1;
+    S.cnt = c.d_cnt.ptr; S.done = c.d_cnt.ptr + nq; S.lo = nullptr; S.w_rows = w_rows; S.dim_pad = dim_pad; S.lut_pitch = lut_pitch; S.cap = cap; S.allow_tc = pages == 1;
     {
         ScanParams probe = base_scan_params(h, mode);
         plan.use_small = h->small_scan >= 0 && mode == TV_SCORE_PERMUTE_DOT && scan_small_supported(probe, int(nq), h->smem_limit);
@@ -1920,7 +1919,7 @@ NoAllocLayout carve_noalloc(unsigned char *base) {
     L.cand = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * kNoAllocCap * 8));           // 256 KiB
     L.thr = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * 8));
     L.topk = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * kNoAllocMaxK * 8));          //   8 KiB
-    L.cnt = reinterpret_cast<uint32_t *>(take(kNoAllocMaxQueries * 4));
+    L.cnt = reinterpret_cast<uint32_t *>(take(2 * kNoAllocMaxQueries * 4));
     static_assert(kNoAllocMaxQueries * kNoAllocMaxDim * 4 + 16 * kNoAllocMaxDim + (kNoAllocMaxDim / 32) * 512 +
                           kNoAllocMaxQueries * (kNoAllocMaxDim / 2) * 32 + kNoAllocMaxQueries * kNoAllocCap * 8 +
                           kNoAllocMaxQueries * kNoAllocMaxK * 8 + 8 * 256 <= kNoAllocScratchBytes,
@@ -1964,7 +1963,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
 
     SearchScratch S{};
     S.q_rot = L.q_rot; S.qscale = L.qscale; S.qbias = L.qbias; S.weights = L.weights; S.wfrag = L.wfrag; S.luts = L.luts;
-    S.cand = L.cand; S.thr = L.thr; S.topk = L.topk; S.cnt = L.cnt; S.lo = nullptr;
+    S.cand = L.cand; S.thr = L.thr; S.topk = L.topk; S.cnt = L.cnt; S.done = L.cnt + nq; S.lo = nullptr;
     S.w_rows = 16; S.dim_pad = kNoAllocMaxDim; S.lut_pitch = size_t((ng + 3) / 4 * 4) * 32; S.cap = int(kNoAllocCap); S.allow_tc = false;
     {
         ScanParams probe = base_scan_params(h, mode);

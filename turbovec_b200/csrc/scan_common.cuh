@@ -22,6 +22,16 @@ __device__ __forceinline__ void push_candidate(const CandidateBuffers &cb, int q
     }
 }
 
+// First chunk of a search (ScanParams::dense): `emit` calls its argument with (query, lane of the block, searched, score,
+// slot) for every key of the block at position `pos`; the keys go to the list position of their place in the chunk.
+template <typename F>
+__device__ __forceinline__ void write_block(const ScanParams &p, uint32_t pos, F emit) {
+    const size_t at = size_t(pos - p.pos_begin) * kLanes;
+    emit([&](int q, int vl, bool on, float score, uint32_t slot) {
+        p.cb.cand[size_t(q) * p.cb.cap + at + vl] = on ? make_key(score, slot) : kEmptyKey;
+    });
+}
+
 // =====================================================================================================
 // PTX helpers: mbarrier + bulk asynchronous copy (no multicast), warp-level int8 MMA
 // =====================================================================================================

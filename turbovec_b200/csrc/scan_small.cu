@@ -208,6 +208,24 @@ scan_small_kernel(ScanParams p, const int8_t *__restrict__ weights, int pitch, c
         if (!ok) break;
 
         // ---- epilogue: accumulator (row, column) = (vector, query) ----
+        auto score_of = [&](int nt, int m, int hrow, int c) {
+            const int isum = accp[nt][m][2 * hrow + c] - accn[nt][m][2 * hrow + c];
+            return __fmul_rn(fmaf(float(isum), qs[nt][c], qb[nt][c]), vs[2 * m + hrow]);
+        };
+        if (p.dense) {
+            // first chunk: every key of the block goes to the list position of its place in the chunk
+            write_block(p, pos, [&](auto put) {
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int m = e >> 2, hrow = (e >> 1) & 1, c = e & 1;
+                        const int vl = 16 * m + 8 * hrow + quad, q = 8 * nt + 2 * t + c;
+                        if (q < p.nq) put(p.q_base + q, vl, base + vl < p.n && ((allow >> vl) & 1u), score_of(nt, m, hrow, c), uint32_t(base + vl));
+                    }
+            });
+            continue;
+        }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -220,9 +238,7 @@ scan_small_kernel(ScanParams p, const int8_t *__restrict__ weights, int pitch, c
                     for (int c = 0; c < 2; ++c) {
                         const int q = 8 * nt + 2 * t + c;
                         if (q >= p.nq) continue;
-                        const int isum = accp[nt][m][2 * hrow + c] - accn[nt][m][2 * hrow + c];
-                        const float score = __fmul_rn(fmaf(float(isum), qs[nt][c], qb[nt][c]), vs[2 * m + hrow]);
-                        push_candidate(p.cb, p.q_base + q, score, uint32_t(base + vl), thr[nt][c], lo[nt][c]);
+                        push_candidate(p.cb, p.q_base + q, score_of(nt, m, hrow, c), uint32_t(base + vl), thr[nt][c], lo[nt][c]);
                     }
                 }
     }

@@ -350,27 +350,30 @@ scan_pd_kernel(ScanParams p) {
             }
             uint32_t allow = 0xffffffffu;
             if (p.mask) allow = reinterpret_cast<const uint32_t *>(p.mask)[blk];
+            write_block(p, pos, [&](auto put) {
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
+                for (int m = 0; m < MT; ++m) {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int ql = 16 * (p.mtile_base + m) + quad + 8 * half;   // query within the prepared batch
-                    if (ql >= p.q_base + p.nq) continue;
-                    const float qs = p.qscale[ql], qb = p.qbias[ql];
-                    const uint64_t thr = p.cb.thr[ql], lo = p.cb.lo ? p.cb.lo[ql] : 0ull;
+                    for (int half = 0; half < 2; ++half) {
+                        const int ql = 16 * (p.mtile_base + m) + quad + 8 * half;   // query within the prepared batch
+                        if (ql >= p.q_base + p.nq) continue;
+                        const float qs = p.qscale[ql], qb = p.qbias[ql];
+                        const uint64_t thr = p.cb.thr[ql], lo = p.cb.lo ? p.cb.lo[ql] : 0ull;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                        for (int j = 0; j < 4; ++j) {
 #pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const int vl = 8 * j + 2 * t + c;
-                            if (base + vl >= p.n || !((allow >> vl) & 1u)) continue;
-                            const int isum = SPLIT ? acc[m][j][2 * half + c] - accn[SPLIT ? m : 0][j][2 * half + c] : acc[m][j][2 * half + c];
-                            const float score = __fmul_rn(fmaf(float(isum), qs, qb), vs[2 * j + c]);
-                            push_candidate(p.cb, ql, score, uint32_t(base + vl), thr, lo);
+                            for (int c = 0; c < 2; ++c) {
+                                const int vl = 8 * j + 2 * t + c;
+                                const bool on = base + vl < p.n && ((allow >> vl) & 1u);
+                                const int isum = SPLIT ? acc[m][j][2 * half + c] - accn[SPLIT ? m : 0][j][2 * half + c] : acc[m][j][2 * half + c];
+                                const float score = __fmul_rn(fmaf(float(isum), qs, qb), vs[2 * j + c]);
+                                if (p.dense) put(ql, vl, on, score, uint32_t(base + vl));
+                                else if (on) push_candidate(p.cb, ql, score, uint32_t(base + vl), thr, lo);
+                            }
                         }
                     }
                 }
-            }
+            });
         }
     }
 }
@@ -457,6 +460,20 @@ __global__ void __launch_bounds__(256) scan_lut_kernel(ScanParams p) {
                 total[q] += mine;
             }
         }
+        auto score_of = [&](int q, float vs) {
+            const float pre = p.mode == kModeLutFlush ? facc[q] : __fadd_rn(__fmul_rn(float(int(total[q])), qs[q]), qb[q]);
+            return __fmul_rn(pre, vs);
+        };
+        if (p.dense) {
+            const bool on = slot < p.n && (!p.mask || ((p.mask[slot >> 6] >> (slot & 63)) & 1ull));
+            const float vs = on ? p.vec_scales[slot] : 0.0f;
+            write_block(p, pos, [&](auto put) {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                    if (q < nq_here) put(p.q_base + q, my_vec, on, score_of(q, vs), uint32_t(slot));
+            });
+            continue;
+        }
         if (slot < p.n) {
             const bool allowed = !p.mask || ((p.mask[slot >> 6] >> (slot & 63)) & 1ull);
             if (allowed) {
@@ -464,9 +481,7 @@ __global__ void __launch_bounds__(256) scan_lut_kernel(ScanParams p) {
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) {
                     if (q >= nq_here) break;
-                    const float pre = p.mode == kModeLutFlush ? facc[q]
-                                                              : __fadd_rn(__fmul_rn(float(int(total[q])), qs[q]), qb[q]);
-                    push_candidate(p.cb, p.q_base + q, __fmul_rn(pre, vs), uint32_t(slot), thr[q], lo[q]);
+                    push_candidate(p.cb, p.q_base + q, score_of(q, vs), uint32_t(slot), thr[q], lo[q]);
                 }
             }
         }
@@ -474,7 +489,7 @@ __global__ void __launch_bounds__(256) scan_lut_kernel(ScanParams p) {
 }
 
 // =====================================================================================================
-// Selection: one CTA per query merges the previous top-k with the new candidates in shared memory.
+// Selection for k above kSelectMaxK (smaller k: select.cu): one CTA per query merges the previous top-k with the new candidates in shared memory.
 // With few entries it is a plain bitonic sort.  With many more entries than k it is a bitonic top-k: sort
 // runs of m = 2^ceil(log2 k) (at least 32) entries in alternating directions, then repeatedly take the
 // element-wise minimum of each ascending/descending pair of runs (the m smallest of the pair, as a bitonic
@@ -736,9 +751,8 @@ static int sort_capacity(int cap, int k) {
     while (n2 < cap + k) n2 <<= 1;
     return n2;
 }
-size_t select_smem_bytes(int cap, int k) { return size_t(sort_capacity(cap, k)) * 8; }
 
-cudaError_t launch_select(const CandidateBuffers &cb, int nq, int dense_count, cudaStream_t s) {
+cudaError_t launch_select_sort(const CandidateBuffers &cb, int nq, int dense_count, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
     const int sort_n = sort_capacity(cb.cap, cb.k);
     const size_t smem = size_t(sort_n) * 8;

@@ -64,11 +64,16 @@ struct CandidateBuffers {
     uint64_t *topk;
     uint32_t *overflow;
     uint32_t *error;               // device-side wait timeouts
+    uint32_t *done;                // per query: parts of a long list selected so far (zero between launches)
     int cap, k;
 };
-size_t select_smem_bytes(int cap, int k);
-// dense_count > 0: every query has exactly that many candidates (written without counting, ScanParams::dense).
-cudaError_t launch_select(const CandidateBuffers &cb, int nq, int dense_count, cudaStream_t s);
+// Selection (select.cu).  dense_blocks > 0: the scan wrote 32 keys for each of the first min(dense_blocks, *n_live)
+// positions (n_live == nullptr: dense_blocks) without counting them (ScanParams::dense).
+constexpr int kSelectMaxK = 512;       // larger k: the bitonic form in search.cu
+constexpr int kSelectSegment = 4096;   // keys one CTA selects from
+int candidate_capacity(size_t k, size_t nq, size_t n);
+cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blocks, const uint32_t *n_live, cudaStream_t s);
+cudaError_t launch_select_sort(const CandidateBuffers &cb, int nq, int dense_count, cudaStream_t s);
 // Result keys (score-descending image << 32 | slot) of a finished search, `offset` added to every slot.
 cudaError_t launch_export_keys(const uint64_t *topk, int64_t count, uint64_t offset, uint64_t *out, cudaStream_t s);
 // keys[n_lists][nq][k] -> per query the k best of all lists, decoded; n_lists * k at most kMergeMaxKeys.
@@ -95,8 +100,8 @@ struct ScanParams {
     const uint32_t *live_blocks;   // or nullptr: positions are block ids
     const uint32_t *n_live;        // device count of live_blocks (when live_blocks != nullptr)
     uint32_t pos_begin, pos_end;   // positions scanned by this launch
-    int dense;                     // tcgen05 scan only: write every key to cand[q][place in chunk] without counting
-                                   // (the chunk holds at most cb.cap vectors; the selection is told the count)
+    int dense;                     // write every key to cand[q][place in chunk] without counting, kEmptyKey for slots that
+                                   // are not searched (the chunk holds at most cb.cap vectors; the selection is told the count)
     CandidateBuffers cb;
     // permute-dot
     const uint32_t *wfrag;
