@@ -121,7 +121,8 @@ struct SearchCtx {
     DeviceFlags *d_flags = nullptr;
     DeviceFlags *h_flags = nullptr;
     DeviceArray<float> d_stage;              // query upload
-    DeviceArray<float> d_qrot, d_qscale, d_qbias;
+    DeviceArray<float> d_qrot;               // tv_rotate
+    DeviceArray<float> d_qscale, d_qbias;
     DeviceArray<uint8_t> d_luts;
     DeviceArray<int8_t> d_weights;
     DeviceArray<uint32_t> d_wfrag;
@@ -748,7 +749,7 @@ struct CtxLease {
 
 // The device buffers one search runs on: the context's arrays, or the fixed array of the allocation-free entry point.
 struct SearchScratch {
-    float *q_rot, *qscale, *qbias;
+    float *qscale, *qbias;
     int8_t *weights;
     uint32_t *wfrag;
     uint8_t *luts;
@@ -955,10 +956,11 @@ int expanded_sync(tv_index *h, cudaStream_t st, const uint32_t level_words[4], b
     return TV_OK;
 }
 
-// Query preparation, then scan + select over a geometric chunk schedule, all enqueued on `st`.
+// Scan + select over a geometric chunk schedule, all enqueued on `st`.
 //   careful: chunks never exceed the candidate capacity, so no list can overflow whatever the data order.
+//   fresh: the selection state is as query preparation left it.
 int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, const ScanPlan &plan, int mode,
-                   size_t nq, size_t kk, const MaskOnDevice &m, uint32_t *d_overflow, uint32_t *d_error, bool careful) {
+                   size_t nq, size_t kk, const MaskOnDevice &m, uint32_t *d_overflow, uint32_t *d_error, bool careful, bool fresh) {
     const size_t n = h->n;
     const int ng = h->ngroups;
     const size_t n_blocks = (n + kBlock - 1) / kBlock;
@@ -978,9 +980,11 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
         if (rc != TV_OK) return rc;
     }
 
-    TV_CUDA(cudaMemsetAsync(S.cnt, 0, 2 * nq * 4, st));
-    TV_CUDA(cudaMemsetAsync(S.thr, 0xff, nq * 8, st));
-    TV_CUDA(cudaMemsetAsync(S.topk, 0xff, nq * kk * 8, st));
+    if (!fresh) {
+        TV_CUDA(cudaMemsetAsync(S.cnt, 0, 2 * nq * 4, st));
+        TV_CUDA(cudaMemsetAsync(S.thr, 0xff, nq * 8, st));
+        TV_CUDA(cudaMemsetAsync(S.topk, 0xff, nq * kk * 8, st));
+    }
     // Chunk 0 holds at most `cap` vectors, so every one of them may pass.  Later chunks grow so that the
     // expected number of candidates per query, k * |chunk| / |seen|, stays near cap / 4.
     // The tensor-memory scan pays for dense candidates (its epilogue re-reads a 32 x 32 tile of scores
@@ -1056,8 +1060,9 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
     return TV_OK;
 }
 
+// Query operands, and the selection state of the batch as enqueue_search wants it (kk results per query).
 int enqueue_query_prep(tv_index *h, cudaStream_t st, const SearchScratch &S, const ScanPlan &plan, int mode, const float *dq,
-                       size_t nq, unsigned long long *d_first_invalid) {
+                       size_t nq, size_t kk, unsigned long long *d_first_invalid) {
     const size_t dim = h->dim;
     const int ng = h->ngroups;
     const int ksteps = (ng + 15) / 16;
@@ -1070,15 +1075,17 @@ int enqueue_query_prep(tv_index *h, cudaStream_t st, const SearchScratch &S, con
     qp.centroids = h->d_codebook.ptr + 16;
     if (!h->shift.empty()) { qp.shift = h->d_calib.ptr; qp.scale_tq = h->d_calib.ptr + dim; }
     qp.level_scale = h->level_scale;
-    qp.q_rot = S.q_rot; qp.qscale = S.qscale; qp.qbias = S.qbias;
+    qp.qscale = S.qscale; qp.qbias = S.qbias;
     qp.luts = S.luts; qp.lut_pitch = int(S.lut_pitch); qp.weights = S.weights; qp.dim_pad = int(S.dim_pad);
-    qp.wfrag = S.wfrag; qp.mtiles_total = mt_total;
+    qp.mtiles_total = mt_total;
     qp.first_invalid = d_first_invalid;
-    if (mode == TV_SCORE_PERMUTE_DOT) {
+    qp.cnt = S.cnt; qp.done = S.done; qp.thr = S.thr; qp.topk = S.topk; qp.k = int(kk);
+    // the tensor-memory scans read whole groups of 256 operand rows and whole K slabs
+    qp.pad_operands = plan.use_tc ? 1 : 0;
+    qp.rows = plan.use_tc ? int(S.w_rows) : int(nq);
+    if (mode == TV_SCORE_PERMUTE_DOT && !plan.use_tc && !plan.use_small) {    // only scan_pd_kernel reads the fragments
+        qp.wfrag = S.wfrag;
         TV_CUDA(cudaMemsetAsync(S.wfrag, 0, size_t(ksteps) * mt_total * 32 * 16, st));
-        if (plan.use_tc) TV_CUDA(cudaMemsetAsync(S.weights, 0, S.w_rows * S.dim_pad, st));
-    } else if (plan.use_tc) {
-        TV_CUDA(cudaMemsetAsync(S.luts, 0, S.w_rows * S.lut_pitch, st));
     }
     TV_CUDA(launch_query_prep(qp, st));
     h->launches++;
@@ -1140,7 +1147,6 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     // ---- buffers ----
     TV_CUDA(injected_failure(h));
     if (!queries_on_device) TV_CUDA(c.d_stage.reserve(nq * dim));
-    TV_CUDA(c.d_qrot.reserve(nq * dim));
     TV_CUDA(c.d_qscale.reserve(nq_pad));
     TV_CUDA(c.d_qbias.reserve(nq_pad));
     const size_t w_rows = (nq + 255) / 256 * 256;
@@ -1164,7 +1170,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     }
 
     SearchScratch S{};
-    S.q_rot = c.d_qrot.ptr; S.qscale = c.d_qscale.ptr; S.qbias = c.d_qbias.ptr; S.weights = c.d_weights.ptr;
+    S.qscale = c.d_qscale.ptr; S.qbias = c.d_qbias.ptr; S.weights = c.d_weights.ptr;
     S.wfrag = c.d_wfrag.ptr; S.luts = c.d_luts.ptr; S.cand = c.d_cand.ptr; S.thr = c.d_thr.ptr; S.topk = c.d_topk.ptr;
     S.cnt = c.d_cnt.ptr; S.done = c.d_cnt.ptr + nq; S.lo = nullptr; S.w_rows = w_rows; S.dim_pad = dim_pad; S.lut_pitch = lut_pitch; S.cap = cap; S.allow_tc = pages == 1;
     {
@@ -1197,7 +1203,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         if (rc != TV_OK) return rc;
     }
 
-    rc = enqueue_query_prep(h, st, S, plan, mode, dq, nq, &c.d_flags->first_invalid);
+    rc = enqueue_query_prep(h, st, S, plan, mode, dq, nq, k_page, &c.d_flags->first_invalid);
     if (rc != TV_OK) return rc;
 
     CandidateBuffers out_cb{};                                  // what finalize reads
@@ -1231,7 +1237,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         S.lo = page == 0 ? nullptr : c.d_floor.ptr;
         for (int attempt = 0; attempt < 2; ++attempt) {
             const bool careful = attempt == 1 || h->force_careful;
-            rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, k_this, m, &c.d_flags->overflow, &c.d_flags->error, careful);
+            rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, k_this, m, &c.d_flags->overflow, &c.d_flags->error, careful, page == 0 && attempt == 0);
             if (rc != TV_OK) { c.marks.used = 0; return rc; }
             if (pages == 1) {
                 rc = finish();                                  // the common case: one submission, one synchronisation
@@ -1899,7 +1905,7 @@ std::mutex g_noalloc_mu;                                 // one call at a time p
 void *g_noalloc_base[64] = {nullptr};                    // device address of the array, per device ordinal
 
 struct NoAllocLayout {
-    float *q_rot, *qscale, *qbias;
+    float *qscale, *qbias;
     int8_t *weights;
     uint32_t *wfrag;
     uint8_t *luts;
@@ -1910,7 +1916,6 @@ NoAllocLayout carve_noalloc(unsigned char *base) {
     NoAllocLayout L;
     size_t off = 0;
     auto take = [&](size_t bytes) { unsigned char *p = base + off; off += (bytes + 255) & ~size_t(255); return p; };
-    L.q_rot = reinterpret_cast<float *>(take(kNoAllocMaxQueries * kNoAllocMaxDim * 4));          // 128 KiB
     L.qscale = reinterpret_cast<float *>(take(16 * 4));
     L.qbias = reinterpret_cast<float *>(take(16 * 4));
     L.weights = reinterpret_cast<int8_t *>(take(16 * kNoAllocMaxDim));                           //  64 KiB
@@ -1920,7 +1925,7 @@ NoAllocLayout carve_noalloc(unsigned char *base) {
     L.thr = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * 8));
     L.topk = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * kNoAllocMaxK * 8));          //   8 KiB
     L.cnt = reinterpret_cast<uint32_t *>(take(2 * kNoAllocMaxQueries * 4));
-    static_assert(kNoAllocMaxQueries * kNoAllocMaxDim * 4 + 16 * kNoAllocMaxDim + (kNoAllocMaxDim / 32) * 512 +
+    static_assert(16 * kNoAllocMaxDim + (kNoAllocMaxDim / 32) * 512 +
                           kNoAllocMaxQueries * (kNoAllocMaxDim / 2) * 32 + kNoAllocMaxQueries * kNoAllocCap * 8 +
                           kNoAllocMaxQueries * kNoAllocMaxK * 8 + 8 * 256 <= kNoAllocScratchBytes,
                   "scratch layout exceeds the static array");
@@ -1962,7 +1967,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
     if (rc != TV_OK) return rc;
 
     SearchScratch S{};
-    S.q_rot = L.q_rot; S.qscale = L.qscale; S.qbias = L.qbias; S.weights = L.weights; S.wfrag = L.wfrag; S.luts = L.luts;
+    S.qscale = L.qscale; S.qbias = L.qbias; S.weights = L.weights; S.wfrag = L.wfrag; S.luts = L.luts;
     S.cand = L.cand; S.thr = L.thr; S.topk = L.topk; S.cnt = L.cnt; S.done = L.cnt + nq; S.lo = nullptr;
     S.w_rows = 16; S.dim_pad = kNoAllocMaxDim; S.lut_pitch = size_t((ng + 3) / 4 * 4) * 32; S.cap = int(kNoAllocCap); S.allow_tc = false;
     {
@@ -1984,7 +1989,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
 
     // The array still holds the previous call's data.  Query preparation clears the query operands it does not
     // overwrite, and the schedule resets counters, thresholds and result keys at its start.
-    rc = enqueue_query_prep(h, st, S, plan, mode, queries_device, nq, &c.d_flags->first_invalid);
+    rc = enqueue_query_prep(h, st, S, plan, mode, queries_device, nq, kk, &c.d_flags->first_invalid);
     if (rc != TV_OK) return rc;
     MaskOnDevice no_mask;
     CandidateBuffers out_cb{};
@@ -1994,7 +1999,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
     // capacity, which cannot overflow; neither schedule needs memory beyond the fixed array.
     for (int attempt = 0; attempt < 2; ++attempt) {
         const bool careful = attempt == 1 || h->force_careful;
-        rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, kk, no_mask, &c.d_flags->overflow, &c.d_flags->error, careful);
+        rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, kk, no_mask, &c.d_flags->overflow, &c.d_flags->error, careful, attempt == 0);
         if (rc != TV_OK) { c.marks.used = 0; return rc; }
         TV_CUDA(launch_finalize(out_cb, int(nq), nullptr, int64_t(n), scores_out_device, slots_out_device, &c.d_flags->k_eff, 0, st));
         h->launches++;
@@ -2406,7 +2411,7 @@ int tv_rotate(tv_index *h, const float *rows, size_t n, size_t dim, float *rotat
     TV_CUDA(c.d_luts.reserve(n * size_t((h->ngroups + 3) / 4 * 4) * 32));
     TV_CUDA(cudaMemcpyAsync(h->d_stage.ptr, rows, n * dim * 4, cudaMemcpyHostToDevice, st));
     QueryPrepParams qp{};
-    qp.queries = h->d_stage.ptr; qp.nq = int(n); qp.dim = int(dim); qp.bits = h->bits; qp.ngroups = h->ngroups;
+    qp.queries = h->d_stage.ptr; qp.nq = qp.rows = int(n); qp.dim = int(dim); qp.bits = h->bits; qp.ngroups = h->ngroups;
     qp.mode = kModeLutMulAdd;
     qp.perm0 = h->d_perm.ptr; qp.perm1 = h->d_perm.ptr + dim; qp.inv_sqrt_block = h->rot.inv_sqrt_block;
     qp.centroids = h->d_codebook.ptr + 16;

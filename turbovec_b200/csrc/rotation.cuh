@@ -57,15 +57,16 @@ __device__ __forceinline__ float gather_one(const float *src, uint16_t pk, bool 
 
 // One round for one row.  src and dst are distinct shared-memory rows of `dim` floats; perm is the
 // packed table (low 15 bits source index, bit 15 = negative sign).  LOG2B in 3..11 selects the
-// register paths, 12 the shared-memory path (valid for every B).
+// register paths, 12 the shared-memory path (valid for every B).  Several warps can share a row: warp `first` of `step`
+// takes the blocks first, first + step, ... (the shared-memory path runs on warp 0 alone).
 template <int LOG2B>
 __device__ __forceinline__ void rotation_round(const float *src, float *dst, const uint16_t *perm, int dim,
-                                               float inv_sqrt_block, bool use_inv, float inv, int lane) {
+                                               float inv_sqrt_block, bool use_inv, float inv, int lane, int first = 0, int step = 1) {
     if constexpr (LOG2B <= 4) {
         // 32 / B whole blocks per pass of the warp; B divides 32 and dim, so a ragged last pass still
         // holds whole blocks and the idle lanes only feed shuffles nobody reads
         constexpr int B = 1 << LOG2B;
-        for (int base = 0; base < dim; base += 32) {
+        for (int base = 32 * first; base < dim; base += 32 * step) {
             const int idx = base + lane;
             const bool active = idx < dim;
             float v[1] = {active ? gather_one(src, perm[idx], use_inv, inv) : 0.0f};
@@ -76,7 +77,7 @@ __device__ __forceinline__ void rotation_round(const float *src, float *dst, con
         constexpr int B = 1 << LOG2B;
         constexpr int R = B / 32;
         const int nblk = dim >> LOG2B;
-        for (int blk = 0; blk < nblk; ++blk) {
+        for (int blk = first; blk < nblk; blk += step) {
             const int base = blk * B + lane;
             float v[R];
 #pragma unroll
@@ -86,7 +87,7 @@ __device__ __forceinline__ void rotation_round(const float *src, float *dst, con
 #pragma unroll
             for (int r = 0; r < R; ++r) dst[base + r * 32] = __fmul_rn(v[r], inv_sqrt_block);
         }
-    } else {
+    } else if (first == 0) {
         const int B = dim & -dim;
         for (int i = lane; i < dim; i += 32) dst[i] = gather_one(src, perm[i], use_inv, inv);
         __syncwarp();

@@ -37,8 +37,82 @@ __device__ __forceinline__ int8_t round_clamp_i8(float v) {
     return int8_t(int(r));
 }
 
+// One CTA prepares one query; with few queries nothing else runs, so the length of its dependent chain is the cost.
+// The blocks of the rotation are spread over the warps, the tables of a half-byte (16 entries) belong to one thread,
+// which computes its entries from the products of its coordinates and stores them as one word, and the sequential bias
+// sum runs beside the table entries.  One query: dim 1536 4-bit 12.8 us before, dim 3072 2-bit 105 us before.
+// The CTA also resets its query's selection state and clears the operand padding that the tensor-memory scans read
+// (CTAs past the last query clear a whole row).
+template <int BITS>
+__device__ __forceinline__ void half_entries(const float *q, const float *centroids, float (&e)[16]) {
+    // entry = sum over the nibble's coordinates of q[d] * centroid[code] (f32, coordinate order, separately rounded)
+    if constexpr (BITS == 2) {
+        float p0[4], p1[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { p0[c] = __fadd_rn(0.0f, __fmul_rn(q[0], centroids[c])); p1[c] = __fmul_rn(q[1], centroids[c]); }
+#pragma unroll
+        for (int nib = 0; nib < 16; ++nib) e[nib] = __fadd_rn(p0[nib >> 2], p1[nib & 3]);
+    } else {
+#pragma unroll
+        for (int nib = 0; nib < 16; ++nib) e[nib] = __fadd_rn(0.0f, __fmul_rn(q[0], centroids[nib & ((1 << BITS) - 1)]));
+    }
+}
+
+template <int BITS>
+__device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mins, const float *centroids, float *red, int q, float bias_corr) {
+    constexpr int kCoords = BITS == 2 ? 2 : 1;                     // per half-byte: 8 / BITS / 2
+    const int ng = p.ngroups, tid = threadIdx.x;
+    float span = 0.0f;
+    for (int h = tid; h < 2 * ng; h += blockDim.x) {               // h = 2*g + half
+        float e[16];
+        half_entries<BITS>(row + h * kCoords, centroids, e);
+        float mn = FLT_MAX, mx = -FLT_MAX;
+#pragma unroll
+        for (int nib = 0; nib < 16; ++nib) {
+            if (e[nib] < mn) mn = e[nib];
+            if (e[nib] > mx) mx = e[nib];
+        }
+        mins[h] = mn;
+        span = fmaxf(span, __fsub_rn(mx, mn));
+    }
+    const float max_span = block_max(span, red, tid, blockDim.x);
+    float scale = max_span > 0.0f ? __fdiv_rn(max_span, 127.0f) : 1.0f;
+    float inv_scale;
+    if (scale >= FLT_MIN) inv_scale = __fdiv_rn(1.0f, scale);
+    else { scale = 1.0f; inv_scale = 1.0f; }
+    if (tid < 32) {
+        if (tid == 0) {
+            float bias = 0.0f;                                      // sequential in g (search.rs:2910)
+            const float2 *m2 = reinterpret_cast<const float2 *>(mins);
+#pragma unroll 16
+            for (int g = 0; g < ng; ++g) bias = __fadd_rn(bias, __fadd_rn(m2[g].x, m2[g].y));
+            p.qscale[q] = scale;
+            p.qbias[q] = __fadd_rn(bias, bias_corr);                // search.rs:3260
+        }
+        return;
+    }
+    uint4 *lut = reinterpret_cast<uint4 *>(p.luts + size_t(q) * p.lut_pitch);
+    for (int h = tid - 32; h < 2 * ng; h += blockDim.x - 32) {
+        float e[16];
+        half_entries<BITS>(row + h * kCoords, centroids, e);
+        const float mn = mins[h];
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int nib = 0; nib < 16; ++nib) {
+            float r = roundf(__fmul_rn(__fsub_rn(e[nib], mn), inv_scale));
+            r = fminf(fmaxf(r, 0.0f), 127.0f);
+            w[nib >> 2] |= uint32_t(int(r)) << (8 * (nib & 3));
+        }
+        lut[h] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (p.pad_operands)                                             // groups past the last one, up to a whole K slab
+        for (int h = 2 * ng + tid - 32; h < p.lut_pitch / 16; h += blockDim.x - 32) lut[h] = make_uint4(0, 0, 0, 0);
+}
+
+constexpr int kPrepThreads = 256;
+
 template <int LOG2B>
-__global__ void __launch_bounds__(128) query_prep_kernel(QueryPrepParams p) {
+__global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int dim = p.dim, ng = p.ngroups, stride = dim + 8;
     float *rowA = reinterpret_cast<float *>(smem_raw);
@@ -46,21 +120,36 @@ __global__ void __launch_bounds__(128) query_prep_kernel(QueryPrepParams p) {
     uint16_t *perm0 = reinterpret_cast<uint16_t *>(rowB + stride);
     uint16_t *perm1 = perm0 + dim;
     float *mins = reinterpret_cast<float *>(perm0);     // reused after the rotation: 2*ng floats <= 4*dim bytes
-    __shared__ float red[4];
+    __shared__ float red[kPrepThreads / 32];
     __shared__ float s_scalar[2];
+    __shared__ float s_centroids[16];
 
     const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (q >= p.nq) {                                    // operand rows past the last query
+        uint4 *row = reinterpret_cast<uint4 *>(p.mode == kModePermuteDot ? reinterpret_cast<uint8_t *>(p.weights) + size_t(q) * p.dim_pad
+                                                                         : p.luts + size_t(q) * p.lut_pitch);
+        const int words = (p.mode == kModePermuteDot ? p.dim_pad : p.lut_pitch) / 16;
+        for (int i = tid; i < words; i += kPrepThreads) row[i] = make_uint4(0, 0, 0, 0);
+        return;
+    }
+    if (p.cnt != nullptr) {
+        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; }
+        for (int i = tid; i < p.k; i += kPrepThreads) p.topk[size_t(q) * p.k + i] = kEmptyKey;
+    }
     const float *src = p.queries + size_t(q) * dim;
-    for (int i = tid; i < dim; i += blockDim.x) {
+    for (int i = tid; i < dim; i += kPrepThreads) {
         const float v = src[i];
         rowA[i] = v;
         if (!(fabsf(v) < 1e16f)) atomicMin(p.first_invalid, (unsigned long long)(size_t(q) * dim + i));
-        perm0[i] = p.perm0[i];
-        perm1[i] = p.perm1[i];
     }
+    // both tables, 16 bytes at a time (dim is a multiple of 8 and the second table follows the first)
+    for (int i = tid; i < dim / 4; i += kPrepThreads) reinterpret_cast<uint4 *>(perm0)[i] = reinterpret_cast<const uint4 *>(p.perm0)[i];
+    if (tid < 16) s_centroids[tid] = tid < (1 << p.bits) ? p.centroids[tid] : 0.0f;
     __syncthreads();
-    if (warp == 0)   // Rotation::apply: no normalisation (search.rs:3237-3242)
-        rotate_row<LOG2B>(rowA, rowB, perm0, perm1, dim, p.inv_sqrt_block, false, 1.0f, lane);
+    // Rotation::apply: no normalisation (search.rs:3237-3242)
+    rotation_round<LOG2B>(rowA, rowB, perm0, dim, p.inv_sqrt_block, false, 1.0f, lane, warp, kPrepThreads / 32);
+    __syncthreads();
+    rotation_round<LOG2B>(rowB, rowA, perm1, dim, p.inv_sqrt_block, false, 1.0f, lane, warp, kPrepThreads / 32);
     __syncthreads();
 
     // TQ+ inverse (search.rs:3154-3186): q[d] / scale[d]; bias correction = -(sum q[d]*shift[d]) in f64,
@@ -74,16 +163,18 @@ __global__ void __launch_bounds__(128) query_prep_kernel(QueryPrepParams p) {
         }
         __syncthreads();
         bias_corr = s_scalar[0];
-        for (int d = tid; d < dim; d += blockDim.x) rowA[d] = __fdiv_rn(rowA[d], p.scale_tq[d]);
+        for (int d = tid; d < dim; d += kPrepThreads) rowA[d] = __fdiv_rn(rowA[d], p.scale_tq[d]);
         __syncthreads();
     }
-    for (int d = tid; d < dim; d += blockDim.x) p.q_rot[size_t(q) * dim + d] = rowA[d];
+
+    if (p.q_rot != nullptr)
+        for (int d = tid; d < dim; d += kPrepThreads) p.q_rot[size_t(q) * dim + d] = rowA[d];
 
     if (p.mode == kModePermuteDot) {
         // search.rs:2806-2846: one scale for the row, weights = clamp(round(q * (1/qs)), +-127)
         float m = 0.0f;
-        for (int d = tid; d < dim; d += blockDim.x) m = fmaxf(m, fabsf(rowA[d]));
-        const float qmax = block_max(m, red, tid, blockDim.x);
+        for (int d = tid; d < dim; d += kPrepThreads) m = fmaxf(m, fabsf(rowA[d]));
+        const float qmax = block_max(m, red, tid, kPrepThreads);
         float qs = __fdiv_rn(qmax, 127.0f), inv_qs;
         if (qs >= FLT_MIN) inv_qs = __fdiv_rn(1.0f, qs);
         else { qs = 1.0f; inv_qs = 1.0f; }
@@ -91,14 +182,25 @@ __global__ void __launch_bounds__(128) query_prep_kernel(QueryPrepParams p) {
             p.qscale[q] = __fmul_rn(p.level_scale, qs);
             p.qbias[q] = __fadd_rn(0.0f, bias_corr);
         }
-        int8_t *wrow = p.weights + size_t(q) * p.dim_pad;
-        for (int d = tid; d < dim; d += blockDim.x) wrow[d ^ 1] = round_clamp_i8(__fmul_rn(rowA[d], inv_qs));
+        // four weights to a word, adjacent coordinates swapped (the nibble order of a code byte)
+        uint32_t *wrow = reinterpret_cast<uint32_t *>(p.weights + size_t(q) * p.dim_pad);
+        const int words = p.pad_operands ? p.dim_pad / 4 : dim / 4;
+        for (int i = tid; i < words; i += kPrepThreads) {
+            uint32_t word = 0;
+            if (4 * i < dim) {
+                const float4 v = reinterpret_cast<const float4 *>(rowA)[i];
+                word = uint32_t(uint8_t(round_clamp_i8(__fmul_rn(v.y, inv_qs)))) | uint32_t(uint8_t(round_clamp_i8(__fmul_rn(v.x, inv_qs)))) << 8 |
+                       uint32_t(uint8_t(round_clamp_i8(__fmul_rn(v.w, inv_qs)))) << 16 | uint32_t(uint8_t(round_clamp_i8(__fmul_rn(v.z, inv_qs)))) << 24;
+            }
+            wrow[i] = word;
+        }
+        if (p.wfrag == nullptr) return;
         // mma.sync A fragments.  k-step ks covers byte-groups 16ks..16ks+15; thread t of a quad owns
         // groups 16ks + t + {0,4,8,12}; register byte order follows the nibble order of a code byte
         // (low nibble = odd coordinate 2g+1, high nibble = even coordinate 2g; search.rs:2787-2790).
         const int ksteps = (ng + 15) / 16;
         const int m_tile = q >> 4, rr = q & 15, r = rr & 7, hi_row = rr >> 3;
-        for (int idx = tid; idx < ksteps * 8; idx += blockDim.x) {
+        for (int idx = tid; idx < ksteps * 8; idx += kPrepThreads) {
             const int ks = idx >> 3, t = (idx >> 1) & 3, half = idx & 1;
             const int ga = 16 * ks + t + 8 * half, gb = ga + 4;
             uint32_t word = 0;
@@ -112,51 +214,12 @@ __global__ void __launch_bounds__(128) query_prep_kernel(QueryPrepParams p) {
             const size_t frag = ((size_t(ks) * p.mtiles_total + m_tile) * 32 + (r * 4 + t)) * 4 + (half * 2 + hi_row);
             p.wfrag[frag] = word;
         }
+    } else if (p.bits == 2) {                                       // search.rs:2856-2994
+        lut_tables<2>(p, rowA, mins, s_centroids, red, q, bias_corr);
+    } else if (p.bits == 3) {
+        lut_tables<3>(p, rowA, mins, s_centroids, red, q, bias_corr);
     } else {
-        // search.rs:2856-2994.  Entry = sum over the nibble's coordinates of q[d]*centroid[code]
-        // (f32, coordinate order, separately rounded multiply and add).
-        const int cpb = 8 / p.bits, cpn = cpb / 2;
-        const unsigned code_mask = (1u << p.bits) - 1u;
-        auto entry = [&](int d0, unsigned nib) {
-            float s = 0.0f;
-            for (int c = 0; c < cpn; ++c) {
-                const unsigned code = (nib >> ((cpn - 1 - c) * p.bits)) & code_mask;
-                s = __fadd_rn(s, __fmul_rn(rowA[d0 + c], p.centroids[code]));
-            }
-            return s;
-        };
-        float span = 0.0f;
-        for (int h = tid; h < 2 * ng; h += blockDim.x) {           // h = 2*g + half
-            const int d0 = (h >> 1) * cpb + (h & 1) * cpn;
-            float mn = FLT_MAX, mx = -FLT_MAX;
-            for (unsigned nib = 0; nib < 16; ++nib) {
-                const float s = entry(d0, nib);
-                if (s < mn) mn = s;
-                if (s > mx) mx = s;
-            }
-            mins[h] = mn;
-            span = fmaxf(span, __fsub_rn(mx, mn));
-        }
-        const float max_span = block_max(span, red, tid, blockDim.x);
-        float scale = max_span > 0.0f ? __fdiv_rn(max_span, 127.0f) : 1.0f;
-        float inv_scale;
-        if (scale >= FLT_MIN) inv_scale = __fdiv_rn(1.0f, scale);
-        else { scale = 1.0f; inv_scale = 1.0f; }
-        if (tid == 0) {
-            float bias = 0.0f;                                      // sequential in g (search.rs:2910)
-            for (int g = 0; g < ng; ++g) bias = __fadd_rn(bias, __fadd_rn(mins[2 * g], mins[2 * g + 1]));
-            p.qscale[q] = scale;
-            p.qbias[q] = __fadd_rn(bias, bias_corr);                // search.rs:3260
-        }
-        uint8_t *lut = p.luts + size_t(q) * p.lut_pitch;
-        for (int e = tid; e < ng * 32; e += blockDim.x) {
-            const int h = e >> 4;
-            const unsigned nib = e & 15;
-            const int d0 = (h >> 1) * cpb + (h & 1) * cpn;
-            float r = roundf(__fmul_rn(__fsub_rn(entry(d0, nib), mins[h]), inv_scale));
-            r = fminf(fmaxf(r, 0.0f), 127.0f);
-            lut[e] = uint8_t(int(r));
-        }
+        lut_tables<4>(p, rowA, mins, s_centroids, red, q, bias_corr);
     }
 }
 
@@ -712,7 +775,7 @@ cudaError_t launch_query_prep(const QueryPrepParams &p, cudaStream_t stream) {
         cudaError_t e = cudaFuncSetAttribute(query_prep_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                              int(smem));                                                       \
         if (e != cudaSuccess) return e;                                                                        \
-        query_prep_kernel<L><<<p.nq, 128, smem, stream>>>(p);                                                  \
+        query_prep_kernel<L><<<p.rows, kPrepThreads, smem, stream>>>(p);                                                \
         break;                                                                                                 \
     }
     switch (rotation_variant(p.dim)) {

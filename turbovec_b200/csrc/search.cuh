@@ -21,14 +21,20 @@ struct QueryPrepParams {
     const float *scale_tq;
     float level_scale;             // cs of search.rs:2815 (permute-dot only)
     // outputs
-    float *q_rot;                  // [nq][dim] rotated (and TQ+-inverted) queries
+    float *q_rot;                  // [nq][dim] rotated (and TQ+-inverted) queries, or nullptr
     float *qscale, *qbias;         // [nq]
     uint8_t *luts;                 // [nq][lut_pitch], ngroups*32 bytes used per query (LUT modes)
     int lut_pitch;                 // bytes between the tables of consecutive queries: 32 * (ngroups rounded up to 4)
     int8_t *weights;               // [rows][dim_pad] row-major, byte d^1 = weight of coordinate d (permute-dot;
                                    // tensor-core operand: the swap matches the nibble order of a code byte)
     int dim_pad;                   // row pitch of `weights`
-    uint32_t *wfrag;               // mma.sync A fragments (permute-dot), see scan kernel
+    uint32_t *wfrag;               // mma.sync A fragments (permute-dot), see scan kernel; nullptr: not wanted
+    int pad_operands;              // clear the columns of the operand rows past the last coordinate / group
+    int rows;                      // operand rows to write: nq, or more (the rest are cleared)
+    // selection state of the batch, reset here (cnt == nullptr: none)
+    uint32_t *cnt, *done;
+    uint64_t *thr, *topk;
+    int k;
     int mtiles_total;              // ceil(nq / 16)
     unsigned long long *first_invalid;  // min flat index of a query coordinate failing |x| < 1e16
 };
