@@ -442,116 +442,6 @@ scan_pd_kernel(ScanParams p) {
 }
 
 // =====================================================================================================
-// LUT scan (2/3-bit, and every geometry the permute-dot family does not cover): CUDA cores.
-// isum = sum_g U[g][byte>>4] + U[g][16 + (byte&15)] exactly; float epilogue per mode:
-//   kModeLutMulAdd: (f32)isum * scale + bias                      (search.rs:1176)
-//   kModeLutFlush : acc = bias; per 256 groups acc = fma(scale, (f32)isum_batch, acc)   (search.rs:1596)
-// One warp per code block; the tables of up to kLutQueriesPerLaunch queries sit in shared memory (the four
-// group rows a warp instruction touches are 32 consecutive words, so its lookups never conflict).
-// =====================================================================================================
-template <int NQ>
-__global__ void __launch_bounds__(256) scan_lut_kernel(ScanParams p) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int ng = p.ngroups;
-    uint8_t *lut = smem_raw;                                  // [NQ][ng*32]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nq_here = min(NQ, p.nq);
-    for (int q = 0; q < nq_here; ++q) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(p.luts + size_t(p.q_base + q) * p.lut_pitch);
-        uint4 *dst = reinterpret_cast<uint4 *>(lut + size_t(q) * ng * 32);
-        for (int i = tid; i < ng * 2; i += blockDim.x) dst[i] = src[i];
-    }
-    __syncthreads();
-    uint32_t pos_end = p.pos_end;
-    if (p.live_blocks != nullptr) pos_end = min(pos_end, *p.n_live);
-    const uint32_t pos_begin = min(p.pos_begin, pos_end);
-    float qs[NQ], qb[NQ];
-    uint64_t thr[NQ], lo[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        const int ql = p.q_base + min(q, nq_here - 1);
-        qs[q] = p.qscale[ql]; qb[q] = p.qbias[ql]; thr[q] = p.cb.thr[ql];
-        lo[q] = p.cb.lo ? p.cb.lo[ql] : 0ull;
-    }
-    const int warps = blockDim.x >> 5;
-    // A warp instruction reads 128 contiguous bytes = four group rows of the block: lane = (row r = lane / 8,
-    // vectors 4 * (lane % 8) .. + 3).  Each lane sums its quarter of the groups for its four vectors; the
-    // integer partial sums of the four lanes that share a vector quad are added by two shuffles (integer
-    // addition: the order does not matter), then lane (quad, r) finishes vector 4 * quad + r.
-    const int row = lane >> 3, quad = lane & 7;
-    const int my_vec = 4 * quad + row;
-    for (uint32_t pos = pos_begin + blockIdx.x * warps + warp; pos < pos_end; pos += gridDim.x * warps) {
-        const uint32_t blk = p.live_blocks ? p.live_blocks[pos] : pos;
-        const uint32_t *codes32 = reinterpret_cast<const uint32_t *>(p.codes + size_t(blk) * ng * kLanes) + lane;
-        const int64_t slot = int64_t(blk) * kLanes + my_vec;
-        float facc[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) facc[q] = qb[q];
-        uint32_t total[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) total[q] = 0;
-        for (int g0 = 0; g0 < ng; g0 += 256) {
-            const int g1 = min(g0 + 256, ng);
-            uint32_t isum[NQ][4];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) isum[q][j] = 0;
-#pragma unroll 4
-            for (int g = g0 + row; g < g1; g += 4) {
-                const uint32_t word = codes32[size_t(g - row) * 8];      // bytes of vectors 4*quad .. +3 in group g
-                const int o = g * 32;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t byte = (word >> (8 * j)) & 255u;
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q)
-                        isum[q][j] += uint32_t(lut[q * ng * 32 + o + (byte >> 4)]) + uint32_t(lut[q * ng * 32 + o + 16 + (byte & 15)]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                uint32_t mine = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint32_t v = isum[q][j];
-                    v += __shfl_xor_sync(kFullMask, v, 8);
-                    v += __shfl_xor_sync(kFullMask, v, 16);
-                    if (j == row) mine = v;
-                }
-                facc[q] = fmaf(qs[q], float(int(mine)), facc[q]);
-                total[q] += mine;
-            }
-        }
-        auto score_of = [&](int q, float vs) {
-            const float pre = p.mode == kModeLutFlush ? facc[q] : __fadd_rn(__fmul_rn(float(int(total[q])), qs[q]), qb[q]);
-            return __fmul_rn(pre, vs);
-        };
-        if (p.dense) {
-            const bool on = slot < p.n && (!p.mask || ((p.mask[slot >> 6] >> (slot & 63)) & 1ull));
-            const float vs = on ? p.vec_scales[slot] : 0.0f;
-            write_block(p, pos, [&](auto put) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q)
-                    if (q < nq_here) put(p.q_base + q, my_vec, on, score_of(q, vs), uint32_t(slot));
-            });
-            continue;
-        }
-        if (slot < p.n) {
-            const bool allowed = !p.mask || ((p.mask[slot >> 6] >> (slot & 63)) & 1ull);
-            if (allowed) {
-                const float vs = p.vec_scales[slot];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    if (q >= nq_here) break;
-                    push_candidate(p.cb, p.q_base + q, score_of(q, vs), uint32_t(slot), thr[q], lo[q]);
-                }
-            }
-        }
-    }
-}
-
-// =====================================================================================================
 // Selection for k above kSelectMaxK (smaller k: select.cu): one CTA per query merges the previous top-k with the new candidates in shared memory.
 // With few entries it is a plain bitonic sort.  With many more entries than k it is a bitonic top-k: sort
 // runs of m = 2^ceil(log2 k) (at least 32) entries in alternating directions, then repeatedly take the
@@ -897,37 +787,6 @@ cudaError_t launch_scan_pd(const ScanParams &p, int sm_count, cudaStream_t s) {
     else if (mt <= 4) TV_LAUNCH_PD(4, false)
     else return cudaErrorInvalidValue;
 #undef TV_LAUNCH_PD
-    return cudaGetLastError();
-}
-
-int scan_lut_width(int ngroups, size_t smem_limit) {
-    const size_t table = size_t(ngroups) * 32;
-    if (table == 0) return 0;
-    const size_t fit = (smem_limit > 1024 ? smem_limit - 1024 : 0) / table;
-    return fit >= 4 ? 4 : (fit >= 2 ? 2 : (fit >= 1 ? 1 : 0));
-}
-
-cudaError_t launch_scan_lut(const ScanParams &p, int sm_count, cudaStream_t s) {
-    if (p.nq <= 0 || p.pos_end <= p.pos_begin) return cudaSuccess;
-    if (p.nq > 4) return cudaErrorInvalidValue;
-    // sized by the kernel's template width: its inner loop reads all NQ tables (unused ones hold garbage
-    // whose sums are discarded), so the allocation must cover them
-    const int width = p.nq == 1 ? 1 : (p.nq == 2 ? 2 : 4);
-    const size_t smem = size_t(width) * p.ngroups * 32;
-    const uint32_t blocks = p.pos_end - p.pos_begin;
-    // resident CTAs per SM: as many as the tables leave room for (the scan hides its lookup latency with warps)
-    const uint32_t per_sm = uint32_t(std::max<size_t>(1, std::min<size_t>(6, (size_t(200) << 10) / (smem + 1024))));
-    const unsigned grid = unsigned(min(uint32_t(sm_count) * per_sm, (blocks + 7) / 8));
-#define TV_LAUNCH_LUT(N)                                                                                             \
-    {                                                                                                                \
-        cudaError_t e = cudaFuncSetAttribute(scan_lut_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
-        if (e != cudaSuccess) return e;                                                                              \
-        scan_lut_kernel<N><<<grid, 256, smem, s>>>(p);                                                               \
-    }
-    if (width == 1) TV_LAUNCH_LUT(1)
-    else if (width == 2) TV_LAUNCH_LUT(2)
-    else TV_LAUNCH_LUT(4)
-#undef TV_LAUNCH_LUT
     return cudaGetLastError();
 }
 
