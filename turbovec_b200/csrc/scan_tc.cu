@@ -31,13 +31,15 @@ struct TcShared {
     uint64_t d_full[2];            // accumulator buffer complete
     uint64_t d_empty[2];           // accumulator buffer read out by the epilogue warps
     uint32_t tmem_base;
-    uint32_t pad[3];
+    uint32_t epilogue_failed;      // a wait of some epilogue warp ran out: all of them leave after the item
+    uint32_t pad[2];
     // per-query parameters of an item, double buffered; 16-byte aligned for float4 loads
     float qscale[2][kMaxTileQueries];
     float qbias[2][kMaxTileQueries];
     float qthr[2][kMaxTileQueries];   // score of the current k-th key (-inf while fewer than k results exist)
     int ibound[2][kMaxTileQueries];   // per query: integer sum below which no vector of the item can be a candidate
     float vs_part[2][8];              // largest vector scale seen by each epilogue warp of the item
+    PushRing ring;                    // candidates of the epilogue warps
 };
 static_assert(offsetof(TcShared, qscale) % 16 == 0, "parameter arrays must be 16-byte aligned");
 
@@ -79,6 +81,8 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
     const uint32_t n_items = n_vtiles * uint32_t(n_qgroups);
 
     if (tid == 0) {
+        sh->ring.n = 0;
+        sh->epilogue_failed = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], kExpandWarps + 1); mbar_init(&sh->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sh->d_full[b], 1); mbar_init(&sh->d_empty[b], kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -152,7 +156,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
         uint32_t vt = blockIdx.x / uint32_t(n_qgroups);
         int qg = int(blockIdx.x % uint32_t(n_qgroups));
         bool ok = true;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++local_item) {
+        for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x, ++local_item) {
             const int buf = local_item % kBufs, pb = local_item & 1;
             int64_t slot[MT];
             float vs[MT];
@@ -177,6 +181,9 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
             for (int o = 16; o > 0; o >>= 1) vs_warp = fmaxf(vs_warp, __shfl_xor_sync(kFullMask, vs_warp, o));
             if (lane == 0) sh->vs_part[pb][warp - 2] = vs_warp;
             asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
+            // every warp is done with the item before; one warp's failure there ends the loop of all
+            if (*reinterpret_cast<volatile uint32_t *>(&sh->epilogue_failed)) break;
+            ring_flush(sh->ring, p.cb, kRingSize / 2, et, kEpilogueWarps * 32);
             // per-query parameters of this item: one query per epilogue thread
             {
                 float vs_max = 0.0f;
@@ -194,8 +201,8 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
             }
             asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
 
-            ok = mbar_wait(&sh->d_full[buf], (local_item / kBufs) & 1, p.cb.error);
-            if (!ok) break;
+            // warp-uniform outcome; a warp whose wait ran out still meets the others at the barriers of the next item
+            ok = __all_sync(kFullMask, mbar_wait(&sh->d_full[buf], (local_item / kBufs) & 1, p.cb.error));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // the two warps of a lane quarter split the columns; below 64 columns the second one has none
             constexpr int kColsPerHalf = kTileQueries >= 64 ? kTileQueries / 2 : kTileQueries;
@@ -204,7 +211,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(buf * MT + m) * kTileQueries + uint32_t(cbase);
-                for (int c0 = 0; c0 < (has_columns ? kColsPerHalf : 0); c0 += 32) {
+                for (int c0 = 0; c0 < (has_columns && ok ? kColsPerHalf : 0); c0 += 32) {
                     uint32_t acc[32];
                     tmem_ld32(taddr + c0, acc);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -217,15 +224,19 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                         continue;
                     }
                     sift_piece<ONEHOT>(acc, &sh->ibound[pb][cbase + c0], &sh->qscale[pb][cbase + c0], &sh->qbias[pb][cbase + c0], &sh->qthr[pb][cbase + c0],
-                                       fused, vs[m], live[m], slot[m], qg * kTileQueries + cbase + c0, taddr + c0, p.cb);
+                                       fused, vs[m], live[m], slot[m], qg * kTileQueries + cbase + c0, taddr + c0,
+                                       [&](int ql, uint64_t key) { ring_push(sh->ring, p.cb, ql, key); });
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh->d_empty[buf]);
+            if (!ok && lane == 0) sh->epilogue_failed = 1;
             vt += vt_step; qg += qg_step;
             if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
         }
+        asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
+        ring_flush(sh->ring, p.cb, 1, et, kEpilogueWarps * 32);
     } else {
         // ------------------------------------------------ expansion: codes -> int8 A slabs -------
         // The (item, slab) pairs of this CTA form one flat sequence; the code words of the next kAhead slabs

@@ -224,15 +224,47 @@ __device__ __forceinline__ void write_piece(const uint32_t (&acc)[32], const flo
     }
 }
 
+// Candidates on their way to the lists.  Appending one takes a global atomic whose result says where it goes, about a
+// microsecond that the epilogue warp would sit out for every single candidate; the warps of a CTA collect candidates in
+// shared memory instead and write them out together, one thread each, when the ring is half full and at the end.  What does
+// not fit goes to its list directly.  Order within a list does not matter.
+constexpr uint32_t kRingSize = 512;
+struct PushRing {
+    uint32_t n;
+    uint32_t pad[3];
+    uint64_t key[kRingSize];
+    uint32_t ql[kRingSize];
+};
+__device__ __forceinline__ void append_candidate(const CandidateBuffers &cb, int ql, uint64_t key) {
+    if (key < cb.thr[ql] && (cb.lo == nullptr || key >= cb.lo[ql])) {
+        const uint32_t at = atomicAdd(&cb.cnt[ql], 1u);
+        if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
+    }
+}
+__device__ __forceinline__ void ring_push(PushRing &ring, const CandidateBuffers &cb, int ql, uint64_t key) {
+    const uint32_t at = atomicAdd(&ring.n, 1u);
+    if (at < kRingSize) { ring.key[at] = key; ring.ql[at] = uint32_t(ql); }
+    else append_candidate(cb, ql, key);
+}
+// Called by every epilogue thread between two of the epilogue's barriers, where nobody pushes: `limit` = smallest fill
+// that is written out.  Uses barrier 1 (`threads` epilogue threads) itself when it writes.
+__device__ __forceinline__ void ring_flush(PushRing &ring, const CandidateBuffers &cb, uint32_t limit, int et, int threads) {
+    const uint32_t n = *reinterpret_cast<volatile uint32_t *>(&ring.n);
+    if (n < limit) return;
+    for (uint32_t i = et; i < min(n, kRingSize); i += threads) append_candidate(cb, int(ring.ql[i]), ring.key[i]);
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+    if (et == 0) ring.n = 0;
+}
+
 // Later chunks: one integer compare per column dismisses the piece unless some column could be a candidate
 // (dismissal_bound).  Each lane keeps the outcome per run of 8 columns; the runs that any lane of the warp flagged are
 // re-read from tensor memory (address `taddr` = the piece's first column) and scored exactly by the lanes that flagged
-// them, and the keys that beat the query's k-th key are appended to its candidate list.  All pointers are at the
-// piece's first column; every lane of the warp must call this.
-template <bool ONEHOT>
+// them, and `push` gets the (query, key) pairs that reach the query's k-th score.  All pointers are at the piece's first
+// column; every lane of the warp must call this.
+template <bool ONEHOT, typename Push>
 __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int *ibound, const float *qscale, const float *qbias,
                                            const float *qthr, bool fused, float vs, bool live, int64_t slot, int ql0, uint32_t taddr,
-                                           const CandidateBuffers &cb) {
+                                           Push push) {
     uint32_t runs = 0;
     const int4 *pi = reinterpret_cast<const int4 *>(ibound);
 #pragma unroll
@@ -256,14 +288,7 @@ __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int 
             for (int e = 0; e < 8; ++e) {
                 const int c = c1 + e;
                 const float score = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs);
-                if (score >= qthr[c]) {
-                    const int ql = ql0 + c;
-                    const uint64_t key = make_key(score, uint32_t(slot));
-                    if (key < cb.thr[ql] && (cb.lo == nullptr || key >= cb.lo[ql])) {
-                        const uint32_t at = atomicAdd(&cb.cnt[ql], 1u);
-                        if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
-                    }
-                }
+                if (score >= qthr[c]) push(ql0 + c, make_key(score, uint32_t(slot)));
             }
         }
     }

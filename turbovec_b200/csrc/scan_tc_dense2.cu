@@ -43,6 +43,7 @@ struct DensePairShared {
     float qthr[kMaxTileQueries];
     int ibound[kMaxTileQueries];      // per query: integer sum below which no vector of the item can be a candidate
     float vs_part[2][4];              // largest vector scale per lane quarter (written by both column halves)
+    PushRing ring;                    // candidates of the epilogue warps
 };
 static_assert(offsetof(DensePairShared, qscale) % 16 == 0, "parameter arrays must be 16-byte aligned");
 
@@ -67,6 +68,7 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
 
     if (tid == 0) {
         sh->epilogue_failed = 0;
+        sh->ring.n = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 2); mbar_init(&sh->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sh->d_full[b], 1); mbar_init(&sh->d_empty[b], 2 * kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -182,8 +184,12 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
                 for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(kFullMask, m, o));
                 if (lane == 0) sh->vs_part[chalf][quarter] = m;
             }
+            // every warp is done with the item before (and its parameters); one warp's failure there ends the loop of all
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            const float vs_max = fmaxf(fmaxf(sh->vs_part[0][0], sh->vs_part[0][1]), fmaxf(sh->vs_part[0][2], sh->vs_part[0][3]));
+            if (*reinterpret_cast<volatile uint32_t *>(&sh->epilogue_failed)) { ok = false; break; }
+            ring_flush(sh->ring, p.cb, kRingSize / 2, et, kEpilogueWarps * 32);
+            const float *vp = sh->vs_part[0];
+            const float vs_max = fmaxf(fmaxf(vp[0], vp[1]), fmaxf(vp[2], vp[3]));
             {
                 const int ql = qg * kTileQueries + et;
                 float qs = 0.f, qb = 0.f, th = INFINITY;
@@ -215,19 +221,19 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
                     continue;
                 }
                 sift_piece<ONEHOT>(acc, sh->ibound + cbase + c0, qscale + c0, qbias + c0, qthr + c0, fused, vs, live, slot,
-                                   qg * kTileQueries + cbase + c0, taddr + c0, p.cb);
+                                   qg * kTileQueries + cbase + c0, taddr + c0,
+                                   [&](int ql, uint64_t key) { ring_push(sh->ring, p.cb, ql, key); });
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->d_empty[buf]), 0));   // the leader's barrier counts both CTAs
-            // the parameters are rewritten for the next item only after every warp is done with them; the barriers of
-            // the next item need all eight warps, so one warp's failure ends the loop of all
+            // the barriers of the next item need all eight warps
             if (!ok && lane == 0) sh->epilogue_failed = 1;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (sh->epilogue_failed) break;
             vt += vt_step; qg += qg_step;
             if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
         }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        ring_flush(sh->ring, p.cb, 1, et, kEpilogueWarps * 32);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

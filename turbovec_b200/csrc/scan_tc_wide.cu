@@ -216,7 +216,8 @@ scan_tc_wide_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int 
                         continue;
                     }
                     sift_piece<ONEHOT>(acc, sh->ibound + half * kTileQueries + c0, qscale + c0, qbias + c0, qthr + c0, fused, vs, live, slot,
-                                       qg * kTileQueries + c0, taddr + c0, p.cb);
+                                       qg * kTileQueries + c0, taddr + c0,
+                                       [&](int ql, uint64_t key) { append_candidate(p.cb, ql, key); });
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
