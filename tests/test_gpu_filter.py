@@ -1,0 +1,60 @@
+"""Batches over 2- and 3-bit codes that go through the filtering scan: identical to the oracle at ragged dimensions, partial
+query groups and chunk ends, under masks, past 256 byte-groups of the flush family, and where the filter lets too much through."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.util import anisotropic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def T():
+    import turbovec_b200
+    return turbovec_b200
+
+
+def built(T, x, bits):
+    enc = O.encode(x, bits)
+    idx = T.TurboQuantIndex(x.shape[1], bits)
+    idx.add(x)
+    return idx, (O.packed_to_blocked(enc["packed"], bits, x.shape[1]), enc["scales"])
+
+
+def check(idx, pre, q, k, mask=None):
+    n, bits = len(idx), idx.bit_width
+    words = None if mask is None else O.pack_mask(mask)
+    want = O.search(q, pre[0], pre[1], n, q.shape[1], bits, k, mask_words=words)
+    s, i = idx.search(q, k, mask=mask)
+    assert np.array_equal(s, want[0]) and np.array_equal(i, want[1]), (n, q.shape, bits, k)
+
+
+# at least 4 MiB of codes each; dim 2072 at 2 bits has 518 byte-groups, not a multiple of four
+@pytest.mark.parametrize("dim,bits,n,nq", [(64, 2, 270_001, 8), (200, 2, 90_017, 70), (200, 3, 45_003, 9), (1536, 2, 11_001, 65),
+                                           (1000, 3, 9_000, 300), (2072, 2, 8_200, 8), (3072, 2, 6_007, 17)])
+def test_filtering_scan_matches_oracle(T, dim, bits, n, nq):
+    x = anisotropic(n, dim, seed=23)
+    idx, pre = built(T, x, bits)
+    q = anisotropic(nq, dim, seed=23, offset=n + 1)
+    for k in (1, 10, 200):
+        check(idx, pre, q, k)
+    rng = np.random.default_rng(n)
+    for share in (0.6, 0.02):
+        mask = rng.random(n) < share
+        check(idx, pre, q[:12], 10, mask)
+    mask = np.zeros(n, bool)
+    mask[rng.choice(n, 7, replace=False)] = True            # fewer allowed than k
+    check(idx, pre, q[:9], 10, mask)
+
+
+@pytest.mark.parametrize("bits", [2, 3])
+def test_filtering_scan_overflows_and_recovers(T, bits):
+    """Every row the same but for a few, and a query that all of them score below zero: nothing can be dismissed."""
+    n, dim = 300_000, 64
+    x = np.repeat(anisotropic(1, dim, seed=2), n, axis=0)
+    x[3::1117] = anisotropic(len(x[3::1117]), dim, seed=6)
+    idx, pre = built(T, x, bits)
+    q = np.concatenate([-x[:1], x[:1], anisotropic(6, dim, seed=7)])
+    check(idx, pre, q, 10)
+    check(idx, pre, np.concatenate([q, np.zeros((1, dim), np.float32)]), 20)

@@ -123,6 +123,7 @@ struct SearchCtx {
     DeviceArray<float> d_stage;              // query upload
     DeviceArray<float> d_qrot;               // tv_rotate
     DeviceArray<float> d_qscale, d_qbias;
+    DeviceArray<float> d_filter;             // affine bound of a filtering scan: scale, middle and upper bias per query
     DeviceArray<uint8_t> d_luts;
     DeviceArray<int8_t> d_weights;
     DeviceArray<uint32_t> d_wfrag;
@@ -412,12 +413,12 @@ int upload_codebook(tv_index *h) {
         h->qgrid.cells = h->d_qgrid.ptr; h->qgrid.a = grid.a; h->qgrid.b = grid.b;
     }
     TV_CUDA(cudaStreamSynchronize(h->stream));
-    if (h->bits == 4) {
+    {
         // search.rs:2812-2819: cs = cmax/127, level = clamp(round(c/cs), +-127)
         float cmax = 0.f;
         for (float c : h->cb.centroids) cmax = std::fmax(cmax, std::fabs(c));
         const float cs = cmax > 0.f ? cmax / 127.0f : 1.0f;
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < int(h->cb.centroids.size()); ++i) {
             float r = std::round(h->cb.centroids[i] / cs);
             r = std::fmin(std::fmax(r, -127.0f), 127.0f);
             h->levels[i] = int8_t(int(r));
@@ -756,6 +757,7 @@ struct SearchScratch {
     uint64_t *cand, *thr, *topk, *lo;      // lo: lowest admissible key per query (paged top-k), or nullptr
     uint32_t *cnt, *done;                  // done follows cnt: both are cleared together
     size_t w_rows, dim_pad, lut_pitch;
+    float *f_scale, *f_mid, *f_max;        // affine bound of a filtering scan
     int cap;
     bool allow_tc;
 };
@@ -873,6 +875,7 @@ ScanParams base_scan_params(const tv_index *h, int mode) {
 struct ScanPlan {
     bool use_tc = false;       // tensor-memory scan (tcgen05)
     bool use_small = false;    // scan_small_kernel (up to 16 permute-dot queries)
+    bool use_filter = false;   // tensor-memory scan over int8 levels in front of the u8-LUT scores (scan_filter.cu)
     int lut_width = 0;         // queries per launch of the CUDA-core LUT scan
 };
 
@@ -900,6 +903,13 @@ int plan_scan(tv_index *h, int mode, size_t nq, bool allow_tc, ScanPlan &plan) {
         }
     }
     return TV_OK;
+}
+
+// Whether a batch goes through the filtering scan instead of the one-hot contraction.
+bool wants_filter(const tv_index *h, int mode, size_t nq, const ScanPlan &plan) {
+    if (!scan_filter_supported(h->bits, mode, h->ngroups, h->smem_limit) || h->mma_min_batch == 0) return false;
+    const bool batch = plan.use_tc || (h->mma_min_batch < 0 && nq >= 8);    // flush geometries beyond 256 groups have no one-hot form
+    return batch && h->n * size_t(h->ngroups) >= (size_t(4) << 20);
 }
 
 // Brings the int8 copy of the index (scan_tc_dense.cu) up to date on `st`: allocates it when policy and free memory
@@ -956,6 +966,43 @@ int expanded_sync(tv_index *h, cudaStream_t st, const uint32_t level_words[4], b
     return TV_OK;
 }
 
+// One search through the filtering scan: the first chunk by approximate score, a threshold from its k best, then the whole
+// index in chunks that append survivors, which are scored exactly and selected.
+int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, ScanParams sp, size_t nq, size_t kk,
+                     const MaskOnDevice &m) {
+    const size_t n_blocks = (h->n + kBlock - 1) / kBlock;
+    const float *qscale = S.qscale, *qbias = S.qbias;
+    auto scan = [&](size_t begin, size_t end, const float *bias, bool dense) -> int {
+        sp.pos_begin = uint32_t(begin); sp.pos_end = uint32_t(end); sp.dense = dense ? 1 : 0;
+        sp.qscale = S.f_scale; sp.qbias = bias; sp.q_base = 0; sp.nq = int(nq);
+        if (marks) marks->begin(st);
+        TV_CUDA(launch_scan_tc(sp, S.weights, int(S.w_rows), int(S.dim_pad), h->sm_count, 1, true, st));
+        if (marks) marks->end(st);
+        h->launches++;
+        sp.qscale = qscale; sp.qbias = qbias;
+        return TV_OK;
+    };
+    const size_t first = std::min(n_blocks, size_t(S.cap) / kBlock);
+    int rc = scan(0, first, S.f_mid, true);
+    if (rc != TV_OK) return rc;
+    TV_CUDA(launch_select(sp.cb, int(nq), uint32_t(first), m.n_live, st));
+    TV_CUDA(launch_bootstrap(sp, int(nq), st));
+    h->launches += 2;
+    // every survivor costs a gather of its bytes, so the chunks grow gently: a chunk of five times the vectors seen so far
+    // brings about five times k results above the threshold and, below it, what the bound cannot tell from them
+    for (size_t begin = 0, seen = first; begin < n_blocks;) {
+        size_t end = std::min(n_blocks, std::max(begin, seen) * 6);
+        if (end + end / 2 >= n_blocks) end = n_blocks;
+        rc = scan(begin, end, S.f_max, false);
+        if (rc != TV_OK) return rc;
+        TV_CUDA(launch_score_survivors(sp, int(nq), h->sm_count, st));
+        TV_CUDA(launch_select(sp.cb, int(nq), 0u, nullptr, st));
+        h->launches += 2;
+        begin = end;
+    }
+    return TV_OK;
+}
+
 // Scan + select over a geometric chunk schedule, all enqueued on `st`.
 //   careful: chunks never exceed the candidate capacity, so no list can overflow whatever the data order.
 //   fresh: the selection state is as query preparation left it.
@@ -980,6 +1027,7 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
         if (rc != TV_OK) return rc;
     }
 
+    if (plan.use_filter) return enqueue_filtered(h, st, marks, S, sp, nq, kk, m);
     if (!fresh) {
         TV_CUDA(cudaMemsetAsync(S.cnt, 0, 2 * nq * 4, st));
         TV_CUDA(cudaMemsetAsync(S.thr, 0xff, nq * 8, st));
@@ -1024,9 +1072,9 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
             else if (wide)
                 TV_CUDA(launch_scan_tc_wide(sp, reinterpret_cast<const int8_t *>(S.luts), int(S.w_rows), int(S.lut_pitch), h->sm_count, st));
             else if (mode == TV_SCORE_PERMUTE_DOT)
-                TV_CUDA(launch_scan_tc(sp, S.weights, int(S.w_rows), int(S.dim_pad), h->sm_count, h->tc_tiles, st));
+                TV_CUDA(launch_scan_tc(sp, S.weights, int(S.w_rows), int(S.dim_pad), h->sm_count, h->tc_tiles, false, st));
             else
-                TV_CUDA(launch_scan_tc(sp, reinterpret_cast<const int8_t *>(S.luts), int(S.w_rows), int(S.lut_pitch), h->sm_count, 1, st));
+                TV_CUDA(launch_scan_tc(sp, reinterpret_cast<const int8_t *>(S.luts), int(S.w_rows), int(S.lut_pitch), h->sm_count, 1, false, st));
             if (marks) marks->end(st);
             h->launches++;
         } else if (use_small) {
@@ -1080,9 +1128,14 @@ int enqueue_query_prep(tv_index *h, cudaStream_t st, const SearchScratch &S, con
     qp.mtiles_total = mt_total;
     qp.first_invalid = d_first_invalid;
     qp.cnt = S.cnt; qp.done = S.done; qp.thr = S.thr; qp.topk = S.topk; qp.k = int(kk);
+    if (plan.use_filter) {
+        qp.filter.weights = S.weights; qp.filter.scale = S.f_scale; qp.filter.bias_mid = S.f_mid; qp.filter.bias_max = S.f_max;
+        for (int i = 0; i < 8; ++i) qp.filter.levels[i] = h->levels[i];
+    }
     // the tensor-memory scans read whole groups of 256 operand rows and whole K slabs
-    qp.pad_operands = plan.use_tc ? 1 : 0;
-    qp.rows = plan.use_tc ? int(S.w_rows) : int(nq);
+    const bool tensor = plan.use_tc || plan.use_filter;
+    qp.pad_operands = tensor ? 1 : 0;
+    qp.rows = tensor ? int(S.w_rows) : int(nq);
     if (mode == TV_SCORE_PERMUTE_DOT && !plan.use_tc && !plan.use_small) {    // only scan_pd_kernel reads the fragments
         qp.wfrag = S.wfrag;
         TV_CUDA(cudaMemsetAsync(S.wfrag, 0, size_t(ksteps) * mt_total * 32 * 16, st));
@@ -1144,14 +1197,17 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     int rc = plan_scan(h, mode, nq, pages == 1, plan);
     if (rc != TV_OK) return rc;
 
+    plan.use_filter = pages == 1 && kk <= size_t(kSelectMaxK) && !h->force_careful && wants_filter(h, mode, nq, plan);
+
     // ---- buffers ----
     TV_CUDA(injected_failure(h));
     if (!queries_on_device) TV_CUDA(c.d_stage.reserve(nq * dim));
     TV_CUDA(c.d_qscale.reserve(nq_pad));
     TV_CUDA(c.d_qbias.reserve(nq_pad));
     const size_t w_rows = (nq + 255) / 256 * 256;
+    if (mode == TV_SCORE_PERMUTE_DOT || plan.use_filter) TV_CUDA(c.d_weights.reserve(w_rows * dim_pad));
+    if (plan.use_filter) TV_CUDA(c.d_filter.reserve(3 * nq_pad));
     if (mode == TV_SCORE_PERMUTE_DOT) {
-        TV_CUDA(c.d_weights.reserve(w_rows * dim_pad));
         TV_CUDA(c.d_wfrag.reserve(size_t(ksteps) * mt_total * 32 * 4));
     } else {
         TV_CUDA(c.d_luts.reserve(w_rows * lut_pitch));           // padded to whole query groups and whole K slabs for the tensor path
@@ -1203,6 +1259,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         if (rc != TV_OK) return rc;
     }
 
+    if (plan.use_filter) { S.f_scale = c.d_filter.ptr; S.f_mid = S.f_scale + nq_pad; S.f_max = S.f_mid + nq_pad; }
     rc = enqueue_query_prep(h, st, S, plan, mode, dq, nq, k_page, &c.d_flags->first_invalid);
     if (rc != TV_OK) return rc;
 
@@ -1235,8 +1292,8 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     for (size_t page = 0; page < pages; ++page) {
         const size_t k_this = pages == 1 ? kk : std::min(kPageK, kk - page * kPageK);
         S.lo = page == 0 ? nullptr : c.d_floor.ptr;
-        for (int attempt = 0; attempt < 2; ++attempt) {
-            const bool careful = attempt == 1 || h->force_careful;
+        for (int attempt = 0; attempt < 3; ++attempt) {
+            const bool careful = attempt == 2 || h->force_careful;
             rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, k_this, m, &c.d_flags->overflow, &c.d_flags->error, careful, page == 0 && attempt == 0);
             if (rc != TV_OK) { c.marks.used = 0; return rc; }
             if (pages == 1) {
@@ -1254,7 +1311,9 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
             if (rc != TV_OK) { c.marks.used = 0; return rc; }
             if (!c.h_flags->overflow) break;
             if (careful) return fail(h, TV_ERR_CUDA, "candidate overflow in the bounded schedule (internal error)");
-            // a chunk produced more candidates than the buffer holds: redo this page with bounded chunks
+            // a chunk produced more candidates than the buffer holds: redo this page without the filter, then with bounded chunks
+            if (!plan.use_filter) attempt = 1;
+            plan.use_filter = false;
             c.h_flags->overflow = 0;
             TV_CUDA(cudaMemcpyAsync(&c.d_flags->overflow, &c.h_flags->overflow, 4, cudaMemcpyHostToDevice, st));
         }

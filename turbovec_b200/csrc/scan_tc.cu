@@ -43,21 +43,29 @@ struct TcShared {
 };
 static_assert(offsetof(TcShared, qscale) % 16 == 0, "parameter arrays must be 16-byte aligned");
 
-// ONEHOT = false: permute-dot.  A rows hold the int8 levels of the codes, B rows the int8 query weights
-// (K = dim).  ONEHOT = true: the u8-LUT scan as a contraction (K = 32 * ngroups): A rows hold, per
+// KIND = kLevels4: permute-dot.  A rows hold the int8 levels of the codes, B rows the int8 query weights
+// (K = dim).  KIND = kOneHot: the u8-LUT scan as a contraction (K = 32 * ngroups): A rows hold, per
 // byte-group, a one-hot of the high nibble (16 bytes) then a one-hot of the low nibble (16 bytes); B rows are
 // the per-query u8 tables exactly as query preparation lays them out ([g][hi 16 | lo 16], entries <= 127),
 // so the int32 accumulator is the reference's integer LUT sum (search.rs:1071-1195) and the epilogue applies
 // (f32)isum * scale + bias (search.rs:1176).
+// KIND = kLevels2 / kLevels3: the 2- and 3-bit codes as int8 levels (K = dim), a filter in front of the u8-LUT scores
+// (scan_filter.cu): the epilogue's score is an approximation in the first chunk, an upper bound in the later ones, which
+// append the surviving slots instead of keys.  What bounds the one-hot form is its K, eight times (2-bit) the coordinates
+// and all of it written to shared memory; here a word of 16 codes becomes 16 levels with four byte permutes.
 // MT = accumulator tiles (of 128 vectors) that share one B slab.  MT = 1: work item 128 x 256, four stages,
 // two accumulator buffers (the epilogue of an item overlaps the MMAs of the next).  MT = 2: work item
 // 256 x 256, three stages, both 256-column halves of TMEM hold one item — half the B traffic per
 // multiply-add, at the price of the MMA pipe idling while the epilogue drains the accumulators.
 // NQT = query columns of a work item (MMA N): 256, or 64 / 32 for small batches, where a full-width item
 // would spend three quarters or more of its tensor time on columns that hold no query.
-template <int MT, bool ONEHOT, int NQT>
+enum ScanKind : int { kLevels4 = 0, kOneHot = 1, kLevels2 = 2, kLevels3 = 3 };
+
+template <int MT, int KIND, int NQT>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_slabs, int n_qgroups) {
+    constexpr bool ONEHOT = KIND == kOneHot;
+    constexpr bool kFilter = KIND == kLevels2 || KIND == kLevels3;
     constexpr int kStages = MT == 1 ? 4 : 3;
     constexpr int kABytes = MT * kATileBytes;
     constexpr int kBBytes = NQT * kSlabK;                     // 32 KB at 256 columns
@@ -183,7 +191,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
             asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
             // every warp is done with the item before; one warp's failure there ends the loop of all
             if (*reinterpret_cast<volatile uint32_t *>(&sh->epilogue_failed)) break;
-            ring_flush(sh->ring, p.cb, kRingSize / 2, et, kEpilogueWarps * 32);
+            ring_flush<kFilter>(sh->ring, p.cb, kRingSize / 2, et, kEpilogueWarps * 32);
             // per-query parameters of this item: one query per epilogue thread
             {
                 float vs_max = 0.0f;
@@ -223,6 +231,10 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                                                 qg * kTileQueries + cbase + c0, p.q_base + p.nq, at, p.cb);
                         continue;
                     }
+                    if constexpr (kFilter)
+                        filter_piece(acc, &sh->ibound[pb][cbase + c0], live[m], slot[m], qg * kTileQueries + cbase + c0, taddr + c0,
+                                     [&](int ql, uint64_t v) { ring_push<true>(sh->ring, p.cb, ql, v); });
+                    else
                     sift_piece<ONEHOT>(acc, &sh->ibound[pb][cbase + c0], &sh->qscale[pb][cbase + c0], &sh->qbias[pb][cbase + c0], &sh->qthr[pb][cbase + c0],
                                        fused, vs[m], live[m], slot[m], qg * kTileQueries + cbase + c0, taddr + c0,
                                        [&](int ql, uint64_t key) { ring_push(sh->ring, p.cb, ql, key); });
@@ -236,14 +248,14 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
             if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
         }
         asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
-        ring_flush(sh->ring, p.cb, 1, et, kEpilogueWarps * 32);
+        ring_flush<kFilter>(sh->ring, p.cb, 1, et, kEpilogueWarps * 32);
     } else {
         // ------------------------------------------------ expansion: codes -> int8 A slabs -------
         // The (item, slab) pairs of this CTA form one flat sequence; the code words of the next kAhead slabs
         // are kept in flight in registers so that global-load latency never reaches the expansion itself.
         // A unit = 4 vectors (one 32-bit column of a code block) x 8 byte-groups (one 16-byte chunk of a row).
         constexpr int kUnits = MT;                        // units per thread and slab
-        constexpr int kAhead = MT == 1 ? 4 : 3;
+        constexpr int kAhead = KIND == kLevels2 ? 8 : (MT == 1 ? 4 : 3);
         const int ew = warp - (2 + kEpilogueWarps);       // 0..7
         const int octet = lane & 7;                       // which 8-group run of the slab = 16-byte chunk index
         const int blk_in_item = MT == 1 ? (ew >> 1) : ew;
@@ -251,7 +263,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
         const uint32_t T[4] = {p.level_words[0], p.level_words[1], p.level_words[2], p.level_words[3]};
         const uint32_t my_items = blockIdx.x < n_items ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
         const uint32_t total = my_items * uint32_t(n_slabs);
-        constexpr int kWords = ONEHOT ? 1 : 8;            // code words per unit and slab
+        constexpr int kWords = ONEHOT ? 1 : (KIND == kLevels2 ? 4 : 8);            // code words per unit and slab
         uint32_t w[kAhead][kUnits][kWords];
         // fetch cursor: walks the same (item, slab) sequence as the consumers
         uint32_t f_item = blockIdx.x, f_vt = blockIdx.x / uint32_t(n_qgroups);
@@ -271,6 +283,13 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                 const int g = f_slab * 4 + (octet >> 1);
 #pragma unroll
                 for (int u = 0; u < kUnits; ++u) dst[u][0] = (f_have && g < ng) ? __ldg(f_src + size_t(g) * 8 + u * 4) : 0u;
+            } else if constexpr (KIND == kLevels2) {
+                // a slab is 32 byte-groups of four coordinates; chunk `octet` = groups 4 octet .. + 3
+                const int g0 = f_slab * (kSlabK / 4) + octet * 4;
+#pragma unroll
+                for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) dst[u][r] = (f_have && g0 + r < ng) ? __ldg(f_src + size_t(g0 + r) * 8 + u * 4) : 0u;
             } else {
                 const int g0 = f_slab * (kSlabK / 2) + octet * 8;
                 const uint32_t *src = f_src + size_t(g0) * 8;
@@ -312,6 +331,20 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                             v[u][j].x = q == 0 ? bit : 0u; v[u][j].y = q == 1 ? bit : 0u;
                             v[u][j].z = q == 2 ? bit : 0u; v[u][j].w = q == 3 ? bit : 0u;
                         }
+                    } else if constexpr (KIND == kLevels2) {
+                        // 4x4 byte transpose: word j = the four groups of vector j.  Its fields at bits 4i (coordinates 3 and 1 of
+                        // a group) and 4i + 2 (coordinates 2 and 0) select levels; the query rows are stored in this order
+                        // (kLevels2Order in search.cu).
+                        const uint32_t *x = w[a][u];
+                        const uint32_t t0 = prmt(x[0], x[1], 0x5140), t1 = prmt(x[0], x[1], 0x7362);
+                        const uint32_t t2 = prmt(x[2], x[3], 0x5140), t3 = prmt(x[2], x[3], 0x7362);
+                        const uint32_t xv[4] = {prmt(t0, t2, 0x5410), prmt(t0, t2, 0x7632), prmt(t1, t3, 0x5410), prmt(t1, t3, 0x7632)};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint32_t e = xv[j] & 0x33333333u, o = (xv[j] >> 2) & 0x33333333u;
+                            v[u][j].x = prmt(T[0], 0u, e); v[u][j].y = prmt(T[0], 0u, mad_hi(e, 0x10000u, 0u));
+                            v[u][j].z = prmt(T[0], 0u, o); v[u][j].w = prmt(T[0], 0u, mad_hi(o, 0x10000u, 0u));
+                        }
                     } else {
                         // 4x4 byte transposes: bytes of vector j of the unit in groups g0..g0+3 (xlo) and g0+4..g0+7 (xhi)
                         const uint32_t *x = w[a][u];
@@ -323,8 +356,13 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                         const uint32_t xhi[4] = {prmt(u0, u2, 0x5410), prmt(u0, u2, 0x7632), prmt(u1, u3, 0x5410), prmt(u1, u3, 0x7632)};
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            expand8(xlo[j], T, v[u][j].x, v[u][j].y);
-                            expand8(xhi[j], T, v[u][j].z, v[u][j].w);
+                            if constexpr (KIND == kLevels3) {        // a nibble below 8 is a selector as it stands
+                                v[u][j].x = prmt(T[0], T[1], xlo[j]); v[u][j].y = prmt(T[0], T[1], mad_hi(xlo[j], 0x10000u, 0u));
+                                v[u][j].z = prmt(T[0], T[1], xhi[j]); v[u][j].w = prmt(T[0], T[1], mad_hi(xhi[j], 0x10000u, 0u));
+                            } else {
+                                expand8(xlo[j], T, v[u][j].x, v[u][j].y);
+                                expand8(xhi[j], T, v[u][j].z, v[u][j].w);
+                            }
                         }
                     }
                 }
@@ -486,12 +524,13 @@ bool scan_tc_supported(int bits, int mode, int ngroups) {
 // pair-swapped (byte 2g = coordinate 2g+1, byte 2g+1 = coordinate 2g) to match the nibble order of a code byte.
 // LUT: weights = the u8 tables [rows][pitch = 32 * ngroups].
 // tiles_per_item: 1 or 2 accumulator tiles of 128 vectors per B slab (see the kernel).
+// filter: weights = int8 weights [rows][pitch] for a filtering scan of 2- or 3-bit codes.
 cudaError_t launch_scan_tc(const ScanParams &p, const int8_t *weights, int rows, int pitch, int sm_count, int tiles_per_item,
-                           cudaStream_t s) {
+                           bool filter, cudaStream_t s) {
     if (p.nq <= 0 || p.pos_end <= p.pos_begin) return cudaSuccess;
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
-    const bool onehot = p.mode != kModePermuteDot;
+    const bool onehot = p.mode != kModePermuteDot && !filter;
     const int nq_all = p.q_base + p.nq;
     // query columns per work item: the tensor time of an item grows with them whether they hold queries or not
     const int nqt = nq_all <= 32 && onehot ? 32 : (nq_all <= 64 ? 64 : kMaxTileQueries);
@@ -507,7 +546,7 @@ cudaError_t launch_scan_tc(const ScanParams &p, const int8_t *weights, int rows,
     const int n_slabs = pitch / kSlabK;
     const int n_qgroups = (nq_all + nqt - 1) / nqt;
     const size_t smem = scan_tc_smem_bytes(nqt);
-    const int mt = (tiles_per_item == 2 && !onehot && nqt == kMaxTileQueries) ? 2 : 1;
+    const int mt = (tiles_per_item == 2 && p.mode == kModePermuteDot && nqt == kMaxTileQueries) ? 2 : 1;
     const uint32_t vtiles = (p.pos_end - p.pos_begin + 4 * mt - 1) / (4 * mt);
     const uint64_t items = uint64_t(vtiles) * n_qgroups;
     // a multiple of the query-group count keeps the CTAs that share a vector tile in step (codes hit L2)
@@ -521,16 +560,20 @@ cudaError_t launch_scan_tc(const ScanParams &p, const int8_t *weights, int rows,
         if (e != cudaSuccess) return e;                                                                                 \
         scan_tc_kernel<M, O, N><<<grid, kThreadsTc, smem, s>>>(p, map, n_slabs, n_qgroups);                             \
     }
-    if (onehot) {
-        if (nqt == 32) TV_LAUNCH_TC(1, true, 32)
-        else if (nqt == 64) TV_LAUNCH_TC(1, true, 64)
-        else TV_LAUNCH_TC(1, true, 256)
+    if (filter) {
+        if (p.bits == 2) { if (nqt == 64) TV_LAUNCH_TC(1, kLevels2, 64) else TV_LAUNCH_TC(1, kLevels2, 256) }
+        else if (p.bits == 3) { if (nqt == 64) TV_LAUNCH_TC(1, kLevels3, 64) else TV_LAUNCH_TC(1, kLevels3, 256) }
+        else return cudaErrorInvalidValue;
+    } else if (onehot) {
+        if (nqt == 32) TV_LAUNCH_TC(1, kOneHot, 32)
+        else if (nqt == 64) TV_LAUNCH_TC(1, kOneHot, 64)
+        else TV_LAUNCH_TC(1, kOneHot, 256)
     } else if (mt == 2) {
-        TV_LAUNCH_TC(2, false, 256)
+        TV_LAUNCH_TC(2, kLevels4, 256)
     } else if (nqt == 64) {
-        TV_LAUNCH_TC(1, false, 64)
+        TV_LAUNCH_TC(1, kLevels4, 64)
     } else {
-        TV_LAUNCH_TC(1, false, 256)
+        TV_LAUNCH_TC(1, kLevels4, 256)
     }
 #undef TV_LAUNCH_TC
     return cudaGetLastError();

@@ -241,19 +241,45 @@ __device__ __forceinline__ void append_candidate(const CandidateBuffers &cb, int
         if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
     }
 }
+// RAW: a survivor of a filtering scan, appended unseen (its exact key is computed later)
+template <bool RAW>
+__device__ __forceinline__ void append_any(const CandidateBuffers &cb, int ql, uint64_t key) {
+    if constexpr (RAW) {
+        const uint32_t at = atomicAdd(&cb.cnt[ql], 1u);
+        if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
+    } else {
+        append_candidate(cb, ql, key);
+    }
+}
+template <bool RAW = false>
 __device__ __forceinline__ void ring_push(PushRing &ring, const CandidateBuffers &cb, int ql, uint64_t key) {
     const uint32_t at = atomicAdd(&ring.n, 1u);
     if (at < kRingSize) { ring.key[at] = key; ring.ql[at] = uint32_t(ql); }
-    else append_candidate(cb, ql, key);
+    else append_any<RAW>(cb, ql, key);
 }
 // Called by every epilogue thread between two of the epilogue's barriers, where nobody pushes: `limit` = smallest fill
 // that is written out.  Uses barrier 1 (`threads` epilogue threads) itself when it writes.
+template <bool RAW = false>
 __device__ __forceinline__ void ring_flush(PushRing &ring, const CandidateBuffers &cb, uint32_t limit, int et, int threads) {
     const uint32_t n = *reinterpret_cast<volatile uint32_t *>(&ring.n);
     if (n < limit) return;
-    for (uint32_t i = et; i < min(n, kRingSize); i += threads) append_candidate(cb, int(ring.ql[i]), ring.key[i]);
+    for (uint32_t i = et; i < min(n, kRingSize); i += threads) append_any<RAW>(cb, int(ring.ql[i]), ring.key[i]);
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
     if (et == 0) ring.n = 0;
+}
+
+// Which runs of 8 of a piece's 32 columns hold a sum at or above the column's bound for this lane's vector (bit = run).
+__device__ __forceinline__ uint32_t surviving_runs(const uint32_t (&acc)[32], const int *ibound, bool live) {
+    uint32_t runs = 0;
+    const int4 *pi = reinterpret_cast<const int4 *>(ibound);
+#pragma unroll
+    for (int j4 = 0; j4 < 8; ++j4) {
+        const int4 b = pi[j4];
+        const bool may = (int(acc[4 * j4 + 0]) >= b.x) | (int(acc[4 * j4 + 1]) >= b.y) | (int(acc[4 * j4 + 2]) >= b.z) |
+                         (int(acc[4 * j4 + 3]) >= b.w);
+        runs |= uint32_t(may) << (j4 >> 1);
+    }
+    return live ? runs : 0u;
 }
 
 // Later chunks: one integer compare per column dismisses the piece unless some column could be a candidate
@@ -265,16 +291,7 @@ template <bool ONEHOT, typename Push>
 __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int *ibound, const float *qscale, const float *qbias,
                                            const float *qthr, bool fused, float vs, bool live, int64_t slot, int ql0, uint32_t taddr,
                                            Push push) {
-    uint32_t runs = 0;
-    const int4 *pi = reinterpret_cast<const int4 *>(ibound);
-#pragma unroll
-    for (int j4 = 0; j4 < 8; ++j4) {
-        const int4 b = pi[j4];
-        const bool may = (int(acc[4 * j4 + 0]) >= b.x) | (int(acc[4 * j4 + 1]) >= b.y) | (int(acc[4 * j4 + 2]) >= b.z) |
-                         (int(acc[4 * j4 + 3]) >= b.w);
-        runs |= uint32_t(may) << (j4 >> 1);
-    }
-    if (!live) runs = 0;
+    const uint32_t runs = surviving_runs(acc, ibound, live);
     const uint32_t warp_runs = __reduce_or_sync(0xffffffffu, runs);
     if (warp_runs == 0) return;
 #pragma unroll 1
@@ -290,6 +307,26 @@ __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int 
                 const float score = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs);
                 if (score >= qthr[c]) push(ql0 + c, make_key(score, uint32_t(slot)));
             }
+        }
+    }
+}
+
+// Filtering scans: `push` gets (query, slot) for every column whose sum reaches the bound; there is no score yet.
+template <typename Push>
+__device__ __forceinline__ void filter_piece(const uint32_t (&acc)[32], const int *ibound, bool live, int64_t slot, int ql0, uint32_t taddr, Push push) {
+    const uint32_t runs = surviving_runs(acc, ibound, live);
+    const uint32_t warp_runs = __reduce_or_sync(0xffffffffu, runs);
+    if (warp_runs == 0) return;
+#pragma unroll 1
+    for (int c1 = 0; c1 < 32; c1 += 8) {
+        if (!((warp_runs >> (c1 >> 3)) & 1u)) continue;
+        uint32_t a8[8];
+        tmem_ld8(taddr + c1, a8);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if ((runs >> (c1 >> 3)) & 1u) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (int(a8[e]) >= ibound[c1 + e]) push(ql0 + c1 + e, uint64_t(slot));
         }
     }
 }

@@ -43,6 +43,8 @@ __device__ __forceinline__ int8_t round_clamp_i8(float v) {
 // sum runs beside the table entries.  One query: dim 1536 4-bit 12.8 us before, dim 3072 2-bit 105 us before.
 // The CTA also resets its query's selection state and clears the operand padding that the tensor-memory scans read
 // (CTAs past the last query clear a whole row).
+constexpr int kPrepThreads = 256;
+
 template <int BITS>
 __device__ __forceinline__ void half_entries(const float *q, const float *centroids, float (&e)[16]) {
     // entry = sum over the nibble's coordinates of q[d] * centroid[code] (f32, coordinate order, separately rounded)
@@ -58,8 +60,18 @@ __device__ __forceinline__ void half_entries(const float *q, const float *centro
     }
 }
 
+// Coordinate (within a chunk of 16) whose level the expansion of 2-bit codes puts at byte b of word w (scan_tc.cu, kLevels2).
+__device__ __forceinline__ int levels2_coord(int w, int b) { return (w & 1) * 8 - (w >> 1) + 4 * (b >> 1) + ((b & 1) ? 1 : 3); }
+
+// The u8 tables of a query and, for a filtering scan (scan_filter.cu), its int8 weights and the affine bound
+//   isum <= alpha * sum_d W[d] * L[code[d]] + beta + D,   with the equality's two sides at most D apart,
+// beta and D summed over the half-bytes from the extremes of U - alpha * (W . L) over the entries.  The entries' deviation
+// is evaluated in f32 (values up to 127: 5e-5 covers it) and summed in f64; 1e-5 of the reference's own bias covers the
+// roundings of its float epilogue, whose terms are that large before they cancel.
 template <int BITS>
 __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mins, const float *centroids, float *red, int q, float bias_corr) {
+    __shared__ double part[2][kPrepThreads / 32];
+    __shared__ float s_bias;
     constexpr int kCoords = BITS == 2 ? 2 : 1;                     // per half-byte: 8 / BITS / 2
     const int ng = p.ngroups, tid = threadIdx.x;
     float span = 0.0f;
@@ -80,6 +92,18 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mi
     float inv_scale;
     if (scale >= FLT_MIN) inv_scale = __fdiv_rn(1.0f, scale);
     else { scale = 1.0f; inv_scale = 1.0f; }
+    const bool filter = BITS != 4 && p.filter.weights != nullptr;
+    float w_scale = 1.0f, w_inv = 1.0f, alpha = 0.0f;
+    if (filter) {
+        float m = 0.0f;
+        for (int d = tid; d < p.dim; d += blockDim.x) m = fmaxf(m, fabsf(row[d]));
+        m = block_max(m, red, tid, blockDim.x);
+        w_scale = __fdiv_rn(m, 127.0f);
+        if (w_scale >= FLT_MIN) w_inv = __fdiv_rn(1.0f, w_scale);
+        else w_scale = 1.0f;
+        alpha = __fdiv_rn(__fmul_rn(w_scale, p.level_scale), scale);
+    }
+    double beta = 0.0, slack = 0.0;
     if (tid < 32) {
         if (tid == 0) {
             float bias = 0.0f;                                      // sequential in g (search.rs:2910)
@@ -87,29 +111,69 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mi
 #pragma unroll 16
             for (int g = 0; g < ng; ++g) bias = __fadd_rn(bias, __fadd_rn(m2[g].x, m2[g].y));
             p.qscale[q] = scale;
-            p.qbias[q] = __fadd_rn(bias, bias_corr);                // search.rs:3260
+            s_bias = p.qbias[q] = __fadd_rn(bias, bias_corr);       // search.rs:3260
         }
-        return;
-    }
-    uint4 *lut = reinterpret_cast<uint4 *>(p.luts + size_t(q) * p.lut_pitch);
-    for (int h = tid - 32; h < 2 * ng; h += blockDim.x - 32) {
-        float e[16];
-        half_entries<BITS>(row + h * kCoords, centroids, e);
-        const float mn = mins[h];
-        uint32_t w[4] = {0, 0, 0, 0};
+    } else {
+        uint4 *lut = reinterpret_cast<uint4 *>(p.luts + size_t(q) * p.lut_pitch);
+        for (int h = tid - 32; h < 2 * ng; h += blockDim.x - 32) {
+            float e[16];
+            half_entries<BITS>(row + h * kCoords, centroids, e);
+            const float mn = mins[h];
+            uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int nib = 0; nib < 16; ++nib) {
-            float r = roundf(__fmul_rn(__fsub_rn(e[nib], mn), inv_scale));
-            r = fminf(fmaxf(r, 0.0f), 127.0f);
-            w[nib >> 2] |= uint32_t(int(r)) << (8 * (nib & 3));
+            for (int nib = 0; nib < 16; ++nib) {
+                float r = roundf(__fmul_rn(__fsub_rn(e[nib], mn), inv_scale));
+                r = fminf(fmaxf(r, 0.0f), 127.0f);
+                e[nib] = r;
+                w[nib >> 2] |= uint32_t(int(r)) << (8 * (nib & 3));
+            }
+            lut[h] = make_uint4(w[0], w[1], w[2], w[3]);
+            if constexpr (BITS != 4) {
+                if (filter) {
+                    float wt[2];
+                    for (int c = 0; c < kCoords; ++c) wt[c] = alpha * float(round_clamp_i8(__fmul_rn(row[h * kCoords + c], w_inv)));
+                    float lo = FLT_MAX, hi = -FLT_MAX;
+#pragma unroll
+                    for (int nib = 0; nib < (BITS == 3 ? 8 : 16); ++nib) {
+                        const float fit = BITS == 2 ? wt[0] * float(p.filter.levels[nib >> 2]) + wt[1] * float(p.filter.levels[nib & 3])
+                                                    : wt[0] * float(p.filter.levels[nib]);
+                        lo = fminf(lo, e[nib] - fit);
+                        hi = fmaxf(hi, e[nib] - fit);
+                    }
+                    beta += 0.5 * (double(hi) + double(lo));
+                    slack += 0.5 * (double(hi) - double(lo)) + 5e-5;
+                }
+            }
         }
-        lut[h] = make_uint4(w[0], w[1], w[2], w[3]);
+        if (p.pad_operands)                                         // groups past the last one, up to a whole K slab
+            for (int h = 2 * ng + tid - 32; h < p.lut_pitch / 16; h += blockDim.x - 32) lut[h] = make_uint4(0, 0, 0, 0);
     }
-    if (p.pad_operands)                                             // groups past the last one, up to a whole K slab
-        for (int h = 2 * ng + tid - 32; h < p.lut_pitch / 16; h += blockDim.x - 32) lut[h] = make_uint4(0, 0, 0, 0);
+    if (!filter) return;
+    uint32_t *wrow = reinterpret_cast<uint32_t *>(p.filter.weights + size_t(q) * p.dim_pad);
+    for (int i = tid; i < p.dim_pad / 4; i += blockDim.x) {
+        uint32_t word = 0;
+        for (int b = 0; b < 4; ++b) {
+            // 3-bit codes lie in nibbles, low nibble = odd coordinate
+            const int d = BITS == 2 ? (i >> 2) * 16 + levels2_coord(i & 3, b) : 4 * i + (b ^ 1);
+            if (d < p.dim) word |= uint32_t(uint8_t(round_clamp_i8(__fmul_rn(row[d], w_inv)))) << (8 * b);
+        }
+        wrow[i] = word;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        beta += __shfl_xor_sync(kFullMask, beta, o);
+        slack += __shfl_xor_sync(kFullMask, slack, o);
+    }
+    if ((tid & 31) == 0) { part[0][tid >> 5] = beta; part[1][tid >> 5] = slack; }
+    __syncthreads();
+    if (tid == 0) {
+        beta = slack = 0.0;
+        for (int w = 0; w < kPrepThreads / 32; ++w) { beta += part[0][w]; slack += part[1][w]; }
+        const double base = double(scale) * beta + double(s_bias);
+        p.filter.scale[q] = float(double(scale) * double(alpha));
+        p.filter.bias_mid[q] = float(base);
+        p.filter.bias_max[q] = float(base + double(scale) * slack * 1.000001 + 1e-5 * fabs(double(s_bias)));
+    }
 }
-
-constexpr int kPrepThreads = 256;
 
 template <int LOG2B>
 __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParams p) {
@@ -130,6 +194,10 @@ __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParam
                                                                          : p.luts + size_t(q) * p.lut_pitch);
         const int words = (p.mode == kModePermuteDot ? p.dim_pad : p.lut_pitch) / 16;
         for (int i = tid; i < words; i += kPrepThreads) row[i] = make_uint4(0, 0, 0, 0);
+        if (p.mode != kModePermuteDot && p.filter.weights != nullptr) {
+            uint4 *w = reinterpret_cast<uint4 *>(p.filter.weights + size_t(q) * p.dim_pad);
+            for (int i = tid; i < p.dim_pad / 16; i += kPrepThreads) w[i] = make_uint4(0, 0, 0, 0);
+        }
         return;
     }
     if (p.cnt != nullptr) {

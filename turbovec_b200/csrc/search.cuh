@@ -19,7 +19,7 @@ struct QueryPrepParams {
     const float *centroids;        // 2^bits
     const float *shift;            // TQ+ pair or nullptr
     const float *scale_tq;
-    float level_scale;             // cs of search.rs:2815 (permute-dot only)
+    float level_scale;             // cs of search.rs:2815: a level is round(centroid / cs)
     // outputs
     float *q_rot;                  // [nq][dim] rotated (and TQ+-inverted) queries, or nullptr
     float *qscale, *qbias;         // [nq]
@@ -31,6 +31,13 @@ struct QueryPrepParams {
     uint32_t *wfrag;               // mma.sync A fragments (permute-dot), see scan kernel; nullptr: not wanted
     int pad_operands;              // clear the columns of the operand rows past the last coordinate / group
     int rows;                      // operand rows to write: nq, or more (the rest are cleared)
+    // operands of a filtering scan over 2- or 3-bit codes (scan_filter.cu); weights == nullptr: not wanted
+    struct Filter {
+        int8_t *weights;           // [rows][dim_pad], coordinates in the order of the expanded levels
+        float *scale;              // [nq] a score is close to fma(W . L, scale, bias_mid) and at most fma(W . L, scale, bias_max)
+        float *bias_mid, *bias_max;
+        int8_t levels[8];
+    } filter;
     // selection state of the batch, reset here (cnt == nullptr: none)
     uint32_t *cnt, *done;
     uint64_t *thr, *topk;
@@ -125,8 +132,14 @@ cudaError_t launch_scan_pd(const ScanParams &p, int sm_count, cudaStream_t s);
 // LUT families: weights = the u8 tables [rows][pitch = 32 * (ngroups rounded up to 4)], rows % 256 == 0, unused
 // tables and the padding groups zero.
 bool scan_tc_supported(int bits, int mode, int ngroups);
+// filter: 2- or 3-bit codes as int8 levels against int8 weights; p.qscale / p.qbias = the affine bound (first chunk: the
+// approximation), later chunks append slots, which launch_score_survivors turns into keys (scan_filter.cu).
 cudaError_t launch_scan_tc(const ScanParams &p, const int8_t *weights, int rows, int pitch, int sm_count,
-                           int tiles_per_item, cudaStream_t s);
+                           int tiles_per_item, bool filter, cudaStream_t s);
+bool scan_filter_supported(int bits, int mode, int ngroups, size_t smem_limit);
+cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cudaStream_t s);
+// topk = best of the first chunk by approximate score -> thr; topk is empty again
+cudaError_t launch_bootstrap(const ScanParams &p, int nq, cudaStream_t s);
 // The same scan for more than 256 queries with every expanded code slab shared by two query groups (scan_tc_wide.cu).
 bool scan_tc_wide_supported(int bits, int mode, int ngroups, int nq_total);
 cudaError_t launch_scan_tc_wide(const ScanParams &p, const int8_t *weights, int rows, int pitch, int sm_count, cudaStream_t s);
