@@ -31,17 +31,10 @@ struct TcShared {
     uint64_t d_full[2];            // accumulator buffer complete
     uint64_t d_empty[2];           // accumulator buffer read out by the epilogue warps
     uint32_t tmem_base;
-    uint32_t epilogue_failed;      // a wait of some epilogue warp ran out: all of them leave after the item
-    uint32_t pad[2];
-    // per-query parameters of an item, double buffered; 16-byte aligned for float4 loads
-    float qscale[2][kMaxTileQueries];
-    float qbias[2][kMaxTileQueries];
-    float qthr[2][kMaxTileQueries];   // score of the current k-th key (-inf while fewer than k results exist)
-    int ibound[2][kMaxTileQueries];   // per query: integer sum below which no vector of the item can be a candidate
-    float vs_part[2][8];              // largest vector scale seen by each epilogue warp of the item
-    PushRing ring;                    // candidates of the epilogue warps
+    uint32_t pad[3];
+    EpilogueShared ep;             // 16-byte aligned for vector loads
 };
-static_assert(offsetof(TcShared, qscale) % 16 == 0, "parameter arrays must be 16-byte aligned");
+static_assert(offsetof(TcShared, ep) % 16 == 0, "parameter arrays must be 16-byte aligned");
 
 // KIND = kLevels4: permute-dot.  A rows hold the int8 levels of the codes, B rows the int8 query weights
 // (K = dim).  KIND = kOneHot: the u8-LUT scan as a contraction (K = 32 * ngroups): A rows hold, per
@@ -89,8 +82,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
     const uint32_t n_items = n_vtiles * uint32_t(n_qgroups);
 
     if (tid == 0) {
-        sh->ring.n = 0;
-        sh->epilogue_failed = 0;
+        for (int w = 0; w < kEpilogueWarps; ++w) sh->ep.ring[w].n = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], kExpandWarps + 1); mbar_init(&sh->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sh->d_full[b], 1); mbar_init(&sh->d_empty[b], kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -160,64 +152,69 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
         const int quarter = warp & 3;                     // TMEM lanes 32*quarter .. +31 are this warp's
         const int half = (warp - 2) >> 2;                 // which 128 of the item's 256 query columns
         const int et = (warp - 2) * 32 + lane;            // 0..255 among the epilogue threads
+        // the two warps of a lane quarter split the columns; below 64 columns the second one has none
+        constexpr int kColsPerHalf = kTileQueries >= 64 ? kTileQueries / 2 : kTileQueries;
+        const int cbase = half * kColsPerHalf;
+        const bool has_columns = cbase < kTileQueries;
+        EpilogueShared &es = sh->ep;
+        WarpRing &ring = es.ring[warp - 2];
+        int *nbound = es.nbound[warp - 2];
+        const float *qscale = es.qscale + cbase, *qbias = es.qbias + cbase, *qthr = es.qthr + cbase;
         uint32_t local_item = 0;
         uint32_t vt = blockIdx.x / uint32_t(n_qgroups);
-        int qg = int(blockIdx.x % uint32_t(n_qgroups));
-        bool ok = true;
+        int qg = int(blockIdx.x % uint32_t(n_qgroups)), qg_here = -1;
+        float u[4], w[4];
+        const bool my_columns = has_columns && 4 * lane < kColsPerHalf;   // lane: columns 4 lane .. + 3 of the warp's
+        bool ok = true;                                   // warp-uniform
+        // this lane's vectors of a tile; the scales of the next item's are on their way while this one is drained
+        struct Row { uint32_t slot; float vs; bool have, live; };
+        auto fetch_row = [&](uint32_t tile, int m) {
+            const int row = m * kMmaM + quarter * 32 + lane;
+            const uint32_t pos = pos_begin + tile * kBlocksPerItem + uint32_t(row >> 5);
+            Row r{0u, 0.0f, pos < pos_end, false};
+            uint32_t blk = 0;
+            if (r.have) blk = p.live_blocks ? p.live_blocks[pos] : pos;
+            r.slot = blk * 32u + uint32_t(row & 31);            // slots are 32-bit
+            r.live = r.have && int64_t(r.slot) < p.n;
+            if (r.live && p.mask) r.live = (p.mask[r.slot >> 6] >> (r.slot & 63)) & 1ull;
+            if (r.live) r.vs = p.vec_scales[r.slot];
+            return r;
+        };
+        Row next[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) next[m] = fetch_row(vt, m);
         for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x, ++local_item) {
-            const int buf = local_item % kBufs, pb = local_item & 1;
-            int64_t slot[MT];
-            float vs[MT];
-            bool live[MT], have_row[MT];
-            float vs_warp = 0.0f;
+            const int buf = local_item % kBufs;
+            if (qg != qg_here) {                          // the same for all epilogue warps; once, unless the grid does not divide evenly
+                asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
+                load_columns<kTileQueries>(es, p, qg, et);
+                asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (my_columns) column_terms(qscale[4 * lane + e], qbias[4 * lane + e], qthr[4 * lane + e], u[e], w[e]);
+                qg_here = qg;
+            }
+            const uint32_t vt_cur = vt;
+            const int ql0 = qg * kTileQueries + cbase;
+            vt += vt_step; qg += qg_step;
+            if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
+            Row cur[MT];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) { cur[m] = next[m]; next[m] = fetch_row(vt, m); }
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const int row = m * kMmaM + quarter * 32 + lane;        // vector within the item
-                const uint32_t pos = pos_begin + vt * kBlocksPerItem + uint32_t(row >> 5);
-                const bool have = pos < pos_end;
-                have_row[m] = have;
-                uint32_t blk = 0;
-                if (have) blk = p.live_blocks ? p.live_blocks[pos] : pos;
-                slot[m] = int64_t(blk) * 32 + (row & 31);
-                live[m] = have && slot[m] < p.n;
-                if (live[m] && p.mask) live[m] = (p.mask[slot[m] >> 6] >> (slot[m] & 63)) & 1ull;
-                vs[m] = live[m] ? p.vec_scales[slot[m]] : 0.0f;
-                vs_warp = fmaxf(vs_warp, vs[m]);
-            }
-            // the largest vector scale of the item, for the integer dismissal bound of every query
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) vs_warp = fmaxf(vs_warp, __shfl_xor_sync(kFullMask, vs_warp, o));
-            if (lane == 0) sh->vs_part[pb][warp - 2] = vs_warp;
-            asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
-            // every warp is done with the item before; one warp's failure there ends the loop of all
-            if (*reinterpret_cast<volatile uint32_t *>(&sh->epilogue_failed)) break;
-            ring_flush<kFilter>(sh->ring, p.cb, kRingSize / 2, et, kEpilogueWarps * 32);
-            // per-query parameters of this item: one query per epilogue thread
-            {
-                float vs_max = 0.0f;
-#pragma unroll
-                for (int i = 0; i < kEpilogueWarps; ++i) vs_max = fmaxf(vs_max, sh->vs_part[pb][i]);
-                const int ql = qg * kTileQueries + et;
-                float qs = 0.f, qb = 0.f, th = INFINITY;
-                if (et < kTileQueries && ql < p.q_base + p.nq) {
-                    qs = p.qscale[ql]; qb = p.qbias[ql];
-                    const uint64_t key = p.cb.thr[ql];
-                    th = key == kEmptyKey ? -INFINITY : desc_bits_to_score(uint32_t(key >> 32));
+                const float vs_max = __uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(fmaxf(cur[m].vs, 0.0f))));
+                const float inv_vs = fminf(1.0f / vs_max, 1e30f);
+                __syncwarp();                             // the bounds of the tile before have been read
+                if (my_columns)
+                    reinterpret_cast<int4 *>(nbound)[lane] = make_int4(negated_bound(u[0], w[0], inv_vs), negated_bound(u[1], w[1], inv_vs),
+                                                                       negated_bound(u[2], w[2], inv_vs), negated_bound(u[3], w[3], inv_vs));
+                __syncwarp();
+                // a warp whose wait ran out drains and waits for nothing more, but still signs for its items and meets the others
+                if (m == 0) {
+                    ok = ok && __all_sync(kFullMask, mbar_wait(&sh->d_full[buf], (local_item / kBufs) & 1, p.cb.error));
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-                sh->qscale[pb][et] = qs; sh->qbias[pb][et] = qb; sh->qthr[pb][et] = th;
-                sh->ibound[pb][et] = dismissal_bound(qs, qb, th, vs_max);
-            }
-            asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
-
-            // warp-uniform outcome; a warp whose wait ran out still meets the others at the barriers of the next item
-            ok = __all_sync(kFullMask, mbar_wait(&sh->d_full[buf], (local_item / kBufs) & 1, p.cb.error));
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // the two warps of a lane quarter split the columns; below 64 columns the second one has none
-            constexpr int kColsPerHalf = kTileQueries >= 64 ? kTileQueries / 2 : kTileQueries;
-            const int cbase = half * kColsPerHalf;
-            const bool has_columns = cbase < kTileQueries;
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
                 const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(buf * MT + m) * kTileQueries + uint32_t(cbase);
                 for (int c0 = 0; c0 < (has_columns && ok ? kColsPerHalf : 0); c0 += 32) {
                     uint32_t acc[32];
@@ -225,30 +222,21 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (p.dense) {
                         // first chunk of a search: every vector's key goes to the list position of its place in the chunk
-                        const uint32_t at = (vt * kBlocksPerItem) * 32u + uint32_t(m * kMmaM + quarter * 32 + lane);
-                        if (have_row[m])
-                            write_piece<ONEHOT>(acc, &sh->qscale[pb][cbase + c0], &sh->qbias[pb][cbase + c0], fused, vs[m], live[m], slot[m],
-                                                qg * kTileQueries + cbase + c0, p.q_base + p.nq, at, p.cb);
+                        const uint32_t at = (vt_cur * kBlocksPerItem) * 32u + uint32_t(m * kMmaM + quarter * 32 + lane);
+                        if (cur[m].have)
+                            write_piece<ONEHOT>(acc, qscale + c0, qbias + c0, fused, cur[m].vs, cur[m].live, cur[m].slot, ql0 + c0, p.q_base + p.nq, at, p.cb);
                         continue;
                     }
-                    if constexpr (kFilter)
-                        filter_piece(acc, &sh->ibound[pb][cbase + c0], live[m], slot[m], qg * kTileQueries + cbase + c0, taddr + c0,
-                                     [&](int ql, uint64_t v) { ring_push<true>(sh->ring, p.cb, ql, v); });
-                    else
-                    sift_piece<ONEHOT>(acc, &sh->ibound[pb][cbase + c0], &sh->qscale[pb][cbase + c0], &sh->qbias[pb][cbase + c0], &sh->qthr[pb][cbase + c0],
-                                       fused, vs[m], live[m], slot[m], qg * kTileQueries + cbase + c0, taddr + c0,
-                                       [&](int ql, uint64_t key) { ring_push(sh->ring, p.cb, ql, key); });
+                    warp_sift<ONEHOT, kFilter>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, fused, cur[m].vs, cur[m].live, cur[m].slot,
+                                               ql0 + c0, taddr + c0, ring, p.cb);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh->d_empty[buf]);
-            if (!ok && lane == 0) sh->epilogue_failed = 1;
-            vt += vt_step; qg += qg_step;
-            if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
+            ring_flush<kFilter>(ring, p.cb, kRingSize / 2, lane);
         }
-        asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
-        ring_flush<kFilter>(sh->ring, p.cb, 1, et, kEpilogueWarps * 32);
+        ring_flush<kFilter>(ring, p.cb, 1, lane);
     } else {
         // ------------------------------------------------ expansion: codes -> int8 A slabs -------
         // The (item, slab) pairs of this CTA form one flat sequence; the code words of the next kAhead slabs

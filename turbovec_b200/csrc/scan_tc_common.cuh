@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda.h>
 
+#include <cfloat>
 #include <climits>
 #include <cstddef>
 
@@ -224,48 +225,11 @@ __device__ __forceinline__ void write_piece(const uint32_t (&acc)[32], const flo
     }
 }
 
-// Candidates on their way to the lists.  Appending one takes a global atomic whose result says where it goes, about a
-// microsecond that the epilogue warp would sit out for every single candidate; the warps of a CTA collect candidates in
-// shared memory instead and write them out together, one thread each, when the ring is half full and at the end.  What does
-// not fit goes to its list directly.  Order within a list does not matter.
-constexpr uint32_t kRingSize = 512;
-struct PushRing {
-    uint32_t n;
-    uint32_t pad[3];
-    uint64_t key[kRingSize];
-    uint32_t ql[kRingSize];
-};
 __device__ __forceinline__ void append_candidate(const CandidateBuffers &cb, int ql, uint64_t key) {
     if (key < cb.thr[ql] && (cb.lo == nullptr || key >= cb.lo[ql])) {
         const uint32_t at = atomicAdd(&cb.cnt[ql], 1u);
         if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
     }
-}
-// RAW: a survivor of a filtering scan, appended unseen (its exact key is computed later)
-template <bool RAW>
-__device__ __forceinline__ void append_any(const CandidateBuffers &cb, int ql, uint64_t key) {
-    if constexpr (RAW) {
-        const uint32_t at = atomicAdd(&cb.cnt[ql], 1u);
-        if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
-    } else {
-        append_candidate(cb, ql, key);
-    }
-}
-template <bool RAW = false>
-__device__ __forceinline__ void ring_push(PushRing &ring, const CandidateBuffers &cb, int ql, uint64_t key) {
-    const uint32_t at = atomicAdd(&ring.n, 1u);
-    if (at < kRingSize) { ring.key[at] = key; ring.ql[at] = uint32_t(ql); }
-    else append_any<RAW>(cb, ql, key);
-}
-// Called by every epilogue thread between two of the epilogue's barriers, where nobody pushes: `limit` = smallest fill
-// that is written out.  Uses barrier 1 (`threads` epilogue threads) itself when it writes.
-template <bool RAW = false>
-__device__ __forceinline__ void ring_flush(PushRing &ring, const CandidateBuffers &cb, uint32_t limit, int et, int threads) {
-    const uint32_t n = *reinterpret_cast<volatile uint32_t *>(&ring.n);
-    if (n < limit) return;
-    for (uint32_t i = et; i < min(n, kRingSize); i += threads) append_any<RAW>(cb, int(ring.ql[i]), ring.key[i]);
-    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-    if (et == 0) ring.n = 0;
 }
 
 // Which runs of 8 of a piece's 32 columns hold a sum at or above the column's bound for this lane's vector (bit = run).
@@ -311,11 +275,109 @@ __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int 
     }
 }
 
-// Filtering scans: `push` gets (query, slot) for every column whose sum reaches the bound; there is no score yet.
-template <typename Push>
-__device__ __forceinline__ void filter_piece(const uint32_t (&acc)[32], const int *ibound, bool live, int64_t slot, int ql0, uint32_t taddr, Push push) {
-    const uint32_t runs = surviving_runs(acc, ibound, live);
-    const uint32_t warp_runs = __reduce_or_sync(0xffffffffu, runs);
+// ---- epilogue of scan_tc.cu and scan_tc_dense2.cu: every warp on its own ------------------------------------------
+// An item with few K slabs leaves the epilogue about a thousand cycles, so it must not be a chain of barriers and
+// dependent loads.  The query group of a CTA stays the same from item to item, so the parameters of its columns are read
+// once; a warp derives the bounds of its columns from the largest scale of its own 32 vectors (a reciprocal and two
+// multiply-adds per column, four columns to a lane), which is also a tighter bound than one over the whole tile, and meets
+// no other warp.  A bound is kept negated: one add-and-max per column tells whether a run of 8 holds a survivor.
+// Candidates go through a ring of the warp: appending one takes a global atomic whose result says where it goes, about a
+// microsecond that the warp would sit out for every single candidate; it writes them out together, one lane each.
+constexpr int kWarpColumns = 128;                             // most columns of one epilogue warp
+constexpr uint32_t kRingSize = 64;
+constexpr int kFar = 1 << 29;                                 // beyond every integer sum (at most 127 * 127 * 16384 in magnitude)
+struct WarpRing {
+    uint64_t key[kRingSize];
+    uint32_t ql[kRingSize];
+    uint32_t n;
+    uint32_t pad;
+};
+struct EpilogueShared {
+    float qscale[kMaxTileQueries];    // per-query parameters of the query group
+    float qbias[kMaxTileQueries];
+    float qthr[kMaxTileQueries];      // score of the current k-th key (-inf while fewer than k results exist)
+    int nbound[kEpilogueWarps][kWarpColumns];   // per warp and column: minus the integer sum below which no vector of the warp is a candidate
+    WarpRing ring[kEpilogueWarps];
+};
+
+// One column's terms of the dismissal bound (see dismissal_bound): bound = u / vs_max - w, less the margin.
+__device__ __forceinline__ void column_terms(float qs, float qb, float t, float &u, float &w) {
+    u = t / qs; w = qb / qs;
+    if (t == INFINITY) { u = 0.0f; w = -1e30f; }                              // no query: nothing passes
+    else if (!(t > 0.0f) || !(qs > 0.0f) || !(u <= FLT_MAX) || !(fabsf(w) <= FLT_MAX)) { u = 0.0f; w = 1e30f; }   // everything passes
+}
+__device__ __forceinline__ int negated_bound(float u, float w, float inv_vs) {
+    const float x = u * inv_vs;
+    const float lo = (x - w) - (1.0e-5f * (x + fabsf(w)) + 2.0f);
+    return -__float2int_rd(fminf(fmaxf(lo, -float(kFar)), float(kFar)));
+}
+
+// Parameters of query group `qg` (NQT columns), by all epilogue threads; barriers on both sides are the caller's.
+template <int NQT>
+__device__ __forceinline__ void load_columns(EpilogueShared &es, const ScanParams &p, int qg, int et) {
+    if (et >= NQT) return;
+    const int ql = qg * NQT + et;
+    float qs = 0.f, qb = 0.f, th = INFINITY;
+    if (ql < p.q_base + p.nq) {
+        qs = p.qscale[ql]; qb = p.qbias[ql];
+        const uint64_t key = p.cb.thr[ql];
+        th = key == kEmptyKey ? -INFINITY : desc_bits_to_score(uint32_t(key >> 32));
+    }
+    es.qscale[et] = qs; es.qbias[et] = qb; es.qthr[et] = th;
+}
+
+// RAW: a survivor of a filtering scan, appended unseen (its exact key is computed later)
+template <bool RAW>
+__device__ __forceinline__ void append_any(const CandidateBuffers &cb, int ql, uint64_t key) {
+    if constexpr (RAW) {
+        const uint32_t at = atomicAdd(&cb.cnt[ql], 1u);
+        if (at < uint32_t(cb.cap)) cb.cand[size_t(ql) * cb.cap + at] = key;
+    } else {
+        append_candidate(cb, ql, key);
+    }
+}
+template <bool RAW>
+__device__ __forceinline__ void ring_push(WarpRing &ring, const CandidateBuffers &cb, int ql, uint64_t key) {
+    const uint32_t at = atomicAdd(&ring.n, 1u);
+    if (at < kRingSize) { ring.key[at] = key; ring.ql[at] = uint32_t(ql); }
+    else append_any<RAW>(cb, ql, key);
+}
+// by the whole warp: writes the ring out when it holds at least `limit` entries
+template <bool RAW>
+__device__ __forceinline__ void ring_flush(WarpRing &ring, const CandidateBuffers &cb, uint32_t limit, int lane) {
+    __syncwarp();
+    const uint32_t n = ring.n;
+    if (n < limit) return;
+    for (uint32_t i = lane; i < min(n, kRingSize); i += 32) append_any<RAW>(cb, int(ring.ql[i]), ring.key[i]);
+    __syncwarp();
+    if (lane == 0) ring.n = 0;
+    __syncwarp();
+}
+
+// One piece (32 accumulator columns of the lane's vector) against the warp's bounds; all pointers at the piece's first
+// column, `taddr` its address in tensor memory.  Runs of 8 columns that any lane of the warp flags are read again: RAW
+// appends (query, slot) of every column at its bound, else the exact score decides.  Every lane must call this.
+template <bool ONEHOT, bool RAW>
+__device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *nbound, const float *qscale, const float *qbias, const float *qthr,
+                                          bool fused, float vs, bool live, int64_t slot, int ql0, uint32_t taddr, WarpRing &ring,
+                                          const CandidateBuffers &cb) {
+    uint32_t runs = 0;
+    const int4 *pn = reinterpret_cast<const int4 *>(nbound);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int4 a = pn[2 * r], b = pn[2 * r + 1];
+        int m = int(acc[8 * r]) + a.x;
+        m = __viaddmax_s32(int(acc[8 * r + 1]), a.y, m);
+        m = __viaddmax_s32(int(acc[8 * r + 2]), a.z, m);
+        m = __viaddmax_s32(int(acc[8 * r + 3]), a.w, m);
+        m = __viaddmax_s32(int(acc[8 * r + 4]), b.x, m);
+        m = __viaddmax_s32(int(acc[8 * r + 5]), b.y, m);
+        m = __viaddmax_s32(int(acc[8 * r + 6]), b.z, m);
+        m = __viaddmax_s32(int(acc[8 * r + 7]), b.w, m);
+        runs |= uint32_t(m >= 0) << r;
+    }
+    if (!live) runs = 0;
+    const uint32_t warp_runs = __reduce_or_sync(kFullMask, runs);
     if (warp_runs == 0) return;
 #pragma unroll 1
     for (int c1 = 0; c1 < 32; c1 += 8) {
@@ -325,8 +387,15 @@ __device__ __forceinline__ void filter_piece(const uint32_t (&acc)[32], const in
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if ((runs >> (c1 >> 3)) & 1u) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (int(a8[e]) >= ibound[c1 + e]) push(ql0 + c1 + e, uint64_t(slot));
+            for (int e = 0; e < 8; ++e) {
+                const int c = c1 + e;
+                if constexpr (RAW) {
+                    if (int(a8[e]) + nbound[c] >= 0) ring_push<true>(ring, cb, ql0 + c, uint64_t(slot));
+                } else {
+                    const float score = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs);
+                    if (score >= qthr[c]) ring_push<false>(ring, cb, ql0 + c, make_key(score, uint32_t(slot)));
+                }
+            }
         }
     }
 }

@@ -36,16 +36,10 @@ struct DensePairShared {
     uint64_t d_full[2];               // per CTA: accumulator buffer complete
     uint64_t d_empty[2];              // leader's copy: buffer drained by the 8 epilogue warps of both CTAs
     uint32_t tmem_base;
-    uint32_t epilogue_failed;         // a wait of some epilogue warp ran out: all of them leave after the item
-    uint32_t pad[2];
-    float qscale[kMaxTileQueries];    // per-query parameters of the item's group
-    float qbias[kMaxTileQueries];
-    float qthr[kMaxTileQueries];
-    int ibound[kMaxTileQueries];      // per query: integer sum below which no vector of the item can be a candidate
-    float vs_part[2][4];              // largest vector scale per lane quarter (written by both column halves)
-    PushRing ring;                    // candidates of the epilogue warps
+    uint32_t pad[3];
+    EpilogueShared ep;
 };
-static_assert(offsetof(DensePairShared, qscale) % 16 == 0, "parameter arrays must be 16-byte aligned");
+static_assert(offsetof(DensePairShared, ep) % 16 == 0, "parameter arrays must be 16-byte aligned");
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap amap128,
@@ -67,8 +61,7 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
     const uint32_t n_items = n_vtiles * uint32_t(n_qgroups);
 
     if (tid == 0) {
-        sh->epilogue_failed = 0;
-        sh->ring.n = 0;
+        for (int w = 0; w < kEpilogueWarps; ++w) sh->ep.ring[w].n = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 2); mbar_init(&sh->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sh->d_full[b], 1); mbar_init(&sh->d_empty[b], 2 * kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -162,51 +155,55 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
         const int quarter = warp & 3;                     // TMEM lanes 32*quarter .. +31 are this warp's
         const int chalf = (warp - kFirstEpilogueWarp) >> 2;   // which 128 of the item's 256 query columns
         const int et = (warp - kFirstEpilogueWarp) * 32 + lane;   // 0..255 among the epilogue threads
+        EpilogueShared &es = sh->ep;
+        const int ew = warp - kFirstEpilogueWarp;
+        WarpRing &ring = es.ring[ew];
+        int *nbound = es.nbound[ew];
+        const int cbase = chalf * 128;                    // first of this warp's columns
+        const float *qscale = es.qscale + cbase, *qbias = es.qbias + cbase, *qthr = es.qthr + cbase;
+        const int row = quarter * 32 + lane;
         uint32_t local_item = 0;
         uint32_t vt = cluster_id / uint32_t(n_qgroups);
-        int qg = int(cluster_id % uint32_t(n_qgroups));
-        bool ok = true;
+        int qg = int(cluster_id % uint32_t(n_qgroups)), qg_here = -1;
+        float u[4], w[4];
+        bool ok = true;                                   // warp-uniform
+        // this lane's vector of a tile; the scale of the next item's is on its way while this one is drained
+        struct Row { uint32_t slot; float vs; bool have, live; };
+        auto fetch_row = [&](uint32_t tile) {
+            const uint32_t pos = pos_begin + (tile * 2 + rank) * kBlocksPerCta + uint32_t(row >> 5);
+            Row r{0u, 0.0f, pos < pos_end, false};
+            uint32_t blk = 0;
+            if (r.have) blk = p.live_blocks ? p.live_blocks[pos] : pos;
+            r.slot = blk * 32u + uint32_t(row & 31);            // slots are 32-bit
+            r.live = r.have && int64_t(r.slot) < p.n;
+            if (r.live && p.mask) r.live = (p.mask[r.slot >> 6] >> (r.slot & 63)) & 1ull;
+            if (r.live) r.vs = p.vec_scales[r.slot];
+            return r;
+        };
+        Row next = fetch_row(vt);
         for (uint32_t item = cluster_id; item < n_items; item += n_clusters, ++local_item) {
             const int buf = local_item & 1;
-            // this lane's vector, and the largest vector scale of this CTA's tile (dismissal_bound)
-            const int row = quarter * 32 + lane;
-            const uint32_t pos = pos_begin + (vt * 2 + rank) * kBlocksPerCta + uint32_t(row >> 5);
-            const bool have_row = pos < pos_end;
-            uint32_t blk = 0;
-            if (have_row) blk = p.live_blocks ? p.live_blocks[pos] : pos;
-            const int64_t slot = int64_t(blk) * 32 + (row & 31);
-            bool live = have_row && slot < p.n;
-            if (live && p.mask) live = (p.mask[slot >> 6] >> (slot & 63)) & 1ull;
-            const float vs = live ? p.vec_scales[slot] : 0.0f;
-            {
-                float m = vs;
+            if (qg != qg_here) {                          // the same for all epilogue warps; once, unless the clusters do not divide evenly
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                load_columns<kTileQueries>(es, p, qg, et);
+                asm volatile("bar.sync 1, 256;" ::: "memory");
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(kFullMask, m, o));
-                if (lane == 0) sh->vs_part[chalf][quarter] = m;
+                for (int e = 0; e < 4; ++e) column_terms(qscale[4 * lane + e], qbias[4 * lane + e], qthr[4 * lane + e], u[e], w[e]);
+                qg_here = qg;
             }
-            // every warp is done with the item before (and its parameters); one warp's failure there ends the loop of all
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (*reinterpret_cast<volatile uint32_t *>(&sh->epilogue_failed)) { ok = false; break; }
-            ring_flush(sh->ring, p.cb, kRingSize / 2, et, kEpilogueWarps * 32);
-            const float *vp = sh->vs_part[0];
-            const float vs_max = fmaxf(fmaxf(vp[0], vp[1]), fmaxf(vp[2], vp[3]));
-            {
-                const int ql = qg * kTileQueries + et;
-                float qs = 0.f, qb = 0.f, th = INFINITY;
-                if (ql < p.q_base + p.nq) {
-                    qs = p.qscale[ql]; qb = p.qbias[ql];
-                    const uint64_t key = p.cb.thr[ql];
-                    th = key == kEmptyKey ? -INFINITY : desc_bits_to_score(uint32_t(key >> 32));
-                }
-                sh->qscale[et] = qs; sh->qbias[et] = qb; sh->qthr[et] = th;
-                sh->ibound[et] = dismissal_bound(qs, qb, th, vs_max);
-            }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-
-            const int cbase = chalf * 128;                               // first of this warp's columns
-            const float *qscale = sh->qscale + cbase, *qbias = sh->qbias + cbase, *qthr = sh->qthr + cbase;
-            // warp-uniform outcome; a warp whose wait ran out still meets the others at the barrier below
-            ok = __all_sync(kFullMask, mbar_wait(&sh->d_full[buf], (local_item >> 1) & 1, p.cb.error));
+            const Row cur = next;
+            const uint32_t vt_cur = vt;
+            const int ql0 = qg * kTileQueries + cbase;
+            vt += vt_step; qg += qg_step;
+            if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
+            next = fetch_row(vt);
+            const float vs_max = __uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(fmaxf(cur.vs, 0.0f))));
+            const float inv_vs = fminf(1.0f / vs_max, 1e30f);
+            reinterpret_cast<int4 *>(nbound)[lane] = make_int4(negated_bound(u[0], w[0], inv_vs), negated_bound(u[1], w[1], inv_vs),
+                                                               negated_bound(u[2], w[2], inv_vs), negated_bound(u[3], w[3], inv_vs));
+            __syncwarp();
+            // a warp whose wait ran out drains and waits for nothing more, but still signs for its items and meets the others
+            ok = ok && __all_sync(kFullMask, mbar_wait(&sh->d_full[buf], (local_item >> 1) & 1, p.cb.error));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(buf) * kTileQueries + uint32_t(cbase);
             for (int c0 = 0; c0 < (ok ? 128 : 0); c0 += 32) {
@@ -215,25 +212,20 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (p.dense) {
                     // first chunk of a search: every vector's key goes to the list position of its place in the chunk
-                    const uint32_t at = ((vt * 2 + rank) * kBlocksPerCta) * 32u + uint32_t(row);
-                    if (have_row)
-                        write_piece<ONEHOT>(acc, qscale + c0, qbias + c0, fused, vs, live, slot, qg * kTileQueries + cbase + c0, p.q_base + p.nq, at, p.cb);
+                    const uint32_t at = ((vt_cur * 2 + rank) * kBlocksPerCta) * 32u + uint32_t(row);
+                    if (cur.have)
+                        write_piece<ONEHOT>(acc, qscale + c0, qbias + c0, fused, cur.vs, cur.live, cur.slot, ql0 + c0, p.q_base + p.nq, at, p.cb);
                     continue;
                 }
-                sift_piece<ONEHOT>(acc, sh->ibound + cbase + c0, qscale + c0, qbias + c0, qthr + c0, fused, vs, live, slot,
-                                   qg * kTileQueries + cbase + c0, taddr + c0,
-                                   [&](int ql, uint64_t key) { ring_push(sh->ring, p.cb, ql, key); });
+                warp_sift<ONEHOT, false>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, fused, cur.vs, cur.live, cur.slot, ql0 + c0,
+                                         taddr + c0, ring, p.cb);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->d_empty[buf]), 0));   // the leader's barrier counts both CTAs
-            // the barriers of the next item need all eight warps
-            if (!ok && lane == 0) sh->epilogue_failed = 1;
-            vt += vt_step; qg += qg_step;
-            if (qg >= n_qgroups) { qg -= n_qgroups; ++vt; }
+            ring_flush<false>(ring, p.cb, kRingSize / 2, lane);
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        ring_flush(sh->ring, p.cb, 1, et, kEpilogueWarps * 32);
+        ring_flush<false>(ring, p.cb, 1, lane);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
