@@ -123,7 +123,7 @@ struct SearchCtx {
     DeviceArray<float> d_stage;              // query upload
     DeviceArray<float> d_qrot;               // tv_rotate
     DeviceArray<float> d_qscale, d_qbias;
-    DeviceArray<float> d_filter;             // affine bound of a filtering scan: scale, middle and upper bias per query
+    DeviceArray<float> d_filter;             // affine bound of a filtering scan per query
     DeviceArray<uint8_t> d_luts;
     DeviceArray<int8_t> d_weights;
     DeviceArray<uint32_t> d_wfrag;
@@ -757,7 +757,7 @@ struct SearchScratch {
     uint64_t *cand, *thr, *topk, *lo;      // lo: lowest admissible key per query (paged top-k), or nullptr
     uint32_t *cnt, *done;                  // done follows cnt: both are cleared together
     size_t w_rows, dim_pad, lut_pitch;
-    float *f_scale, *f_mid, *f_max;        // affine bound of a filtering scan
+    float *f_scale, *f_mid, *f_max, *f_alpha, *f_suffix;   // affine bound of a filtering scan
     int cap;
     bool allow_tc;
 };
@@ -972,6 +972,7 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
                      const MaskOnDevice &m) {
     const size_t n_blocks = (h->n + kBlock - 1) / kBlock;
     const float *qscale = S.qscale, *qbias = S.qbias;
+    sp.f_weights = S.weights; sp.f_pitch = int(S.dim_pad); sp.f_alpha = S.f_alpha; sp.f_suffix = S.f_suffix;
     auto scan = [&](size_t begin, size_t end, const float *bias, bool dense) -> int {
         sp.pos_begin = uint32_t(begin); sp.pos_end = uint32_t(end); sp.dense = dense ? 1 : 0;
         sp.qscale = S.f_scale; sp.qbias = bias; sp.q_base = 0; sp.nq = int(nq);
@@ -1130,6 +1131,7 @@ int enqueue_query_prep(tv_index *h, cudaStream_t st, const SearchScratch &S, con
     qp.cnt = S.cnt; qp.done = S.done; qp.thr = S.thr; qp.topk = S.topk; qp.k = int(kk);
     if (plan.use_filter) {
         qp.filter.weights = S.weights; qp.filter.scale = S.f_scale; qp.filter.bias_mid = S.f_mid; qp.filter.bias_max = S.f_max;
+        qp.filter.alpha = S.f_alpha; qp.filter.suffix = S.f_suffix;
         for (int i = 0; i < 8; ++i) qp.filter.levels[i] = h->levels[i];
     }
     // the tensor-memory scans read whole groups of 256 operand rows and whole K slabs
@@ -1206,7 +1208,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     TV_CUDA(c.d_qbias.reserve(nq_pad));
     const size_t w_rows = (nq + 255) / 256 * 256;
     if (mode == TV_SCORE_PERMUTE_DOT || plan.use_filter) TV_CUDA(c.d_weights.reserve(w_rows * dim_pad));
-    if (plan.use_filter) TV_CUDA(c.d_filter.reserve(3 * nq_pad));
+    if (plan.use_filter) TV_CUDA(c.d_filter.reserve((4 + kFilterBatches) * nq_pad));
     if (mode == TV_SCORE_PERMUTE_DOT) {
         TV_CUDA(c.d_wfrag.reserve(size_t(ksteps) * mt_total * 32 * 4));
     } else {
@@ -1259,7 +1261,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         if (rc != TV_OK) return rc;
     }
 
-    if (plan.use_filter) { S.f_scale = c.d_filter.ptr; S.f_mid = S.f_scale + nq_pad; S.f_max = S.f_mid + nq_pad; }
+    if (plan.use_filter) { S.f_scale = c.d_filter.ptr; S.f_mid = S.f_scale + nq_pad; S.f_max = S.f_mid + nq_pad; S.f_alpha = S.f_max + nq_pad; S.f_suffix = S.f_alpha + nq_pad; }
     rc = enqueue_query_prep(h, st, S, plan, mode, dq, nq, k_page, &c.d_flags->first_invalid);
     if (rc != TV_OK) return rc;
 

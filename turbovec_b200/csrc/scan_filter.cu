@@ -15,11 +15,13 @@
 // They are found again by the filtering scans, which cover the first chunk as well.
 //
 // What bounds the scoring is the gather: a vector's bytes lie 32 apart (one per sector) in its code block, so every byte
-// costs a sector.  A warp scores four survivors at a time to keep enough of them in flight.
+// costs a sector.  A warp scores four survivors at a time to keep enough of them in flight, and leaves a survivor as soon
+// as it can no longer reach the threshold: after every 128 byte-groups the bound is the exact sum so far, plus alpha times
+// what W . L has left, plus the largest deviations of the remaining half-bytes (suffix sums from query preparation).  The
+// sum of deviations is what let most survivors through, and it shrinks with every batch.
 #include <algorithm>
 
-#include "search.cuh"
-#include "tv_common.cuh"
+#include "scan_tc_common.cuh"
 
 namespace tv {
 namespace {
@@ -28,42 +30,82 @@ constexpr int kScoreThreads = 256;
 constexpr int kScoreWarps = kScoreThreads / 32;
 constexpr int kTogether = 4;               // survivors per warp and step
 
-// The exact keys of up to kTogether slots; valid in every lane.
-template <typename Emit>
-__device__ __forceinline__ void exact_keys(const ScanParams &p, const uint8_t *lut, int q, const uint32_t (&slot)[kTogether], int lane, Emit emit) {
+// The exact keys of up to kTogether slots, valid in every lane.  EXIT: `sum` = W . L of each; a survivor that drops out on
+// the way gets kEmptyKey.
+template <bool EXIT, typename Emit>
+__device__ __forceinline__ void exact_keys(const ScanParams &p, const uint8_t *lut, const uint32_t *wq, int q, const uint32_t (&slot)[kTogether],
+                                           const int (&sum)[kTogether], uint64_t thr, int lane, Emit emit) {
     const int ng = p.ngroups;
     const uint8_t *src[kTogether];
-#pragma unroll
-    for (int j = 0; j < kTogether; ++j) src[j] = p.codes + size_t(slot[j] >> 5) * ng * 32 + (slot[j] & 31u);
-    float facc[kTogether];
-    int total[kTogether];
+    float facc[kTogether], vs[kTogether];
+    int total[kTogether], need[kTogether], left[kTogether];
     const float qs = p.qscale[q], qb = p.qbias[q];
+    const float alpha = EXIT ? p.f_alpha[q] : 0.0f;
+    const float t = thr == kEmptyKey ? -INFINITY : desc_bits_to_score(uint32_t(thr >> 32));
+    uint32_t alive = (1u << kTogether) - 1u;
 #pragma unroll
-    for (int j = 0; j < kTogether; ++j) { facc[j] = qb; total[j] = 0; }
-    for (int g0 = 0; g0 < ng; g0 += 256) {
-        const int g1 = min(g0 + 256, ng);
-        int sum[kTogether];
+    for (int j = 0; j < kTogether; ++j) {
+        src[j] = p.codes + size_t(slot[j] >> 5) * ng * 32 + (slot[j] & 31u);
+        vs[j] = p.vec_scales[slot[j]];
+        facc[j] = qb; total[j] = 0; left[j] = sum[j];
+        need[j] = EXIT ? dismissal_bound(qs, qb, t, vs[j]) : 0;
+    }
+    for (int g0 = 0; g0 < ng && alive; g0 += 256) {
+        int part[kTogether];
 #pragma unroll
-        for (int j = 0; j < kTogether; ++j) sum[j] = 0;
-#pragma unroll 4
-        for (int g = g0 + lane; g < g1; g += 32) {
+        for (int j = 0; j < kTogether; ++j) part[j] = 0;
+#pragma unroll
+        for (int h0 = g0; h0 < g0 + 256; h0 += kFilterBatch) {
+            if (h0 >= ng || !alive) break;
+            int s[kTogether], w[kTogether];
+#pragma unroll
+            for (int j = 0; j < kTogether; ++j) { s[j] = 0; w[j] = 0; }
+            uint32_t byte[kFilterBatch / 32][kTogether];
+#pragma unroll
+            for (int i = 0; i < kFilterBatch / 32; ++i)
+#pragma unroll
+                for (int j = 0; j < kTogether; ++j) {
+                    const int g = h0 + 32 * i + lane;
+                    byte[i][j] = g < ng && ((alive >> j) & 1u) ? __ldg(src[j] + size_t(g) * 32) : 0u;
+                }
+#pragma unroll
+            for (int i = 0; i < kFilterBatch / 32; ++i) {
+                const int g = h0 + 32 * i + lane;
+                if (g >= ng) continue;
+                const uint32_t wg = EXIT ? wq[g] : 0u;
+#pragma unroll
+                for (int j = 0; j < kTogether; ++j) {
+                    const uint32_t b = byte[i][j];
+                    s[j] += int(lut[g * 32 + (b >> 4)]) + int(lut[g * 32 + 16 + (b & 15u)]);
+                    if constexpr (EXIT) {
+                        // selectors of the byte's levels, in the order of wq
+                        const uint32_t sel = p.bits == 2 ? (b & 0x33u) | ((b >> 2) & 0x33u) << 8 : b;
+                        w[j] = __dp4a(int(__byte_perm(p.level_words[0], p.level_words[1], sel)), int(wg), w[j]);
+                    }
+                }
+            }
+            const float rest = EXIT ? p.f_suffix[size_t(q) * kFilterBatches + h0 / kFilterBatch + 1] : 0.0f;
 #pragma unroll
             for (int j = 0; j < kTogether; ++j) {
-                const uint32_t byte = __ldg(src[j] + size_t(g) * 32);
-                sum[j] += int(lut[g * 32 + (byte >> 4)]) + int(lut[g * 32 + 16 + (byte & 15u)]);
+                part[j] += __reduce_add_sync(kFullMask, s[j]);
+                if constexpr (EXIT) {
+                    left[j] -= __reduce_add_sync(kFullMask, w[j]);
+                    // 1e-3 + 1e-6 of the terms: their roundings
+                    const float more = alpha * float(left[j]);
+                    if (float(total[j] + part[j]) + more + rest + (1e-3f + 1e-6f * (fabsf(more) + fabsf(rest))) < float(need[j])) alive &= ~(1u << j);
+                }
             }
         }
 #pragma unroll
         for (int j = 0; j < kTogether; ++j) {
-            sum[j] = __reduce_add_sync(kFullMask, sum[j]);
-            facc[j] = fmaf(qs, float(sum[j]), facc[j]);
-            total[j] += sum[j];
+            facc[j] = fmaf(qs, float(part[j]), facc[j]);
+            total[j] += part[j];
         }
     }
 #pragma unroll
     for (int j = 0; j < kTogether; ++j) {
         const float pre = p.mode == kModeLutFlush ? facc[j] : __fadd_rn(__fmul_rn(float(total[j]), qs), qb);
-        emit(j, make_key(__fmul_rn(pre, p.vec_scales[slot[j]]), slot[j]));
+        emit(j, (alive >> j) & 1u ? make_key(__fmul_rn(pre, vs[j]), slot[j]) : kEmptyKey);
     }
 }
 
@@ -72,22 +114,41 @@ __device__ __forceinline__ void load_tables(const ScanParams &p, int q, uint4 *l
     for (int i = threadIdx.x; i < p.ngroups * 2; i += kScoreThreads) lut[i] = src[i];
 }
 
-// cand[q][i] = slot -> exact key, or kEmptyKey when it does not beat the k-th best.  Grid (shares of a list, queries).
+// The int8 weights of a byte-group in one word, in the order of its levels: 2-bit coordinates 3, 1, 2, 0; 3-bit 1, 0.
+__device__ __forceinline__ void load_weights(const ScanParams &p, int q, uint32_t *wq) {
+    const uint8_t *row = reinterpret_cast<const uint8_t *>(p.f_weights) + size_t(q) * p.f_pitch;
+    for (int g = threadIdx.x; g < p.ngroups; g += kScoreThreads) {
+        if (p.bits == 2) {                                // rows of levels2_coord order: pairs of bytes in words w and w + 2 of a chunk
+            const uint8_t *c = row + (g >> 2) * 16 + ((g >> 1) & 1) * 4 + (g & 1) * 2;
+            wq[g] = uint32_t(*reinterpret_cast<const uint16_t *>(c)) | uint32_t(*reinterpret_cast<const uint16_t *>(c + 8)) << 16;
+        } else {
+            wq[g] = *reinterpret_cast<const uint16_t *>(row + 2 * g);
+        }
+    }
+}
+
+// cand[q][i] = (W . L, slot) -> exact key, or kEmptyKey when it does not beat the k-th best.  Grid (shares of a list, queries).
 __global__ void __launch_bounds__(kScoreThreads) score_survivors_kernel(ScanParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint32_t *wq = reinterpret_cast<uint32_t *>(smem_raw + size_t(p.ngroups) * 32);
     const int q = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = min(p.cb.cnt[q], uint32_t(p.cb.cap));
     if (blockIdx.x * kScoreWarps * kTogether >= n) return;
     load_tables(p, q, reinterpret_cast<uint4 *>(smem_raw));
+    load_weights(p, q, wq);
     __syncthreads();
     uint64_t *list = p.cb.cand + size_t(q) * p.cb.cap;
     const uint64_t thr = p.cb.thr[q];
     for (uint32_t i = (blockIdx.x * kScoreWarps + warp) * kTogether; i < n; i += gridDim.x * kScoreWarps * kTogether) {
         uint32_t slot[kTogether];
+        int sum[kTogether];
 #pragma unroll
-        for (int j = 0; j < kTogether; ++j) slot[j] = uint32_t(list[min(i + j, n - 1)]);
+        for (int j = 0; j < kTogether; ++j) {
+            const uint64_t v = list[min(i + j, n - 1)];
+            slot[j] = uint32_t(v); sum[j] = int(uint32_t(v >> 32));
+        }
         __syncwarp();                                     // every lane has read the slots before lane 0 puts keys there
-        exact_keys(p, smem_raw, q, slot, lane, [&](int j, uint64_t key) {
+        exact_keys<true>(p, smem_raw, wq, q, slot, sum, thr, lane, [&](int j, uint64_t key) {
             if (lane == 0 && i + j < n) list[i + j] = key < thr ? key : kEmptyKey;
         });
     }
@@ -110,7 +171,8 @@ __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) 
             uint32_t slot[kTogether];
 #pragma unroll
             for (int j = 0; j < kTogether; ++j) slot[j] = uint32_t(top[min(i + j, k - 1)]);
-            exact_keys(p, smem_raw, q, slot, lane, [&](int, uint64_t key) { mine = max(mine, key); });
+            const int none[kTogether] = {};
+            exact_keys<false>(p, smem_raw, nullptr, q, slot, none, kEmptyKey, lane, [&](int, uint64_t key) { mine = max(mine, key); });
         }
     }
     if (lane == 0) worst[warp] = mine;
@@ -125,11 +187,11 @@ __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) 
 }  // namespace
 
 bool scan_filter_supported(int bits, int mode, int ngroups, size_t smem_limit) {
-    return tensor_map_encoder() != nullptr && (bits == 2 || bits == 3) && (mode == kModeLutMulAdd || mode == kModeLutFlush) && size_t(ngroups) * 32 + 1024 <= smem_limit;
+    return tensor_map_encoder() != nullptr && (bits == 2 || bits == 3) && (mode == kModeLutMulAdd || mode == kModeLutFlush) && size_t(ngroups) * 36 + 1024 <= smem_limit && ngroups <= kFilterBatch * (kFilterBatches - 1);
 }
 
 cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cudaStream_t s) {
-    const size_t smem = size_t(p.ngroups) * 32;
+    const size_t smem = size_t(p.ngroups) * 36;
     cudaError_t e = cudaFuncSetAttribute(score_survivors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     for (int q0 = 0; q0 < nq; q0 += 32768) {
@@ -137,6 +199,7 @@ cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cu
         ScanParams part = p;
         part.cb.cand += size_t(q0) * p.cb.cap; part.cb.cnt += q0; part.cb.thr += q0;
         part.luts += size_t(q0) * p.lut_pitch; part.qscale += q0; part.qbias += q0;
+        part.f_alpha += q0; part.f_suffix += size_t(q0) * kFilterBatches; part.f_weights += size_t(q0) * p.f_pitch;
         // about eight CTAs per SM over all queries, at least one per query, none without a first step of its own
         const unsigned shares = unsigned(std::max(1, std::min(8 * sm_count / here, p.cb.cap / (kScoreWarps * kTogether))));
         score_survivors_kernel<<<dim3(shares, unsigned(here)), kScoreThreads, smem, s>>>(part);

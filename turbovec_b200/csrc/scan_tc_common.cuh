@@ -356,7 +356,7 @@ __device__ __forceinline__ void ring_flush(WarpRing &ring, const CandidateBuffer
 
 // One piece (32 accumulator columns of the lane's vector) against the warp's bounds; all pointers at the piece's first
 // column, `taddr` its address in tensor memory.  Runs of 8 columns that any lane of the warp flags are read again: RAW
-// appends (query, slot) of every column at its bound, else the exact score decides.  Every lane must call this.
+// appends (sum, slot) of every column at its bound, else the exact score decides.  Every lane must call this.
 template <bool ONEHOT, bool RAW>
 __device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *nbound, const float *qscale, const float *qbias, const float *qthr,
                                           bool fused, float vs, bool live, int64_t slot, int ql0, uint32_t taddr, WarpRing &ring,
@@ -390,7 +390,10 @@ __device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *
             for (int e = 0; e < 8; ++e) {
                 const int c = c1 + e;
                 if constexpr (RAW) {
-                    if (int(a8[e]) + nbound[c] >= 0) ring_push<true>(ring, cb, ql0 + c, uint64_t(slot));
+                    // the bound with the vector's own scale in place of the warp's largest; the margin covers its roundings
+                    const float up = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs), t = qthr[c];
+                    if (int(a8[e]) + nbound[c] >= 0 && up + 1.0e-5f * (fabsf(up) + fabsf(t)) >= t)
+                        ring_push<true>(ring, cb, ql0 + c, uint64_t(a8[e]) << 32 | uint64_t(slot));
                 } else {
                     const float score = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs);
                     if (score >= qthr[c]) ring_push<false>(ring, cb, ql0 + c, make_key(score, uint32_t(slot)));

@@ -69,8 +69,9 @@ __device__ __forceinline__ int levels2_coord(int w, int b) { return (w & 1) * 8 
 // is evaluated in f32 (values up to 127: 5e-5 covers it) and summed in f64; 1e-5 of the reference's own bias covers the
 // roundings of its float epilogue, whose terms are that large before they cancel.
 template <int BITS>
-__device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mins, const float *centroids, float *red, int q, float bias_corr) {
+__device__ void lut_tables(const QueryPrepParams &p, const float *row, float *dev, float *mins, const float *centroids, float *red, int q, float bias_corr) {
     __shared__ double part[2][kPrepThreads / 32];
+    __shared__ double batch_sum[kFilterBatches];
     __shared__ float s_bias;
     constexpr int kCoords = BITS == 2 ? 2 : 1;                     // per half-byte: 8 / BITS / 2
     const int ng = p.ngroups, tid = threadIdx.x;
@@ -140,6 +141,7 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mi
                         lo = fminf(lo, e[nib] - fit);
                         hi = fmaxf(hi, e[nib] - fit);
                     }
+                    dev[h] = hi + 5e-5f;
                     beta += 0.5 * (double(hi) + double(lo));
                     slack += 0.5 * (double(hi) - double(lo)) + 5e-5;
                 }
@@ -165,11 +167,25 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *mi
     }
     if ((tid & 31) == 0) { part[0][tid >> 5] = beta; part[1][tid >> 5] = slack; }
     __syncthreads();
+    // suffix sums of the largest deviations by batches of byte-groups
+    const int batches = (ng + kFilterBatch - 1) / kFilterBatch;
+    for (int b = tid >> 5; b < batches; b += kPrepThreads / 32) {
+        double sum = 0.0;
+        for (int h = 2 * kFilterBatch * b + (tid & 31); h < min(2 * kFilterBatch * (b + 1), 2 * ng); h += 32) sum += double(dev[h]);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
+        if ((tid & 31) == 0) batch_sum[b] = sum;
+    }
+    __syncthreads();
     if (tid == 0) {
         beta = slack = 0.0;
         for (int w = 0; w < kPrepThreads / 32; ++w) { beta += part[0][w]; slack += part[1][w]; }
         const double base = double(scale) * beta + double(s_bias);
         p.filter.scale[q] = float(double(scale) * double(alpha));
+        double rest = 0.0;
+        float *suffix = p.filter.suffix + size_t(q) * kFilterBatches;
+        suffix[batches] = 0.0f;
+        for (int b = batches - 1; b >= 0; --b) { rest += batch_sum[b]; suffix[b] = float(rest + 1e-2 + 1e-6 * fabs(rest)); }
+        p.filter.alpha[q] = alpha;
         p.filter.bias_mid[q] = float(base);
         p.filter.bias_max[q] = float(base + double(scale) * slack * 1.000001 + 1e-5 * fabs(double(s_bias)));
     }
@@ -283,11 +299,11 @@ __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParam
             p.wfrag[frag] = word;
         }
     } else if (p.bits == 2) {                                       // search.rs:2856-2994
-        lut_tables<2>(p, rowA, mins, s_centroids, red, q, bias_corr);
+        lut_tables<2>(p, rowA, rowB, mins, s_centroids, red, q, bias_corr);
     } else if (p.bits == 3) {
-        lut_tables<3>(p, rowA, mins, s_centroids, red, q, bias_corr);
+        lut_tables<3>(p, rowA, rowB, mins, s_centroids, red, q, bias_corr);
     } else {
-        lut_tables<4>(p, rowA, mins, s_centroids, red, q, bias_corr);
+        lut_tables<4>(p, rowA, rowB, mins, s_centroids, red, q, bias_corr);
     }
 }
 

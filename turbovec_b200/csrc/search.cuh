@@ -10,6 +10,10 @@ namespace tv {
 // Float epilogues of the reference's kernel families (turbovec/src/search.rs:1523, 1176, 1596).
 enum ScoreMode : int { kModePermuteDot = 1, kModeLutMulAdd = 2, kModeLutFlush = 3 };
 
+// Batches of byte-groups after which the exact scoring of a filtering scan's survivors looks at the bound again; together
+// they cover every geometry whose tables fit in shared memory.
+constexpr int kFilterBatch = 128, kFilterBatches = 66;
+
 struct QueryPrepParams {
     const float *queries;          // [nq][dim] device
     int nq, dim, bits, ngroups;
@@ -36,6 +40,9 @@ struct QueryPrepParams {
         int8_t *weights;           // [rows][dim_pad], coordinates in the order of the expanded levels
         float *scale;              // [nq] a score is close to fma(W . L, scale, bias_mid) and at most fma(W . L, scale, bias_max)
         float *bias_mid, *bias_max;
+        float *alpha;              // [nq] isum is close to alpha * (W . L) + a constant
+        float *suffix;             // [nq][kFilterBatches] largest deviations from that, summed over the byte-groups from
+                                   // kFilterBatch * i on (and 0 past the last one)
         int8_t levels[8];
     } filter;
     // selection state of the batch, reset here (cnt == nullptr: none)
@@ -124,6 +131,10 @@ struct ScanParams {
     // LUT
     const uint8_t *luts;
     int lut_pitch;                 // bytes between the tables of consecutive queries
+    // exact scoring behind a filtering scan (QueryPrepParams::Filter)
+    const int8_t *f_weights;
+    int f_pitch;
+    const float *f_alpha, *f_suffix;
 };
 // Permute-dot scan on mma.sync (int8 x int8 -> int32), up to 64 queries per launch.
 cudaError_t launch_scan_pd(const ScanParams &p, int sm_count, cudaStream_t s);
