@@ -82,7 +82,6 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
     const uint32_t n_items = n_vtiles * uint32_t(n_qgroups);
 
     if (tid == 0) {
-        for (int w = 0; w < kEpilogueWarps; ++w) sh->ep.ring[w].n = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], kExpandWarps + 1); mbar_init(&sh->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sh->d_full[b], 1); mbar_init(&sh->d_empty[b], kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -164,6 +163,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
         uint32_t vt = blockIdx.x / uint32_t(n_qgroups);
         int qg = int(blockIdx.x % uint32_t(n_qgroups)), qg_here = -1;
         float u[4], w[4];
+        uint32_t fill = 0;                                // entries in the warp's ring
         const bool my_columns = has_columns && 4 * lane < kColsPerHalf;   // lane: columns 4 lane .. + 3 of the warp's
         bool ok = true;                                   // warp-uniform
         // this lane's vectors of a tile; the scales of the next item's are on their way while this one is drained
@@ -228,15 +228,15 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                         continue;
                     }
                     warp_sift<ONEHOT, kFilter>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, fused, cur[m].vs, cur[m].live, cur[m].slot,
-                                               ql0 + c0, taddr + c0, ring, p.cb);
+                                               ql0 + c0, ring, fill, p.cb, lane);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh->d_empty[buf]);
-            ring_flush<kFilter>(ring, p.cb, kRingSize / 2, lane);
+            ring_flush<kFilter>(ring, fill, p.cb, kRingSize / 2, lane);
         }
-        ring_flush<kFilter>(ring, p.cb, 1, lane);
+        ring_flush<kFilter>(ring, fill, p.cb, 1, lane);
     } else {
         // ------------------------------------------------ expansion: codes -> int8 A slabs -------
         // The (item, slab) pairs of this CTA form one flat sequence; the code words of the next kAhead slabs

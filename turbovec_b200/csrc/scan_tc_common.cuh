@@ -286,11 +286,9 @@ __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int 
 constexpr int kWarpColumns = 128;                             // most columns of one epilogue warp
 constexpr uint32_t kRingSize = 64;
 constexpr int kFar = 1 << 29;                                 // beyond every integer sum (at most 127 * 127 * 16384 in magnitude)
-struct WarpRing {
+struct WarpRing {                    // the warp keeps the fill count in a register
     uint64_t key[kRingSize];
     uint32_t ql[kRingSize];
-    uint32_t n;
-    uint32_t pad;
 };
 struct EpilogueShared {
     float qscale[kMaxTileQueries];    // per-query parameters of the query group
@@ -336,31 +334,35 @@ __device__ __forceinline__ void append_any(const CandidateBuffers &cb, int ql, u
         append_candidate(cb, ql, key);
     }
 }
+// by the whole warp: lanes with `on` add their entry; `fill` (warp-uniform) counts the entries
 template <bool RAW>
-__device__ __forceinline__ void ring_push(WarpRing &ring, const CandidateBuffers &cb, int ql, uint64_t key) {
-    const uint32_t at = atomicAdd(&ring.n, 1u);
-    if (at < kRingSize) { ring.key[at] = key; ring.ql[at] = uint32_t(ql); }
-    else append_any<RAW>(cb, ql, key);
+__device__ __forceinline__ void ring_push(WarpRing &ring, uint32_t &fill, const CandidateBuffers &cb, bool on, int ql, uint64_t key, int lane) {
+    const uint32_t who = __ballot_sync(kFullMask, on);
+    if (on) {
+        const uint32_t at = fill + __popc(who & ((1u << lane) - 1u));
+        if (at < kRingSize) { ring.key[at] = key; ring.ql[at] = uint32_t(ql); }
+        else append_any<RAW>(cb, ql, key);
+    }
+    fill = min(fill + __popc(who), kRingSize);
 }
 // by the whole warp: writes the ring out when it holds at least `limit` entries
 template <bool RAW>
-__device__ __forceinline__ void ring_flush(WarpRing &ring, const CandidateBuffers &cb, uint32_t limit, int lane) {
+__device__ __forceinline__ void ring_flush(WarpRing &ring, uint32_t &fill, const CandidateBuffers &cb, uint32_t limit, int lane) {
+    if (fill < limit) return;
     __syncwarp();
-    const uint32_t n = ring.n;
-    if (n < limit) return;
-    for (uint32_t i = lane; i < min(n, kRingSize); i += 32) append_any<RAW>(cb, int(ring.ql[i]), ring.key[i]);
+    for (uint32_t i = lane; i < fill; i += 32) append_any<RAW>(cb, int(ring.ql[i]), ring.key[i]);
     __syncwarp();
-    if (lane == 0) ring.n = 0;
-    __syncwarp();
+    fill = 0;
 }
 
 // One piece (32 accumulator columns of the lane's vector) against the warp's bounds; all pointers at the piece's first
-// column, `taddr` its address in tensor memory.  Runs of 8 columns that any lane of the warp flags are read again: RAW
-// appends (sum, slot) of every column at its bound, else the exact score decides.  Every lane must call this.
+// column.  Of a run of 8 columns that any lane of the warp flags, every lane takes its own surviving columns one after the
+// other (hardly ever more than one): the vector's own scale decides, by the exact score or, RAW, by the bound on it, whose
+// margin covers its roundings; then (sum, slot) is appended.  Every lane must call this.
 template <bool ONEHOT, bool RAW>
 __device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *nbound, const float *qscale, const float *qbias, const float *qthr,
-                                          bool fused, float vs, bool live, int64_t slot, int ql0, uint32_t taddr, WarpRing &ring,
-                                          const CandidateBuffers &cb) {
+                                          bool fused, float vs, bool live, uint32_t slot, int ql0, WarpRing &ring, uint32_t &fill,
+                                          const CandidateBuffers &cb, int lane) {
     uint32_t runs = 0;
     const int4 *pn = reinterpret_cast<const int4 *>(nbound);
 #pragma unroll
@@ -379,26 +381,33 @@ __device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *
     if (!live) runs = 0;
     const uint32_t warp_runs = __reduce_or_sync(kFullMask, runs);
     if (warp_runs == 0) return;
-#pragma unroll 1
-    for (int c1 = 0; c1 < 32; c1 += 8) {
-        if (!((warp_runs >> (c1 >> 3)) & 1u)) continue;
-        uint32_t a8[8];
-        tmem_ld8(taddr + c1, a8);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if ((runs >> (c1 >> 3)) & 1u) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int c = c1 + e;
-                if constexpr (RAW) {
-                    // the bound with the vector's own scale in place of the warp's largest; the margin covers its roundings
-                    const float up = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs), t = qthr[c];
-                    if (int(a8[e]) + nbound[c] >= 0 && up + 1.0e-5f * (fabsf(up) + fabsf(t)) >= t)
-                        ring_push<true>(ring, cb, ql0 + c, uint64_t(a8[e]) << 32 | uint64_t(slot));
-                } else {
-                    const float score = final_score<ONEHOT>(fused, a8[e], qscale[c], qbias[c], vs);
-                    if (score >= qthr[c]) ring_push<false>(ring, cb, ql0 + c, make_key(score, uint32_t(slot)));
-                }
+    for (int r = 0; r < 4; ++r) {
+        if (!((warp_runs >> r) & 1u)) continue;
+        const int4 a = pn[2 * r], b = pn[2 * r + 1];
+        uint32_t mine = uint32_t(int(acc[8 * r]) + a.x >= 0) | uint32_t(int(acc[8 * r + 1]) + a.y >= 0) << 1 |
+                        uint32_t(int(acc[8 * r + 2]) + a.z >= 0) << 2 | uint32_t(int(acc[8 * r + 3]) + a.w >= 0) << 3 |
+                        uint32_t(int(acc[8 * r + 4]) + b.x >= 0) << 4 | uint32_t(int(acc[8 * r + 5]) + b.y >= 0) << 5 |
+                        uint32_t(int(acc[8 * r + 6]) + b.z >= 0) << 6 | uint32_t(int(acc[8 * r + 7]) + b.w >= 0) << 7;
+        if (!live) mine = 0;
+        while (__any_sync(kFullMask, mine != 0)) {
+            const int e = mine ? __ffs(int(mine)) - 1 : 0;
+            uint32_t sum = acc[8 * r];
+#pragma unroll
+            for (int i = 1; i < 8; ++i) sum = e == i ? acc[8 * r + i] : sum;
+            const int c = 8 * r + e;
+            const float score = final_score<ONEHOT>(fused, sum, qscale[c], qbias[c], vs), t = qthr[c];
+            bool on = mine != 0;
+            uint64_t key;
+            if constexpr (RAW) {
+                on = on && score + 1.0e-5f * (fabsf(score) + fabsf(t)) >= t;
+                key = uint64_t(sum) << 32 | slot;
+            } else {
+                on = on && score >= t;
+                key = make_key(score, slot);
             }
+            ring_push<RAW>(ring, fill, cb, on, ql0 + c, key, lane);
+            mine &= mine - 1;
         }
     }
 }

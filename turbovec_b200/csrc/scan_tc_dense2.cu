@@ -61,7 +61,6 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
     const uint32_t n_items = n_vtiles * uint32_t(n_qgroups);
 
     if (tid == 0) {
-        for (int w = 0; w < kEpilogueWarps; ++w) sh->ep.ring[w].n = 0;
         for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 2); mbar_init(&sh->empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&sh->d_full[b], 1); mbar_init(&sh->d_empty[b], 2 * kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -166,6 +165,7 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
         uint32_t vt = cluster_id / uint32_t(n_qgroups);
         int qg = int(cluster_id % uint32_t(n_qgroups)), qg_here = -1;
         float u[4], w[4];
+        uint32_t fill = 0;                                // entries in the warp's ring
         bool ok = true;                                   // warp-uniform
         // this lane's vector of a tile; the scale of the next item's is on its way while this one is drained
         struct Row { uint32_t slot; float vs; bool have, live; };
@@ -218,14 +218,14 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
                     continue;
                 }
                 warp_sift<ONEHOT, false>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, fused, cur.vs, cur.live, cur.slot, ql0 + c0,
-                                         taddr + c0, ring, p.cb);
+                                         ring, fill, p.cb, lane);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->d_empty[buf]), 0));   // the leader's barrier counts both CTAs
-            ring_flush<false>(ring, p.cb, kRingSize / 2, lane);
+            ring_flush<false>(ring, fill, p.cb, kRingSize / 2, lane);
         }
-        ring_flush<false>(ring, p.cb, 1, lane);
+        ring_flush<false>(ring, fill, p.cb, 1, lane);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
