@@ -30,6 +30,19 @@ using namespace tv;
 
 thread_local std::string g_create_error;
 
+// Frees the workspaces that wait for the next handle (WorkSetPool below); false when there were none.
+bool release_idle_workspaces();
+
+// cudaMalloc that gives idle workspaces back before it reports that memory ran out.
+cudaError_t device_alloc(void **ptr, size_t bytes) {
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && release_idle_workspaces()) {
+        cudaGetLastError();
+        e = cudaMalloc(ptr, bytes);
+    }
+    return e;
+}
+
 template <typename T>
 struct DeviceArray {
     T *ptr = nullptr;
@@ -44,21 +57,27 @@ struct DeviceArray {
     cudaError_t reserve(size_t n) {
         if (n <= cap) return cudaSuccess;
         release();
-        cudaError_t e = cudaMalloc(&ptr, std::max<size_t>(n, 1) * sizeof(T));
+        cudaError_t e = device_alloc(reinterpret_cast<void **>(&ptr), std::max<size_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess) cap = n;
         return e;
     }
+    size_t bytes() const { return cap * sizeof(T); }
 };
 
 template <typename T>
 struct PinnedArray {
     T *ptr = nullptr;
     size_t cap = 0;
-    ~PinnedArray() { if (ptr) cudaFreeHost(ptr); }
+    ~PinnedArray() { release(); }
+    void release() {
+        if (ptr) cudaFreeHost(ptr);
+        ptr = nullptr;
+        cap = 0;
+    }
+    size_t bytes() const { return cap * sizeof(T); }
     cudaError_t reserve(size_t n) {
         if (n <= cap) return cudaSuccess;
-        if (ptr) cudaFreeHost(ptr);
-        ptr = nullptr; cap = 0;
+        release();
         cudaError_t e = cudaMallocHost(&ptr, std::max<size_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess) cap = n;
         return e;
@@ -138,6 +157,12 @@ struct SearchCtx {
     DeviceArray<uint64_t> d_keys_tmp;        // staging of tv_search_device_keys when the shard holds fewer than k vectors
     PinnedArray<float> h_scores;
     PinnedArray<int64_t> h_slots;
+    template <typename F>
+    void each_array(F f) {
+        f(d_stage); f(d_qrot); f(d_qscale); f(d_qbias); f(d_filter); f(d_luts); f(d_weights); f(d_wfrag); f(d_mask); f(d_mask_bool); f(d_slots_in); f(d_live); f(d_allow_ids); f(d_cand); f(d_thr); f(d_topk); f(d_floor); f(d_keys_all); f(d_cnt); f(d_scores); f(d_slots); f(d_keys_tmp);
+    }
+    template <typename F>
+    void each_pinned(F f) { f(h_scores); f(h_slots); }
     cudaError_t init() {
         cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&ev0);
@@ -162,6 +187,117 @@ struct SearchCtx {
     }
 };
 constexpr int kSearchCtxs = 2;
+
+// What a handle works with besides its data: streams, events, status words, staging buffers and the search contexts.
+// Making one costs about 15 ms (page-locked allocations take 2 - 20 ms each on this class of machine, device allocations
+// 0.4 - 3 ms), as much as encoding two million vectors, so a destroyed handle leaves its workspace for the next one on
+// the device.  At most kIdleSets wait per device, each trimmed to kIdleDeviceBytes and kIdlePinnedBytes, and all of them
+// are freed when an allocation fails.  A workspace belongs to one handle at a time, and its streams are idle in between.
+struct WorkSet {
+    cudaStream_t stream = nullptr;           // mutations and accessors
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_mut = nullptr;            // recorded on `stream` after every mutation; searches wait for it
+    Marks marks;                             // ingest launches of the last add
+    DeviceFlags *d_flags = nullptr;
+    DeviceFlags *h_flags = nullptr;
+    // host-memory adds: two pinned + two device staging buffers, a copy stream and per-buffer events
+    PinnedArray<float> h_add[2];
+    DeviceArray<float> d_add[2];
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_consumed[2] = {nullptr, nullptr};
+    SearchCtx ctx[kSearchCtxs];
+
+    cudaError_t init() {
+        cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreate(&ev0);
+        if (e == cudaSuccess) e = cudaEventCreate(&ev1);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_mut, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void **>(&d_flags), sizeof(DeviceFlags));
+        if (e == cudaSuccess) e = cudaMallocHost(&h_flags, sizeof(DeviceFlags));
+        for (int i = 0; i < kSearchCtxs && e == cudaSuccess; ++i) e = ctx[i].init();
+        return e;
+    }
+    // Waits for the streams and cuts the buffers down to what an idle workspace may hold; false when something failed.
+    bool retire() {
+        bool ok = stream && cudaStreamSynchronize(stream) == cudaSuccess;
+        if (ok && copy_stream) ok = cudaStreamSynchronize(copy_stream) == cudaSuccess;
+        marks.used = 0;
+        size_t device = 0, pinned = 0;
+        for (SearchCtx &c : ctx) {
+            ok = ok && c.stream && cudaStreamSynchronize(c.stream) == cudaSuccess;
+            c.busy = false;
+            c.marks.used = 0;
+            c.each_array([&](auto &a) { device += a.bytes(); if (device > kIdleDeviceBytes) { device -= a.bytes(); a.release(); } });
+            c.each_pinned([&](auto &a) { pinned += a.bytes(); if (pinned > kIdlePinnedBytes) { pinned -= a.bytes(); a.release(); } });
+        }
+        for (int b = 0; b < 2; ++b) {
+            device += d_add[b].bytes(); if (device > kIdleDeviceBytes) { device -= d_add[b].bytes(); d_add[b].release(); }
+            pinned += h_add[b].bytes(); if (pinned > kIdlePinnedBytes) { pinned -= h_add[b].bytes(); h_add[b].release(); }
+        }
+        return ok;
+    }
+    ~WorkSet() {
+        if (stream) cudaStreamSynchronize(stream);
+        if (d_flags) cudaFree(d_flags);
+        if (h_flags) cudaFreeHost(h_flags);
+        if (ev0) cudaEventDestroy(ev0);
+        if (ev1) cudaEventDestroy(ev1);
+        if (ev_mut) cudaEventDestroy(ev_mut);
+        for (int b = 0; b < 2; ++b) {
+            if (ev_copied[b]) cudaEventDestroy(ev_copied[b]);
+            if (ev_consumed[b]) cudaEventDestroy(ev_consumed[b]);
+        }
+        if (copy_stream) cudaStreamDestroy(copy_stream);
+        if (stream) cudaStreamDestroy(stream);
+    }
+    static constexpr size_t kIdleDeviceBytes = size_t(96) << 20, kIdlePinnedBytes = size_t(40) << 20;
+};
+
+struct WorkSetPool {
+    static constexpr size_t kIdleSets = 2;
+    std::mutex mu;
+    std::unordered_map<int, std::vector<WorkSet *>> idle;    // by device
+};
+WorkSetPool &workset_pool() {
+    static WorkSetPool *pool = new WorkSetPool;              // never destroyed: the driver may be gone by then
+    return *pool;
+}
+// The device is current.
+WorkSet *acquire_workset(int device, cudaError_t *err) {
+    WorkSetPool &pool = workset_pool();
+    {
+        std::lock_guard<std::mutex> g(pool.mu);
+        auto &list = pool.idle[device];
+        if (!list.empty()) { WorkSet *w = list.back(); list.pop_back(); return w; }
+    }
+    WorkSet *w = new WorkSet;
+    *err = w->init();
+    if (*err != cudaSuccess) { delete w; return nullptr; }
+    return w;
+}
+void return_workset(int device, WorkSet *w) {
+    if (!w) return;
+    if (w->retire()) {
+        WorkSetPool &pool = workset_pool();
+        std::lock_guard<std::mutex> g(pool.mu);
+        auto &list = pool.idle[device];
+        if (list.size() < WorkSetPool::kIdleSets) { list.push_back(w); return; }
+    }
+    delete w;
+}
+bool release_idle_workspaces() {
+    std::vector<WorkSet *> all;
+    {
+        WorkSetPool &pool = workset_pool();
+        std::lock_guard<std::mutex> g(pool.mu);
+        for (auto &entry : pool.idle) {
+            all.insert(all.end(), entry.second.begin(), entry.second.end());
+            entry.second.clear();
+        }
+    }
+    for (WorkSet *w : all) delete w;
+    return !all.empty();
+}
 
 // Device copy of the id -> slot table, kept for large allowlists (search.cu: idtab_*_kernel).  The host tables stay the
 // authority; this copy is brought up to date lazily, by the first allowlist search after a change.
@@ -260,12 +396,9 @@ struct tv_index {
     int dense_pair = 1;          // 1: the scan over the int8 copy runs on CTA pairs (cta_group::2)
     int fail_next = 0;           // test hook (TV_OPT_FAIL_NEXT): the next device allocation / upload of a call reports failure
 
-    cudaStream_t stream = nullptr;           // mutations and accessors
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t ev_mut = nullptr;            // recorded on `stream` after every mutation; searches wait for it
+    WorkSet *ws = nullptr;                   // streams, events, staging and search contexts
     std::atomic<uint64_t> launches{0};
     float last_ms = 0.f;
-    Marks marks;                             // ingest launches of the last add
     float last_main_ms = 0.f;
     int last_main_launches = 0;
 
@@ -294,16 +427,8 @@ struct tv_index {
     // scratch of the mutating calls
     DeviceArray<float> d_stage;              // ingest staging (calibration sample)
     DeviceArray<uint8_t> d_row;              // one row's byte-groups (get_row / set_row)
-    // host-memory adds: two pinned + two device staging buffers, a copy stream and per-buffer events
-    PinnedArray<float> h_add[2];
-    DeviceArray<float> d_add[2];
-    cudaStream_t copy_stream = nullptr;
-    cudaEvent_t ev_copied[2] = {nullptr, nullptr}, ev_consumed[2] = {nullptr, nullptr};
-    DeviceFlags *d_flags = nullptr;
-    DeviceFlags *h_flags = nullptr;
 
-    // search contexts
-    SearchCtx ctx[kSearchCtxs];
+    // hands out the search contexts of the workspace
     std::mutex ctx_mu;
     std::condition_variable ctx_cv;
     PreparedMask prepared;
@@ -327,20 +452,10 @@ struct tv_index {
 
     ~tv_index() {
         cudaSetDevice(device);
-        if (stream) cudaStreamSynchronize(stream);
+        if (ws && ws->stream) cudaStreamSynchronize(ws->stream);
         if (d_codes) cudaFree(d_codes);
         if (d_scales) cudaFree(d_scales);
-        if (d_flags) cudaFree(d_flags);
-        if (h_flags) cudaFreeHost(h_flags);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        if (ev_mut) cudaEventDestroy(ev_mut);
-        for (int b = 0; b < 2; ++b) {
-            if (ev_copied[b]) cudaEventDestroy(ev_copied[b]);
-            if (ev_consumed[b]) cudaEventDestroy(ev_consumed[b]);
-        }
-        if (copy_stream) cudaStreamDestroy(copy_stream);
-        if (stream) cudaStreamDestroy(stream);
+        return_workset(device, ws);
     }
 };
 
@@ -357,18 +472,18 @@ int fail(tv_index *h, int code, const std::string &msg) {
 }
 
 // Brackets one ingest launch with two events from the handle's pool.
-void mark_begin(tv_index *h) { h->marks.begin(h->stream); }
-void mark_end(tv_index *h) { h->marks.end(h->stream); }
+void mark_begin(tv_index *h) { h->ws->marks.begin(h->ws->stream); }
+void mark_end(tv_index *h) { h->ws->marks.end(h->ws->stream); }
 void collect_marks(tv_index *h) {
-    h->marks.collect();
-    h->last_main_ms = h->marks.total_ms;
-    h->last_main_launches = h->marks.launches;
+    h->ws->marks.collect();
+    h->last_main_ms = h->ws->marks.total_ms;
+    h->last_main_launches = h->ws->marks.launches;
 }
 
 // Called at the end of every call that changed device state on the handle's stream: searches run on their own
 // streams and wait for this event first.  Also drops a prepared mask, which describes the index as it was.
 void mutation_done(tv_index *h) {
-    cudaEventRecord(h->ev_mut, h->stream);
+    cudaEventRecord(h->ws->ev_mut, h->ws->stream);
     h->prepared.valid = false;
 }
 
@@ -403,16 +518,16 @@ int upload_codebook(tv_index *h) {
     for (size_t i = 0; i < h->cb.boundaries.size(); ++i) cbuf[i] = h->cb.boundaries[i];
     for (size_t i = 0; i < h->cb.centroids.size(); ++i) cbuf[16 + i] = h->cb.centroids[i];
     TV_CUDA(h->d_codebook.reserve(32));
-    TV_CUDA(cudaMemcpyAsync(h->d_codebook.ptr, cbuf, sizeof cbuf, cudaMemcpyHostToDevice, h->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_codebook.ptr, cbuf, sizeof cbuf, cudaMemcpyHostToDevice, h->ws->stream));
     QuantGridHost grid;
     h->qgrid = QuantGrid{};
     if (build_quant_grid(h->cb.boundaries.data(), int(h->cb.boundaries.size()), grid)) {
         static_assert(sizeof(QuantCell) == sizeof(uint2), "grid cells are uploaded as they are");
         TV_CUDA(h->d_qgrid.reserve(grid.cells.size()));
-        TV_CUDA(cudaMemcpyAsync(h->d_qgrid.ptr, grid.cells.data(), grid.cells.size() * sizeof(uint2), cudaMemcpyHostToDevice, h->stream));
+        TV_CUDA(cudaMemcpyAsync(h->d_qgrid.ptr, grid.cells.data(), grid.cells.size() * sizeof(uint2), cudaMemcpyHostToDevice, h->ws->stream));
         h->qgrid.cells = h->d_qgrid.ptr; h->qgrid.a = grid.a; h->qgrid.b = grid.b;
     }
-    TV_CUDA(cudaStreamSynchronize(h->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     {
         // search.rs:2812-2819: cs = cmax/127, level = clamp(round(c/cs), +-127)
         float cmax = 0.f;
@@ -436,17 +551,17 @@ int ensure_tables(tv_index *h) {
     h->rot = build_rotation_tables(dim);
     h->cb = codebook(h->bits, dim);
     TV_CUDA(h->d_perm.reserve(size_t(2) * dim));
-    TV_CUDA(cudaMemcpyAsync(h->d_perm.ptr, h->rot.packed[0].data(), size_t(dim) * 2, cudaMemcpyHostToDevice, h->stream));
-    TV_CUDA(cudaMemcpyAsync(h->d_perm.ptr + dim, h->rot.packed[1].data(), size_t(dim) * 2, cudaMemcpyHostToDevice, h->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_perm.ptr, h->rot.packed[0].data(), size_t(dim) * 2, cudaMemcpyHostToDevice, h->ws->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_perm.ptr + dim, h->rot.packed[1].data(), size_t(dim) * 2, cudaMemcpyHostToDevice, h->ws->stream));
     // bank-conflict-free exchange layout of the pipelined ingest kernel (vectors of up to 48 registers per lane: beyond that the kernel has no registers for the offsets)
     h->exchange_ready = false;
     ExchangeLayoutHost ex;
     if (dim % 32 == 0 && dim / 32 <= 48 && build_exchange_layout(int(dim), h->rot.packed[1].data(), ex)) {
         TV_CUDA(h->d_store_bank.reserve(dim));
         TV_CUDA(h->d_perm1_exchange.reserve(dim));
-        TV_CUDA(cudaMemcpyAsync(h->d_store_bank.ptr, ex.store_bank.data(), dim, cudaMemcpyHostToDevice, h->stream));
-        TV_CUDA(cudaMemcpyAsync(h->d_perm1_exchange.ptr, ex.perm1_exchange.data(), size_t(dim) * 2, cudaMemcpyHostToDevice, h->stream));
-        TV_CUDA(cudaStreamSynchronize(h->stream));     // `ex` goes out of scope
+        TV_CUDA(cudaMemcpyAsync(h->d_store_bank.ptr, ex.store_bank.data(), dim, cudaMemcpyHostToDevice, h->ws->stream));
+        TV_CUDA(cudaMemcpyAsync(h->d_perm1_exchange.ptr, ex.perm1_exchange.data(), size_t(dim) * 2, cudaMemcpyHostToDevice, h->ws->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));     // `ex` goes out of scope
         h->exchange_ready = true;
     }
     int rc = upload_codebook(h);
@@ -465,8 +580,8 @@ int upload_calibration(tv_index *h) {
         buf[2 * dim + d] = 1.0f / h->scale_tq[d];     // encode.rs:593
     }
     TV_CUDA(h->d_calib.reserve(3 * dim));
-    TV_CUDA(cudaMemcpyAsync(h->d_calib.ptr, buf.data(), buf.size() * 4, cudaMemcpyHostToDevice, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_calib.ptr, buf.data(), buf.size() * 4, cudaMemcpyHostToDevice, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     return TV_OK;
 }
 
@@ -480,17 +595,17 @@ int ensure_capacity(tv_index *h, size_t n_total) {
         size_t new_cap = std::max(blocks, h->code_blocks_cap + h->code_blocks_cap / 2);
         new_cap = std::max<size_t>(new_cap, 64);
         uint8_t *fresh = nullptr;
-        cudaError_t e = cudaMalloc(&fresh, new_cap * block_bytes);
+        cudaError_t e = device_alloc(reinterpret_cast<void **>(&fresh), new_cap * block_bytes);
         if (e != cudaSuccess && new_cap > blocks) {      // retry with the exact size before giving up
             cudaGetLastError();
             new_cap = blocks;
-            e = cudaMalloc(&fresh, new_cap * block_bytes);
+            e = device_alloc(reinterpret_cast<void **>(&fresh), new_cap * block_bytes);
         }
         TV_CUDA(e);
         const size_t used = ((h->n + kBlock - 1) / kBlock) * block_bytes;
-        if (used) TV_CUDA(cudaMemcpyAsync(fresh, h->d_codes, used, cudaMemcpyDeviceToDevice, h->stream));
-        TV_CUDA(cudaMemsetAsync(fresh + used, 0, new_cap * block_bytes - used, h->stream));
-        TV_CUDA(cudaStreamSynchronize(h->stream));
+        if (used) TV_CUDA(cudaMemcpyAsync(fresh, h->d_codes, used, cudaMemcpyDeviceToDevice, h->ws->stream));
+        TV_CUDA(cudaMemsetAsync(fresh + used, 0, new_cap * block_bytes - used, h->ws->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));
         if (h->d_codes) cudaFree(h->d_codes);
         h->d_codes = fresh;
         h->code_blocks_cap = new_cap;
@@ -500,9 +615,9 @@ int ensure_capacity(tv_index *h, size_t n_total) {
         size_t new_cap = std::max(n_total, h->scales_cap + h->scales_cap / 2);
         new_cap = std::max<size_t>(new_cap, 2048);
         float *fresh = nullptr;
-        TV_CUDA(cudaMalloc(&fresh, new_cap * sizeof(float)));
-        if (h->n) TV_CUDA(cudaMemcpyAsync(fresh, h->d_scales, h->n * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
-        TV_CUDA(cudaStreamSynchronize(h->stream));
+        TV_CUDA(device_alloc(reinterpret_cast<void **>(&fresh), new_cap * sizeof(float)));
+        if (h->n) TV_CUDA(cudaMemcpyAsync(fresh, h->d_scales, h->n * sizeof(float), cudaMemcpyDeviceToDevice, h->ws->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));
         if (h->d_scales) cudaFree(h->d_scales);
         h->d_scales = fresh;
         h->scales_cap = new_cap;
@@ -571,10 +686,10 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
     const int V = ingest_vectors_per_pass(int(dim), h->ngroups, h->smem_limit);
     if (V == 0) return fail(h, TV_ERR_UNSUPPORTED, "dim too large for the ingest kernel's shared memory");
 
-    h->h_flags->first_invalid = ~0ull;
-    h->h_flags->error = 0;
-    TV_CUDA(cudaMemcpyAsync(&h->d_flags->first_invalid, &h->h_flags->first_invalid, 8, cudaMemcpyHostToDevice, h->stream));
-    TV_CUDA(cudaMemcpyAsync(&h->d_flags->error, &h->h_flags->error, 4, cudaMemcpyHostToDevice, h->stream));
+    h->ws->h_flags->first_invalid = ~0ull;
+    h->ws->h_flags->error = 0;
+    TV_CUDA(cudaMemcpyAsync(&h->ws->d_flags->first_invalid, &h->ws->h_flags->first_invalid, 8, cudaMemcpyHostToDevice, h->ws->stream));
+    TV_CUDA(cudaMemcpyAsync(&h->ws->d_flags->error, &h->ws->h_flags->error, 4, cudaMemcpyHostToDevice, h->ws->stream));
 
     IngestParams p{};
     p.dim = int(dim); p.bits = h->bits; p.ngroups = h->ngroups;
@@ -583,33 +698,31 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
     p.boundaries = h->d_codebook.ptr; p.centroids = h->d_codebook.ptr + 16;
     if (!h->shift.empty()) { p.shift = h->d_calib.ptr; p.scale_tq = h->d_calib.ptr + dim; p.inv_scale_tq = h->d_calib.ptr + 2 * dim; }
     p.codes = h->d_codes; p.scales = h->d_scales;
-    p.first_invalid = &h->d_flags->first_invalid;
+    p.first_invalid = &h->ws->d_flags->first_invalid;
 
-    // Device input is encoded in place.  Host input goes through pinned staging in chunks of about 64 MB,
-    // double buffered: host threads copy chunk i+1 into pinned memory while chunk i crosses the bus on the copy
+    // Device input is encoded in place.  Host input goes through pinned staging in chunks of about 16 MB,
+    // double buffered (page-locking 16 MB takes 12 ms): host threads copy chunk i+1 into pinned memory while chunk i crosses the bus on the copy
     // stream and chunk i-1 is encoded on the handle's stream.
-    const size_t chunk_rows = on_device ? n : std::max<size_t>(1, std::min<size_t>(n, (size_t(64) << 20) / (dim * 4)));
-    if (!on_device) {
-        if (!h->copy_stream) {
-            TV_CUDA(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-            for (int b = 0; b < 2; ++b) {
-                TV_CUDA(cudaEventCreateWithFlags(&h->ev_copied[b], cudaEventDisableTiming));
-                TV_CUDA(cudaEventCreateWithFlags(&h->ev_consumed[b], cudaEventDisableTiming));
-            }
-        }
-        for (int b = 0; b < 2; ++b) {
-            TV_CUDA(h->h_add[b].reserve(chunk_rows * dim));
-            TV_CUDA(h->d_add[b].reserve(chunk_rows * dim));
-        }
-    }
-    const size_t copy_threads = std::min<size_t>(16, std::max(1u, std::thread::hardware_concurrency()));
-    // page-locked input (cudaHostAlloc / cudaHostRegister) is read by the copy engine directly
+    const size_t chunk_rows = on_device ? n : std::max<size_t>(1, std::min<size_t>(n, (size_t(16) << 20) / (dim * 4)));
     bool src_pinned = false;
     if (!on_device) {
+        if (!h->ws->copy_stream) {
+            TV_CUDA(cudaStreamCreateWithFlags(&h->ws->copy_stream, cudaStreamNonBlocking));
+            for (int b = 0; b < 2; ++b) {
+                TV_CUDA(cudaEventCreateWithFlags(&h->ws->ev_copied[b], cudaEventDisableTiming));
+                TV_CUDA(cudaEventCreateWithFlags(&h->ws->ev_consumed[b], cudaEventDisableTiming));
+            }
+        }
+        // page-locked input (cudaHostAlloc / cudaHostRegister) is read by the copy engine directly
         cudaPointerAttributes attr{};
         if (cudaPointerGetAttributes(&attr, x) == cudaSuccess) src_pinned = attr.type == cudaMemoryTypeHost;
         else cudaGetLastError();
+        for (int b = 0; b < (n > chunk_rows ? 2 : 1); ++b) {
+            if (!src_pinned) TV_CUDA(h->ws->h_add[b].reserve(chunk_rows * dim));
+            TV_CUDA(h->ws->d_add[b].reserve(chunk_rows * dim));
+        }
     }
+    const size_t copy_threads = std::min<size_t>(16, std::max(1u, std::thread::hardware_concurrency()));
     // A failure after the first launch leaves bytes in lanes past `len`: they are cleared again before the
     // call returns, so that a failed add leaves the index exactly as it was (lib.rs:889-930).
     cudaError_t step_err = cudaSuccess;
@@ -619,7 +732,7 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
         step_err = (expr);                                         \
         if (step_err != cudaSuccess) { step_what = #expr; break; } \
     }
-    TV_CUDA(cudaEventRecord(h->ev0, h->stream));
+    TV_CUDA(cudaEventRecord(h->ws->ev0, h->ws->stream));
     size_t chunk_index = 0;
     for (size_t done = 0; done < n; done += chunk_rows, ++chunk_index) {
         const size_t rows = std::min(chunk_rows, n - done);
@@ -627,25 +740,25 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
         TV_STEP(injected_failure(h));
         if (!on_device) {
             const int b = int(chunk_index & 1);
-            if (chunk_index >= 2) TV_STEP(cudaEventSynchronize(h->ev_consumed[b]));   // the encode of chunk i-2 has read d_add[b]
+            if (chunk_index >= 2) TV_STEP(cudaEventSynchronize(h->ws->ev_consumed[b]));   // the encode of chunk i-2 has read d_add[b]
             const size_t bytes = rows * dim * 4;
-            const float *h_src = h->h_add[b].ptr;
+            const float *h_src = h->ws->h_add[b].ptr;
             if (src_pinned) {
                 h_src = src;
             } else if (bytes < (size_t(4) << 20) || copy_threads == 1) {
-                std::memcpy(h->h_add[b].ptr, src, bytes);
+                std::memcpy(h->ws->h_add[b].ptr, src, bytes);
             } else {
                 std::vector<std::thread> pool;
                 for (size_t t = 0; t < copy_threads; ++t) {
                     const size_t lo = bytes * t / copy_threads / 64 * 64, hi = t + 1 == copy_threads ? bytes : bytes * (t + 1) / copy_threads / 64 * 64;
-                    pool.emplace_back([=] { std::memcpy(reinterpret_cast<char *>(h->h_add[b].ptr) + lo, reinterpret_cast<const char *>(src) + lo, hi - lo); });
+                    pool.emplace_back([=] { std::memcpy(reinterpret_cast<char *>(h->ws->h_add[b].ptr) + lo, reinterpret_cast<const char *>(src) + lo, hi - lo); });
                 }
                 for (auto &th : pool) th.join();
             }
-            TV_STEP(cudaMemcpyAsync(h->d_add[b].ptr, h_src, bytes, cudaMemcpyHostToDevice, h->copy_stream));
-            TV_STEP(cudaEventRecord(h->ev_copied[b], h->copy_stream));
-            TV_STEP(cudaStreamWaitEvent(h->stream, h->ev_copied[b], 0));
-            src = h->d_add[b].ptr;
+            TV_STEP(cudaMemcpyAsync(h->ws->d_add[b].ptr, h_src, bytes, cudaMemcpyHostToDevice, h->ws->copy_stream));
+            TV_STEP(cudaEventRecord(h->ws->ev_copied[b], h->ws->copy_stream));
+            TV_STEP(cudaStreamWaitEvent(h->ws->stream, h->ws->ev_copied[b], 0));
+            src = h->ws->d_add[b].ptr;
         }
         p.x = src; p.n = int64_t(rows); p.slot0 = int64_t(h->n + done); p.row_base = int64_t(done);
         // rows that complete a partly filled block go through the block-at-a-time kernel, whole blocks
@@ -657,7 +770,7 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
         if (head > 0) {
             p.n = head;
             mark_begin(h);
-            TV_STEP(launch_ingest(p, V, h->stream));
+            TV_STEP(launch_ingest(p, V, h->ws->stream));
             mark_end(h);
             h->launches++;
         }
@@ -666,43 +779,43 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
             p.exact_sums = h->ingest_pipeline == 2;
             if (h->exchange_ready) { p.store_bank = h->d_store_bank.ptr; p.perm1_exchange = h->d_perm1_exchange.ptr; }
             mark_begin(h);
-            TV_STEP(launch_ingest_fast(p, h->qgrid, h->sm_count, h->smem_limit, &h->d_flags->error, h->stream));
+            TV_STEP(launch_ingest_fast(p, h->qgrid, h->sm_count, h->smem_limit, &h->ws->d_flags->error, h->ws->stream));
             mark_end(h);
             h->launches++;
         }
-        if (!on_device) TV_STEP(cudaEventRecord(h->ev_consumed[chunk_index & 1], h->stream));
+        if (!on_device) TV_STEP(cudaEventRecord(h->ws->ev_consumed[chunk_index & 1], h->ws->stream));
     }
 #undef TV_STEP
     if (step_err != cudaSuccess) {
         cudaGetLastError();
-        cudaStreamSynchronize(h->stream);
-        if (h->copy_stream) cudaStreamSynchronize(h->copy_stream);
+        cudaStreamSynchronize(h->ws->stream);
+        if (h->ws->copy_stream) cudaStreamSynchronize(h->ws->copy_stream);
         const int64_t total = int64_t(n) * h->ngroups;
-        clear_slots_kernel<<<unsigned(std::min<int64_t>((total + 255) / 256, 65535)), 256, 0, h->stream>>>(
+        clear_slots_kernel<<<unsigned(std::min<int64_t>((total + 255) / 256, 65535)), 256, 0, h->ws->stream>>>(
             h->d_codes, h->ngroups, int64_t(h->n), int64_t(h->n + n));
-        cudaStreamSynchronize(h->stream);
-        h->marks.used = 0;
+        cudaStreamSynchronize(h->ws->stream);
+        h->ws->marks.used = 0;
         if (was_lazy) { h->dim = 0; h->tables_ready = false; }
         return fail(h, step_err == cudaErrorMemoryAllocation ? TV_ERR_OUT_OF_MEMORY : TV_ERR_CUDA,
                     std::string(step_what) + ": " + cudaGetErrorString(step_err));
     }
-    TV_CUDA(cudaEventRecord(h->ev1, h->stream));
-    TV_CUDA(cudaMemcpyAsync(&h->h_flags->first_invalid, &h->d_flags->first_invalid, 8, cudaMemcpyDeviceToHost, h->stream));
-    TV_CUDA(cudaMemcpyAsync(&h->h_flags->error, &h->d_flags->error, 4, cudaMemcpyDeviceToHost, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
-    cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
+    TV_CUDA(cudaEventRecord(h->ws->ev1, h->ws->stream));
+    TV_CUDA(cudaMemcpyAsync(&h->ws->h_flags->first_invalid, &h->ws->d_flags->first_invalid, 8, cudaMemcpyDeviceToHost, h->ws->stream));
+    TV_CUDA(cudaMemcpyAsync(&h->ws->h_flags->error, &h->ws->d_flags->error, 4, cudaMemcpyDeviceToHost, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
+    cudaEventElapsedTime(&h->last_ms, h->ws->ev0, h->ws->ev1);
     collect_marks(h);
-    if (h->h_flags->error != 0) {
+    if (h->ws->h_flags->error != 0) {
         if (was_lazy) { h->dim = 0; h->tables_ready = false; }
-        return fail(h, TV_ERR_DEVICE_TIMEOUT, "the ingest kernel gave up waiting for a staged row (code " + std::to_string(h->h_flags->error) + ")");
+        return fail(h, TV_ERR_DEVICE_TIMEOUT, "the ingest kernel gave up waiting for a staged row (code " + std::to_string(h->ws->h_flags->error) + ")");
     }
-    if (h->h_flags->first_invalid != ~0ull) {
+    if (h->ws->h_flags->first_invalid != ~0ull) {
         // roll back: the new lanes must read as zero again, nothing else was touched
         const int64_t total = int64_t(n) * h->ngroups;
-        clear_slots_kernel<<<unsigned(std::min<int64_t>((total + 255) / 256, 65535)), 256, 0, h->stream>>>(
+        clear_slots_kernel<<<unsigned(std::min<int64_t>((total + 255) / 256, 65535)), 256, 0, h->ws->stream>>>(
             h->d_codes, h->ngroups, int64_t(h->n), int64_t(h->n + n));
-        cudaStreamSynchronize(h->stream);
-        const unsigned long long flat = h->h_flags->first_invalid;
+        cudaStreamSynchronize(h->ws->stream);
+        const unsigned long long flat = h->ws->h_flags->first_invalid;
         h->err_vec = size_t(flat / dim); h->err_coord = size_t(flat % dim);
         if (on_device) cudaMemcpy(&h->err_value, x + flat, 4, cudaMemcpyDeviceToHost);
         else h->err_value = x[flat];
@@ -736,7 +849,7 @@ struct CtxLease {
         std::unique_lock<std::mutex> g(h->ctx_mu);
         for (;;) {
             for (int i = 0; i < kSearchCtxs; ++i)
-                if (!h->ctx[i].busy) { c = &h->ctx[i]; break; }
+                if (!h->ws->ctx[i].busy) { c = &h->ws->ctx[i]; break; }
             if (c) break;
             h->ctx_cv.wait(g);
         }
@@ -1237,7 +1350,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     }
 
     // ---- inputs ----
-    TV_CUDA(cudaStreamWaitEvent(st, h->ev_mut, 0));          // after every mutation enqueued on the handle's stream
+    TV_CUDA(cudaStreamWaitEvent(st, h->ws->ev_mut, 0));          // after every mutation enqueued on the handle's stream
     const float *dq = queries;
     if (!queries_on_device) {
         TV_CUDA(cudaMemcpyAsync(c.d_stage.ptr, queries, nq * dim * 4, cudaMemcpyHostToDevice, st));
@@ -1495,19 +1608,13 @@ int tv_index_create(size_t dim, int bit_width, int kind, int device, tv_index **
         return int(TV_ERR_CUDA);
     };
     if ((e = cudaSetDevice(device)) != cudaSuccess) return bail("cudaSetDevice", e);
-    cudaDeviceProp prop{};
-    if ((e = cudaGetDeviceProperties(&prop, device)) != cudaSuccess) return bail("cudaGetDeviceProperties", e);
-    h->sm_count = prop.multiProcessorCount;
-    h->smem_limit = prop.sharedMemPerBlockOptin;
-    if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess) return bail("cudaStreamCreate", e);
-    if ((e = cudaEventCreate(&h->ev0)) != cudaSuccess) return bail("cudaEventCreate", e);
-    if ((e = cudaEventCreate(&h->ev1)) != cudaSuccess) return bail("cudaEventCreate", e);
-    if ((e = cudaEventCreateWithFlags(&h->ev_mut, cudaEventDisableTiming)) != cudaSuccess) return bail("cudaEventCreate", e);
-    if ((e = cudaEventRecord(h->ev_mut, h->stream)) != cudaSuccess) return bail("cudaEventRecord", e);
-    if ((e = cudaMalloc(&h->d_flags, sizeof(DeviceFlags))) != cudaSuccess) return bail("cudaMalloc", e);
-    if ((e = cudaMallocHost(&h->h_flags, sizeof(DeviceFlags))) != cudaSuccess) return bail("cudaMallocHost", e);
-    for (int i = 0; i < kSearchCtxs; ++i)
-        if ((e = h->ctx[i].init()) != cudaSuccess) return bail("search context", e);
+    // two attributes, not cudaGetDeviceProperties: that takes 2.6 ms
+    int smem_optin = 0;
+    if ((e = cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return bail("cudaDeviceGetAttribute", e);
+    if ((e = cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) != cudaSuccess) return bail("cudaDeviceGetAttribute", e);
+    h->smem_limit = size_t(smem_optin);
+    if (!(h->ws = acquire_workset(device, &e))) return bail("workspace", e);
+    if ((e = cudaEventRecord(h->ws->ev_mut, h->ws->stream)) != cudaSuccess) return bail("cudaEventRecord", e);
     *out = h;
     return TV_OK;
 }
@@ -1645,7 +1752,7 @@ int tv_swap_remove(tv_index *h, size_t slot, size_t *moved_from) {
     if (slot >= h->n) return fail(h, TV_ERR_SLOT_OUT_OF_RANGE, "index " + std::to_string(slot) + " out of bounds (n_vectors = " + std::to_string(h->n) + ")");
     TV_CUDA(cudaSetDevice(h->device));
     const size_t last = h->n - 1;
-    move_lane_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->stream>>>(h->d_codes, h->d_scales, h->ngroups, int64_t(last), int64_t(slot));
+    move_lane_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->ws->stream>>>(h->d_codes, h->d_scales, h->ngroups, int64_t(last), int64_t(slot));
     h->launches++;
     TV_CUDA(cudaGetLastError());
     // no synchronisation: the result is known on the host, and every later call on this handle runs on the
@@ -1669,7 +1776,7 @@ int tv_remove(tv_index *h, uint64_t id, int *removed) {
     if (it == h->id_to_slot.end()) return TV_OK;                       // id_map.rs:521-523
     const size_t slot = it->second, last = h->n - 1;
     TV_CUDA(cudaSetDevice(h->device));
-    move_lane_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->stream>>>(h->d_codes, h->d_scales, h->ngroups, int64_t(last), int64_t(slot));
+    move_lane_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->ws->stream>>>(h->d_codes, h->d_scales, h->ngroups, int64_t(last), int64_t(slot));
     h->launches++;
     TV_CUDA(cudaGetLastError());
     h->mark_dirty(slot);
@@ -1699,12 +1806,12 @@ int tv_get_row(const tv_index *hc, size_t slot, uint8_t *groups_out, size_t capa
     if (capacity < size_t(h->ngroups)) return fail(h, TV_ERR_INVALID_ARGUMENT, "output buffer too small");
     TV_CUDA(cudaSetDevice(h->device));
     TV_CUDA(h->d_row.reserve(size_t(h->ngroups)));
-    gather_row_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->stream>>>(h->d_codes, h->ngroups, int64_t(slot), h->d_row.ptr);
+    gather_row_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->ws->stream>>>(h->d_codes, h->ngroups, int64_t(slot), h->d_row.ptr);
     h->launches++;
     TV_CUDA(cudaGetLastError());
-    TV_CUDA(cudaMemcpyAsync(groups_out, h->d_row.ptr, size_t(h->ngroups), cudaMemcpyDeviceToHost, h->stream));
-    TV_CUDA(cudaMemcpyAsync(scale_out, h->d_scales + slot, 4, cudaMemcpyDeviceToHost, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
+    TV_CUDA(cudaMemcpyAsync(groups_out, h->d_row.ptr, size_t(h->ngroups), cudaMemcpyDeviceToHost, h->ws->stream));
+    TV_CUDA(cudaMemcpyAsync(scale_out, h->d_scales + slot, 4, cudaMemcpyDeviceToHost, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     return TV_OK;
 }
 
@@ -1716,12 +1823,12 @@ int tv_set_row(tv_index *h, size_t slot, const uint8_t *groups, size_t count, fl
     if (!(scale >= 0.0f) || !std::isfinite(scale)) return fail(h, TV_ERR_PARTS_INVALID, "scale is negative or not finite");
     TV_CUDA(cudaSetDevice(h->device));
     TV_CUDA(h->d_row.reserve(count));
-    TV_CUDA(cudaMemcpyAsync(h->d_row.ptr, groups, count, cudaMemcpyHostToDevice, h->stream));
-    scatter_row_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->stream>>>(h->d_codes, h->ngroups, int64_t(slot), h->d_row.ptr);
+    TV_CUDA(cudaMemcpyAsync(h->d_row.ptr, groups, count, cudaMemcpyHostToDevice, h->ws->stream));
+    scatter_row_kernel<<<(h->ngroups + 255) / 256, 256, 0, h->ws->stream>>>(h->d_codes, h->ngroups, int64_t(slot), h->d_row.ptr);
     h->launches++;
     TV_CUDA(cudaGetLastError());
-    TV_CUDA(cudaMemcpyAsync(h->d_scales + slot, &scale, 4, cudaMemcpyHostToDevice, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_scales + slot, &scale, 4, cudaMemcpyHostToDevice, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     h->mark_dirty(slot);
     h->expanded.touch(slot);
     mutation_done(h);
@@ -1840,18 +1947,18 @@ int prepare_mask(tv_index *h, const MaskSpec &spec) {
     if (h->dim == 0 || h->n == 0) return fail(h, TV_ERR_INVALID_ARGUMENT, "the index is empty: nothing to prepare a mask for");
     TV_CUDA(cudaSetDevice(h->device));
     TV_CUDA(h->prepared.counts.reserve(2));
-    TV_CUDA(cudaMemsetAsync(h->prepared.counts.ptr, 0, 16, h->stream));
+    TV_CUDA(cudaMemsetAsync(h->prepared.counts.ptr, 0, 16, h->ws->stream));
     MaskOnDevice m;
-    TV_CUDA(cudaMemsetAsync(&h->d_flags->first_unknown, 0xff, 8, h->stream));
-    int rc = build_mask(h, h->stream, spec, h->prepared.words, h->ctx[0].d_mask_bool, h->ctx[0].d_slots_in, h->prepared.live,
-                        h->ctx[0].d_allow_ids, &h->d_flags->first_unknown,
+    TV_CUDA(cudaMemsetAsync(&h->ws->d_flags->first_unknown, 0xff, 8, h->ws->stream));
+    int rc = build_mask(h, h->ws->stream, spec, h->prepared.words, h->ws->ctx[0].d_mask_bool, h->ws->ctx[0].d_slots_in, h->prepared.live,
+                        h->ws->ctx[0].d_allow_ids, &h->ws->d_flags->first_unknown,
                         h->prepared.counts.ptr, reinterpret_cast<uint32_t *>(h->prepared.counts.ptr + 1), m);
     if (rc != TV_OK) return rc;
-    TV_CUDA(cudaEventRecord(h->ev_mut, h->stream));             // searches run on other streams: order them after this
-    TV_CUDA(cudaMemcpyAsync(&h->h_flags->first_unknown, &h->d_flags->first_unknown, 8, cudaMemcpyDeviceToHost, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
-    if (spec.ids_host && h->h_flags->first_unknown != ~0ull) {
-        const uint64_t bad = spec.ids_host[h->h_flags->first_unknown];
+    TV_CUDA(cudaEventRecord(h->ws->ev_mut, h->ws->stream));             // searches run on other streams: order them after this
+    TV_CUDA(cudaMemcpyAsync(&h->ws->h_flags->first_unknown, &h->ws->d_flags->first_unknown, 8, cudaMemcpyDeviceToHost, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
+    if (spec.ids_host && h->ws->h_flags->first_unknown != ~0ull) {
+        const uint64_t bad = spec.ids_host[h->ws->h_flags->first_unknown];
         { std::lock_guard<std::mutex> g(h->stat_mu); h->err_id = bad; }
         return fail(h, TV_ERR_UNKNOWN_ID, "allowlist id " + std::to_string(bad) + " is not in the index");
     }
@@ -2041,7 +2148,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
     CtxLease lease(h);
     SearchCtx &c = *lease.c;
     cudaStream_t st = c.stream;
-    TV_CUDA(cudaStreamWaitEvent(st, h->ev_mut, 0));
+    TV_CUDA(cudaStreamWaitEvent(st, h->ws->ev_mut, 0));
     DeviceFlags init{};
     init.first_invalid = ~0ull;
     *c.h_flags = init;
@@ -2122,9 +2229,9 @@ int tv_export_blocked(const tv_index *hc, uint8_t *blocked_out, size_t blocked_c
     if ((blocked_out && blocked_capacity < bytes) || (scales_out && scales_capacity < h->n)) return fail(h, TV_ERR_INVALID_ARGUMENT, "output buffer too small");
     if (h->n == 0) return TV_OK;
     TV_CUDA(cudaSetDevice(h->device));
-    if (blocked_out) TV_CUDA(cudaMemcpyAsync(blocked_out, h->d_codes, bytes, cudaMemcpyDeviceToHost, h->stream));
-    if (scales_out) TV_CUDA(cudaMemcpyAsync(scales_out, h->d_scales, h->n * 4, cudaMemcpyDeviceToHost, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
+    if (blocked_out) TV_CUDA(cudaMemcpyAsync(blocked_out, h->d_codes, bytes, cudaMemcpyDeviceToHost, h->ws->stream));
+    if (scales_out) TV_CUDA(cudaMemcpyAsync(scales_out, h->d_scales, h->n * 4, cudaMemcpyDeviceToHost, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     return TV_OK;
 }
 
@@ -2173,9 +2280,9 @@ int tv_import_packed(tv_index *h, size_t dim, const uint8_t *packed, size_t n, c
     if (rc != TV_OK) { if (was_lazy) { h->dim = 0; h->tables_ready = false; } return rc; }
     std::vector<uint8_t> blocked;
     packed_to_blocked(packed, n, h->bits, int(dim), blocked);
-    TV_CUDA(cudaMemcpyAsync(h->d_codes, blocked.data(), blocked.size(), cudaMemcpyHostToDevice, h->stream));
-    TV_CUDA(cudaMemcpyAsync(h->d_scales, scales, n * 4, cudaMemcpyHostToDevice, h->stream));
-    TV_CUDA(cudaStreamSynchronize(h->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_codes, blocked.data(), blocked.size(), cudaMemcpyHostToDevice, h->ws->stream));
+    TV_CUDA(cudaMemcpyAsync(h->d_scales, scales, n * 4, cudaMemcpyHostToDevice, h->ws->stream));
+    TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     h->n = n;
     h->expanded.reset();
     mutation_done(h);
@@ -2204,9 +2311,9 @@ int gather_parts(tv_index *h, V7Parts &p) {
     p.scales.resize(h->n);
     if (h->n) {
         TV_CUDA(cudaSetDevice(h->device));
-        TV_CUDA(cudaMemcpyAsync(p.blocked.data(), h->d_codes, p.blocked.size(), cudaMemcpyDeviceToHost, h->stream));
-        TV_CUDA(cudaMemcpyAsync(p.scales.data(), h->d_scales, h->n * 4, cudaMemcpyDeviceToHost, h->stream));
-        TV_CUDA(cudaStreamSynchronize(h->stream));
+        TV_CUDA(cudaMemcpyAsync(p.blocked.data(), h->d_codes, p.blocked.size(), cudaMemcpyDeviceToHost, h->ws->stream));
+        TV_CUDA(cudaMemcpyAsync(p.scales.data(), h->d_scales, h->n * 4, cudaMemcpyDeviceToHost, h->ws->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     }
     if (h->kind == TV_KIND_IDMAP) p.ids = h->slot_to_id;
     return TV_OK;
@@ -2271,9 +2378,9 @@ int index_from_image(const uint8_t *data, size_t len, int expect_kind, int devic
     if (rc == TV_OK && p.n) rc = ensure_capacity(h, p.n);
     if (rc != TV_OK) return bail(rc);
     if (p.n) {
-        if (cudaMemcpyAsync(h->d_codes, p.blocked.data(), p.blocked.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-            cudaMemcpyAsync(h->d_scales, p.scales.data(), p.n * 4, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-            cudaStreamSynchronize(h->stream) != cudaSuccess) {
+        if (cudaMemcpyAsync(h->d_codes, p.blocked.data(), p.blocked.size(), cudaMemcpyHostToDevice, h->ws->stream) != cudaSuccess ||
+            cudaMemcpyAsync(h->d_scales, p.scales.data(), p.n * 4, cudaMemcpyHostToDevice, h->ws->stream) != cudaSuccess ||
+            cudaStreamSynchronize(h->ws->stream) != cudaSuccess) {
             h->last_error = "upload of the image failed";
             return bail(TV_ERR_CUDA);
         }
@@ -2369,13 +2476,13 @@ int tv_sync(tv_index *h, const char *path) {
             while (j < need.size() && need[j] == need[j - 1] + 1) ++j;
             const size_t first = need[i], rows_end = std::min(h->n, (need[j - 1] + 1) * kBlock);
             TV_CUDA(cudaMemcpyAsync(codes.data() + i * rb * kBlock, h->d_codes + first * rb * kBlock, (j - i) * rb * kBlock,
-                                    cudaMemcpyDeviceToHost, h->stream));
+                                    cudaMemcpyDeviceToHost, h->ws->stream));
             if (rows_end > first * kBlock)
                 TV_CUDA(cudaMemcpyAsync(scales.data() + i * kBlock, h->d_scales + first * kBlock, (rows_end - first * kBlock) * 4,
-                                        cudaMemcpyDeviceToHost, h->stream));
+                                        cudaMemcpyDeviceToHost, h->ws->stream));
             i = j;
         }
-        TV_CUDA(cudaStreamSynchronize(h->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));
         src.block = [&](size_t block, const uint8_t *&c, const float *&sc) {
             const size_t i = size_t(std::lower_bound(need.begin(), need.end(), block) - need.begin());
             c = codes.data() + i * rb * kBlock;
@@ -2462,8 +2569,8 @@ int tv_rotate(tv_index *h, const float *rows, size_t n, size_t dim, float *rotat
     TV_CUDA(cudaSetDevice(h->device));
     int rc = ensure_tables(h);
     if (rc != TV_OK) return rc;
-    cudaStream_t st = h->stream;
-    SearchCtx &c = h->ctx[0];                                  // the lock is exclusive: no search holds it
+    cudaStream_t st = h->ws->stream;
+    SearchCtx &c = h->ws->ctx[0];                                  // the lock is exclusive: no search holds it
     const size_t nq_pad = (n + 15) / 16 * 16;
     TV_CUDA(h->d_stage.reserve(n * dim));
     TV_CUDA(c.d_qrot.reserve(n * dim));
@@ -2478,7 +2585,7 @@ int tv_rotate(tv_index *h, const float *rows, size_t n, size_t dim, float *rotat
     qp.centroids = h->d_codebook.ptr + 16;
     qp.q_rot = c.d_qrot.ptr; qp.qscale = c.d_qscale.ptr; qp.qbias = c.d_qbias.ptr; qp.luts = c.d_luts.ptr;
     qp.lut_pitch = (h->ngroups + 3) / 4 * 4 * 32;
-    qp.first_invalid = &h->d_flags->first_invalid;
+    qp.first_invalid = &h->ws->d_flags->first_invalid;
     TV_CUDA(launch_query_prep(qp, st));
     h->launches++;
     TV_CUDA(cudaMemcpyAsync(rotated_out, c.d_qrot.ptr, n * dim * 4, cudaMemcpyDeviceToHost, st));
@@ -2549,22 +2656,22 @@ int tv_calibrate(tv_index *h, const float *sample, size_t n, size_t dim) {
     const size_t chunk_rows = std::max<size_t>(1, std::min<size_t>(n, (size_t(128) << 20) / (dim * 4)));
     TV_CUDA(h->d_stage.reserve(chunk_rows * dim));
     TV_CUDA(d_rot.reserve((on_device ? n : chunk_rows) * dim));
-    h->h_flags->first_invalid = ~0ull;
-    TV_CUDA(cudaMemcpyAsync(&h->d_flags->first_invalid, &h->h_flags->first_invalid, 8, cudaMemcpyHostToDevice, h->stream));
+    h->ws->h_flags->first_invalid = ~0ull;
+    TV_CUDA(cudaMemcpyAsync(&h->ws->d_flags->first_invalid, &h->ws->h_flags->first_invalid, 8, cudaMemcpyHostToDevice, h->ws->stream));
     IngestParams p{};
     p.dim = int(dim); p.bits = h->bits; p.ngroups = h->ngroups;
     p.perm0 = h->d_perm.ptr; p.perm1 = h->d_perm.ptr + dim; p.inv_sqrt_block = h->rot.inv_sqrt_block;
     p.boundaries = h->d_codebook.ptr; p.centroids = h->d_codebook.ptr + 16;
-    p.first_invalid = &h->d_flags->first_invalid;
+    p.first_invalid = &h->ws->d_flags->first_invalid;
     for (size_t done = 0; done < n; done += chunk_rows) {
         const size_t rows = std::min(chunk_rows, n - done);
-        TV_CUDA(cudaMemcpyAsync(h->d_stage.ptr, sample + done * dim, rows * dim * 4, cudaMemcpyHostToDevice, h->stream));
+        TV_CUDA(cudaMemcpyAsync(h->d_stage.ptr, sample + done * dim, rows * dim * 4, cudaMemcpyHostToDevice, h->ws->stream));
         p.x = h->d_stage.ptr; p.n = int64_t(rows); p.slot0 = 0; p.row_base = int64_t(done);
         p.rot_out = on_device ? d_rot.ptr + done * dim : d_rot.ptr;
-        TV_CUDA(launch_ingest(p, V, h->stream));
+        TV_CUDA(launch_ingest(p, V, h->ws->stream));
         h->launches++;
-        if (!on_device) TV_CUDA(cudaMemcpyAsync(rotated.data() + done * dim, d_rot.ptr, rows * dim * 4, cudaMemcpyDeviceToHost, h->stream));
-        TV_CUDA(cudaStreamSynchronize(h->stream));           // the staging buffer is reused by the next chunk
+        if (!on_device) TV_CUDA(cudaMemcpyAsync(rotated.data() + done * dim, d_rot.ptr, rows * dim * 4, cudaMemcpyDeviceToHost, h->ws->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));           // the staging buffer is reused by the next chunk
     }
 
     // anchor: probability mass inside the outermost centroid (encode.rs:364-369)
@@ -2579,10 +2686,10 @@ int tv_calibrate(tv_index *h, const float *sample, size_t n, size_t dim) {
     if (on_device) {
         DeviceArray<float> d_q;
         TV_CUDA(d_q.reserve(2 * dim));
-        TV_CUDA(launch_quantile_pair(d_rot.ptr, int64_t(n), int(dim), int64_t(lo_idx), int64_t(hi_idx), d_q.ptr, d_q.ptr + dim, h->stream));
+        TV_CUDA(launch_quantile_pair(d_rot.ptr, int64_t(n), int(dim), int64_t(lo_idx), int64_t(hi_idx), d_q.ptr, d_q.ptr + dim, h->ws->stream));
         h->launches++;
-        TV_CUDA(cudaMemcpyAsync(qe.data(), d_q.ptr, 2 * dim * 4, cudaMemcpyDeviceToHost, h->stream));
-        TV_CUDA(cudaStreamSynchronize(h->stream));
+        TV_CUDA(cudaMemcpyAsync(qe.data(), d_q.ptr, 2 * dim * 4, cudaMemcpyDeviceToHost, h->ws->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     } else {
         for (size_t d = 0; d < dim; ++d) {
             for (size_t i = 0; i < n; ++i) col[i] = rotated[i * dim + d];
@@ -2609,17 +2716,17 @@ int tv_calibrate(tv_index *h, const float *sample, size_t n, size_t dim) {
         for (size_t d = 0; d < dim; ++d) { pair[d] = shift[d]; pair[dim + d] = scale[d]; pair[2 * dim + d] = 1.0f / scale[d]; }
         DeviceArray<float> d_new;
         TV_CUDA(d_new.reserve(3 * dim));
-        TV_CUDA(cudaMemcpyAsync(d_new.ptr, pair.data(), pair.size() * 4, cudaMemcpyHostToDevice, h->stream));
+        TV_CUDA(cudaMemcpyAsync(d_new.ptr, pair.data(), pair.size() * 4, cudaMemcpyHostToDevice, h->ws->stream));
         ReencodeParams rp{};
         rp.codes = h->d_codes; rp.scales = h->d_scales; rp.n = int64_t(h->n);
         rp.dim = int(dim); rp.bits = h->bits; rp.ngroups = h->ngroups;
         rp.boundaries = h->d_codebook.ptr; rp.centroids = h->d_codebook.ptr + 16;
         if (!h->shift.empty()) { rp.old_shift = h->d_calib.ptr; rp.old_inv = h->d_calib.ptr + 2 * dim; }
         rp.new_shift = d_new.ptr; rp.new_scale = d_new.ptr + dim; rp.new_inv = d_new.ptr + 2 * dim;
-        TV_CUDA(launch_reencode(rp, h->stream));
+        TV_CUDA(launch_reencode(rp, h->ws->stream));
         h->expanded.reset();                       // every stored code changed
         h->launches++;
-        TV_CUDA(cudaStreamSynchronize(h->stream));
+        TV_CUDA(cudaStreamSynchronize(h->ws->stream));
     }
     h->shift = shift;
     h->scale_tq = scale;
