@@ -84,16 +84,6 @@ struct PinnedArray {
     }
 };
 
-struct DeviceFlags {        // one pinned + one device copy of the status words of a call
-    unsigned long long first_invalid;
-    unsigned long long n_allowed;
-    unsigned long long first_unknown;   // smallest allowlist index whose id the device table does not hold
-    uint32_t n_live;
-    uint32_t overflow;
-    uint32_t error;
-    uint32_t k_eff;
-};
-
 // CUDA events around the launches of the dominant kernel (scan, ingest) of one call.
 struct Marks {
     std::vector<cudaEvent_t> pool;
@@ -139,6 +129,7 @@ struct SearchCtx {
     Marks marks;
     DeviceFlags *d_flags = nullptr;
     DeviceFlags *h_flags = nullptr;
+    bool flags_clean = false;                // *d_flags is as a new search wants it (the last selection of a search leaves it so)
     DeviceArray<float> d_stage;              // query upload
     DeviceArray<float> d_qrot;               // tv_rotate
     DeviceArray<float> d_qscale, d_qbias;
@@ -157,12 +148,13 @@ struct SearchCtx {
     DeviceArray<uint64_t> d_keys_tmp;        // staging of tv_search_device_keys when the shard holds fewer than k vectors
     PinnedArray<float> h_scores;
     PinnedArray<int64_t> h_slots;
+    PinnedArray<float> h_queries;            // a small batch: query preparation reads it from here
     template <typename F>
     void each_array(F f) {
         f(d_stage); f(d_qrot); f(d_qscale); f(d_qbias); f(d_filter); f(d_luts); f(d_weights); f(d_wfrag); f(d_mask); f(d_mask_bool); f(d_slots_in); f(d_live); f(d_allow_ids); f(d_cand); f(d_thr); f(d_topk); f(d_floor); f(d_keys_all); f(d_cnt); f(d_scores); f(d_slots); f(d_keys_tmp);
     }
     template <typename F>
-    void each_pinned(F f) { f(h_scores); f(h_slots); }
+    void each_pinned(F f) { f(h_scores); f(h_slots); f(h_queries); }
     cudaError_t init() {
         cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&ev0);
@@ -176,6 +168,15 @@ struct SearchCtx {
             if (e == cudaSuccess) marks.pool.push_back(ev);
         }
         return e;
+    }
+    // the status words of a new search, through `stream`
+    cudaError_t reset_flags() {
+        if (flags_clean) return cudaSuccess;
+        DeviceFlags init{};
+        init.first_invalid = ~0ull;
+        init.first_unknown = ~0ull;
+        *h_flags = init;
+        return cudaMemcpyAsync(d_flags, h_flags, sizeof(DeviceFlags), cudaMemcpyHostToDevice, stream);
     }
     ~SearchCtx() {
         if (stream) cudaStreamSynchronize(stream);
@@ -376,6 +377,8 @@ struct tv_index {
     // Readers and writers: searches hold the lock shared and take a SearchCtx from the pool; every call that changes
     // the index, and the accessors that use the handle's own stream, hold it exclusively.
     std::shared_mutex mu;
+    std::mutex mut_mu;
+    bool mut_pending = false;    // under mut_mu or the exclusive lock: the handle's stream has work that ev_mut does not cover
     std::mutex stat_mu;          // error text / detail and the timing figures of the last call
     std::string last_error;
     size_t err_vec = 0, err_coord = 0;
@@ -483,8 +486,18 @@ void collect_marks(tv_index *h) {
 // Called at the end of every call that changed device state on the handle's stream: searches run on their own
 // streams and wait for this event first.  Also drops a prepared mask, which describes the index as it was.
 void mutation_done(tv_index *h) {
-    cudaEventRecord(h->ws->ev_mut, h->ws->stream);
+    h->mut_pending = true;                   // the event is recorded by the next search: one for a row of removals
     h->prepared.valid = false;
+}
+// Makes `st` wait for every mutation enqueued on the handle's stream.
+cudaError_t wait_for_mutations(tv_index *h, cudaStream_t st) {
+    std::lock_guard<std::mutex> g(h->mut_mu);
+    if (h->mut_pending) {
+        cudaError_t e = cudaEventRecord(h->ws->ev_mut, h->ws->stream);
+        if (e != cudaSuccess) return e;
+        h->mut_pending = false;
+    }
+    return cudaStreamWaitEvent(st, h->ws->ev_mut, 0);
 }
 
 // Test hook: with TV_OPT_FAIL_NEXT set, the next guarded allocation or upload of a call reports
@@ -868,7 +881,7 @@ struct SearchScratch {
     uint32_t *wfrag;
     uint8_t *luts;
     uint64_t *cand, *thr, *topk, *lo;      // lo: lowest admissible key per query (paged top-k), or nullptr
-    uint32_t *cnt, *done;                  // done follows cnt: both are cleared together
+    uint32_t *cnt, *done;                  // done (nq + 1 counters) follows cnt: both are cleared together
     size_t w_rows, dim_pad, lut_pitch;
     float *f_scale, *f_mid, *f_max, *f_alpha, *f_suffix;   // affine bound of a filtering scan
     int cap;
@@ -1082,7 +1095,7 @@ int expanded_sync(tv_index *h, cudaStream_t st, const uint32_t level_words[4], b
 // One search through the filtering scan: the first chunk by approximate score, a threshold from its k best, then the whole
 // index in chunks that append survivors, which are scored exactly and selected.
 int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, ScanParams sp, size_t nq, size_t kk,
-                     const MaskOnDevice &m) {
+                     const MaskOnDevice &m, const SearchOutput *out) {
     const size_t n_blocks = (h->n + kBlock - 1) / kBlock;
     const float *qscale = S.qscale, *qbias = S.qbias;
     sp.f_weights = S.weights; sp.f_pitch = int(S.dim_pad); sp.f_alpha = S.f_alpha; sp.f_suffix = S.f_suffix;
@@ -1099,7 +1112,7 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
     const size_t first = std::min(n_blocks, size_t(S.cap) / kBlock);
     int rc = scan(0, first, S.f_mid, true);
     if (rc != TV_OK) return rc;
-    TV_CUDA(launch_select(sp.cb, int(nq), uint32_t(first), m.n_live, st));
+    TV_CUDA(launch_select(sp.cb, int(nq), uint32_t(first), m.n_live, nullptr, st));
     TV_CUDA(launch_bootstrap(sp, int(nq), st));
     h->launches += 2;
     // every survivor costs a gather of its bytes, so the chunks grow gently: a chunk of five times the vectors seen so far
@@ -1110,7 +1123,7 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
         rc = scan(begin, end, S.f_max, false);
         if (rc != TV_OK) return rc;
         TV_CUDA(launch_score_survivors(sp, int(nq), h->sm_count, st));
-        TV_CUDA(launch_select(sp.cb, int(nq), 0u, nullptr, st));
+        TV_CUDA(launch_select(sp.cb, int(nq), 0u, nullptr, end == n_blocks ? out : nullptr, st));
         h->launches += 2;
         begin = end;
     }
@@ -1120,8 +1133,10 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
 // Scan + select over a geometric chunk schedule, all enqueued on `st`.
 //   careful: chunks never exceed the candidate capacity, so no list can overflow whatever the data order.
 //   fresh: the selection state is as query preparation left it.
+//   out: what the last selection finishes the search with, or nullptr.
 int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, const ScanPlan &plan, int mode,
-                   size_t nq, size_t kk, const MaskOnDevice &m, uint32_t *d_overflow, uint32_t *d_error, bool careful, bool fresh) {
+                   size_t nq, size_t kk, const MaskOnDevice &m, uint32_t *d_overflow, uint32_t *d_error, bool careful, bool fresh,
+                   const SearchOutput *out) {
     const size_t n = h->n;
     const int ng = h->ngroups;
     const size_t n_blocks = (n + kBlock - 1) / kBlock;
@@ -1141,9 +1156,9 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
         if (rc != TV_OK) return rc;
     }
 
-    if (plan.use_filter) return enqueue_filtered(h, st, marks, S, sp, nq, kk, m);
+    if (plan.use_filter) return enqueue_filtered(h, st, marks, S, sp, nq, kk, m, out);
     if (!fresh) {
-        TV_CUDA(cudaMemsetAsync(S.cnt, 0, 2 * nq * 4, st));
+        TV_CUDA(cudaMemsetAsync(S.cnt, 0, (2 * nq + 1) * 4, st));
         TV_CUDA(cudaMemsetAsync(S.thr, 0xff, nq * 8, st));
         TV_CUDA(cudaMemsetAsync(S.topk, 0xff, nq * kk * 8, st));
     }
@@ -1215,7 +1230,7 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
                 h->launches++;
             }
         }
-        TV_CUDA(launch_select(cb, int(nq), dense ? uint32_t(end) : 0u, m.n_live, st));
+        TV_CUDA(launch_select(cb, int(nq), dense ? uint32_t(end) : 0u, m.n_live, end >= n_blocks ? out : nullptr, st));
         h->launches++;
         begin = end;
     }
@@ -1316,7 +1331,11 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
 
     // ---- buffers ----
     TV_CUDA(injected_failure(h));
-    if (!queries_on_device) TV_CUDA(c.d_stage.reserve(nq * dim));
+    // A few queries are read by the preparation kernel straight from page-locked memory (48 KB: 2 us at the bus's rate),
+    // which saves a copy of about 10 us; more of them go through the copy engine.
+    const bool small_upload = !queries_on_device && nq * dim * 4 <= (size_t(48) << 10);
+    if (small_upload) TV_CUDA(c.h_queries.reserve(size_t(12) << 10));
+    else if (!queries_on_device) TV_CUDA(c.d_stage.reserve(nq * dim));
     TV_CUDA(c.d_qscale.reserve(nq_pad));
     TV_CUDA(c.d_qbias.reserve(nq_pad));
     const size_t w_rows = (nq + 255) / 256 * 256;
@@ -1328,14 +1347,14 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         TV_CUDA(c.d_luts.reserve(w_rows * lut_pitch));           // padded to whole query groups and whole K slabs for the tensor path
     }
     TV_CUDA(c.d_cand.reserve(nq * size_t(cap)));
-    TV_CUDA(c.d_cnt.reserve(2 * nq));                            // candidate counts, then the selection's part counters
+    TV_CUDA(c.d_cnt.reserve(2 * nq + 1));                        // candidate counts, then the selection's part counters, then the count of finished queries
     TV_CUDA(c.d_thr.reserve(nq));
     TV_CUDA(c.d_topk.reserve(nq * k_page));
     if (pages > 1) {
         TV_CUDA(c.d_floor.reserve(nq));
         TV_CUDA(c.d_keys_all.reserve(nq * kk));
     }
-    if (!out_scores_dev) {
+    if (!out_scores_dev && (pages > 1 || kk > size_t(kSelectMaxK) || out_keys_dev)) {
         TV_CUDA(c.d_scores.reserve(nq * kk));
         TV_CUDA(c.d_slots.reserve(nq * kk));
     }
@@ -1350,17 +1369,19 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     }
 
     // ---- inputs ----
-    TV_CUDA(cudaStreamWaitEvent(st, h->ws->ev_mut, 0));          // after every mutation enqueued on the handle's stream
+    TV_CUDA(wait_for_mutations(h, st));                      // after every mutation enqueued on the handle's stream
     const float *dq = queries;
     if (!queries_on_device) {
-        TV_CUDA(cudaMemcpyAsync(c.d_stage.ptr, queries, nq * dim * 4, cudaMemcpyHostToDevice, st));
-        dq = c.d_stage.ptr;
+        if (small_upload) {
+            std::memcpy(c.h_queries.ptr, queries, nq * dim * 4);
+            dq = c.h_queries.ptr;
+        } else {
+            TV_CUDA(cudaMemcpyAsync(c.d_stage.ptr, queries, nq * dim * 4, cudaMemcpyHostToDevice, st));
+            dq = c.d_stage.ptr;
+        }
     }
-    DeviceFlags init{};
-    init.first_invalid = ~0ull;
-    init.first_unknown = ~0ull;
-    *c.h_flags = init;
-    TV_CUDA(cudaMemcpyAsync(c.d_flags, c.h_flags, sizeof(DeviceFlags), cudaMemcpyHostToDevice, st));
+    TV_CUDA(c.reset_flags());
+    c.flags_clean = false;                                   // until this search has ended well
     TV_CUDA(cudaEventRecord(c.ev0, st));
 
     MaskOnDevice m;
@@ -1382,19 +1403,35 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     out_cb.topk = pages == 1 ? c.d_topk.ptr : c.d_keys_all.ptr;
     out_cb.k = int(kk);
     uint32_t *d_keff = &c.d_flags->k_eff;
+    // In the common case the last selection decodes the rows and publishes the status words, for a host search straight
+    // into page-locked memory; larger k, paged searches and key exports take separate steps.
+    const bool fused = pages == 1 && kk <= size_t(kSelectMaxK) && !out_keys_dev;
+    SearchOutput out{};
+    if (!out_scores_dev && !out_keys_dev) {
+        TV_CUDA(c.h_scores.reserve(nq * kk));
+        TV_CUDA(c.h_slots.reserve(nq * kk));
+    }
+    if (fused) {
+        out.scores = out_scores_dev ? out_scores_dev : c.h_scores.ptr;
+        out.slots = out_scores_dev ? out_slots_dev : c.h_slots.ptr;
+        out.n_allowed = m.n_allowed; out.n = int64_t(n); out.stride_is_k = out_scores_dev ? 0 : 1;
+        out.flags = c.d_flags; out.flags_host = c.h_flags; out.finished = c.d_cnt.ptr + 2 * nq; out.nq = int(nq);
+    }
     // decode / export of the finished rows, the status words and (host searches) the results, then one synchronisation
     auto finish = [&]() -> int {
         if (out_keys_dev) TV_CUDA(launch_export_keys(out_cb.topk, int64_t(nq * kk), key_offset, out_keys_dev, st));
-        if (out_scores_dev) TV_CUDA(launch_finalize(out_cb, int(nq), m.n_allowed, int64_t(n), out_scores_dev, out_slots_dev, d_keff, 0, st));
-        else TV_CUDA(launch_finalize(out_cb, int(nq), m.n_allowed, int64_t(n), c.d_scores.ptr, c.d_slots.ptr, d_keff, 1, st));
-        h->launches++;
+        if (!fused) {
+            if (out_scores_dev) TV_CUDA(launch_finalize(out_cb, int(nq), m.n_allowed, int64_t(n), out_scores_dev, out_slots_dev, d_keff, 0, st));
+            else TV_CUDA(launch_finalize(out_cb, int(nq), m.n_allowed, int64_t(n), c.d_scores.ptr, c.d_slots.ptr, d_keff, 1, st));
+            h->launches++;
+        }
         TV_CUDA(cudaEventRecord(c.ev1, st));
-        TV_CUDA(cudaMemcpyAsync(c.h_flags, c.d_flags, sizeof(DeviceFlags), cudaMemcpyDeviceToHost, st));
-        if (!out_scores_dev && !out_keys_dev) {
-            TV_CUDA(c.h_scores.reserve(nq * kk));
-            TV_CUDA(c.h_slots.reserve(nq * kk));
-            TV_CUDA(cudaMemcpyAsync(c.h_scores.ptr, c.d_scores.ptr, nq * kk * 4, cudaMemcpyDeviceToHost, st));
-            TV_CUDA(cudaMemcpyAsync(c.h_slots.ptr, c.d_slots.ptr, nq * kk * 8, cudaMemcpyDeviceToHost, st));
+        if (!fused) {
+            TV_CUDA(cudaMemcpyAsync(c.h_flags, c.d_flags, sizeof(DeviceFlags), cudaMemcpyDeviceToHost, st));
+            if (!out_scores_dev && !out_keys_dev) {
+                TV_CUDA(cudaMemcpyAsync(c.h_scores.ptr, c.d_scores.ptr, nq * kk * 4, cudaMemcpyDeviceToHost, st));
+                TV_CUDA(cudaMemcpyAsync(c.h_slots.ptr, c.d_slots.ptr, nq * kk * 8, cudaMemcpyDeviceToHost, st));
+            }
         }
         TV_CUDA(cudaStreamSynchronize(st));
         float ms = 0.f;
@@ -1409,7 +1446,8 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         S.lo = page == 0 ? nullptr : c.d_floor.ptr;
         for (int attempt = 0; attempt < 3; ++attempt) {
             const bool careful = attempt == 2 || h->force_careful;
-            rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, k_this, m, &c.d_flags->overflow, &c.d_flags->error, careful, page == 0 && attempt == 0);
+            rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, k_this, m, &c.d_flags->overflow, &c.d_flags->error, careful, page == 0 && attempt == 0,
+                                fused ? &out : nullptr);
             if (rc != TV_OK) { c.marks.used = 0; return rc; }
             if (pages == 1) {
                 rc = finish();                                  // the common case: one submission, one synchronisation
@@ -1445,6 +1483,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         }
     }
     *k_eff_out = c.h_flags->k_eff;
+    c.flags_clean = fused;
     return TV_OK;
 }
 
@@ -2092,7 +2131,7 @@ NoAllocLayout carve_noalloc(unsigned char *base) {
     L.cand = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * kNoAllocCap * 8));           // 256 KiB
     L.thr = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * 8));
     L.topk = reinterpret_cast<uint64_t *>(take(kNoAllocMaxQueries * kNoAllocMaxK * 8));          //   8 KiB
-    L.cnt = reinterpret_cast<uint32_t *>(take(2 * kNoAllocMaxQueries * 4));
+    L.cnt = reinterpret_cast<uint32_t *>(take((2 * kNoAllocMaxQueries + 1) * 4));
     static_assert(16 * kNoAllocMaxDim + (kNoAllocMaxDim / 32) * 512 +
                           kNoAllocMaxQueries * (kNoAllocMaxDim / 2) * 32 + kNoAllocMaxQueries * kNoAllocCap * 8 +
                           kNoAllocMaxQueries * kNoAllocMaxK * 8 + 8 * 256 <= kNoAllocScratchBytes,
@@ -2148,11 +2187,9 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
     CtxLease lease(h);
     SearchCtx &c = *lease.c;
     cudaStream_t st = c.stream;
-    TV_CUDA(cudaStreamWaitEvent(st, h->ws->ev_mut, 0));
-    DeviceFlags init{};
-    init.first_invalid = ~0ull;
-    *c.h_flags = init;
-    TV_CUDA(cudaMemcpyAsync(c.d_flags, c.h_flags, sizeof(DeviceFlags), cudaMemcpyHostToDevice, st));
+    TV_CUDA(wait_for_mutations(h, st));
+    TV_CUDA(c.reset_flags());
+    c.flags_clean = false;
     TV_CUDA(cudaEventRecord(c.ev0, st));
 
     // The array still holds the previous call's data.  Query preparation clears the query operands it does not
@@ -2167,7 +2204,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
     // capacity, which cannot overflow; neither schedule needs memory beyond the fixed array.
     for (int attempt = 0; attempt < 2; ++attempt) {
         const bool careful = attempt == 1 || h->force_careful;
-        rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, kk, no_mask, &c.d_flags->overflow, &c.d_flags->error, careful, attempt == 0);
+        rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, kk, no_mask, &c.d_flags->overflow, &c.d_flags->error, careful, attempt == 0, nullptr);
         if (rc != TV_OK) { c.marks.used = 0; return rc; }
         TV_CUDA(launch_finalize(out_cb, int(nq), nullptr, int64_t(n), scores_out_device, slots_out_device, &c.d_flags->k_eff, 0, st));
         h->launches++;

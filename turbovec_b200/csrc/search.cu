@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParam
         return;
     }
     if (p.cnt != nullptr) {
-        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; }
+        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; if (q == 0) p.done[p.nq] = 0; }
         for (int i = tid; i < p.k; i += kPrepThreads) p.topk[size_t(q) * p.k + i] = kEmptyKey;
     }
     const float *src = p.queries + size_t(q) * dim;

@@ -46,7 +46,7 @@ struct QueryPrepParams {
         int8_t levels[8];
     } filter;
     // selection state of the batch, reset here (cnt == nullptr: none)
-    uint32_t *cnt, *done;
+    uint32_t *cnt, *done;          // done[nq] = SearchOutput::finished
     uint64_t *thr, *topk;
     int k;
     int mtiles_total;              // ceil(nq / 16)
@@ -71,6 +71,17 @@ cudaError_t launch_idtab_upsert(uint64_t *keys, uint32_t *vals, int log2cap, con
 cudaError_t launch_idtab_lookup(const uint64_t *keys, const uint32_t *vals, int log2cap, const uint64_t *ids, int64_t n, uint64_t *words,
                                 unsigned long long *first_unknown, cudaStream_t s);
 
+// Status words of one call on the device; the host's copy arrives when the call ends.
+struct DeviceFlags {
+    unsigned long long first_invalid;
+    unsigned long long n_allowed;
+    unsigned long long first_unknown;   // smallest allowlist index whose id the device table does not hold
+    uint32_t n_live;
+    uint32_t overflow;
+    uint32_t error;
+    uint32_t k_eff;
+};
+
 // ---- candidate machinery ----
 // Scan kernels append the key of every (query, slot) whose key is below thr[query] to
 // cand[query*cap ...]; cnt[query] counts appends (it may exceed cap: the excess is dropped and the
@@ -92,7 +103,21 @@ struct CandidateBuffers {
 constexpr int kSelectMaxK = 512;       // larger k: the bitonic form in search.cu
 constexpr int kSelectSegment = 4096;   // keys one CTA selects from
 int candidate_capacity(size_t k, size_t nq, size_t n);
-cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blocks, const uint32_t *n_live, cudaStream_t s);
+// The last selection of a search can finish it: `out` receives the decoded rows as launch_finalize writes them, in device
+// or page-locked host memory, and the CTA that ends last copies the status words to flags_host and, unless a list
+// overflowed, leaves the device's copy as a new search wants it.
+struct SearchOutput {
+    float *scores;
+    int64_t *slots;
+    const unsigned long long *n_allowed;   // or nullptr: all n
+    int64_t n;
+    int stride_is_k;
+    DeviceFlags *flags, *flags_host;
+    uint32_t *finished;                    // queries finished (zero between launches)
+    int nq;
+    int q0;                                // first query of the launch (set by launch_select)
+};
+cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blocks, const uint32_t *n_live, const SearchOutput *out, cudaStream_t s);
 cudaError_t launch_select_sort(const CandidateBuffers &cb, int nq, int dense_count, cudaStream_t s);
 // Result keys (score-descending image << 32 | slot) of a finished search, `offset` added to every slot.
 cudaError_t launch_export_keys(const uint64_t *topk, int64_t count, uint64_t offset, uint64_t *out, cudaStream_t s);

@@ -145,7 +145,7 @@ __device__ int block_smallest(const uint64_t (&key)[kSelKeysPerThread], int k, S
 
 // dense_blocks > 0: the scan wrote 32 keys per scanned block without counting them, for the first min(dense_blocks,
 // *n_live) positions, and there are no earlier results.
-__global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuffers cb, uint32_t dense_blocks, const uint32_t *n_live) {
+__global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuffers cb, uint32_t dense_blocks, const uint32_t *n_live, SearchOutput out) {
     __shared__ SelectShared sh;
     const int q = blockIdx.y, tid = threadIdx.x;
     const uint32_t part = blockIdx.x;
@@ -193,6 +193,29 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
         cb.thr[q] = m == cb.k ? sh.sorted[cb.k - 1] : kEmptyKey;        // kEmptyKey until k results exist: everything still passes
         cb.cnt[q] = 0;
     }
+    if (out.scores == nullptr) return;
+    const unsigned long long allowed = out.n_allowed ? *reinterpret_cast<const volatile unsigned long long *>(out.n_allowed) : (unsigned long long)out.n;
+    const int k_eff = int(min((unsigned long long)cb.k, min((unsigned long long)out.n, allowed)));
+    const size_t row = (size_t(q) + out.q0) * (out.stride_is_k ? cb.k : k_eff);
+    for (int i = tid; i < k_eff; i += kSelThreads) {
+        // (-inf, 0) padding as search.rs:4341-4352
+        out.scores[row + i] = i < m ? desc_bits_to_score(uint32_t(sh.sorted[i] >> 32)) : -INFINITY;
+        out.slots[row + i] = i < m ? int64_t(sh.sorted[i] & 0xffffffffu) : 0;
+    }
+    __threadfence_system();                                             // the rows may lie in host memory
+    __syncthreads();
+    if (tid != 0 || atomicAdd(out.finished, 1u) != uint32_t(out.nq) - 1u) return;
+    __threadfence();
+    *out.finished = 0;
+    volatile DeviceFlags *f = out.flags, *host = out.flags_host;
+    const uint32_t overflow = f->overflow;
+    host->first_invalid = f->first_invalid; host->n_allowed = f->n_allowed; host->first_unknown = f->first_unknown;
+    host->n_live = f->n_live; host->overflow = overflow; host->error = f->error; host->k_eff = uint32_t(k_eff);
+    if (overflow == 0) {
+        f->first_invalid = ~0ull; f->n_allowed = 0; f->first_unknown = ~0ull;
+        f->n_live = 0; f->error = 0; f->k_eff = 0;
+    }
+    __threadfence_system();
 }
 
 }  // namespace
@@ -209,8 +232,9 @@ int candidate_capacity(size_t k, size_t nq, size_t n) {
     return int(parts * kSelectSegment);
 }
 
-cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blocks, const uint32_t *n_live, cudaStream_t s) {
+cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blocks, const uint32_t *n_live, const SearchOutput *out, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
+    if (cb.k > kSelectMaxK && out != nullptr) return cudaErrorInvalidValue;
     if (cb.k > kSelectMaxK) return launch_select_sort(cb, nq, int(dense_blocks) * 32, s);
     const uint32_t list = dense_blocks > 0 ? std::min<uint32_t>(dense_blocks * 32u, uint32_t(cb.cap)) : uint32_t(cb.cap);
     const uint32_t parts = (list + kSelectSegment - 1) / kSelectSegment;
@@ -218,8 +242,10 @@ cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blo
     // queries on grid.y would stop at 65,535: larger batches in slices
     for (int q0 = 0; q0 < nq; q0 += 32768) {
         CandidateBuffers part = cb;
+        SearchOutput o{};
+        if (out != nullptr) { o = *out; o.q0 = q0; }
         part.cand += size_t(q0) * cb.cap; part.cnt += q0; part.thr += q0; part.topk += size_t(q0) * cb.k; part.done += q0;
-        select_parts_kernel<<<dim3(parts, unsigned(std::min(nq - q0, 32768))), kSelThreads, 0, s>>>(part, dense_blocks, n_live);
+        select_parts_kernel<<<dim3(parts, unsigned(std::min(nq - q0, 32768))), kSelThreads, 0, s>>>(part, dense_blocks, n_live, o);
     }
     return cudaGetLastError();
 }
