@@ -105,6 +105,23 @@ __device__ __forceinline__ float max_nan(float a, float b) {   // NaN wins, unli
 }
 
 
+// Two f32 operations in one instruction, each rounded on its own exactly like the scalar one.  The rotation warps are short
+// of issue slots, not of arithmetic.
+__device__ __forceinline__ void add2(float &a, float &b, float x0, float x1, float y0, float y1) {
+    asm("{\n\t.reg .b64 x, y, d;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 d, x, y;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(a), "=f"(b) : "f"(x0), "f"(x1), "f"(y0), "f"(y1));
+}
+__device__ __forceinline__ void mul2(float &a, float &b, float x0, float x1, float y) {
+    asm("{\n\t.reg .b64 x, y, d;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmul.rn.f32x2 d, x, y;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(a), "=f"(b) : "f"(x0), "f"(x1), "f"(y));
+}
+// x * y + z with one y for both
+__device__ __forceinline__ void fma2(float &a, float &b, float x0, float x1, float y, float z0, float z1) {
+    asm("{\n\t.reg .b64 x, y, z, d;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmov.b64 z, {%5, %6};\n\tfma.rn.f32x2 d, x, y, z;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(a), "=f"(b) : "f"(x0), "f"(x1), "f"(y), "f"(z0), "f"(z1));
+}
+
+
 // Vectors per wave = rotation warps: 8 (three warpgroups, 384 threads), or 4 (two warpgroups, 256 threads) for
 // dimensions whose rows would not fit twice eight times in shared memory.  Warps V .. V+3 are the service
 // warps: norm (even waves), staging, norm (odd waves), copy.
@@ -184,11 +201,18 @@ __device__ __forceinline__ void wht_blocks(float (&v)[R * NBLK], int lane) {
         for (int b = 0; b < NBLK; ++b) {
 #pragma unroll
             for (int i = 0; i < R; i += 2 * len) {
+                if (len == 1) {
+                    const float x = v[b * R + i], y = v[b * R + i + 1];
+                    v[b * R + i] = __fadd_rn(x, y);
+                    v[b * R + i + 1] = __fsub_rn(x, y);
+                } else {
 #pragma unroll
-                for (int j = i; j < i + len; ++j) {
-                    const float x = v[b * R + j], y = v[b * R + j + len];
-                    v[b * R + j] = __fadd_rn(x, y);
-                    v[b * R + j + len] = __fsub_rn(x, y);
+                    for (int j = i; j < i + len; j += 2) {   // register pairs; x - y as the exact -y plus x, rounded once
+                        float *a = &v[b * R + j], *c = &v[b * R + j + len];
+                        const float x0 = a[0], x1 = a[1], y0 = c[0], y1 = c[1];
+                        add2(a[0], a[1], x0, x1, y0, y1);
+                        fma2(c[0], c[1], y0, y1, -1.0f, x0, x1);
+                    }
                 }
             }
         }
@@ -204,6 +228,16 @@ __device__ __forceinline__ void wht_blocks(float (&v)[R * NBLK], int lane) {
             for (int r0 = 0; r0 < R; ++r0) {
                 if (r0 & t) continue;
                 const int r1 = r0 | t;
+                if (t > 1) {                                  // two neighbouring pairs at a time
+                    if (r0 & 1) continue;
+                    float *a = &v[b * R + r0], *c = &v[b * R + r1];
+                    const float keep0 = upper ? c[0] : a[0], keep1 = upper ? c[1] : a[1];
+                    const float send0 = upper ? -a[0] : c[0], send1 = upper ? -a[1] : c[1];
+                    const float recv0 = __shfl_xor_sync(kFullMask, send0, 1 << i), recv1 = __shfl_xor_sync(kFullMask, send1, 1 << i);
+                    fma2(a[0], a[1], recv0, recv1, cs, keep0, keep1);
+                    fma2(c[0], c[1], keep0, keep1, -cs, recv0, recv1);
+                    continue;
+                }
                 const float keep = upper ? v[b * R + r1] : v[b * R + r0];
                 const float send = upper ? -v[b * R + r0] : v[b * R + r1];
                 const float recv = __shfl_xor_sync(kFullMask, send, 1 << i);
@@ -332,9 +366,10 @@ __global__ void __launch_bounds__((V + 4) * 32, 1) ingest_fast_kernel(IngestPara
                     wht_blocks<R, NBLK>(v, lane);
 #pragma unroll
                     for (int k = 0; k < T; ++k) {
+                        if ((k & 1) == 0) mul2(v[k], v[k + 1], v[k], v[k + 1], isb);
                         uint32_t at = rl;
                         if constexpr (kExchange) at = rb + __byte_perm(sbank[k >> 2], 0, 0x4440 + (k & 3));
-                        sts_f32(at + row_of<R>(k) * 128, __fmul_rn(v[k], isb));
+                        sts_f32(at + row_of<R>(k) * 128, v[k]);
                     }
                     __syncwarp();
                     // round 2
@@ -352,8 +387,8 @@ __global__ void __launch_bounds__((V + 4) * 32, 1) ingest_fast_kernel(IngestPara
                     double tabs = 0.0;                                // sum |term| of this lane (calibrated)
 #pragma unroll
                     for (int k = 0; k < T; ++k) {
-                        const float y = __fmul_rn(v[k], isb);
-                        v[k] = y;
+                        if ((k & 1) == 0) mul2(v[k], v[k + 1], v[k], v[k + 1], isb);
+                        const float y = v[k];
                         const int kk = row_of<R>(k);               // this register holds coordinate kk * 32 + lane
                         float c = y, sh = 0.0f;
                         if constexpr (CALIB) {                     // (rot + shift) * scale, encode.rs:1447
