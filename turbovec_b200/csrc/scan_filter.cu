@@ -48,7 +48,7 @@ __device__ __forceinline__ void exact_keys(const ScanParams &p, const uint8_t *l
         src[j] = p.codes + size_t(slot[j] >> 5) * ng * 32 + (slot[j] & 31u);
         vs[j] = p.vec_scales[slot[j]];
         facc[j] = qb; total[j] = 0; left[j] = sum[j];
-        need[j] = EXIT ? dismissal_bound(qs, qb, t, vs[j]) : 0;
+        need[j] = 0;
     }
     for (int g0 = 0; g0 < ng && alive; g0 += 256) {
         int part[kTogether];
@@ -83,6 +83,10 @@ __device__ __forceinline__ void exact_keys(const ScanParams &p, const uint8_t *l
                         w[j] = __dp4a(int(__byte_perm(p.level_words[0], p.level_words[1], sel)), int(wg), w[j]);
                     }
                 }
+            }
+            if (EXIT && h0 == 0) {                       // only now: the scales were requested with the first bytes
+#pragma unroll
+                for (int j = 0; j < kTogether; ++j) need[j] = dismissal_bound(qs, qb, t, vs[j]);
             }
             const float rest = EXIT ? p.f_suffix[size_t(q) * kFilterBatches + h0 / kFilterBatch + 1] : 0.0f;
 #pragma unroll
@@ -128,7 +132,7 @@ __device__ __forceinline__ void load_weights(const ScanParams &p, int q, uint32_
 }
 
 // cand[q][i] = (W . L, slot) -> exact key, or kEmptyKey when it does not beat the k-th best.  Grid (shares of a list, queries).
-__global__ void __launch_bounds__(kScoreThreads) score_survivors_kernel(ScanParams p) {
+__global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t *wq = reinterpret_cast<uint32_t *>(smem_raw + size_t(p.ngroups) * 32);
     const int q = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

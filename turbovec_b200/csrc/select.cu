@@ -202,9 +202,11 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
         out.scores[row + i] = i < m ? desc_bits_to_score(uint32_t(sh.sorted[i] >> 32)) : -INFINITY;
         out.slots[row + i] = i < m ? int64_t(sh.sorted[i] & 0xffffffffu) : 0;
     }
-    __threadfence_system();                                             // the rows may lie in host memory
+    // (the host reads the rows after the kernel has ended; only the status words are passed on between CTAs)
     __syncthreads();
-    if (tid != 0 || atomicAdd(out.finished, 1u) != uint32_t(out.nq) - 1u) return;
+    if (tid != 0) return;
+    __threadfence();
+    if (atomicAdd(out.finished, 1u) != uint32_t(out.nq) - 1u) return;
     __threadfence();
     *out.finished = 0;
     volatile DeviceFlags *f = out.flags, *host = out.flags_host;
@@ -215,7 +217,6 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
         f->first_invalid = ~0ull; f->n_allowed = 0; f->first_unknown = ~0ull;
         f->n_live = 0; f->error = 0; f->k_eff = 0;
     }
-    __threadfence_system();
 }
 
 }  // namespace
