@@ -1115,10 +1115,11 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
     TV_CUDA(launch_select(sp.cb, int(nq), uint32_t(first), m.n_live, nullptr, st));
     TV_CUDA(launch_bootstrap(sp, int(nq), st));
     h->launches += 2;
-    // every survivor costs a gather of its bytes, so the chunks grow gently: a chunk of five times the vectors seen so far
-    // brings about five times k results above the threshold and, below it, what the bound cannot tell from them
+    // every survivor costs a gather of its bytes, so the chunks grow gently: a chunk of three times the vectors seen so far
+    // brings about three times k results above the threshold and, below it, what the bound cannot tell from them
+    // (x4 / x6 / x9 / x14: 1,155 / 1,195 / 1,186 / 1,452 us for 1.2 M x 200 2-bit, batch 1,024)
     for (size_t begin = 0, seen = first; begin < n_blocks;) {
-        size_t end = std::min(n_blocks, std::max(begin, seen) * 6);
+        size_t end = std::min(n_blocks, std::max(begin, seen) * 4);
         if (end + end / 2 >= n_blocks) end = n_blocks;
         rc = scan(begin, end, S.f_max, false);
         if (rc != TV_OK) return rc;

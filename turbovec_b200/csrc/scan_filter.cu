@@ -122,11 +122,13 @@ __device__ __forceinline__ void load_tables(const ScanParams &p, int q, uint4 *l
 __device__ __forceinline__ void load_weights(const ScanParams &p, int q, uint32_t *wq) {
     const uint8_t *row = reinterpret_cast<const uint8_t *>(p.f_weights) + size_t(q) * p.f_pitch;
     for (int g = threadIdx.x; g < p.ngroups; g += kScoreThreads) {
-        if (p.bits == 2) {                                // rows of levels2_coord order: pairs of bytes in words w and w + 2 of a chunk
-            const uint8_t *c = row + (g >> 2) * 16 + ((g >> 1) & 1) * 4 + (g & 1) * 2;
-            wq[g] = uint32_t(*reinterpret_cast<const uint16_t *>(c)) | uint32_t(*reinterpret_cast<const uint16_t *>(c + 8)) << 16;
+        // rows in filter_coord order (search.cu)
+        if (p.bits == 2) {
+            const int c = g & 7, i = (g >> 3) & 3;
+            const uint8_t *at = row + (g >> 5) * 128 + c * 16 + (i >> 1) * 4 + (i & 1) * 2;
+            wq[g] = uint32_t(*reinterpret_cast<const uint16_t *>(at)) | uint32_t(*reinterpret_cast<const uint16_t *>(at + 8)) << 16;
         } else {
-            wq[g] = *reinterpret_cast<const uint16_t *>(row + 2 * g);
+            wq[g] = *reinterpret_cast<const uint16_t *>(row + (g >> 6) * 128 + (g & 7) * 16 + ((g >> 3) & 7) * 2);
         }
     }
 }

@@ -272,12 +272,25 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
 #pragma unroll
                 for (int u = 0; u < kUnits; ++u) dst[u][0] = (f_have && g < ng) ? __ldg(f_src + size_t(g) * 8 + u * 4) : 0u;
             } else if constexpr (KIND == kLevels2) {
-                // a slab is 32 byte-groups of four coordinates; chunk `octet` = groups 4 octet .. + 3
-                const int g0 = f_slab * (kSlabK / 4) + octet * 4;
+                // a slab is 32 byte-groups of four coordinates; chunk `octet` = groups octet + 8r, so that a load instruction
+                // of the warp reads eight neighbouring groups (two lines) and not one of every four (eight lines: the tag
+                // lookups took 288 of 1,018 cycles a slab)
+                const int g0 = f_slab * (kSlabK / 4) + octet;
+                const uint32_t *src = f_src + g0 * 8;
+                if (f_have && g0 + 24 < ng) {
 #pragma unroll
-                for (int u = 0; u < kUnits; ++u)
+                    for (int r = 0; r < 4; ++r) dst[0][r] = __ldg(src + r * 64);
+                } else {
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) dst[u][r] = (f_have && g0 + r < ng) ? __ldg(f_src + size_t(g0 + r) * 8 + u * 4) : 0u;
+                    for (int r = 0; r < 4; ++r) dst[0][r] = (f_have && g0 + 8 * r < ng) ? __ldg(src + r * 64) : 0u;
+                }
+            } else if constexpr (KIND == kLevels3) {
+                // 64 byte-groups of two coordinates; chunk `octet` = groups octet + 8r
+                const int g0 = f_slab * (kSlabK / 2) + octet;
+                const uint32_t *src = f_src + g0 * 8;
+                const bool whole = f_have && g0 + 56 < ng;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) dst[0][r] = (whole || (f_have && g0 + 8 * r < ng)) ? __ldg(src + r * 64) : 0u;
             } else {
                 const int g0 = f_slab * (kSlabK / 2) + octet * 8;
                 const uint32_t *src = f_src + size_t(g0) * 8;
@@ -297,79 +310,114 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
 #pragma unroll
         for (int a = 0; a < kAhead; ++a) fetch(w[a]);
         bool ok = true;
-        for (uint32_t f0 = 0; f0 < total && ok; f0 += kAhead) {
+        if constexpr (KIND == kLevels2) {
+            // two slabs to a step: one wait for the stores to become visible to the MMAs, and twice the independent work
+            static_assert(kAhead % 2 == 0 && kStages % 2 == 0, "slabs go in pairs");
+            for (uint32_t f0 = 0; f0 < total && ok; f0 += kAhead) {
 #pragma unroll
-            for (int a = 0; a < kAhead; ++a) {
-                const uint32_t f = f0 + uint32_t(a);
-                if (f >= total || !ok) break;
-                const int st = f % kStages;
-                uint4 v[kUnits][4];
+                for (int a = 0; a < kAhead; a += 2) {
+                    const uint32_t f = f0 + uint32_t(a);
+                    if (f >= total || !ok) break;
+                    uint4 v[2][4];
 #pragma unroll
-                for (int u = 0; u < kUnits; ++u) {
-                    if constexpr (ONEHOT) {
-                        // byte j of the word = code byte of vector j in this chunk's group; its high (even chunk)
-                        // or low (odd chunk) nibble n becomes a 16-byte one-hot: byte n = 1
-                        const uint32_t word = w[a][u][0];
-                        const uint32_t nibs = (octet & 1) ? (word & 0x0f0f0f0fu) : ((word >> 4) & 0x0f0f0f0fu);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const uint32_t n = (nibs >> (8 * j)) & 15u;
-                            const uint32_t bit = 1u << ((n & 3u) * 8u);
-                            const uint32_t q = n >> 2;
-                            v[u][j].x = q == 0 ? bit : 0u; v[u][j].y = q == 1 ? bit : 0u;
-                            v[u][j].z = q == 2 ? bit : 0u; v[u][j].w = q == 3 ? bit : 0u;
-                        }
-                    } else if constexpr (KIND == kLevels2) {
+                    for (int h = 0; h < 2; ++h) {
                         // 4x4 byte transpose: word j = the four groups of vector j.  Its fields at bits 4i (coordinates 3 and 1 of
                         // a group) and 4i + 2 (coordinates 2 and 0) select levels; the query rows are stored in this order
-                        // (kLevels2Order in search.cu).
-                        const uint32_t *x = w[a][u];
+                        // (filter_coord in search.cu).
+                        const uint32_t *x = w[a + h][0];
                         const uint32_t t0 = prmt(x[0], x[1], 0x5140), t1 = prmt(x[0], x[1], 0x7362);
                         const uint32_t t2 = prmt(x[2], x[3], 0x5140), t3 = prmt(x[2], x[3], 0x7362);
                         const uint32_t xv[4] = {prmt(t0, t2, 0x5410), prmt(t0, t2, 0x7632), prmt(t1, t3, 0x5410), prmt(t1, t3, 0x7632)};
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const uint32_t e = xv[j] & 0x33333333u, o = (xv[j] >> 2) & 0x33333333u;
-                            v[u][j].x = prmt(T[0], 0u, e); v[u][j].y = prmt(T[0], 0u, mad_hi(e, 0x10000u, 0u));
-                            v[u][j].z = prmt(T[0], 0u, o); v[u][j].w = prmt(T[0], 0u, mad_hi(o, 0x10000u, 0u));
+                            v[h][j].x = prmt(T[0], 0u, e); v[h][j].y = prmt(T[0], 0u, mad_hi(e, 0x10000u, 0u));
+                            v[h][j].z = prmt(T[0], 0u, o); v[h][j].w = prmt(T[0], 0u, mad_hi(o, 0x10000u, 0u));
                         }
-                    } else {
-                        // 4x4 byte transposes: bytes of vector j of the unit in groups g0..g0+3 (xlo) and g0+4..g0+7 (xhi)
-                        const uint32_t *x = w[a][u];
-                        const uint32_t t0 = prmt(x[0], x[1], 0x5140), t1 = prmt(x[0], x[1], 0x7362);
-                        const uint32_t t2 = prmt(x[2], x[3], 0x5140), t3 = prmt(x[2], x[3], 0x7362);
-                        const uint32_t u0 = prmt(x[4], x[5], 0x5140), u1 = prmt(x[4], x[5], 0x7362);
-                        const uint32_t u2 = prmt(x[6], x[7], 0x5140), u3 = prmt(x[6], x[7], 0x7362);
-                        const uint32_t xlo[4] = {prmt(t0, t2, 0x5410), prmt(t0, t2, 0x7632), prmt(t1, t3, 0x5410), prmt(t1, t3, 0x7632)};
-                        const uint32_t xhi[4] = {prmt(u0, u2, 0x5410), prmt(u0, u2, 0x7632), prmt(u1, u3, 0x5410), prmt(u1, u3, 0x7632)};
+                        fetch(w[a + h]);                  // refill these ring slots (slab f + h + kAhead)
+                    }
+                    const int slabs = min(2u, total - f);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (h >= slabs || !ok) break;
+                        const int st = (f + h) % kStages;
+                        ok = mbar_wait(&sh->empty[st], (((f + h) / kStages) & 1) ^ 1, p.cb.error);
+                        if (!ok) break;
+                        unsigned char *a_stage = stages + size_t(st) * kStageBytes;
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            if constexpr (KIND == kLevels3) {        // a nibble below 8 is a selector as it stands
-                                v[u][j].x = prmt(T[0], T[1], xlo[j]); v[u][j].y = prmt(T[0], T[1], mad_hi(xlo[j], 0x10000u, 0u));
-                                v[u][j].z = prmt(T[0], T[1], xhi[j]); v[u][j].w = prmt(T[0], T[1], mad_hi(xhi[j], 0x10000u, 0u));
-                            } else {
-                                expand8(xlo[j], T, v[u][j].x, v[u][j].y);
-                                expand8(xhi[j], T, v[u][j].z, v[u][j].w);
+                            const int row = blk_in_item * 32 + quad0 * 4 + j;
+                            *reinterpret_cast<uint4 *>(a_stage + (row >> 3) * 1024 + (row & 7) * 128 + ((octet ^ (row & 7)) << 4)) = v[h][j];
+                        }
+                    }
+                    if (!ok) break;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA
+                    __syncwarp();
+                    if (lane == 0)
+                        for (int h = 0; h < slabs; ++h) mbar_arrive(&sh->full[(f + h) % kStages]);
+                }
+            }
+        } else {
+            for (uint32_t f0 = 0; f0 < total && ok; f0 += kAhead) {
+#pragma unroll
+                for (int a = 0; a < kAhead; ++a) {
+                    const uint32_t f = f0 + uint32_t(a);
+                    if (f >= total || !ok) break;
+                    const int st = f % kStages;
+                    uint4 v[kUnits][4];
+#pragma unroll
+                    for (int u = 0; u < kUnits; ++u) {
+                        if constexpr (ONEHOT) {
+                            // byte j of the word = code byte of vector j in this chunk's group; its high (even chunk)
+                            // or low (odd chunk) nibble n becomes a 16-byte one-hot: byte n = 1
+                            const uint32_t word = w[a][u][0];
+                            const uint32_t nibs = (octet & 1) ? (word & 0x0f0f0f0fu) : ((word >> 4) & 0x0f0f0f0fu);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const uint32_t n = (nibs >> (8 * j)) & 15u;
+                                const uint32_t bit = 1u << ((n & 3u) * 8u);
+                                const uint32_t q = n >> 2;
+                                v[u][j].x = q == 0 ? bit : 0u; v[u][j].y = q == 1 ? bit : 0u;
+                                v[u][j].z = q == 2 ? bit : 0u; v[u][j].w = q == 3 ? bit : 0u;
+                            }
+                        } else {
+                            // 4x4 byte transposes: bytes of vector j of the unit in groups g0..g0+3 (xlo) and g0+4..g0+7 (xhi)
+                            const uint32_t *x = w[a][u];
+                            const uint32_t t0 = prmt(x[0], x[1], 0x5140), t1 = prmt(x[0], x[1], 0x7362);
+                            const uint32_t t2 = prmt(x[2], x[3], 0x5140), t3 = prmt(x[2], x[3], 0x7362);
+                            const uint32_t u0 = prmt(x[4], x[5], 0x5140), u1 = prmt(x[4], x[5], 0x7362);
+                            const uint32_t u2 = prmt(x[6], x[7], 0x5140), u3 = prmt(x[6], x[7], 0x7362);
+                            const uint32_t xlo[4] = {prmt(t0, t2, 0x5410), prmt(t0, t2, 0x7632), prmt(t1, t3, 0x5410), prmt(t1, t3, 0x7632)};
+                            const uint32_t xhi[4] = {prmt(u0, u2, 0x5410), prmt(u0, u2, 0x7632), prmt(u1, u3, 0x5410), prmt(u1, u3, 0x7632)};
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                if constexpr (KIND == kLevels3) {        // a nibble below 8 is a selector as it stands
+                                    v[u][j].x = prmt(T[0], T[1], xlo[j]); v[u][j].y = prmt(T[0], T[1], mad_hi(xlo[j], 0x10000u, 0u));
+                                    v[u][j].z = prmt(T[0], T[1], xhi[j]); v[u][j].w = prmt(T[0], T[1], mad_hi(xhi[j], 0x10000u, 0u));
+                                } else {
+                                    expand8(xlo[j], T, v[u][j].x, v[u][j].y);
+                                    expand8(xhi[j], T, v[u][j].z, v[u][j].w);
+                                }
                             }
                         }
                     }
+                    fetch(w[a]);                              // refill this ring slot (slab f + kAhead)
+                    ok = mbar_wait(&sh->empty[st], ((f / kStages) & 1) ^ 1, p.cb.error);
+                    if (!ok) break;
+                    unsigned char *a_stage = stages + size_t(st) * kStageBytes;
+#pragma unroll
+                    for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int row = blk_in_item * 32 + (quad0 + 4 * u) * 4 + j;   // vector within the item
+                            const int r = row & (kMmaM - 1);
+                            // accumulator tile row>>7; 128-byte swizzle: 16-byte chunk c of row r sits at chunk position c ^ (r % 8)
+                            *reinterpret_cast<uint4 *>(a_stage + (row >> 7) * kATileBytes + (r >> 3) * 1024 + (r & 7) * 128 + ((octet ^ (r & 7)) << 4)) = v[u][j];
+                        }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh->full[st]);
                 }
-                fetch(w[a]);                              // refill this ring slot (slab f + kAhead)
-                ok = mbar_wait(&sh->empty[st], ((f / kStages) & 1) ^ 1, p.cb.error);
-                if (!ok) break;
-                unsigned char *a_stage = stages + size_t(st) * kStageBytes;
-#pragma unroll
-                for (int u = 0; u < kUnits; ++u)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int row = blk_in_item * 32 + (quad0 + 4 * u) * 4 + j;   // vector within the item
-                        const int r = row & (kMmaM - 1);
-                        // accumulator tile row>>7; 128-byte swizzle: 16-byte chunk c of row r sits at chunk position c ^ (r % 8)
-                        *reinterpret_cast<uint4 *>(a_stage + (row >> 7) * kATileBytes + (r >> 3) * 1024 + (r & 7) * 128 + ((octet ^ (r & 7)) << 4)) = v[u][j];
-                    }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh->full[st]);
             }
         }
     }

@@ -60,8 +60,19 @@ __device__ __forceinline__ void half_entries(const float *q, const float *centro
     }
 }
 
-// Coordinate (within a chunk of 16) whose level the expansion of 2-bit codes puts at byte b of word w (scan_tc.cu, kLevels2).
-__device__ __forceinline__ int levels2_coord(int w, int b) { return (w & 1) * 8 - (w >> 1) + 4 * (b >> 1) + ((b & 1) ? 1 : 3); }
+// Coordinate whose level the expansion of a filtering scan (scan_tc.cu, kLevels2 / kLevels3) puts at byte b of word i of a
+// row: 16-byte chunk c of a 128-byte slab holds the byte-groups c, c + 8, c + 16, ... of the slab.
+template <int BITS>
+__device__ __forceinline__ int filter_coord(int i, int b) {
+    const int slab = i >> 5, c = (i >> 2) & 7, w = i & 3;
+    if constexpr (BITS == 2) {                                      // words 0, 1: coordinates 3 and 1 of two groups; 2, 3: 2 and 0
+        const int group = c + 8 * ((w & 1) * 2 + (b >> 1));
+        return slab * 128 + 4 * group + (w < 2 ? ((b & 1) ? 1 : 3) : ((b & 1) ? 0 : 2));
+    } else {                                                        // two groups a word, coordinate 1 before coordinate 0
+        const int group = c + 8 * (2 * w + (b >> 1));
+        return slab * 128 + 2 * group + ((b & 1) ^ 1);
+    }
+}
 
 // The u8 tables of a query and, for a filtering scan (scan_filter.cu), its int8 weights and the affine bound
 //   isum <= alpha * sum_d W[d] * L[code[d]] + beta + D,   with the equality's two sides at most D apart,
@@ -155,8 +166,7 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *de
     for (int i = tid; i < p.dim_pad / 4; i += blockDim.x) {
         uint32_t word = 0;
         for (int b = 0; b < 4; ++b) {
-            // 3-bit codes lie in nibbles, low nibble = odd coordinate
-            const int d = BITS == 2 ? (i >> 2) * 16 + levels2_coord(i & 3, b) : 4 * i + (b ^ 1);
+            const int d = filter_coord<BITS == 2 ? 2 : 3>(i, b);
             if (d < p.dim) word |= uint32_t(uint8_t(round_clamp_i8(__fmul_rn(row[d], w_inv)))) << (8 * b);
         }
         wrow[i] = word;
