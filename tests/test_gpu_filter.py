@@ -58,3 +58,20 @@ def test_filtering_scan_overflows_and_recovers(T, bits):
     q = np.concatenate([-x[:1], x[:1], anisotropic(6, dim, seed=7)])
     check(idx, pre, q, 10)
     check(idx, pre, np.concatenate([q, np.zeros((1, dim), np.float32)]), 20)
+
+
+@pytest.mark.parametrize("bits,n", [(2, 33_001), (3, 17_003)])
+def test_filtering_scan_of_a_calibrated_index(T, bits, n):
+    """The TQ+ pair moves the queries' coordinates and their bias; the bound has to follow."""
+    dim = 512
+    x = anisotropic(n, dim, seed=51) * np.float32(3.0)
+    x[:, ::7] *= np.float32(2.5)
+    sh, sc = O.fit_calibration(x[:4000], bits)
+    idx = T.TurboQuantIndex(dim, bits)
+    idx.calibrate(x[:4000])
+    idx.add(x)
+    enc = O.encode(x, bits, sh, sc)
+    q = anisotropic(20, dim, seed=51, offset=n + 3)
+    want = O.search(q, O.packed_to_blocked(enc["packed"], bits, dim), enc["scales"], n, dim, bits, 10, shift=sh, scale=sc)
+    s, i = idx.search(q, 10)
+    assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
