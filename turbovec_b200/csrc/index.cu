@@ -1031,11 +1031,42 @@ int plan_scan(tv_index *h, int mode, size_t nq, bool allow_tc, ScanPlan &plan) {
     return TV_OK;
 }
 
-// Whether a batch goes through the filtering scan instead of the one-hot contraction.
-bool wants_filter(const tv_index *h, int mode, size_t nq, const ScanPlan &plan) {
+// Whether a batch goes through the filtering scan: when its expected time is well below that of the form it replaces.
+// The filter saves contraction (an eighth of the one-hot K) and pays for survivors, whose number depends on how far the
+// threshold of the vectors seen so far stands above the width of the bound.  With scores spread like a normal
+// distribution, the k-th best of m scores lies at z = Q^-1(k / m) standard deviations, and Q(z - delta) of a chunk survive;
+// delta, the bound's width, grows with the square root of the dimension (0.020 for 2-bit, 0.033 for 3-bit codes, plus
+// the spread of the vector scales).  Rates measured on 1.5 k - 1 M vectors of 200 - 3,072 dimensions (us): one-hot 5.3e-6
+// a byte-group per 256 queries, register lookups 1e-6 a byte-group per 4 queries, filter 0.7e-6 a byte-group per 256
+// queries, epilogue of either contraction 6e-7 a sum, survivors 3e-6 a byte-group, launches of the filter 120 against 60.
+// Both sides, filter / one-hot, us: 640 k x 200 2-bit, 8 queries 155 / 241, 512 queries 518 / 750; 160 k x 200, 64 queries
+// 142 / 146; 32 k x 1536, 64 queries 169 / 135; 100 k x 3072, 64 queries 518 / 512, 512 queries 5,887 / 1,167 (short lists of
+// many queries leave a loose threshold); 48 k x 768 3-bit, 512 queries 1,068 / 437; 1 M x 3072, 64 queries 1,160 / 3,750.
+bool wants_filter(const tv_index *h, int mode, size_t nq, size_t k, int cap, bool masked, const ScanPlan &plan) {
     if (!scan_filter_supported(h->bits, mode, h->ngroups, h->smem_limit) || h->mma_min_batch == 0) return false;
-    const bool batch = plan.use_tc || (h->mma_min_batch < 0 && nq >= 8);    // flush geometries beyond 256 groups have no one-hot form
-    return batch && h->n * size_t(h->ngroups) >= (size_t(4) << 20);
+    // flush geometries beyond 256 groups have no one-hot form; a batch size set by the caller decides alone
+    const bool by_caller = h->mma_min_batch > 0;
+    if (!plan.use_tc && int64_t(nq) < (by_caller ? h->mma_min_batch : 8)) return false;
+    if (by_caller) return true;
+    const double n = double(h->n), bytes = n * h->ngroups, groups = std::ceil(double(nq) / 256.0);
+    const double delta = (h->bits == 2 ? 0.020 : 0.033) * std::sqrt(double(h->dim)) + 0.2;
+    auto upper_tail = [](double x) { return 0.5 * std::erfc(x * 0.70710678118654752); };
+    auto quantile = [](double p) {                             // Abramowitz and Stegun 26.2.23
+        const double t = std::sqrt(-2.0 * std::log(std::min(p, 0.5)));
+        return t - (2.515517 + 0.802853 * t + 0.010328 * t * t) / (1.0 + 1.432788 * t + 0.189269 * t * t + 0.001308 * t * t * t);
+    };
+    // the chunks of enqueue_filtered; under a mask an unknown share of the vectors counts, taken as an eighth
+    double survivors = 0.0;
+    for (double begin = 0.0, seen = std::min(double(cap), n); begin < n;) {
+        const double end = std::max(begin, seen) * 5.9 >= n ? n : std::max(begin, seen) * 4.0;   // (a short tail joins the chunk before)
+        survivors += (end - begin) * upper_tail(quantile(double(k) / (std::max(begin, seen) * (masked ? 0.125 : 1.0))) - delta);
+        begin = end;
+    }
+    const double sums = n * double(nq) * 6e-7;
+    const double filter = 120.0 + bytes * 0.7e-6 * groups * (1.0 + std::min(1.0, double(cap) / n)) + sums +
+                          survivors * double(nq) * h->ngroups * 3e-6;
+    const double other = 60.0 + (plan.use_tc ? bytes * 5.3e-6 * groups + sums : bytes * 1e-6 * std::ceil(double(nq) / 4.0));
+    return other > 1.3 * filter;
 }
 
 // Brings the int8 copy of the index (scan_tc_dense.cu) up to date on `st`: allocates it when policy and free memory
@@ -1328,7 +1359,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     int rc = plan_scan(h, mode, nq, pages == 1, plan);
     if (rc != TV_OK) return rc;
 
-    plan.use_filter = pages == 1 && kk <= size_t(kSelectMaxK) && !h->force_careful && wants_filter(h, mode, nq, plan);
+    plan.use_filter = pages == 1 && kk <= size_t(kSelectMaxK) && !h->force_careful && wants_filter(h, mode, nq, kk, cap, mask.any(), plan);
 
     // ---- buffers ----
     TV_CUDA(injected_failure(h));
