@@ -1,0 +1,46 @@
+"""Several handles in one process: what they share (kernel attributes, the pool of workspaces) does not let one disturb another."""
+import threading
+
+import numpy as np
+import pytest
+
+from tests.util import anisotropic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def T():
+    import turbovec_b200
+    return turbovec_b200
+
+
+def test_handles_of_different_sizes_searched_from_two_threads(T):
+    """The tables of the two handles need 2 KB and 96 KB of shared memory in the same kernels: neither's limit is the other's.
+    A launch above a limit is refused by the runtime before anything runs."""
+    shapes = [(64, 2, 4), (3072, 2, 4), (64, 3, 1), (3072, 3, 1)]
+    work = []
+    for dim, bits, nq in shapes:
+        idx = T.TurboQuantIndex(dim, bits)
+        idx.add(anisotropic(700, dim, seed=5))
+        q = anisotropic(nq, dim, seed=5, offset=9)
+        work.append((idx, q, idx.search(q, 5)))
+    errors = []
+    start = threading.Barrier(len(work))
+
+    def search(idx, q, want):
+        start.wait()
+        for _ in range(800):
+            try:
+                s, i = idx.search(q, 5)
+                assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+            except Exception as e:  # noqa: BLE001
+                errors.append(repr(e))
+                return
+
+    threads = [threading.Thread(target=search, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors

@@ -188,3 +188,21 @@ def test_sync_planner_matches_a_restatement():
     many = set(range(0, 4000, 3))
     assert len(many) > 1024 and plan(4096, 4096, set(), many) == 93
     assert plan(4096, 4096, set(), set(list(many)[:1024]))[1] == sorted(list(many)[:1024])
+
+
+def test_shared_memory_limits_of_kernels_do_not_depend_on_the_call():
+    """The dynamic shared memory limit is state of a kernel on a device, shared by all handles of the process: a launcher that
+    sets it to its own call's size can lower it between another thread's call and its launch, which the runtime then refuses
+    ("invalid argument").  Sizes that follow the geometry go through allow_dynamic_shared, which sets one value per kernel."""
+    csrc = os.path.join(ROOT, "turbovec_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        lines = open(os.path.join(csrc, name)).read().splitlines()
+        size = ""
+        for at, line in enumerate(lines):
+            if re.search(r"size_t smem = ", line):
+                size = line.split("size_t smem = ")[1]
+            if "cudaFuncAttributeMaxDynamicSharedMemorySize" not in line:
+                continue
+            value = (line + (lines[at + 1] if at + 1 < len(lines) else "")).split("cudaFuncAttributeMaxDynamicSharedMemorySize,")[1]
+            if "int(smem)" in value:
+                assert not re.search(r"\bp\.|ngroups|\bdim\b|\bng\b", size), f"{name}:{at + 1}: limit set to {size}"

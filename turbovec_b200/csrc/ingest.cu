@@ -304,8 +304,7 @@ cudaError_t launch_ingest(const IngestParams &p, int V, cudaStream_t stream) {
     const int variant = rotation_variant(p.dim);
 #define TV_LAUNCH_INGEST(L)                                                                               \
     case L: {                                                                                             \
-        cudaError_t e = cudaFuncSetAttribute(ingest_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                             int(smem));                                                  \
+        cudaError_t e = allow_dynamic_shared(ingest_kernel<L>);                                           \
         if (e != cudaSuccess) return e;                                                                   \
         ingest_kernel<L><<<grid, V * 32, smem, stream>>>(p);                                              \
         break;                                                                                            \

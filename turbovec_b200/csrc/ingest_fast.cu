@@ -757,7 +757,7 @@ cudaError_t launch_ingest_fast(const IngestParams &p, const QuantGrid &grid, int
     const unsigned nctas = unsigned(std::min<int64_t>(nblocks, int64_t(sm_count)));   // one CTA per SM: it owns the register file
 #define TV_LAUNCH_FAST_VC(L2B, NB, VV, CC)                                                                           \
     {                                                                                                                \
-        cudaError_t e = cudaFuncSetAttribute(ingest_fast_kernel<L2B, NB, VV, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
+        cudaError_t e = allow_dynamic_shared(ingest_fast_kernel<L2B, NB, VV, CC>);                                   \
         if (e != cudaSuccess) return e;                                                                              \
         ingest_fast_kernel<L2B, NB, VV, CC><<<nctas, (VV + 4) * 32, smem, stream>>>(p, grid, error);                 \
     }

@@ -198,7 +198,7 @@ bool scan_filter_supported(int bits, int mode, int ngroups, size_t smem_limit) {
 
 cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cudaStream_t s) {
     const size_t smem = size_t(p.ngroups) * 36;
-    cudaError_t e = cudaFuncSetAttribute(score_survivors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_dynamic_shared(score_survivors_kernel);
     if (e != cudaSuccess) return e;
     for (int q0 = 0; q0 < nq; q0 += 32768) {
         const int here = std::min(nq - q0, 32768);
@@ -215,7 +215,7 @@ cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cu
 
 cudaError_t launch_bootstrap(const ScanParams &p, int nq, cudaStream_t s) {
     const size_t smem = size_t(p.ngroups) * 32;
-    cudaError_t e = cudaFuncSetAttribute(bootstrap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_dynamic_shared(bootstrap_kernel, 1024);
     if (e != cudaSuccess) return e;
     bootstrap_kernel<<<nq, kScoreThreads, smem, s>>>(p);
     return cudaGetLastError();

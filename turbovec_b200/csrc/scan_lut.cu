@@ -170,8 +170,7 @@ template <int NQ, int NB>
 static cudaError_t launch_lut(const ScanParams &p, int sm_count, cudaStream_t s) {
     const size_t smem = size_t(NQ) * p.ngroups * 32;
     auto kern = scan_lut_kernel<NQ, NB>;
-    // the attribute belongs to the current device: set on every launch (a host-side table write)
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_dynamic_shared(kern);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLutThreads, smem);

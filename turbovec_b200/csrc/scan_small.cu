@@ -258,7 +258,7 @@ cudaError_t launch_variant(const ScanParams &p, const int8_t *weights, int pitch
                            cudaStream_t s) {
     const size_t smem = small_smem_bytes(NT, STAGES, p.ngroups);
     auto kern = scan_small_kernel<NT, STAGES, SWZ, CTAS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_dynamic_shared(kern, 1024);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = p.pos_end - p.pos_begin;
     const unsigned grid = unsigned(min(uint32_t(sm_count) * CTAS, (blocks + kSmallWarps - 1) / kSmallWarps));

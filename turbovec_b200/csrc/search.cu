@@ -756,8 +756,7 @@ cudaError_t launch_query_prep(const QueryPrepParams &p, cudaStream_t stream) {
     const size_t smem = query_prep_smem_bytes(p.dim);
 #define TV_LAUNCH_QP(L)                                                                                        \
     case L: {                                                                                                  \
-        cudaError_t e = cudaFuncSetAttribute(query_prep_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                             int(smem));                                                       \
+        cudaError_t e = allow_dynamic_shared(query_prep_kernel<L>, 2048);                                      \
         if (e != cudaSuccess) return e;                                                                        \
         query_prep_kernel<L><<<p.rows, kPrepThreads, smem, stream>>>(p);                                                \
         break;                                                                                                 \

@@ -38,4 +38,13 @@ __host__ __device__ inline uint64_t make_key(float score, uint32_t slot) {
 }
 constexpr uint64_t kEmptyKey = 0xffffffffffffffffull;   // sorts after every real key; "no result yet"
 
+// Lets `kern` be launched with any dynamic shared memory that a block of sm_100 can have next to `static_bytes` of its own.
+// The limit is state of the kernel on the device, which every thread of the process shares: two handles whose launches
+// want different sizes must set it to the same value, or one lowers it between the other's call and its launch.
+constexpr int kBlockSharedBytes = 227 * 1024;
+template <typename Kernel>
+cudaError_t allow_dynamic_shared(Kernel *kern, int static_bytes = 0) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBlockSharedBytes - static_bytes);
+}
+
 }  // namespace tv
