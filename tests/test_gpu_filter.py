@@ -77,3 +77,18 @@ def test_filtering_scan_of_a_calibrated_index(T, bits, n):
     want = O.search(q, O.packed_to_blocked(enc["packed"], bits, dim), enc["scales"], n, dim, bits, 10, shift=sh, scale=sc)
     s, i = idx.search(q, 10)
     assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+
+
+def test_filtering_scan_of_rows_with_unused_bits_set(T):
+    """set_row takes any bytes; bit 3 of a 3-bit nibble does not count in the exact score and must not in the filter."""
+    n, dim = 20_011, 256
+    x = anisotropic(n, dim, seed=61)
+    idx, pre = built(T, x, 3)
+    q = anisotropic(12, dim, seed=61, offset=4)
+    want = O.search(q, pre[0], pre[1], n, dim, 3, 10)
+    for slot in np.unique(np.concatenate([want[1].ravel(), np.arange(5, n, 997)])):
+        groups, scale = idx.get_row(int(slot))
+        idx.set_row(int(slot), groups | np.random.default_rng(slot).choice(np.array([0x08, 0x80, 0x88], np.uint8), groups.size), scale)
+    for batch in (q, q[:1]):
+        s, i = idx.search(batch, 10)
+        assert np.array_equal(i, want[1][:len(batch)]) and np.array_equal(s, want[0][:len(batch)])

@@ -79,7 +79,7 @@ __device__ __forceinline__ void exact_keys(const ScanParams &p, const uint8_t *l
                     s[j] += int(lut[g * 32 + (b >> 4)]) + int(lut[g * 32 + 16 + (b & 15u)]);
                     if constexpr (EXIT) {
                         // selectors of the byte's levels, in the order of wq
-                        const uint32_t sel = p.bits == 2 ? (b & 0x33u) | ((b >> 2) & 0x33u) << 8 : b;
+                        const uint32_t sel = p.bits == 2 ? (b & 0x33u) | ((b >> 2) & 0x33u) << 8 : b & 0x77u;
                         w[j] = __dp4a(int(__byte_perm(p.level_words[0], p.level_words[1], sel)), int(wg), w[j]);
                     }
                 }

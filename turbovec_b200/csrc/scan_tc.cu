@@ -391,9 +391,12 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                             const uint32_t xhi[4] = {prmt(u0, u2, 0x5410), prmt(u0, u2, 0x7632), prmt(u1, u3, 0x5410), prmt(u1, u3, 0x7632)};
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
-                                if constexpr (KIND == kLevels3) {        // a nibble below 8 is a selector as it stands
-                                    v[u][j].x = prmt(T[0], T[1], xlo[j]); v[u][j].y = prmt(T[0], T[1], mad_hi(xlo[j], 0x10000u, 0u));
-                                    v[u][j].z = prmt(T[0], T[1], xhi[j]); v[u][j].w = prmt(T[0], T[1], mad_hi(xhi[j], 0x10000u, 0u));
+                                if constexpr (KIND == kLevels3) {
+                                    // a nibble below 8 is a selector as it stands; a row set from outside may have bit 3 of
+                                    // a nibble on, which the tables of the exact score ignore
+                                    const uint32_t lo = xlo[j] & 0x77777777u, hi = xhi[j] & 0x77777777u;
+                                    v[u][j].x = prmt(T[0], T[1], lo); v[u][j].y = prmt(T[0], T[1], mad_hi(lo, 0x10000u, 0u));
+                                    v[u][j].z = prmt(T[0], T[1], hi); v[u][j].w = prmt(T[0], T[1], mad_hi(hi, 0x10000u, 0u));
                                 } else {
                                     expand8(xlo[j], T, v[u][j].x, v[u][j].y);
                                     expand8(xhi[j], T, v[u][j].z, v[u][j].w);
