@@ -92,3 +92,22 @@ def test_filtering_scan_of_rows_with_unused_bits_set(T):
     for batch in (q, q[:1]):
         s, i = idx.search(batch, 10)
         assert np.array_equal(i, want[1][:len(batch)]) and np.array_equal(s, want[0][:len(batch)])
+
+
+@pytest.mark.parametrize("n,k", [(20_011, 10), (300, 300)])
+def test_filtering_scan_of_scores_that_overflow(T, n, k):
+    """Scales and queries are bounded each on its own; their product can be infinite, of either sign, for the k-th result too."""
+    dim = 64
+    x = anisotropic(n, dim, seed=71)
+    idx, pre = built(T, x, 2)
+    scales = pre[1].copy()
+    for slot in range(0, n, max(1, n // 300)):
+        groups, _ = idx.get_row(slot)
+        scales[slot] = 3e38
+        idx.set_row(slot, groups, 3e38)
+    q = anisotropic(9, dim, seed=71, offset=4) * np.float32(1000.0)
+    with np.errstate(over="ignore"):
+        want = O.search(q, pre[0], scales, n, dim, 2, k)
+    assert np.isinf(want[0]).any()
+    s, i = idx.search(q, k)
+    assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])

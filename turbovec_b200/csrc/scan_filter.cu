@@ -20,6 +20,7 @@
 // what W . L has left, plus the largest deviations of the remaining half-bytes (suffix sums from query preparation).  The
 // sum of deviations is what let most survivors through, and it shrinks with every batch.
 #include <algorithm>
+#include <cfloat>
 
 #include "scan_tc_common.cuh"
 
@@ -161,7 +162,8 @@ __global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanP
 }
 
 // topk[q] = the k best of the first chunk by approximate score -> thr[q] just above the worst of their exact keys; the
-// running top-k is empty again.  Fewer than k entries: no threshold.
+// running top-k is empty again.  Fewer than k entries, or a k-th score that overflowed: no threshold (the filtering scans
+// take an infinite one for a column without a query, and these k vectors have yet to be found).
 __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t worst[kScoreWarps];
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) 
     for (int i = threadIdx.x; i < k; i += kScoreThreads) top[i] = kEmptyKey;
     if (threadIdx.x == 0) {
         for (int w = 0; w < kScoreWarps; ++w) mine = max(mine, worst[w]);
-        p.cb.thr[q] = full ? mine + 1 : kEmptyKey;
+        p.cb.thr[q] = full && fabsf(desc_bits_to_score(uint32_t(mine >> 32))) <= FLT_MAX ? mine + 1 : kEmptyKey;
     }
 }
 

@@ -400,7 +400,7 @@ __device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *
             bool on = mine != 0;
             uint64_t key;
             if constexpr (RAW) {
-                on = on && score + 1.0e-5f * (fabsf(score) + fabsf(t)) >= t;
+                on = on && !(score + 1.0e-5f * (fabsf(score) + fabsf(t)) < t);   // (an infinite score compares with nothing: kept)
                 key = uint64_t(sum) << 32 | slot;
             } else {
                 on = on && score >= t;
