@@ -99,8 +99,8 @@ enum {
     TV_OPT_SCORE_MODE = 1,      /* one of TV_SCORE_* */
     TV_OPT_MMA_MIN_BATCH = 2,   /* query batches of at least this size use the tensor-memory scan; 0 = never;
                                  * -1 (default) = measured switch points: permute-dot 17 with the int8 copy of the index
-                                 * (TV_OPT_TC_EXPANDED) and 33 without it, u8-LUT families 8, and for 2- and 3-bit codes the
-                                 * int8 filter in front of the exact scores where it is expected to pay (set: always) */
+                                 * (TV_OPT_TC_EXPANDED) and 33 without it, u8-LUT families 8 (as a one-hot contraction, unless
+                                 * TV_OPT_FILTER takes the batch) */
     TV_OPT_FORCE_CAREFUL = 3,   /* 1: run the candidate-overflow recovery schedule always (testing) */
     TV_OPT_TC_TILES = 4,        /* accumulator tiles of 128 vectors per query slab in the tensor-memory scan: 1 or 2 */
     TV_OPT_INGEST_PIPELINE = 5, /* 1 (default): whole code blocks are encoded by the pipelined ingest kernel; 0: never;
@@ -121,8 +121,14 @@ enum {
                                  * copy); 2: always, a search fails when it does not fit.  The copy is built and kept current
                                  * lazily by the searches that use it.  Identical results. */
     TV_OPT_EXPANDED_BYTES = 12, /* read-only: bytes the int8 copy holds right now (0 = none) */
-    TV_OPT_DENSE_PAIR = 13      /* 1 (default): the scan over the int8 copy runs on CTA pairs (tcgen05 cta_group::2: half the
+    TV_OPT_DENSE_PAIR = 13,     /* 1 (default): the scan over the int8 copy runs on CTA pairs (tcgen05 cta_group::2: half the
                                  * query bytes per SM); 0: one CTA per work item.  Identical results. */
+    TV_OPT_FILTER = 14,         /* 2- and 3-bit codes, k <= 512: an int8 contraction that bounds the scores from above in front of
+                                 * the exact scores.  1 (default): batches for which it is expected to pay, as long as
+                                 * TV_OPT_MMA_MIN_BATCH is -1; 0: never; 2: always (not with TV_OPT_MMA_MIN_BATCH = 0).
+                                 * Identical results. */
+    TV_OPT_FILTER_REDONE = 15   /* read-only: queries of the last search that the filter left with too many survivors and that
+                                 * were searched again without it; -1: that search did not use the filter */
 };
 
 /* ---- construction: TurboQuantIndex::new / new_lazy (lib.rs:629, 670), IdMapIndex::new (id_map.rs:278) ---- */

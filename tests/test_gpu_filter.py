@@ -5,6 +5,7 @@ import pytest
 
 from oracle import oracle as O
 from tests.util import anisotropic
+from turbovec_b200 import OPT_FILTER_REDONE
 
 pytestmark = pytest.mark.gpu
 
@@ -19,16 +20,17 @@ def built(T, x, bits):
     enc = O.encode(x, bits)
     idx = T.TurboQuantIndex(x.shape[1], bits)
     idx.add(x)
-    idx.set_option(T.OPT_MMA_MIN_BATCH, 1)                  # the filter whatever its expected time
+    idx.set_option(T.OPT_FILTER, 2)                         # whatever its expected time
     return idx, (O.packed_to_blocked(enc["packed"], bits, x.shape[1]), enc["scales"])
 
 
-def check(idx, pre, q, k, mask=None):
+def check(idx, pre, q, k, mask=None, redone=0):
     n, bits = len(idx), idx.bit_width
     words = None if mask is None else O.pack_mask(mask)
     want = O.search(q, pre[0], pre[1], n, q.shape[1], bits, k, mask_words=words)
     s, i = idx.search(q, k, mask=mask)
     assert np.array_equal(s, want[0]) and np.array_equal(i, want[1]), (n, q.shape, bits, k)
+    assert idx.get_option(OPT_FILTER_REDONE) == redone, "the filter did not take this batch, or not to its end"
 
 
 # dim 2072 at 2 bits has 518 byte-groups, not a multiple of four
@@ -57,8 +59,8 @@ def test_filtering_scan_overflows_and_recovers(T, bits):
     x[3::1117] = anisotropic(len(x[3::1117]), dim, seed=6)
     idx, pre = built(T, x, bits)
     q = np.concatenate([-x[:1], x[:1], anisotropic(6, dim, seed=7)])
-    check(idx, pre, q, 10)
-    check(idx, pre, np.concatenate([q, np.zeros((1, dim), np.float32)]), 20)
+    check(idx, pre, q, 10, redone=len(q))
+    check(idx, pre, np.concatenate([q, np.zeros((1, dim), np.float32)]), 20, redone=len(q) + 1)
 
 
 @pytest.mark.parametrize("bits,n", [(2, 33_001), (3, 17_003)])
@@ -71,12 +73,13 @@ def test_filtering_scan_of_a_calibrated_index(T, bits, n):
     idx = T.TurboQuantIndex(dim, bits)
     idx.calibrate(x[:4000])
     idx.add(x)
-    idx.set_option(T.OPT_MMA_MIN_BATCH, 1)
+    idx.set_option(T.OPT_FILTER, 2)
     enc = O.encode(x, bits, sh, sc)
     q = anisotropic(20, dim, seed=51, offset=n + 3)
     want = O.search(q, O.packed_to_blocked(enc["packed"], bits, dim), enc["scales"], n, dim, bits, 10, shift=sh, scale=sc)
     s, i = idx.search(q, 10)
     assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+    assert idx.get_option(T.OPT_FILTER_REDONE) == 0
 
 
 def test_filtering_scan_of_rows_with_unused_bits_set(T):
@@ -111,3 +114,23 @@ def test_filtering_scan_of_scores_that_overflow(T, n, k):
     assert np.isinf(want[0]).any()
     s, i = idx.search(q, k)
     assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+
+
+@pytest.mark.parametrize("dim,bits,n,nq", [(1536, 2, 3000, 9), (1024, 3, 1500, 70), (64, 2, 40_000, 513), (3072, 2, 1500, 300)])
+def test_one_hot_form_of_wide_batches_is_still_reached(T, dim, bits, n, nq):
+    """A batch size that the caller sets selects the one-hot contraction, above 256 queries two query groups to a work item."""
+    x = anisotropic(n, dim, seed=43)
+    idx, pre = built(T, x, bits)
+    idx.set_option(T.OPT_SCORE_MODE, T.SCORE_LUT_MULADD)
+    idx.set_option(T.OPT_FILTER, 1)
+    idx.set_option(T.OPT_MMA_MIN_BATCH, 1)
+    q = anisotropic(nq, dim, seed=43, offset=7)
+    want = O.search(q, pre[0], pre[1], n, dim, bits, 10, mode=O.MODE_LUT_MULADD)
+    s, i = idx.search(q, 10)
+    assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+    assert idx.get_option(T.OPT_FILTER_REDONE) == -1
+    idx.set_option(T.OPT_MMA_MIN_BATCH, -1)
+    idx.set_option(T.OPT_FILTER, 0)
+    s, i = idx.search(q, 10)
+    assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+    assert idx.get_option(T.OPT_FILTER_REDONE) == -1

@@ -396,6 +396,8 @@ struct tv_index {
                                  // (5 = four-stage rings, two CTAs per SM, swizzled tensor copies: the fastest measured)
     int tc_wide = 1;             // 1: batches above 256 queries share every expanded code slab between two query groups
     int tc_expanded = 1;         // 1: large permute-dot batches scan an int8 copy of the index when device memory has room for it; 0 never; 2 always (fail if it does not fit)
+    int filter = 1;              // filtering scan of 2- and 3-bit codes: 1 where it is expected to pay, 0 never, 2 always
+    int64_t filter_redone = -1;  // under stat_mu: queries that the last search did again without the filter, -1: it had none
     int dense_pair = 1;          // 1: the scan over the int8 copy runs on CTA pairs (cta_group::2)
     int fail_next = 0;           // test hook (TV_OPT_FAIL_NEXT): the next device allocation / upload of a call reports failure
 
@@ -1043,11 +1045,10 @@ int plan_scan(tv_index *h, int mode, size_t nq, bool allow_tc, ScanPlan &plan) {
 // 142 / 146; 32 k x 1536, 64 queries 169 / 135; 100 k x 3072, 64 queries 518 / 512, 512 queries 5,887 / 1,167 (short lists of
 // many queries leave a loose threshold); 48 k x 768 3-bit, 512 queries 1,068 / 437; 1 M x 3072, 64 queries 1,160 / 3,750.
 bool wants_filter(const tv_index *h, int mode, size_t nq, size_t k, int cap, bool masked, const ScanPlan &plan) {
-    if (!scan_filter_supported(h->bits, mode, h->ngroups, h->smem_limit) || h->mma_min_batch == 0) return false;
-    // flush geometries beyond 256 groups have no one-hot form; a batch size set by the caller decides alone
-    const bool by_caller = h->mma_min_batch > 0;
-    if (!plan.use_tc && int64_t(nq) < (by_caller ? h->mma_min_batch : 8)) return false;
-    if (by_caller) return true;
+    if (!scan_filter_supported(h->bits, mode, h->ngroups, h->smem_limit) || h->filter == 0 || h->mma_min_batch == 0) return false;
+    if (h->filter == 2) return true;
+    if (h->mma_min_batch > 0) return false;                    // the caller asked for the one-hot form
+    if (!plan.use_tc && nq < 8) return false;                  // (flush geometries beyond 256 groups have no one-hot form)
     const double n = double(h->n), bytes = n * h->ngroups, groups = std::ceil(double(nq) / 256.0);
     const double delta = (h->bits == 2 ? 0.020 : 0.033) * std::sqrt(double(h->dim)) + 0.2;
     auto upper_tail = [](double x) { return 0.5 * std::erfc(x * 0.70710678118654752); };
@@ -1360,6 +1361,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     if (rc != TV_OK) return rc;
 
     plan.use_filter = pages == 1 && kk <= size_t(kSelectMaxK) && !h->force_careful && wants_filter(h, mode, nq, kk, cap, mask.any(), plan);
+    int64_t redone = plan.use_filter ? 0 : -1;               // TV_OPT_FILTER_REDONE
 
     // ---- buffers ----
     TV_CUDA(injected_failure(h));
@@ -1471,6 +1473,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         c.marks.collect();
         std::lock_guard<std::mutex> g(h->stat_mu);
         h->last_ms = ms; h->last_main_ms = c.marks.total_ms; h->last_main_launches = c.marks.launches;
+        h->filter_redone = redone;
         return TV_OK;
     };
     for (size_t page = 0; page < pages; ++page) {
@@ -1498,6 +1501,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
             if (careful) return fail(h, TV_ERR_CUDA, "candidate overflow in the bounded schedule (internal error)");
             // a chunk produced more candidates than the buffer holds: redo this page without the filter, then with bounded chunks
             if (!plan.use_filter) attempt = 1;
+            else redone = int64_t(nq);
             plan.use_filter = false;
             c.h_flags->overflow = 0;
             TV_CUDA(cudaMemcpyAsync(&c.d_flags->overflow, &c.h_flags->overflow, 4, cudaMemcpyHostToDevice, st));
@@ -1736,6 +1740,7 @@ int tv_set_option(tv_index *h, int option, int64_t value) {
         case TV_OPT_FAIL_NEXT: h->fail_next = value < 0 ? 0 : int(value); return TV_OK;
         case TV_OPT_TC_WIDE: h->tc_wide = value != 0; return TV_OK;
         case TV_OPT_DENSE_PAIR: h->dense_pair = value != 0; return TV_OK;
+        case TV_OPT_FILTER: h->filter = value < 0 || value > 2 ? 1 : int(value); return TV_OK;
         case TV_OPT_TC_EXPANDED:
             h->tc_expanded = value < 0 || value > 2 ? 1 : int(value);
             if (h->tc_expanded == 0) { std::lock_guard<std::mutex> g(h->expanded.mu); h->expanded.drop(); }
@@ -1758,6 +1763,8 @@ int64_t tv_get_option(const tv_index *h, int option) {
         case TV_OPT_TC_WIDE: return h->tc_wide;
         case TV_OPT_TC_EXPANDED: return h->tc_expanded;
         case TV_OPT_DENSE_PAIR: return h->dense_pair;
+        case TV_OPT_FILTER: return h->filter;
+        case TV_OPT_FILTER_REDONE: { std::lock_guard<std::mutex> g(const_cast<tv_index *>(h)->stat_mu); return h->filter_redone; }
         case TV_OPT_EXPANDED_BYTES: return h->expanded.levels.ptr ? int64_t(h->expanded.rows_cap * size_t(h->expanded.pitch)) : 0;
         default: return -1;
     }
