@@ -30,7 +30,8 @@ def check(idx, pre, q, k, mask=None, redone=0):
     want = O.search(q, pre[0], pre[1], n, q.shape[1], bits, k, mask_words=words)
     s, i = idx.search(q, k, mask=mask)
     assert np.array_equal(s, want[0]) and np.array_equal(i, want[1]), (n, q.shape, bits, k)
-    assert idx.get_option(OPT_FILTER_REDONE) == redone, "the filter did not take this batch, or not to its end"
+    if redone is not None:
+        assert idx.get_option(OPT_FILTER_REDONE) == redone, "the filter did not take this batch, or not to its end"
 
 
 # dim 2072 at 2 bits has 518 byte-groups, not a multiple of four
@@ -59,8 +60,52 @@ def test_filtering_scan_overflows_and_recovers(T, bits):
     x[3::1117] = anisotropic(len(x[3::1117]), dim, seed=6)
     idx, pre = built(T, x, bits)
     q = np.concatenate([-x[:1], x[:1], anisotropic(6, dim, seed=7)])
-    check(idx, pre, q, 10, redone=len(q))
-    check(idx, pre, np.concatenate([q, np.zeros((1, dim), np.float32)]), 20, redone=len(q) + 1)
+    for batch, k in ((q, 10), (np.concatenate([q, np.zeros((1, dim), np.float32)]), 20)):
+        check(idx, pre, batch, k, redone=None)
+        assert idx.get_option(OPT_FILTER_REDONE) > 0
+
+
+@pytest.mark.parametrize("bits", [2, 3])
+def test_queries_that_the_filter_cannot_finish_are_redone_alone(T, bits):
+    """Half of the rows are copies of one row: more ties at the k-th place than a list holds for the queries near it, none that
+    matter for the others.  A zero query ties with every row, and the slots alone decide."""
+    n, dim = 300_000, 64
+    x = anisotropic(n, dim, seed=81)
+    x[::2] = x[0]
+    idx, pre = built(T, x, bits)
+    q = anisotropic(16, dim, seed=81, offset=5)
+    q[3] = 0.0
+    check(idx, pre, q, 10)
+    q[[0, 9]] = x[0]
+    q[9] *= np.float32(3.0)
+    mask = np.random.default_rng(1).random(n) < 0.97
+    for m in (None, mask):
+        check(idx, pre, q, 10, m, redone=2)
+    q[:12] = x[0]                                                   # most of the batch: all of it
+    check(idx, pre, q, 10, redone=16)
+
+
+def test_redone_queries_reach_every_kind_of_output(T):
+    import torch
+    n, dim, k = 300_000, 64, 10
+    x = anisotropic(n, dim, seed=82)
+    x[::2] = x[0]
+    idx, pre = built(T, x, 2)
+    q = anisotropic(16, dim, seed=82, offset=5)
+    q[[2, 7]] = x[0]
+    want = O.search(q, pre[0], pre[1], n, dim, 2, k)
+    dq = torch.from_numpy(q).cuda()
+    s = torch.empty((16, k), device="cuda")
+    i = torch.empty((16, k), dtype=torch.int64, device="cuda")
+    assert idx.search_device(dq.data_ptr(), 16, k, s.data_ptr(), i.data_ptr()) == k
+    assert idx.get_option(OPT_FILTER_REDONE) == 2
+    assert np.array_equal(s.cpu().numpy(), want[0]) and np.array_equal(i.cpu().numpy(), want[1])
+    keys = torch.empty((16, k), dtype=torch.int64, device="cuda")
+    idx.search_device_keys(dq.data_ptr(), 16, k, keys.data_ptr(), 1000)
+    assert idx.get_option(OPT_FILTER_REDONE) == 2
+    assert np.array_equal((keys.cpu().numpy() & 0xffffffff) - 1000, want[1])
+    idx.search(q[:1], k)                                            # a search after one that was redone
+    check(idx, pre, q[3:7], k)
 
 
 @pytest.mark.parametrize("bits,n", [(2, 33_001), (3, 17_003)])

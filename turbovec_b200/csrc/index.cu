@@ -145,13 +145,16 @@ struct SearchCtx {
     DeviceArray<uint32_t> d_cnt;
     DeviceArray<float> d_scores;
     DeviceArray<int64_t> d_slots;
+    DeviceArray<float> d_redo_queries;       // queries that a filtering scan could not finish, and their rows of results
+    DeviceArray<uint32_t> d_redo_who;
+    DeviceArray<uint64_t> d_redo_topk;
     DeviceArray<uint64_t> d_keys_tmp;        // staging of tv_search_device_keys when the shard holds fewer than k vectors
     PinnedArray<float> h_scores;
     PinnedArray<int64_t> h_slots;
     PinnedArray<float> h_queries;            // a small batch: query preparation reads it from here
     template <typename F>
     void each_array(F f) {
-        f(d_stage); f(d_qrot); f(d_qscale); f(d_qbias); f(d_filter); f(d_luts); f(d_weights); f(d_wfrag); f(d_mask); f(d_mask_bool); f(d_slots_in); f(d_live); f(d_allow_ids); f(d_cand); f(d_thr); f(d_topk); f(d_floor); f(d_keys_all); f(d_cnt); f(d_scores); f(d_slots); f(d_keys_tmp);
+        f(d_stage); f(d_qrot); f(d_qscale); f(d_qbias); f(d_filter); f(d_luts); f(d_weights); f(d_wfrag); f(d_mask); f(d_mask_bool); f(d_slots_in); f(d_live); f(d_allow_ids); f(d_cand); f(d_thr); f(d_topk); f(d_floor); f(d_keys_all); f(d_cnt); f(d_scores); f(d_slots); f(d_redo_queries); f(d_redo_who); f(d_redo_topk); f(d_keys_tmp);
     }
     template <typename F>
     void each_pinned(F f) { f(h_scores); f(h_slots); f(h_queries); }
@@ -884,6 +887,7 @@ struct SearchScratch {
     uint8_t *luts;
     uint64_t *cand, *thr, *topk, *lo;      // lo: lowest admissible key per query (paged top-k), or nullptr
     uint32_t *cnt, *done;                  // done (nq + 1 counters) follows cnt: both are cleared together
+    uint32_t *over;                        // filtering scans: marks of the queries whose lists overflowed; else nullptr
     size_t w_rows, dim_pad, lut_pitch;
     float *f_scale, *f_mid, *f_max, *f_alpha, *f_suffix;   // affine bound of a filtering scan
     int cap;
@@ -1131,6 +1135,8 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
     const size_t n_blocks = (h->n + kBlock - 1) / kBlock;
     const float *qscale = S.qscale, *qbias = S.qbias;
     sp.f_weights = S.weights; sp.f_pitch = int(S.dim_pad); sp.f_alpha = S.f_alpha; sp.f_suffix = S.f_suffix;
+    sp.cb.over = S.over;
+    sp.give_up = uint32_t(nq / 2);                             // beyond that search_core starts the whole batch again
     auto scan = [&](size_t begin, size_t end, const float *bias, bool dense) -> int {
         sp.pos_begin = uint32_t(begin); sp.pos_end = uint32_t(end); sp.dense = dense ? 1 : 0;
         sp.qscale = S.f_scale; sp.qbias = bias; sp.q_base = 0; sp.nq = int(nq);
@@ -1289,7 +1295,7 @@ int enqueue_query_prep(tv_index *h, cudaStream_t st, const SearchScratch &S, con
     qp.luts = S.luts; qp.lut_pitch = int(S.lut_pitch); qp.weights = S.weights; qp.dim_pad = int(S.dim_pad);
     qp.mtiles_total = mt_total;
     qp.first_invalid = d_first_invalid;
-    qp.cnt = S.cnt; qp.done = S.done; qp.thr = S.thr; qp.topk = S.topk; qp.k = int(kk);
+    qp.cnt = S.cnt; qp.done = S.done; qp.over = plan.use_filter ? S.over : nullptr; qp.thr = S.thr; qp.topk = S.topk; qp.k = int(kk);
     if (plan.use_filter) {
         qp.filter.weights = S.weights; qp.filter.scale = S.f_scale; qp.filter.bias_mid = S.f_mid; qp.filter.bias_max = S.f_max;
         qp.filter.alpha = S.f_alpha; qp.filter.suffix = S.f_suffix;
@@ -1381,7 +1387,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         TV_CUDA(c.d_luts.reserve(w_rows * lut_pitch));           // padded to whole query groups and whole K slabs for the tensor path
     }
     TV_CUDA(c.d_cand.reserve(nq * size_t(cap)));
-    TV_CUDA(c.d_cnt.reserve(2 * nq + 1));                        // candidate counts, then the selection's part counters, then the count of finished queries
+    TV_CUDA(c.d_cnt.reserve(3 * nq + 1));                        // candidate counts, then the selection's part counters, then the count of finished queries, then overflow marks
     TV_CUDA(c.d_thr.reserve(nq));
     TV_CUDA(c.d_topk.reserve(nq * k_page));
     if (pages > 1) {
@@ -1396,7 +1402,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     SearchScratch S{};
     S.qscale = c.d_qscale.ptr; S.qbias = c.d_qbias.ptr; S.weights = c.d_weights.ptr;
     S.wfrag = c.d_wfrag.ptr; S.luts = c.d_luts.ptr; S.cand = c.d_cand.ptr; S.thr = c.d_thr.ptr; S.topk = c.d_topk.ptr;
-    S.cnt = c.d_cnt.ptr; S.done = c.d_cnt.ptr + nq; S.lo = nullptr; S.w_rows = w_rows; S.dim_pad = dim_pad; S.lut_pitch = lut_pitch; S.cap = cap; S.allow_tc = pages == 1;
+    S.cnt = c.d_cnt.ptr; S.done = c.d_cnt.ptr + nq; S.over = c.d_cnt.ptr + 2 * nq + 1; S.lo = nullptr; S.w_rows = w_rows; S.dim_pad = dim_pad; S.lut_pitch = lut_pitch; S.cap = cap; S.allow_tc = pages == 1;
     {
         ScanParams probe = base_scan_params(h, mode);
         plan.use_small = h->small_scan >= 0 && mode == TV_SCORE_PERMUTE_DOT && scan_small_supported(probe, int(nq), h->smem_limit);
@@ -1439,7 +1445,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     uint32_t *d_keff = &c.d_flags->k_eff;
     // In the common case the last selection decodes the rows and publishes the status words, for a host search straight
     // into page-locked memory; larger k, paged searches and key exports take separate steps.
-    const bool fused = pages == 1 && kk <= size_t(kSelectMaxK) && !out_keys_dev;
+    bool fused = pages == 1 && kk <= size_t(kSelectMaxK) && !out_keys_dev;
     SearchOutput out{};
     if (!out_scores_dev && !out_keys_dev) {
         TV_CUDA(c.h_scores.reserve(nq * kk));
@@ -1476,6 +1482,43 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         h->filter_redone = redone;
         return TV_OK;
     };
+    // Searches the queries `who` again, without the filter, by themselves; their rows then replace those of the batch.
+    auto redo = [&](const std::vector<uint32_t> &who) -> int {
+        const size_t count = who.size();
+        SearchScratch R = S;
+        ScanPlan again;
+        rc = plan_scan(h, mode, count, true, again);
+        if (rc != TV_OK) return rc;
+        R.cap = candidate_capacity(kk, count, n);
+        TV_CUDA(c.d_cand.reserve(count * size_t(R.cap)));
+        TV_CUDA(c.d_redo_queries.reserve(count * dim));
+        TV_CUDA(c.d_redo_who.reserve(count));
+        TV_CUDA(c.d_redo_topk.reserve(count * kk));
+        if (!out_scores_dev && !out_keys_dev) {
+            TV_CUDA(c.d_scores.reserve(nq * kk));
+            TV_CUDA(c.d_slots.reserve(nq * kk));
+        }
+        R.cand = c.d_cand.ptr; R.topk = c.d_redo_topk.ptr; R.done = R.cnt + count; R.over = nullptr; R.w_rows = (count + 255) / 256 * 256;
+        TV_CUDA(cudaMemcpyAsync(c.d_redo_who.ptr, who.data(), count * 4, cudaMemcpyHostToDevice, st));   // pageable: staged before the call returns
+        TV_CUDA(launch_gather_rows(dq, c.d_redo_who.ptr, int(count), int(dim), c.d_redo_queries.ptr, st));
+        rc = enqueue_query_prep(h, st, R, again, mode, c.d_redo_queries.ptr, count, kk, &c.d_flags->first_invalid);
+        if (rc != TV_OK) return rc;
+        h->launches += 2;
+        for (bool careful : {false, true}) {
+            rc = enqueue_search(h, st, &c.marks, R, again, mode, count, kk, m, &c.d_flags->overflow, &c.d_flags->error, careful, !careful, nullptr);
+            if (rc != TV_OK) return rc;
+            TV_CUDA(cudaMemcpyAsync(c.h_flags, c.d_flags, sizeof(DeviceFlags), cudaMemcpyDeviceToHost, st));
+            TV_CUDA(cudaStreamSynchronize(st));
+            rc = check_flags(h, c.h_flags, queries, queries_on_device, st);
+            if (rc != TV_OK || !c.h_flags->overflow) break;
+            if (careful) return fail(h, TV_ERR_CUDA, "candidate overflow in the bounded schedule (internal error)");
+            TV_CUDA(cudaMemsetAsync(&c.d_flags->overflow, 0, 4, st));
+        }
+        if (rc != TV_OK) return rc;
+        TV_CUDA(launch_scatter_rows(c.d_redo_topk.ptr, c.d_redo_who.ptr, int(count), int(kk), c.d_topk.ptr, st));
+        fused = false;                                         // the rows are decoded from d_topk
+        return finish();
+    };
     for (size_t page = 0; page < pages; ++page) {
         const size_t k_this = pages == 1 ? kk : std::min(kPageK, kk - page * kPageK);
         S.lo = page == 0 ? nullptr : c.d_floor.ptr;
@@ -1499,12 +1542,22 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
             if (rc != TV_OK) { c.marks.used = 0; return rc; }
             if (!c.h_flags->overflow) break;
             if (careful) return fail(h, TV_ERR_CUDA, "candidate overflow in the bounded schedule (internal error)");
-            // a chunk produced more candidates than the buffer holds: redo this page without the filter, then with bounded chunks
-            if (!plan.use_filter) attempt = 1;
-            else redone = int64_t(nq);
+            // A chunk produced more candidates than the buffer holds.  Behind a filter that is a matter of single queries (more
+            // vectors tie with their k-th result, or come closer than the bound can tell, than a list holds): those are searched
+            // again without it, or the whole batch when they are most of it.  Without a filter: again with bounded chunks.
+            TV_CUDA(cudaMemsetAsync(&c.d_flags->overflow, 0, 4, st));
+            if (!plan.use_filter) { attempt = 1; continue; }
             plan.use_filter = false;
-            c.h_flags->overflow = 0;
-            TV_CUDA(cudaMemcpyAsync(&c.d_flags->overflow, &c.h_flags->overflow, 4, cudaMemcpyHostToDevice, st));
+            std::vector<uint32_t> over(nq), who;
+            TV_CUDA(cudaMemcpyAsync(over.data(), S.over, nq * 4, cudaMemcpyDeviceToHost, st));
+            TV_CUDA(cudaStreamSynchronize(st));
+            for (size_t q = 0; q < nq; ++q) if (over[q]) who.push_back(uint32_t(q));
+            redone = int64_t(who.size() <= nq / 2 ? who.size() : nq);
+            if (who.size() <= nq / 2) {
+                rc = redo(who);
+                if (rc != TV_OK) { c.marks.used = 0; return rc; }
+                break;
+            }
         }
         if (pages > 1) {
             // this page's keys into their columns of the full rows; its last key bounds the next page from below

@@ -114,6 +114,7 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *de
         if (w_scale >= FLT_MIN) w_inv = __fdiv_rn(1.0f, w_scale);
         else w_scale = 1.0f;
         alpha = __fdiv_rn(__fmul_rn(w_scale, p.level_scale), scale);
+        if (!(max_span > 0.0f)) w_inv = 0.0f;                       // a zero query: every sum is zero, and so is every weight
     }
     double beta = 0.0, slack = 0.0;
     if (tid < 32) {
@@ -197,7 +198,8 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *de
         for (int b = batches - 1; b >= 0; --b) { rest += batch_sum[b]; suffix[b] = float(rest + 1e-2 + 1e-6 * fabs(rest)); }
         p.filter.alpha[q] = alpha;
         p.filter.bias_mid[q] = float(base);
-        p.filter.bias_max[q] = float(base + double(scale) * slack * 1.000001 + 1e-5 * fabs(double(s_bias)));
+        // a zero query's bound is its exact score: all vectors tie, and only their slots decide
+        p.filter.bias_max[q] = max_span > 0.0f ? float(base + double(scale) * slack * 1.000001 + 1e-5 * fabs(double(s_bias))) : s_bias;
     }
 }
 
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParam
         return;
     }
     if (p.cnt != nullptr) {
-        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; if (q == 0) p.done[p.nq] = 0; }
+        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; if (p.over != nullptr) p.over[q] = 0; if (q == 0) p.done[p.nq] = 0; }
         for (int i = tid; i < p.k; i += kPrepThreads) p.topk[size_t(q) * p.k + i] = kEmptyKey;
     }
     const float *src = p.queries + size_t(q) * dim;
@@ -744,6 +746,15 @@ __global__ void __launch_bounds__(256) merge_keys_kernel(const uint64_t *keys_in
     }
 }
 
+__global__ void gather_rows_kernel(const float *src, const uint32_t *who, int dim, float *dst) {
+    const size_t from = size_t(who[blockIdx.x]) * dim, to = size_t(blockIdx.x) * dim;
+    for (int i = threadIdx.x; i < dim; i += blockDim.x) dst[to + i] = src[from + i];
+}
+__global__ void scatter_rows_kernel(const uint64_t *src, const uint32_t *who, int k, uint64_t *dst) {
+    const size_t from = size_t(blockIdx.x) * k, to = size_t(who[blockIdx.x]) * k;
+    for (int i = threadIdx.x; i < k; i += blockDim.x) dst[to + i] = src[from + i];
+}
+
 }  // namespace
 
 // =====================================================================================================
@@ -855,6 +866,15 @@ cudaError_t launch_finalize(const CandidateBuffers &cb, int nq, const unsigned l
     const int64_t total = int64_t(nq) * cb.k;
     finalize_kernel<<<unsigned((total + 255) / 256 + (total == 0)), 256, 0, s>>>(cb, nq, n_allowed, n, scores, slots,
                                                                                  k_eff_out, out_stride_is_k);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gather_rows(const float *src, const uint32_t *who, int count, int dim, float *dst, cudaStream_t s) {
+    gather_rows_kernel<<<unsigned(count), 128, 0, s>>>(src, who, dim, dst);
+    return cudaGetLastError();
+}
+cudaError_t launch_scatter_rows(const uint64_t *src, const uint32_t *who, int count, int k, uint64_t *dst, cudaStream_t s) {
+    scatter_rows_kernel<<<unsigned(count), 128, 0, s>>>(src, who, k, dst);
     return cudaGetLastError();
 }
 

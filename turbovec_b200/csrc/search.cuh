@@ -47,6 +47,7 @@ struct QueryPrepParams {
     } filter;
     // selection state of the batch, reset here (cnt == nullptr: none)
     uint32_t *cnt, *done;          // done[nq] = SearchOutput::finished
+    uint32_t *over;                // or nullptr
     uint64_t *thr, *topk;
     int k;
     int mtiles_total;              // ceil(nq / 16)
@@ -96,6 +97,7 @@ struct CandidateBuffers {
     uint32_t *overflow;
     uint32_t *error;               // device-side wait timeouts
     uint32_t *done;                // per query: parts of a long list selected so far (zero between launches)
+    uint32_t *over;                // filtering scans: per query whether a list of it overflowed, *overflow counts them; else nullptr
     int cap, k;
 };
 // Selection (select.cu).  dense_blocks > 0: the scan wrote 32 keys for each of the first min(dense_blocks, *n_live)
@@ -160,6 +162,7 @@ struct ScanParams {
     const int8_t *f_weights;
     int f_pitch;
     const float *f_alpha, *f_suffix;
+    uint32_t give_up;              // a filtering scan does nothing when more queries than this have overflowed already
 };
 // Permute-dot scan on mma.sync (int8 x int8 -> int32), up to 64 queries per launch.
 cudaError_t launch_scan_pd(const ScanParams &p, int sm_count, cudaStream_t s);
@@ -208,6 +211,9 @@ cudaError_t launch_scan_small(const ScanParams &p, const int8_t *weights, int pi
 // each): scan_lut_width gives how many fit (4, 2, 1, or 0 when not even one does); p.nq must not exceed it.
 int scan_lut_width(int ngroups, size_t smem_limit);
 cudaError_t launch_scan_lut(const ScanParams &p, int sm_count, cudaStream_t s);
+// Rows who[0 .. count) of src -> rows 0 .. of dst; and back: rows 0 .. of src -> rows who[..] of dst.
+cudaError_t launch_gather_rows(const float *src, const uint32_t *who, int count, int dim, float *dst, cudaStream_t s);
+cudaError_t launch_scatter_rows(const uint64_t *src, const uint32_t *who, int count, int k, uint64_t *dst, cudaStream_t s);
 // lo[q] = thr[q] + 1, or the empty key when thr[q] is empty (fewer results than asked for: nothing more can follow).
 cudaError_t launch_advance_floor(const uint64_t *thr, uint64_t *lo, int nq, cudaStream_t s);
 

@@ -155,7 +155,8 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
     const uint32_t ncand = min(raw, uint32_t(cb.cap));
     const uint32_t parts = max(1u, (ncand + kSelectSegment - 1) / kSelectSegment);
     if (part >= parts) return;                                          // (a late CTA may see the count already cleared: same outcome)
-    if (part == 0 && tid == 0 && raw > uint32_t(cb.cap)) atomicExch(cb.overflow, 1u);
+    const bool spilled = raw > uint32_t(cb.cap);
+    if (part == 0 && tid == 0 && spilled && (cb.over == nullptr || atomicExch(&cb.over[q], 1u) == 0u)) atomicAdd(cb.overflow, 1u);
     uint64_t *list = cb.cand + size_t(q) * cb.cap;
     uint64_t *seg = list + size_t(part) * kSelectSegment;
     const uint32_t here = min(uint32_t(kSelectSegment), ncand - min(ncand, part * kSelectSegment));
@@ -190,7 +191,10 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
     }
     for (int i = tid; i < cb.k; i += kSelThreads) cb.topk[size_t(q) * cb.k + i] = i < m ? sh.sorted[i] : kEmptyKey;
     if (tid == 0) {
-        cb.thr[q] = m == cb.k ? sh.sorted[cb.k - 1] : kEmptyKey;        // kEmptyKey until k results exist: everything still passes
+        // kEmptyKey until k results exist: everything still passes.  A query that the filter has lost is searched again by
+        // itself: until then nothing of it need survive.
+        if (spilled && cb.over != nullptr) cb.thr[q] = make_key(INFINITY, 0u);
+        else cb.thr[q] = m == cb.k ? sh.sorted[cb.k - 1] : kEmptyKey;
         cb.cnt[q] = 0;
     }
     if (out.scores == nullptr) return;
@@ -246,6 +250,7 @@ cudaError_t launch_select(const CandidateBuffers &cb, int nq, uint32_t dense_blo
         SearchOutput o{};
         if (out != nullptr) { o = *out; o.q0 = q0; }
         part.cand += size_t(q0) * cb.cap; part.cnt += q0; part.thr += q0; part.topk += size_t(q0) * cb.k; part.done += q0;
+        if (part.over != nullptr) part.over += q0;
         select_parts_kernel<<<dim3(parts, unsigned(std::min(nq - q0, 32768))), kSelThreads, 0, s>>>(part, dense_blocks, n_live, o);
     }
     return cudaGetLastError();
