@@ -135,6 +135,10 @@ enum {
 /* dim == 0 creates a lazy index whose dimension is fixed by the first add.  device = CUDA ordinal. */
 int tv_index_create(size_t dim, int bit_width, int kind, int device, tv_index **out);
 void tv_index_destroy(tv_index *h);
+/* A destroyed handle leaves its streams, events and scratch (at most 96 MB of device and 40 MB of page-locked memory) for the
+ * next handle on the device; at most two wait per device.  This frees those that wait and returns how many there were.  The
+ * library does so by itself when one of its own allocations fails. */
+size_t tv_release_workspaces(void);
 
 /* Message of the most recent failing call on this handle (or of the last failed create when h == NULL). */
 const char *tv_last_error(const tv_index *h);

@@ -3,6 +3,7 @@
 // uniform quantiser) plus a scale, so that tv_get_row / tv_set_row move exactly what the real index moves; a score
 // is scale * sum_d q[d] * (code_d - 8), accumulated in double and rounded once.  Keys use an order-preserving image
 // of the score so that ascending key order = (score descending, slot ascending), as the real library's do.
+#include "cuda_runtime.h"
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -71,6 +72,9 @@ int tv_add(tv_index *h, const float *x, size_t n, size_t dim) {
     }
     return TV_OK;
 }
+// workspaces of destroyed handles: fake_hold makes every allocation fail until they are released
+size_t tv_release_workspaces(void) { const size_t held = fake_held_workspaces; fake_held_workspaces = 0; return held; }
+void fake_hold(size_t workspaces) { fake_held_workspaces = workspaces; }
 int tv_swap_remove(tv_index *h, size_t slot, size_t *moved_from) {
     if (slot >= h->codes.size()) return fail(h, TV_ERR_SLOT_OUT_OF_RANGE, "slot out of range");
     const size_t last = h->codes.size() - 1;

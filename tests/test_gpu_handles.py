@@ -44,3 +44,27 @@ def test_handles_of_different_sizes_searched_from_two_threads(T):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_idle_workspaces_are_bounded_and_given_back(T):
+    import torch
+    T.release_workspaces()
+    x = anisotropic(9000, 512, seed=7)
+    for _ in range(2):
+        handles = [T.TurboQuantIndex(512, 4) for _ in range(4)]
+        want = None
+        for idx in handles:
+            idx.add(x)
+            got = idx.search(x[:40], 7)
+            want = got if want is None else want
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        del handles, idx
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    assert T.release_workspaces() == 2
+    assert torch.cuda.mem_get_info()[0] > before + (8 << 20)
+    assert T.release_workspaces() == 0
+    idx = T.TurboQuantIndex(512, 4)
+    idx.add(x)
+    got = idx.search(x[:40], 7)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])

@@ -188,3 +188,14 @@ def test_failed_add_is_taken_back_from_every_shard(lib):
     assert ids_handle.add(bad, ids[100:600]) == 17
     assert len(ids_handle) == 100 and np.array_equal(ids_handle.ids(), ids[:100])            # the id tables were rolled back too
     assert ids_handle.add(x[100:600], ids[100:600]) == 0 and len(ids_handle) == 600
+
+
+def test_scratch_of_a_search_takes_the_memory_of_destroyed_handles(lib):
+    """Allocations fail while the (fake) workspaces of destroyed handles hold the memory: the search gives those back and goes on."""
+    dim = 16
+    x, q = _rows(300, dim, 11), _rows(2, dim, 12)
+    many, one = Handle(lib, dim, 3), Handle(lib, dim, 1)
+    assert many.add(x) == 0 and one.add(x) == 0
+    want = one.search(q, 5)
+    lib.fake_hold(C.c_size_t(2))
+    assert _same(many.search(q, 5), want)

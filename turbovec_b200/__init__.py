@@ -604,6 +604,12 @@ def measure_int8_peak(device: int = 0, seconds: float = 0.0) -> float:
     return float(out.value)
 
 
+def release_workspaces() -> int:
+    """Frees the scratch memory, streams and events that destroyed indexes have left for the next one (at most two sets of 96 MB
+    of device and 40 MB of page-locked memory per device), for another library's sake; returns the number of sets."""
+    return int(_native.load().tv_release_workspaces())
+
+
 def merge_keys_device(keys_ptr: int, n_lists: int, nq: int, k: int, scores_ptr: int, slots_ptr: int, *, device: int = 0,
                       stream: int = 0, chunk_slots: int = 0) -> None:
     """keys[n_lists][nq][k] (device memory, e.g. all-gathered search_device_keys rows) -> per query the k best,

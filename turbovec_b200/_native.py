@@ -52,6 +52,7 @@ SIGNATURES = {
     "tv_quantise_grid_lookup": (C.c_int, [C.POINTER(C.c_float), C.c_int, C.POINTER(C.c_float), C.c_size_t, C.POINTER(C.c_uint8)]),
     "tv_index_create": (C.c_int, [C.c_size_t, C.c_int, C.c_int, C.c_int, C.POINTER(_H)]),
     "tv_index_destroy": (None, [_H]),
+    "tv_release_workspaces": (C.c_size_t, []),
     "tv_last_error": (C.c_char_p, [_H]),
     "tv_error_detail": (None, [_H, _szp, _szp, _f32p, _u64p]),
     "tv_len": (C.c_size_t, [_H]),

@@ -30,17 +30,24 @@ using namespace tv;
 
 thread_local std::string g_create_error;
 
-// Frees the workspaces that wait for the next handle (WorkSetPool below); false when there were none.
-bool release_idle_workspaces();
+// Frees the workspaces that wait for the next handle (WorkSetPool below); returns how many there were.
+size_t release_idle_workspaces();
 
-// cudaMalloc that gives idle workspaces back before it reports that memory ran out.
-cudaError_t device_alloc(void **ptr, size_t bytes) {
-    cudaError_t e = cudaMalloc(ptr, bytes);
-    if (e == cudaErrorMemoryAllocation && release_idle_workspaces()) {
+// Allocations that give idle workspaces back before they report that memory ran out.
+template <typename Alloc>
+cudaError_t alloc_or_release(Alloc alloc) {
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && release_idle_workspaces() > 0) {
         cudaGetLastError();
-        e = cudaMalloc(ptr, bytes);
+        e = alloc();
     }
     return e;
+}
+cudaError_t device_alloc(void **ptr, size_t bytes) {
+    return alloc_or_release([&] { return cudaMalloc(ptr, bytes); });
+}
+cudaError_t pinned_alloc(void **ptr, size_t bytes) {
+    return alloc_or_release([&] { return cudaMallocHost(ptr, bytes); });
 }
 
 template <typename T>
@@ -78,7 +85,7 @@ struct PinnedArray {
     cudaError_t reserve(size_t n) {
         if (n <= cap) return cudaSuccess;
         release();
-        cudaError_t e = cudaMallocHost(&ptr, std::max<size_t>(n, 1) * sizeof(T));
+        cudaError_t e = pinned_alloc(reinterpret_cast<void **>(&ptr), std::max<size_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess) cap = n;
         return e;
     }
@@ -116,6 +123,11 @@ struct Marks {
         total_ms = total;
         launches = int(used / 2);
         used = 0;
+    }
+    // nothing is bracketed any more; a call of many launches leaves no more events behind than one of few
+    void trim() {
+        used = 0;
+        while (pool.size() > 64) { cudaEventDestroy(pool.back()); pool.pop_back(); }
     }
 };
 
@@ -162,8 +174,8 @@ struct SearchCtx {
         cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&ev0);
         if (e == cudaSuccess) e = cudaEventCreate(&ev1);
-        if (e == cudaSuccess) e = cudaMalloc(&d_flags, sizeof(DeviceFlags));
-        if (e == cudaSuccess) e = cudaMallocHost(&h_flags, sizeof(DeviceFlags));
+        if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void **>(&d_flags), sizeof(DeviceFlags));
+        if (e == cudaSuccess) e = pinned_alloc(reinterpret_cast<void **>(&h_flags), sizeof(DeviceFlags));
         // the event pool of the common schedules up front, so that a search creates nothing
         for (int i = 0; i < 64 && e == cudaSuccess; ++i) {
             cudaEvent_t ev;
@@ -195,8 +207,9 @@ constexpr int kSearchCtxs = 2;
 // What a handle works with besides its data: streams, events, status words, staging buffers and the search contexts.
 // Making one costs about 15 ms (page-locked allocations take 2 - 20 ms each on this class of machine, device allocations
 // 0.4 - 3 ms), as much as encoding two million vectors, so a destroyed handle leaves its workspace for the next one on
-// the device.  At most kIdleSets wait per device, each trimmed to kIdleDeviceBytes and kIdlePinnedBytes, and all of them
-// are freed when an allocation fails.  A workspace belongs to one handle at a time, and its streams are idle in between.
+// the device.  At most kIdleSets wait per device, each trimmed to kIdleDeviceBytes and kIdlePinnedBytes.  All of them are
+// freed when an allocation of this library fails, and by tv_release_workspaces for the sake of others in the process.  A
+// workspace belongs to one handle at a time, and its streams are idle in between.
 struct WorkSet {
     cudaStream_t stream = nullptr;           // mutations and accessors
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -217,7 +230,7 @@ struct WorkSet {
         if (e == cudaSuccess) e = cudaEventCreate(&ev1);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_mut, cudaEventDisableTiming);
         if (e == cudaSuccess) e = device_alloc(reinterpret_cast<void **>(&d_flags), sizeof(DeviceFlags));
-        if (e == cudaSuccess) e = cudaMallocHost(&h_flags, sizeof(DeviceFlags));
+        if (e == cudaSuccess) e = pinned_alloc(reinterpret_cast<void **>(&h_flags), sizeof(DeviceFlags));
         for (int i = 0; i < kSearchCtxs && e == cudaSuccess; ++i) e = ctx[i].init();
         return e;
     }
@@ -225,12 +238,12 @@ struct WorkSet {
     bool retire() {
         bool ok = stream && cudaStreamSynchronize(stream) == cudaSuccess;
         if (ok && copy_stream) ok = cudaStreamSynchronize(copy_stream) == cudaSuccess;
-        marks.used = 0;
+        marks.trim();
         size_t device = 0, pinned = 0;
         for (SearchCtx &c : ctx) {
             ok = ok && c.stream && cudaStreamSynchronize(c.stream) == cudaSuccess;
             c.busy = false;
-            c.marks.used = 0;
+            c.marks.trim();
             c.each_array([&](auto &a) { device += a.bytes(); if (device > kIdleDeviceBytes) { device -= a.bytes(); a.release(); } });
             c.each_pinned([&](auto &a) { pinned += a.bytes(); if (pinned > kIdlePinnedBytes) { pinned -= a.bytes(); a.release(); } });
         }
@@ -266,41 +279,48 @@ WorkSetPool &workset_pool() {
     static WorkSetPool *pool = new WorkSetPool;              // never destroyed: the driver may be gone by then
     return *pool;
 }
-// The device is current.
-WorkSet *acquire_workset(int device, cudaError_t *err) {
+// An idle workspace of the device, or of any device (device < 0); nullptr when none waits.
+WorkSet *take_idle_workset(int device) {
     WorkSetPool &pool = workset_pool();
-    {
-        std::lock_guard<std::mutex> g(pool.mu);
-        auto &list = pool.idle[device];
-        if (!list.empty()) { WorkSet *w = list.back(); list.pop_back(); return w; }
+    std::lock_guard<std::mutex> g(pool.mu);
+    for (auto &entry : pool.idle) {
+        if ((device >= 0 && entry.first != device) || entry.second.empty()) continue;
+        WorkSet *w = entry.second.back();
+        entry.second.pop_back();
+        return w;
+    }
+    return nullptr;
+}
+// The device is current.  The handle's mutations are ordered from here on (ev_mut).
+WorkSet *acquire_workset(int device, cudaError_t *err) {
+    while (WorkSet *w = take_idle_workset(device)) {
+        if (cudaEventRecord(w->ev_mut, w->stream) == cudaSuccess) return w;
+        cudaGetLastError();                                  // left from a context that is gone
+        delete w;
     }
     WorkSet *w = new WorkSet;
     *err = w->init();
+    if (*err == cudaSuccess) *err = cudaEventRecord(w->ev_mut, w->stream);
     if (*err != cudaSuccess) { delete w; return nullptr; }
     return w;
 }
 void return_workset(int device, WorkSet *w) {
     if (!w) return;
     if (w->retire()) {
-        WorkSetPool &pool = workset_pool();
-        std::lock_guard<std::mutex> g(pool.mu);
-        auto &list = pool.idle[device];
-        if (list.size() < WorkSetPool::kIdleSets) { list.push_back(w); return; }
+        try {
+            WorkSetPool &pool = workset_pool();
+            std::lock_guard<std::mutex> g(pool.mu);
+            auto &list = pool.idle[device];
+            if (list.size() < WorkSetPool::kIdleSets) { list.push_back(w); return; }
+        } catch (const std::bad_alloc &) {
+        }                                                    // no room to remember it: freed
     }
     delete w;
 }
-bool release_idle_workspaces() {
-    std::vector<WorkSet *> all;
-    {
-        WorkSetPool &pool = workset_pool();
-        std::lock_guard<std::mutex> g(pool.mu);
-        for (auto &entry : pool.idle) {
-            all.insert(all.end(), entry.second.begin(), entry.second.end());
-            entry.second.clear();
-        }
-    }
-    for (WorkSet *w : all) delete w;
-    return !all.empty();
+size_t release_idle_workspaces() {
+    size_t released = 0;
+    for (; WorkSet *w = take_idle_workset(-1); ++released) delete w;
+    return released;
 }
 
 // Device copy of the id -> slot table, kept for large allowlists (search.cu: idtab_*_kernel).  The host tables stay the
@@ -1092,6 +1112,7 @@ int expanded_sync(tv_index *h, cudaStream_t st, const uint32_t level_words[4], b
         TV_CUDA(cudaMemGetInfo(&free_b, &total_b));
         // keep a tenth of the device (at least 1 GiB) free for scratch and for the growth of the index
         const size_t keep = std::max<size_t>(total_b / 10, size_t(1) << 30);
+        if (free_b < bytes + keep && release_idle_workspaces() > 0) TV_CUDA(cudaMemGetInfo(&free_b, &total_b));
         x.drop();
         cudaError_t e = cudaErrorMemoryAllocation;
         if (h->tc_expanded == 2 || free_b >= bytes + keep) e = x.levels.reserve(bytes);
@@ -1742,12 +1763,13 @@ int tv_index_create(size_t dim, int bit_width, int kind, int device, tv_index **
     if ((e = cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) != cudaSuccess) return bail("cudaDeviceGetAttribute", e);
     h->smem_limit = size_t(smem_optin);
     if (!(h->ws = acquire_workset(device, &e))) return bail("workspace", e);
-    if ((e = cudaEventRecord(h->ws->ev_mut, h->ws->stream)) != cudaSuccess) return bail("cudaEventRecord", e);
     *out = h;
     return TV_OK;
 }
 
 void tv_index_destroy(tv_index *h) { delete h; }
+
+size_t tv_release_workspaces(void) { return release_idle_workspaces(); }
 
 const char *tv_last_error(const tv_index *h) { return h ? h->last_error.c_str() : g_create_error.c_str(); }
 

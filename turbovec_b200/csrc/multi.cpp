@@ -49,6 +49,10 @@ cudaError_t grow(T *&ptr, size_t &cap, size_t n) {
     if (ptr) cudaFree(ptr);
     ptr = nullptr; cap = 0;
     cudaError_t e = cudaMalloc(&ptr, std::max<size_t>(n, 1) * sizeof(T));
+    if (e == cudaErrorMemoryAllocation && tv_release_workspaces() > 0) {     // memory that destroyed handles have left
+        cudaGetLastError();
+        e = cudaMalloc(&ptr, std::max<size_t>(n, 1) * sizeof(T));
+    }
     if (e == cudaSuccess) cap = n;
     return e;
 }
