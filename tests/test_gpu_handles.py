@@ -68,3 +68,21 @@ def test_idle_workspaces_are_bounded_and_given_back(T):
     idx.add(x)
     got = idx.search(x[:40], 7)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("before", [0, 5, 32])
+def test_host_add_in_chunks_of_whole_code_blocks(T, before):
+    """16 MB of rows at a time: one launch per chunk, and one more only for rows that complete a block begun earlier."""
+    n, dim = 12_001, 1536
+    x = anisotropic(n + before, dim, seed=91)
+    idx = T.TurboQuantIndex(dim, 4)
+    if before:
+        idx.add(x[:before])
+    at = idx.launch_count
+    idx.add(x[before:])
+    chunks = -(-(n + before % 32) // (2730 // 32 * 32))
+    assert idx.launch_count - at == chunks + (before % 32 != 0)
+    whole = T.TurboQuantIndex(dim, 4)
+    whole.set_option(T.OPT_INGEST_PIPELINE, 0)
+    whole.add(x)
+    assert np.array_equal(idx.codes_blocked_seq(), whole.codes_blocked_seq()) and np.array_equal(idx.scales(), whole.scales())

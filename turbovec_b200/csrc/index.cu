@@ -741,7 +741,13 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
     // Device input is encoded in place.  Host input goes through pinned staging in chunks of about 16 MB,
     // double buffered (page-locking 16 MB takes 12 ms): host threads copy chunk i+1 into pinned memory while chunk i crosses the bus on the copy
     // stream and chunk i-1 is encoded on the handle's stream.
-    const size_t chunk_rows = on_device ? n : std::max<size_t>(1, std::min<size_t>(n, (size_t(16) << 20) / (dim * 4)));
+    // Several chunks meet at borders of code blocks, so that only the first one can have rows for a partly filled block.
+    size_t chunk_rows = on_device ? n : std::min<size_t>(n, (size_t(16) << 20) / (dim * 4));
+    size_t first_rows = chunk_rows;
+    if (chunk_rows < n) {                                    // (16 MB hold at least 256 rows)
+        chunk_rows -= chunk_rows % kBlock;
+        first_rows = chunk_rows - h->n % kBlock;
+    }
     bool src_pinned = false;
     if (!on_device) {
         if (!h->ws->copy_stream) {
@@ -772,8 +778,7 @@ int add_rows(tv_index *h, const float *x, size_t n, size_t dim, bool on_device) 
     }
     TV_CUDA(cudaEventRecord(h->ws->ev0, h->ws->stream));
     size_t chunk_index = 0;
-    for (size_t done = 0; done < n; done += chunk_rows, ++chunk_index) {
-        const size_t rows = std::min(chunk_rows, n - done);
+    for (size_t done = 0, rows = first_rows; done < n; done += rows, rows = std::min(chunk_rows, n - done), ++chunk_index) {
         const float *src = x + done * dim;
         TV_STEP(injected_failure(h));
         if (!on_device) {
