@@ -1229,9 +1229,9 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
     }
     // Chunk 0 holds at most `cap` vectors, so every one of them may pass.  Later chunks grow so that the
     // expected number of candidates per query, k * |chunk| / |seen|, stays near cap / 4.
-    // The tensor-memory scan pays for dense candidates (its epilogue re-reads a 32 x 32 tile of scores
-    // whenever one of them passes), so its first three chunks grow x6 each (measured against x24, x10 and others on
-    // 10 M and 1.25 M vectors), then by the list-capacity rule.
+    // The tensor-memory scan pays for dense candidates (its epilogue scores every flagged run of 8 columns exactly), so its
+    // first three chunks grow x6 each (x4 / x6 / x9 / x14: 14.7 / 14.2 / 13.9 / 14.4 ms on 10 M x 1536, batch 1,024, and
+    // 367 / 345 / 350 / 358 us on 1.2 M x 200, batch 100), then by the list-capacity rule.
     const size_t first = size_t(S.cap) / kBlock;
     const double growth = std::max(0.5, double(S.cap) / (4.0 * double(kk)));
     size_t begin = 0;
@@ -1312,7 +1312,7 @@ int enqueue_query_prep(tv_index *h, cudaStream_t st, const SearchScratch &S, con
     QueryPrepParams qp{};
     qp.queries = dq; qp.nq = int(nq); qp.dim = int(dim); qp.bits = h->bits; qp.ngroups = ng;
     qp.mode = mode;
-    qp.perm0 = h->d_perm.ptr; qp.perm1 = h->d_perm.ptr + dim;
+    qp.perms = h->d_perm.ptr;
     qp.inv_sqrt_block = h->rot.inv_sqrt_block;
     qp.centroids = h->d_codebook.ptr + 16;
     if (!h->shift.empty()) { qp.shift = h->d_calib.ptr; qp.scale_tq = h->d_calib.ptr + dim; }
@@ -1364,8 +1364,9 @@ int check_flags(tv_index *h, const DeviceFlags *f, const float *queries, bool qu
     return TV_OK;
 }
 
-// The whole search on a context's stream.  Results land in c.d_scores / c.d_slots (row stride k) unless
-// out_scores_dev is given (row stride k_eff).  The caller holds the handle's lock (shared is enough).
+// The whole search on a context's stream.  Results land in the page-locked c.h_scores / c.h_slots (row stride k: written
+// there by the last selection, or copied from c.d_scores / c.d_slots) unless out_scores_dev is given (row stride k_eff).
+// The caller holds the handle's lock (shared is enough).
 int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on_device, size_t nq, size_t k, const MaskSpec &mask,
                 float *out_scores_dev, int64_t *out_slots_dev, size_t *k_eff_out, uint64_t *out_keys_dev = nullptr,
                 uint64_t key_offset = 0) {
@@ -2312,7 +2313,7 @@ int tv_search_device_noalloc(tv_index *h, const float *queries_device, size_t nq
     TV_CUDA(cudaEventRecord(c.ev0, st));
 
     // The array still holds the previous call's data.  Query preparation clears the query operands it does not
-    // overwrite, and the schedule resets counters, thresholds and result keys at its start.
+    // overwrite and resets counters, thresholds and result keys (a repeated schedule resets them again).
     rc = enqueue_query_prep(h, st, S, plan, mode, queries_device, nq, kk, &c.d_flags->first_invalid);
     if (rc != TV_OK) return rc;
     MaskOnDevice no_mask;
@@ -2737,7 +2738,7 @@ int tv_rotate(tv_index *h, const float *rows, size_t n, size_t dim, float *rotat
     QueryPrepParams qp{};
     qp.queries = h->d_stage.ptr; qp.nq = qp.rows = int(n); qp.dim = int(dim); qp.bits = h->bits; qp.ngroups = h->ngroups;
     qp.mode = kModeLutMulAdd;
-    qp.perm0 = h->d_perm.ptr; qp.perm1 = h->d_perm.ptr + dim; qp.inv_sqrt_block = h->rot.inv_sqrt_block;
+    qp.perms = h->d_perm.ptr; qp.inv_sqrt_block = h->rot.inv_sqrt_block;
     qp.centroids = h->d_codebook.ptr + 16;
     qp.q_rot = c.d_qrot.ptr; qp.qscale = c.d_qscale.ptr; qp.qbias = c.d_qbias.ptr; qp.luts = c.d_luts.ptr;
     qp.lut_pitch = (h->ngroups + 3) / 4 * 4 * 32;

@@ -210,8 +210,9 @@ __device__ __forceinline__ int dismissal_bound(float qs, float qb, float t, floa
 }
 
 
-// First chunk of an unfiltered search: the 32 accumulator columns of a piece (queries ql0 .. ql0 + 31 of one vector) go to
-// position `at` of their queries' candidate lists, every one of them.  qscale / qbias point at the piece's first column.
+// First chunk of a search: the 32 accumulator columns of a piece (queries ql0 .. ql0 + 31 of one vector) go to position `at`
+// of their queries' candidate lists, every one of them (kEmptyKey for a slot that the mask does not allow).  qscale / qbias
+// point at the piece's first column.
 template <bool ONEHOT>
 __device__ __forceinline__ void write_piece(const uint32_t (&acc)[32], const float *qscale, const float *qbias, bool fused, float vs,
                                             bool live, int64_t slot, int ql0, int nq_end, uint32_t at, const CandidateBuffers &cb) {

@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParam
         rowA[i] = v;
         if (!(fabsf(v) < 1e16f)) atomicMin(p.first_invalid, (unsigned long long)(size_t(q) * dim + i));
     }
-    // both tables, 16 bytes at a time (dim is a multiple of 8 and the second table follows the first)
-    for (int i = tid; i < dim / 4; i += kPrepThreads) reinterpret_cast<uint4 *>(perm0)[i] = reinterpret_cast<const uint4 *>(p.perm0)[i];
+    // both tables, 16 bytes at a time (dim is a multiple of 8)
+    for (int i = tid; i < dim / 4; i += kPrepThreads) reinterpret_cast<uint4 *>(perm0)[i] = reinterpret_cast<const uint4 *>(p.perms)[i];
     if (tid < 16) s_centroids[tid] = tid < (1 << p.bits) ? p.centroids[tid] : 0.0f;
     __syncthreads();
     // Rotation::apply: no normalisation (search.rs:3237-3242)

@@ -18,7 +18,7 @@ struct QueryPrepParams {
     const float *queries;          // [nq][dim] device
     int nq, dim, bits, ngroups;
     int mode;                      // ScoreMode
-    const uint16_t *perm0, *perm1;
+    const uint16_t *perms;         // the packed permutations of both rounds, [2][dim]
     float inv_sqrt_block;
     const float *centroids;        // 2^bits
     const float *shift;            // TQ+ pair or nullptr
