@@ -179,3 +179,19 @@ def test_one_hot_form_of_wide_batches_is_still_reached(T, dim, bits, n, nq):
     s, i = idx.search(q, 10)
     assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
     assert idx.get_option(T.OPT_FILTER_REDONE) == -1
+
+
+@pytest.mark.parametrize("n,dim,bits,nq,k,chosen", [(500_000, 200, 2, 64, 10, True), (200_000, 1536, 2, 64, 10, True), (3_000, 3072, 2, 300, 10, False),
+                                                    (100_000, 768, 3, 512, 200, False), (60_000, 2072, 2, 64, 10, True)])
+def test_default_choice_on_both_sides_of_the_switch(T, n, dim, bits, nq, k, chosen):
+    """Clearly inside and outside of the region where the filter pays; the results do not depend on it."""
+    idx = T.TurboQuantIndex(dim, bits)
+    for lo in range(0, n, 20_000):
+        idx.add(anisotropic(min(20_000, n - lo), dim, seed=95, offset=lo))
+    q = anisotropic(nq, dim, seed=95, offset=n + 1)
+    s, i = idx.search(q, k)
+    assert (idx.get_option(T.OPT_FILTER_REDONE) >= 0) == chosen
+    idx.set_option(T.OPT_FILTER, 0)
+    s0, i0 = idx.search(q, k)
+    assert idx.get_option(T.OPT_FILTER_REDONE) == -1
+    assert np.array_equal(i, i0) and np.array_equal(s, s0)

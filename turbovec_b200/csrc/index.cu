@@ -1062,41 +1062,65 @@ int plan_scan(tv_index *h, int mode, size_t nq, bool allow_tc, ScanPlan &plan) {
     return TV_OK;
 }
 
-// Whether a batch goes through the filtering scan: when its expected time is well below that of the form it replaces.
+// Blocks [begin, end) of one scan of a filtering search over n_blocks, `first` of which were ranked ahead.  Every survivor costs
+// a gather of its bytes, so the chunks grow gently: one of three times the vectors seen so far brings about three times k
+// results above the threshold and, below it, what the bound cannot tell from them (x4 / x6 / x9 / x14: 1,155 / 1,195 / 1,186 /
+// 1,452 us for 1.2 M x 200 2-bit, batch 1,024).  A short tail joins the chunk before it.
+size_t filter_chunk_end(size_t begin, size_t first, size_t n_blocks) {
+    const size_t end = std::min(n_blocks, std::max(begin, first) * 4);
+    return end + end / 2 >= n_blocks ? n_blocks : end;
+}
+
+// Whether a batch goes through the filtering scan: when its expected time is below that of the form it replaces by more than
+// the estimate's own error, and no chunk is expected to fill the lists (an overflow repeats queries).
 // The filter saves contraction (an eighth of the one-hot K) and pays for survivors, whose number depends on how far the
 // threshold of the vectors seen so far stands above the width of the bound.  With scores spread like a normal
 // distribution, the k-th best of m scores lies at z = Q^-1(k / m) standard deviations, and Q(z - delta) of a chunk survive;
 // delta, the bound's width, grows with the square root of the dimension (0.020 for 2-bit, 0.033 for 3-bit codes, plus
-// the spread of the vector scales).  Rates measured on 1.5 k - 1 M vectors of 200 - 3,072 dimensions (us): one-hot 5.3e-6
-// a byte-group per 256 queries, register lookups 1e-6 a byte-group per 4 queries, filter 0.7e-6 a byte-group per 256
-// queries, epilogue of either contraction 6e-7 a sum, survivors 3e-6 a byte-group, launches of the filter 120 against 60.
-// Both sides, filter / one-hot, us: 640 k x 200 2-bit, 8 queries 155 / 241, 512 queries 518 / 750; 160 k x 200, 64 queries
-// 142 / 146; 32 k x 1536, 64 queries 169 / 135; 100 k x 3072, 64 queries 518 / 512, 512 queries 5,887 / 1,167 (short lists of
-// many queries leave a loose threshold); 48 k x 768 3-bit, 512 queries 1,068 / 437; 1 M x 3072, 64 queries 1,160 / 3,750.
+// the spread of the vector scales).  Rates fitted to both forms at 57 points (us): one-hot 4.5e-6 a byte-group per 256 queries
+// and 8e-4 a candidate, register lookups 1e-6 a byte-group per 4 queries, filter 0.65e-6 a byte-group per 256 queries, epilogue
+// of either contraction 5e-7 a sum, survivors 2e-4 and 1.1e-6 a byte-group (most leave early), launches 100 against 60.
+// Filter / one-hot, us, where the two are close or far apart (k = 10 unless said): 1 M x 3072 2-bit, batch 64 1,055 / 3,642,
+// 256 2,630 / 4,085, 512 4,753 / 7,551, 1,024 13,286 / 14,742 (a list of 4,096 overflows for 16 queries), 128 with k = 100
+// 4,453 / 4,116; 1 M x 1536 2-bit, 1,024 3,496 / 7,717, 128 with k = 100 1,702 / 2,173, 256 with k = 100 3,208 / 2,188;
+// 1 M x 768 3-bit, 1,024 3,447 / 7,716, 512 with k = 100 7,442 / 4,561; 1.2 M x 200 2-bit, 1,024 with k = 100 2,485 / 3,497;
+// 100 k x 3072, 64 295 / 491, 512 1,730 / 1,148; 100 k x 768 3-bit, 512 682 / 673.  At 142 other points the choice was never the
+// slower one by more than 1 %; at 15 it left the faster one, mostly small indexes (30 k x 768 3-bit, 300, k = 1: 159 / 302).
+double one_hot_us(double bytes, double queries, double sums) { return bytes * 4.5e-6 * std::ceil(queries / 256.0) + sums * 5e-7; }
+double filter_us(double bytes, double queries, double sums) { return bytes * 0.65e-6 * std::ceil(queries / 256.0) + sums * 5e-7; }
+double lookup_us(double bytes, double queries) { return bytes * 1e-6 * std::ceil(queries / 4.0); }
 bool wants_filter(const tv_index *h, int mode, size_t nq, size_t k, int cap, bool masked, const ScanPlan &plan) {
     if (!scan_filter_supported(h->bits, mode, h->ngroups, h->smem_limit) || h->filter == 0 || h->mma_min_batch == 0) return false;
     if (h->filter == 2) return true;
     if (h->mma_min_batch > 0) return false;                    // the caller asked for the one-hot form
     if (!plan.use_tc && nq < 8) return false;                  // (flush geometries beyond 256 groups have no one-hot form)
-    const double n = double(h->n), bytes = n * h->ngroups, groups = std::ceil(double(nq) / 256.0);
+    const double n = double(h->n), queries = double(nq), bytes = n * h->ngroups, sums = n * queries;
     const double delta = (h->bits == 2 ? 0.020 : 0.033) * std::sqrt(double(h->dim)) + 0.2;
     auto upper_tail = [](double x) { return 0.5 * std::erfc(x * 0.70710678118654752); };
     auto quantile = [](double p) {                             // Abramowitz and Stegun 26.2.23
         const double t = std::sqrt(-2.0 * std::log(std::min(p, 0.5)));
         return t - (2.515517 + 0.802853 * t + 0.010328 * t * t) / (1.0 + 1.432788 * t + 0.189269 * t * t + 0.001308 * t * t * t);
     };
-    // the chunks of enqueue_filtered; under a mask an unknown share of the vectors counts, taken as an eighth
-    double survivors = 0.0;
-    for (double begin = 0.0, seen = std::min(double(cap), n); begin < n;) {
-        const double end = std::max(begin, seen) * 5.9 >= n ? n : std::max(begin, seen) * 4.0;   // (a short tail joins the chunk before)
-        survivors += (end - begin) * upper_tail(quantile(double(k) / (std::max(begin, seen) * (masked ? 0.125 : 1.0))) - delta);
+    // Under a mask an unknown share of the vectors counts: the threshold is taken from an eighth of them, and the rest leans to
+    // the other form, since launches weigh more the fewer blocks are live.
+    const size_t n_blocks = (h->n + kBlock - 1) / kBlock, first = std::min(n_blocks, size_t(cap) / kBlock);
+    double survivors = 0.0, fullest = 0.0;
+    for (size_t begin = 0; begin < n_blocks;) {
+        const size_t end = filter_chunk_end(begin, first, n_blocks);
+        const double seen = double(std::max(begin, first) * kBlock) * (masked ? 0.125 : 1.0);
+        const double here = double((end - begin) * kBlock) * upper_tail(quantile(double(k) / seen) - delta);
+        survivors += here;
+        fullest = std::max(fullest, here);
         begin = end;
     }
-    const double sums = n * double(nq) * 6e-7;
-    const double filter = 120.0 + bytes * 0.7e-6 * groups * (1.0 + std::min(1.0, double(cap) / n)) + sums +
-                          survivors * double(nq) * h->ngroups * 3e-6;
-    const double other = 60.0 + (plan.use_tc ? bytes * 5.3e-6 * groups + sums : bytes * 1e-6 * std::ceil(double(nq) / 4.0));
-    return other > 1.3 * filter;
+    if (plan.use_tc && !masked && fullest > 0.8 * cap) return false;
+    const double ranked = std::min(1.0, double(cap) / n);      // the first chunk is scanned twice
+    const double filter = 100.0 + filter_us(bytes * (1.0 + ranked), queries, sums) +
+                          survivors * queries * (masked ? 3e-6 * h->ngroups : 2e-4 + 1.1e-6 * h->ngroups);
+    // chunks of the one-hot form grow x6, with about 5 k candidates in each
+    const double candidates = queries * 5.0 * double(k) * std::max(0.0, std::log(n / cap) / std::log(6.0));
+    const double other = 60.0 + (!plan.use_tc ? lookup_us(bytes, queries) : one_hot_us(bytes, queries, sums) + (masked ? 0.0 : candidates * 8e-4));
+    return other > (masked ? 1.3 : 1.15) * filter;
 }
 
 // Brings the int8 copy of the index (scan_tc_dense.cu) up to date on `st`: allocates it when policy and free memory
@@ -1179,12 +1203,8 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
     TV_CUDA(launch_select(sp.cb, int(nq), uint32_t(first), m.n_live, nullptr, st));
     TV_CUDA(launch_bootstrap(sp, int(nq), st));
     h->launches += 2;
-    // every survivor costs a gather of its bytes, so the chunks grow gently: a chunk of three times the vectors seen so far
-    // brings about three times k results above the threshold and, below it, what the bound cannot tell from them
-    // (x4 / x6 / x9 / x14: 1,155 / 1,195 / 1,186 / 1,452 us for 1.2 M x 200 2-bit, batch 1,024)
-    for (size_t begin = 0, seen = first; begin < n_blocks;) {
-        size_t end = std::min(n_blocks, std::max(begin, seen) * 4);
-        if (end + end / 2 >= n_blocks) end = n_blocks;
+    for (size_t begin = 0; begin < n_blocks;) {
+        const size_t end = filter_chunk_end(begin, first, n_blocks);
         rc = scan(begin, end, S.f_max, false);
         if (rc != TV_OK) return rc;
         TV_CUDA(launch_score_survivors(sp, int(nq), h->sm_count, st));
