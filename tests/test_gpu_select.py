@@ -54,3 +54,24 @@ def test_selection_of_equal_scores(T):
     idx.add(x)
     for k in (1, 10, 500, 600):
         check(idx, pre, np.concatenate([x[:1], -x[:1], anisotropic(1, DIM, seed=9)]), k, n, 4)
+
+
+@pytest.mark.parametrize("bits,expanded", [(4, 1), (4, 0), (2, 1), (3, 1)])
+@pytest.mark.parametrize("nq", [70, 300])
+def test_batches_next_to_copies_of_a_row(T, bits, expanded, nq):
+    """Half of the rows are copies of one row, and every query lies next to it: each copy ties with the k-th result of all columns
+    of the tensor-memory scans, and the slots decide.  Some queries elsewhere, and copies with a smaller slot than a result's."""
+    n, dim = 50_003, 200
+    x = anisotropic(n, dim, seed=29)
+    x[20_000::2] = x[0]
+    x[7::5000] = x[0]
+    pre = oracle_of(x, bits)
+    idx = T.TurboQuantIndex(dim, bits)
+    idx.add(x)
+    idx.set_option(T.OPT_TC_EXPANDED, expanded)
+    idx.set_option(T.OPT_MMA_MIN_BATCH, 8)                   # (2 and 3 bits: the one-hot form)
+    q = x[:1] + np.float32(0.01) * anisotropic(nq, dim, seed=29, offset=3)
+    q[::9] = anisotropic(len(q[::9]), dim, seed=29, offset=8)
+    for k in (1, 10, 100):
+        check(idx, pre, q, k, n, bits)
+    check(idx, pre, q, 30, n, bits, np.random.default_rng(1).random(n) < 0.5)

@@ -160,6 +160,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
         WarpRing &ring = es.ring[warp - 2];
         int *nbound = es.nbound[warp - 2];
         const float *qscale = es.qscale + cbase, *qbias = es.qbias + cbase, *qthr = es.qthr + cbase;
+        const uint32_t *qslot = es.qslot + cbase;
         uint32_t local_item = 0;
         uint32_t vt = blockIdx.x / uint32_t(n_qgroups);
         int qg = int(blockIdx.x % uint32_t(n_qgroups)), qg_here = -1;
@@ -228,7 +229,7 @@ scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_sla
                             write_piece<ONEHOT>(acc, qscale + c0, qbias + c0, fused, cur[m].vs, cur[m].live, cur[m].slot, ql0 + c0, p.q_base + p.nq, at, p.cb);
                         continue;
                     }
-                    warp_sift<ONEHOT, kFilter>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, fused, cur[m].vs, cur[m].live, cur[m].slot,
+                    warp_sift<ONEHOT, kFilter>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, qslot + c0, fused, cur[m].vs, cur[m].live, cur[m].slot,
                                                ql0 + c0, ring, fill, p.cb, lane);
                 }
             }

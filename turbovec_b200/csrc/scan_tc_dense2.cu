@@ -160,6 +160,7 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
         int *nbound = es.nbound[ew];
         const int cbase = chalf * 128;                    // first of this warp's columns
         const float *qscale = es.qscale + cbase, *qbias = es.qbias + cbase, *qthr = es.qthr + cbase;
+        const uint32_t *qslot = es.qslot + cbase;
         const int row = quarter * 32 + lane;
         uint32_t local_item = 0;
         uint32_t vt = cluster_id / uint32_t(n_qgroups);
@@ -217,7 +218,7 @@ scan_tc_dense_pair_kernel(ScanParams p, const __grid_constant__ CUtensorMap amap
                         write_piece<ONEHOT>(acc, qscale + c0, qbias + c0, fused, cur.vs, cur.live, cur.slot, ql0 + c0, p.q_base + p.nq, at, p.cb);
                     continue;
                 }
-                warp_sift<ONEHOT, false>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, fused, cur.vs, cur.live, cur.slot, ql0 + c0,
+                warp_sift<ONEHOT, false>(acc, nbound + c0, qscale + c0, qbias + c0, qthr + c0, qslot + c0, fused, cur.vs, cur.live, cur.slot, ql0 + c0,
                                          ring, fill, p.cb, lane);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
