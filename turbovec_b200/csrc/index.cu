@@ -1184,7 +1184,7 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
                      const MaskOnDevice &m, const SearchOutput *out) {
     const size_t n_blocks = (h->n + kBlock - 1) / kBlock;
     const float *qscale = S.qscale, *qbias = S.qbias;
-    sp.f_weights = S.weights; sp.f_pitch = int(S.dim_pad); sp.f_alpha = S.f_alpha; sp.f_suffix = S.f_suffix;
+    sp.f_weights = S.weights; sp.f_pitch = int(S.dim_pad); sp.f_alpha = S.f_alpha; sp.f_suffix = S.f_suffix; sp.f_scale = S.f_scale;
     sp.cb.over = S.over;
     sp.give_up = uint32_t(nq / 2);                             // beyond that search_core starts the whole batch again
     auto scan = [&](size_t begin, size_t end, const float *bias, bool dense) -> int {

@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanP
 
 // topk[q] = the k best of the first chunk by approximate score -> thr[q] just above the worst of their exact keys; the
 // running top-k is empty again.  Fewer than k entries, or a k-th score that overflowed: no threshold (the filtering scans
-// take an infinite one for a column without a query, and these k vectors have yet to be found).
+// take an infinite one for a column without a query, and these k vectors have yet to be found).  A zero query ties with
+// every vector: without a mask, whose blocks come in any order, the first k are its results, and nothing more need survive.
 __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t worst[kScoreWarps];
@@ -171,6 +172,10 @@ __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) 
     uint64_t *top = p.cb.topk + size_t(q) * p.cb.k;
     const int k = p.cb.k;
     const bool full = top[k - 1] != kEmptyKey;
+    if (full && p.f_scale[q] == 0.0f && p.live_blocks == nullptr) {
+        if (threadIdx.x == 0) p.cb.thr[q] = make_key(INFINITY, 0u);
+        return;
+    }
     if (full) load_tables(p, q, reinterpret_cast<uint4 *>(smem_raw));
     __syncthreads();
     uint64_t mine = 0;

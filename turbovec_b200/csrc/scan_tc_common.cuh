@@ -431,9 +431,7 @@ __device__ __forceinline__ void warp_sift(const uint32_t (&acc)[32], const int *
             bool on = mine != 0;
             uint64_t key;
             if constexpr (RAW) {
-                const float most = score + 1.0e-5f * (fabsf(score) + fabsf(t));
-                on = on && !(most < t);                               // (an infinite score compares with nothing: kept)
-                if (on && most == t) on = slot < uint32_t(cb.thr[ql0 + c]);   // at best a tie, which the smaller slot wins
+                on = on && !(score + 1.0e-5f * (fabsf(score) + fabsf(t)) < t);   // (an infinite score compares with nothing: kept)
                 key = uint64_t(sum) << 32 | slot;
             } else {
                 on = on && score >= t;

@@ -114,7 +114,6 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *de
         if (w_scale >= FLT_MIN) w_inv = __fdiv_rn(1.0f, w_scale);
         else w_scale = 1.0f;
         alpha = __fdiv_rn(__fmul_rn(w_scale, p.level_scale), scale);
-        if (!(max_span > 0.0f)) w_inv = 0.0f;                       // a zero query: every sum is zero, and so is every weight
     }
     double beta = 0.0, slack = 0.0;
     if (tid < 32) {
@@ -191,15 +190,15 @@ __device__ void lut_tables(const QueryPrepParams &p, const float *row, float *de
         beta = slack = 0.0;
         for (int w = 0; w < kPrepThreads / 32; ++w) { beta += part[0][w]; slack += part[1][w]; }
         const double base = double(scale) * beta + double(s_bias);
-        p.filter.scale[q] = float(double(scale) * double(alpha));
+        // a scale of zero marks a zero query: its scores are all zero, and the smallest slots win (bootstrap_kernel)
+        p.filter.scale[q] = !(max_span > 0.0f) && s_bias == 0.0f ? 0.0f : fmaxf(float(double(scale) * double(alpha)), 1e-45f);
         double rest = 0.0;
         float *suffix = p.filter.suffix + size_t(q) * kFilterBatches;
         suffix[batches] = 0.0f;
         for (int b = batches - 1; b >= 0; --b) { rest += batch_sum[b]; suffix[b] = float(rest + 1e-2 + 1e-6 * fabs(rest)); }
         p.filter.alpha[q] = alpha;
         p.filter.bias_mid[q] = float(base);
-        // a zero query's bound is its exact score: all vectors tie, and only their slots decide
-        p.filter.bias_max[q] = max_span > 0.0f ? float(base + double(scale) * slack * 1.000001 + 1e-5 * fabs(double(s_bias))) : s_bias;
+        p.filter.bias_max[q] = float(base + double(scale) * slack * 1.000001 + 1e-5 * fabs(double(s_bias)));
     }
 }
 

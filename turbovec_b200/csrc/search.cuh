@@ -161,7 +161,7 @@ struct ScanParams {
     // exact scoring behind a filtering scan (QueryPrepParams::Filter)
     const int8_t *f_weights;
     int f_pitch;
-    const float *f_alpha, *f_suffix;
+    const float *f_alpha, *f_suffix, *f_scale;
     uint32_t give_up;              // a filtering scan does nothing when more queries than this have overflowed already
 };
 // Permute-dot scan on mma.sync (int8 x int8 -> int32), up to 64 queries per launch.

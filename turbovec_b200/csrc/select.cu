@@ -192,8 +192,9 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
     for (int i = tid; i < cb.k; i += kSelThreads) cb.topk[size_t(q) * cb.k + i] = i < m ? sh.sorted[i] : kEmptyKey;
     if (tid == 0) {
         // kEmptyKey until k results exist: everything still passes.  A query that the filter has lost is searched again by
-        // itself: until then nothing of it need survive.
-        if (spilled && cb.over != nullptr) cb.thr[q] = make_key(INFINITY, 0u);
+        // itself: until then nothing of it need survive, in this scan or a later one.
+        const uint64_t nothing = make_key(INFINITY, 0u);
+        if (cb.over != nullptr && (spilled || cb.thr[q] == nothing)) cb.thr[q] = nothing;
         else cb.thr[q] = m == cb.k ? sh.sorted[cb.k - 1] : kEmptyKey;
         cb.cnt[q] = 0;
     }
