@@ -195,3 +195,36 @@ def test_default_choice_on_both_sides_of_the_switch(T, n, dim, bits, nq, k, chos
     s0, i0 = idx.search(q, k)
     assert idx.get_option(T.OPT_FILTER_REDONE) == -1
     assert np.array_equal(i, i0) and np.array_equal(s, s0)
+
+
+@pytest.mark.parametrize("api", ["host", "device"])
+@pytest.mark.parametrize("n,dim,nq,share,masked", [(300_000, 200, 600, 0.01, False), (100_000, 1024, 40, 0.3, False), (300_000, 200, 600, 0.01, True)])
+def test_filter_that_does_not_pay_is_given_up(T, n, dim, nq, share, masked, api):
+    """Where all queries lie near a tight cluster, every vector of it survives the filter: the default decides that on what the
+    scans counted, keeps the results of the chunks before (some, or none in the second case) and goes on without the filter."""
+    import torch
+    k = 10
+    rng = np.random.default_rng(3)
+    x = anisotropic(n, dim, seed=97)
+    near = rng.random(n) < share
+    x[near] = x[0] + np.float32(1e-3) * x[near]
+    idx, pre = built(T, x, 2)
+    idx.set_option(T.OPT_FILTER, 1)
+    q = x[:1] + np.float32(0.01) * anisotropic(nq, dim, seed=97, offset=5)
+    q[1] = 0.0
+    mask = rng.random(n) < 0.9 if masked else None
+    want = O.search(q, pre[0], pre[1], n, dim, 2, k, mask_words=None if mask is None else O.pack_mask(mask))
+    if api == "host":
+        s, i = idx.search(q, k, mask=mask)
+    else:
+        words = 0 if mask is None else torch.from_numpy(O.pack_mask(mask).view(np.int64)).cuda()
+        dq, ds = torch.from_numpy(q).cuda(), torch.empty((nq, k), device="cuda")
+        di = torch.empty((nq, k), dtype=torch.int64, device="cuda")
+        assert idx.search_device(dq.data_ptr(), nq, k, ds.data_ptr(), di.data_ptr(), 0 if mask is None else words.data_ptr()) == k
+        s, i = ds.cpu().numpy(), di.cpu().numpy()
+    assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])
+    if not masked:
+        assert idx.get_option(T.OPT_FILTER_REDONE) > 0
+    s, i = idx.search(anisotropic(9, dim, seed=97, offset=11), k)
+    want = O.search(anisotropic(9, dim, seed=97, offset=11), pre[0], pre[1], n, dim, 2, k)
+    assert np.array_equal(i, want[1]) and np.array_equal(s, want[0])

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <cmath>
 #include <condition_variable>
 #include <cstdio>
@@ -1086,8 +1087,18 @@ size_t filter_chunk_end(size_t begin, size_t first, size_t n_blocks) {
 // 1 M x 768 3-bit, 1,024 3,447 / 7,716, 512 with k = 100 7,442 / 4,561; 1.2 M x 200 2-bit, 1,024 with k = 100 2,485 / 3,497;
 // 100 k x 3072, 64 295 / 491, 512 1,730 / 1,148; 100 k x 768 3-bit, 512 682 / 673.  At 142 other points the choice was never the
 // slower one by more than 1 %; at 15 it left the faster one, mostly small indexes (30 k x 768 3-bit, 300, k = 1: 159 / 302).
+// Survivors per query that a scan of `vectors` is expected to let through, with the k-th best of `seen` as the threshold.
+double expected_survivors(const tv_index *h, double k, double seen, double vectors) {
+    const double delta = (h->bits == 2 ? 0.020 : 0.033) * std::sqrt(double(h->dim)) + 0.2;
+    // Q^-1: Abramowitz and Stegun 26.2.23
+    const double t = std::sqrt(-2.0 * std::log(std::min(k / seen, 0.5)));
+    const double z = t - (2.515517 + 0.802853 * t + 0.010328 * t * t) / (1.0 + 1.432788 * t + 0.189269 * t * t + 0.001308 * t * t * t);
+    return vectors * 0.5 * std::erfc((z - delta) * 0.70710678118654752);
+}
 double one_hot_us(double bytes, double queries, double sums) { return bytes * 4.5e-6 * std::ceil(queries / 256.0) + sums * 5e-7; }
 double filter_us(double bytes, double queries, double sums) { return bytes * 0.65e-6 * std::ceil(queries / 256.0) + sums * 5e-7; }
+// (the chunks of the one-hot form grow x6, with about 5 k candidates in each)
+double one_hot_candidates_us(double queries, double k, double n, double cap) { return queries * 5.0 * k * std::max(0.0, std::log(n / cap) / std::log(6.0)) * 8e-4; }
 double lookup_us(double bytes, double queries) { return bytes * 1e-6 * std::ceil(queries / 4.0); }
 bool wants_filter(const tv_index *h, int mode, size_t nq, size_t k, int cap, bool masked, const ScanPlan &plan) {
     if (!scan_filter_supported(h->bits, mode, h->ngroups, h->smem_limit) || h->filter == 0 || h->mma_min_batch == 0) return false;
@@ -1095,20 +1106,13 @@ bool wants_filter(const tv_index *h, int mode, size_t nq, size_t k, int cap, boo
     if (h->mma_min_batch > 0) return false;                    // the caller asked for the one-hot form
     if (!plan.use_tc && nq < 8) return false;                  // (flush geometries beyond 256 groups have no one-hot form)
     const double n = double(h->n), queries = double(nq), bytes = n * h->ngroups, sums = n * queries;
-    const double delta = (h->bits == 2 ? 0.020 : 0.033) * std::sqrt(double(h->dim)) + 0.2;
-    auto upper_tail = [](double x) { return 0.5 * std::erfc(x * 0.70710678118654752); };
-    auto quantile = [](double p) {                             // Abramowitz and Stegun 26.2.23
-        const double t = std::sqrt(-2.0 * std::log(std::min(p, 0.5)));
-        return t - (2.515517 + 0.802853 * t + 0.010328 * t * t) / (1.0 + 1.432788 * t + 0.189269 * t * t + 0.001308 * t * t * t);
-    };
     // Under a mask an unknown share of the vectors counts: the threshold is taken from an eighth of them, and the rest leans to
     // the other form, since launches weigh more the fewer blocks are live.
     const size_t n_blocks = (h->n + kBlock - 1) / kBlock, first = std::min(n_blocks, size_t(cap) / kBlock);
     double survivors = 0.0, fullest = 0.0;
     for (size_t begin = 0; begin < n_blocks;) {
         const size_t end = filter_chunk_end(begin, first, n_blocks);
-        const double seen = double(std::max(begin, first) * kBlock) * (masked ? 0.125 : 1.0);
-        const double here = double((end - begin) * kBlock) * upper_tail(quantile(double(k) / seen) - delta);
+        const double here = expected_survivors(h, double(k), double(std::max(begin, first) * kBlock) * (masked ? 0.125 : 1.0), double((end - begin) * kBlock));
         survivors += here;
         fullest = std::max(fullest, here);
         begin = end;
@@ -1117,9 +1121,8 @@ bool wants_filter(const tv_index *h, int mode, size_t nq, size_t k, int cap, boo
     const double ranked = std::min(1.0, double(cap) / n);      // the first chunk is scanned twice
     const double filter = 100.0 + filter_us(bytes * (1.0 + ranked), queries, sums) +
                           survivors * queries * (masked ? 3e-6 * h->ngroups : 2e-4 + 1.1e-6 * h->ngroups);
-    // chunks of the one-hot form grow x6, with about 5 k candidates in each
-    const double candidates = queries * 5.0 * double(k) * std::max(0.0, std::log(n / cap) / std::log(6.0));
-    const double other = 60.0 + (!plan.use_tc ? lookup_us(bytes, queries) : one_hot_us(bytes, queries, sums) + (masked ? 0.0 : candidates * 8e-4));
+    const double candidates = masked ? 0.0 : one_hot_candidates_us(queries, double(k), n, cap);
+    const double other = 60.0 + (plan.use_tc ? one_hot_us(bytes, queries, sums) + candidates : lookup_us(bytes, queries));
     return other > (masked ? 1.3 : 1.15) * filter;
 }
 
@@ -1180,13 +1183,23 @@ int expanded_sync(tv_index *h, cudaStream_t st, const uint32_t level_words[4], b
 
 // One search through the filtering scan: the first chunk by approximate score, a threshold from its k best, then the whole
 // index in chunks that append survivors, which are scored exactly and selected.
-int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, ScanParams sp, size_t nq, size_t kk,
+int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, const ScanPlan &plan, ScanParams sp, size_t nq,
                      const MaskOnDevice &m, const SearchOutput *out) {
     const size_t n_blocks = (h->n + kBlock - 1) / kBlock;
     const float *qscale = S.qscale, *qbias = S.qbias;
     sp.f_weights = S.weights; sp.f_pitch = int(S.dim_pad); sp.f_alpha = S.f_alpha; sp.f_suffix = S.f_suffix; sp.f_scale = S.f_scale;
     sp.cb.over = S.over;
     sp.give_up = uint32_t(nq / 2);                             // beyond that search_core starts the whole batch again
+    // what the scoring weighs its survivors against; one that never leaves early costs 3.2e-6 us a byte-group, the others about
+    // a third of it
+    const double bytes = double(n_blocks) * kBlock * h->ngroups, sums = double(n_blocks) * kBlock * double(nq);
+    const bool always = h->filter == 2;
+    sp.f_positions = uint32_t(n_blocks);
+    sp.f_mid = S.f_mid; sp.f_max = S.f_max;
+    sp.f_tally = reinterpret_cast<float *>(S.over + nq + 1);
+    sp.f_survivor_us = float(2e-4 + 2e-6 * h->ngroups);
+    sp.f_redo_us = float(lookup_us(bytes, 1.0));
+    sp.f_redo_group_us = float(plan.use_tc ? one_hot_us(bytes, 1.0, 0.0) : 64.0 * lookup_us(bytes, 1.0));
     auto scan = [&](size_t begin, size_t end, const float *bias, bool dense) -> int {
         sp.pos_begin = uint32_t(begin); sp.pos_end = uint32_t(end); sp.dense = dense ? 1 : 0;
         sp.qscale = S.f_scale; sp.qbias = bias; sp.q_base = 0; sp.nq = int(nq);
@@ -1201,12 +1214,31 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
     int rc = scan(0, first, S.f_mid, true);
     if (rc != TV_OK) return rc;
     TV_CUDA(launch_select(sp.cb, int(nq), uint32_t(first), m.n_live, nullptr, st));
+    auto set_budget = [&](size_t begin, size_t end) {          // for the scan of [begin, end)
+        const double rest = double(n_blocks - begin) / double(n_blocks), after = double(n_blocks - end) / double(n_blocks);
+        const double other = plan.use_tc ? one_hot_us(bytes * rest, double(nq), sums * rest) + one_hot_candidates_us(double(nq), sp.cb.k, double(h->n), S.cap) * rest
+                                         : lookup_us(bytes * rest, double(nq));
+        sp.f_budget_us = always ? FLT_MAX : float(other - filter_us(bytes * after, double(nq), sums * after));
+        sp.f_scan_us = float(filter_us(bytes * (rest - after), double(nq), sums * (rest - after)));
+        sp.f_chunks = 1.0f;
+        for (size_t b = end; b < n_blocks; b = filter_chunk_end(b, first, n_blocks)) sp.f_chunks += 1.0f;
+    };
+    set_budget(0, filter_chunk_end(0, first, n_blocks));
+    // The estimate from the first chunk and the count of the survivors take a few us each: not for a scan of little of the index.
+    auto is_small = [&](size_t begin, size_t end) { return (end - begin) * 16 < n_blocks; };
+    if (is_small(0, filter_chunk_end(0, first, n_blocks))) sp.f_budget_us = FLT_MAX;
+    sp.f_ahead = uint32_t(std::min(h->n, filter_chunk_end(0, first, n_blocks) * kBlock));
     TV_CUDA(launch_bootstrap(sp, int(nq), st));
     h->launches += 2;
     for (size_t begin = 0; begin < n_blocks;) {
         const size_t end = filter_chunk_end(begin, first, n_blocks);
+        set_budget(begin, end);
+        if (is_small(begin, end)) sp.f_budget_us = FLT_MAX;
         rc = scan(begin, end, S.f_max, false);
         if (rc != TV_OK) return rc;
+        // many times the survivors to be expected: not a hard query (those reach about six times) but copies of a result
+        sp.cb.unusual = float(16.0 * expected_survivors(h, sp.cb.k, double(std::max(begin, first) * kBlock) * (m.words ? 0.125 : 1.0), double((end - begin) * kBlock)));
+        sp.cb.ahead = always || end == n_blocks ? 0.0f : float(double(filter_chunk_end(end, first, n_blocks) - end) / double(end - begin));
         TV_CUDA(launch_score_survivors(sp, int(nq), h->sm_count, st));
         TV_CUDA(launch_select(sp.cb, int(nq), 0u, nullptr, end == n_blocks ? out : nullptr, st));
         h->launches += 2;
@@ -1219,9 +1251,10 @@ int enqueue_filtered(tv_index *h, cudaStream_t st, Marks *marks, const SearchScr
 //   careful: chunks never exceed the candidate capacity, so no list can overflow whatever the data order.
 //   fresh: the selection state is as query preparation left it.
 //   out: what the last selection finishes the search with, or nullptr.
+//   from: > 0: the blocks before it have been searched, and the selection state holds their results.
 int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScratch &S, const ScanPlan &plan, int mode,
                    size_t nq, size_t kk, const MaskOnDevice &m, uint32_t *d_overflow, uint32_t *d_error, bool careful, bool fresh,
-                   const SearchOutput *out) {
+                   const SearchOutput *out, size_t from = 0) {
     const size_t n = h->n;
     const int ng = h->ngroups;
     const size_t n_blocks = (n + kBlock - 1) / kBlock;
@@ -1241,8 +1274,8 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
         if (rc != TV_OK) return rc;
     }
 
-    if (plan.use_filter) return enqueue_filtered(h, st, marks, S, sp, nq, kk, m, out);
-    if (!fresh) {
+    if (plan.use_filter) return enqueue_filtered(h, st, marks, S, plan, sp, nq, m, out);
+    if (!fresh && from == 0) {
         TV_CUDA(cudaMemsetAsync(S.cnt, 0, (2 * nq + 1) * 4, st));
         TV_CUDA(cudaMemsetAsync(S.thr, 0xff, nq * 8, st));
         TV_CUDA(cudaMemsetAsync(S.topk, 0xff, nq * kk * 8, st));
@@ -1254,8 +1287,8 @@ int enqueue_search(tv_index *h, cudaStream_t st, Marks *marks, const SearchScrat
     // 367 / 345 / 350 / 358 us on 1.2 M x 200, batch 100), then by the list-capacity rule.
     const size_t first = size_t(S.cap) / kBlock;
     const double growth = std::max(0.5, double(S.cap) / (4.0 * double(kk)));
-    size_t begin = 0;
-    int stage = 0;
+    size_t begin = from;
+    int stage = from == 0 ? 0 : 1;
     while (begin < n_blocks) {
         size_t len = first;
         if (!careful && begin > 0) {
@@ -1408,6 +1441,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
     const size_t dim_pad = (dim + 127) / 128 * 128;
     const int ksteps = (ng + 15) / 16;
     const size_t lut_pitch = size_t((ng + 3) / 4 * 4) * 32;
+    const size_t n_blocks = (n + kBlock - 1) / kBlock;
 
     ScanPlan plan;
     int rc = plan_scan(h, mode, nq, pages == 1, plan);
@@ -1418,8 +1452,9 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
 
     // ---- buffers ----
     TV_CUDA(injected_failure(h));
-    // A few queries are read by the preparation kernel straight from page-locked memory (48 KB: 2 us at the bus's rate),
-    // which saves a copy of about 10 us; more of them go through the copy engine.
+    // A few queries are read by the preparation kernel straight from page-locked memory, which saves a copy: rows of 256
+    // coordinates 68 against 77 us a call at 3 KB, 87 / 107 at 48 KB, 98 / 117 at 96 KB, 118 / 123 at 192 KB, 162 / 146 at
+    // 384 KB; rows of 1,536 within 3 us of each other up to 192 KB.
     const bool small_upload = !queries_on_device && nq * dim * 4 <= (size_t(48) << 10);
     if (small_upload) TV_CUDA(c.h_queries.reserve(size_t(12) << 10));
     else if (!queries_on_device) TV_CUDA(c.d_stage.reserve(nq * dim));
@@ -1434,7 +1469,7 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         TV_CUDA(c.d_luts.reserve(w_rows * lut_pitch));           // padded to whole query groups and whole K slabs for the tensor path
     }
     TV_CUDA(c.d_cand.reserve(nq * size_t(cap)));
-    TV_CUDA(c.d_cnt.reserve(3 * nq + 1));                        // candidate counts, then the selection's part counters, then the count of finished queries, then overflow marks
+    TV_CUDA(c.d_cnt.reserve(3 * nq + 5));                        // candidate counts, then the selection's part counters, then the count of finished queries, then overflow marks, where a filter stopped and its tally
     TV_CUDA(c.d_thr.reserve(nq));
     TV_CUDA(c.d_topk.reserve(nq * k_page));
     if (pages > 1) {
@@ -1541,10 +1576,6 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         TV_CUDA(c.d_redo_queries.reserve(count * dim));
         TV_CUDA(c.d_redo_who.reserve(count));
         TV_CUDA(c.d_redo_topk.reserve(count * kk));
-        if (!out_scores_dev && !out_keys_dev) {
-            TV_CUDA(c.d_scores.reserve(nq * kk));
-            TV_CUDA(c.d_slots.reserve(nq * kk));
-        }
         R.cand = c.d_cand.ptr; R.topk = c.d_redo_topk.ptr; R.done = R.cnt + count; R.over = nullptr; R.w_rows = (count + 255) / 256 * 256;
         TV_CUDA(cudaMemcpyAsync(c.d_redo_who.ptr, who.data(), count * 4, cudaMemcpyHostToDevice, st));   // pageable: staged before the call returns
         TV_CUDA(launch_gather_rows(dq, c.d_redo_who.ptr, int(count), int(dim), c.d_redo_queries.ptr, st));
@@ -1563,7 +1594,15 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
         }
         if (rc != TV_OK) return rc;
         TV_CUDA(launch_scatter_rows(c.d_redo_topk.ptr, c.d_redo_who.ptr, int(count), int(kk), c.d_topk.ptr, st));
-        fused = false;                                         // the rows are decoded from d_topk
+        return TV_OK;
+    };
+    // decodes the rows from d_topk
+    auto finish_apart = [&]() -> int {
+        if (!out_scores_dev && !out_keys_dev) {
+            TV_CUDA(c.d_scores.reserve(nq * kk));
+            TV_CUDA(c.d_slots.reserve(nq * kk));
+        }
+        fused = false;
         return finish();
     };
     for (size_t page = 0; page < pages; ++page) {
@@ -1589,22 +1628,37 @@ int search_core(tv_index *h, SearchCtx &c, const float *queries, bool queries_on
             if (rc != TV_OK) { c.marks.used = 0; return rc; }
             if (!c.h_flags->overflow) break;
             if (careful) return fail(h, TV_ERR_CUDA, "candidate overflow in the bounded schedule (internal error)");
-            // A chunk produced more candidates than the buffer holds.  Behind a filter that is a matter of single queries (more
-            // vectors tie with their k-th result, or come closer than the bound can tell, than a list holds): those are searched
-            // again without it, or the whole batch when they are most of it.  Without a filter: again with bounded chunks.
+            // A chunk produced more candidates than the buffer holds: again with bounded chunks.
             TV_CUDA(cudaMemsetAsync(&c.d_flags->overflow, 0, 4, st));
             if (!plan.use_filter) { attempt = 1; continue; }
+            // Behind a filter that is a matter of single queries (more vectors tie with their k-th result, or come closer than
+            // the bound can tell, than a list holds): those are searched again without it, or the whole batch when they are
+            // most of it.  Or the filter was given up on the way: the rest is searched without it.
             plan.use_filter = false;
-            std::vector<uint32_t> over(nq), who;
-            TV_CUDA(cudaMemcpyAsync(over.data(), S.over, nq * 4, cudaMemcpyDeviceToHost, st));
+            std::vector<uint32_t> over(nq + 1), who;
+            TV_CUDA(cudaMemcpyAsync(over.data(), S.over, over.size() * 4, cudaMemcpyDeviceToHost, st));
             TV_CUDA(cudaStreamSynchronize(st));
             for (size_t q = 0; q < nq; ++q) if (over[q]) who.push_back(uint32_t(q));
-            redone = int64_t(who.size() <= nq / 2 ? who.size() : nq);
-            if (who.size() <= nq / 2) {
-                rc = redo(who);
+            const size_t from = over[nq] ? over[nq] - 1 : n_blocks;
+            redone = int64_t(from < n_blocks || who.size() > nq / 2 ? nq : who.size());
+            if (from == 0 || who.size() > nq / 2) continue;    // nothing to keep
+            if (from < n_blocks) {
+                rc = enqueue_search(h, st, &c.marks, S, plan, mode, nq, kk, m, &c.d_flags->overflow, &c.d_flags->error, false, false, nullptr, from);
                 if (rc != TV_OK) { c.marks.used = 0; return rc; }
-                break;
+                TV_CUDA(cudaMemcpyAsync(c.h_flags, c.d_flags, sizeof(DeviceFlags), cudaMemcpyDeviceToHost, st));
+                TV_CUDA(cudaStreamSynchronize(st));
+                rc = check_flags(h, c.h_flags, queries, queries_on_device, st);
+                if (rc != TV_OK) { c.marks.used = 0; return rc; }
+                if (c.h_flags->overflow) {
+                    TV_CUDA(cudaMemsetAsync(&c.d_flags->overflow, 0, 4, st));
+                    attempt = 1;
+                    continue;
+                }
             }
+            if (!who.empty()) rc = redo(who);
+            if (rc == TV_OK) rc = finish_apart();
+            if (rc != TV_OK) { c.marks.used = 0; return rc; }
+            break;
         }
         if (pages > 1) {
             // this page's keys into their columns of the full rows; its last key bounds the next page from below

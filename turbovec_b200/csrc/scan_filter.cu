@@ -30,6 +30,7 @@ namespace {
 constexpr int kScoreThreads = 256;
 constexpr int kScoreWarps = kScoreThreads / 32;
 constexpr int kTogether = 4;               // survivors per warp and step
+constexpr int kSample = 1024;              // vectors of the first chunk by which the next scan's survivors are estimated
 
 // The exact keys of up to kTogether slots, valid in every lane.  EXIT: `sum` = W . L of each; a survivor that drops out on
 // the way gets kEmptyKey.
@@ -134,8 +135,33 @@ __device__ __forceinline__ void load_weights(const ScanParams &p, int q, uint32_
     }
 }
 
+// Whether scoring this chunk's survivors, and redoing the queries whose lists overflowed, would take longer than the form
+// without the filter saves from here on (filter_hopeless).  How many survive depends on the data (copies and tight clusters near the k-th
+// result all do) and is known only now; a scan without its scoring costs a seventh of the other form, so giving up here
+// costs little, and the results of the chunks before stay.  By the whole block.
+__device__ bool not_worth_while(const ScanParams &p, const uint32_t *all_cnt, int all_queries) {
+    __shared__ float part[2][kScoreWarps];
+    if (p.f_budget_us >= FLT_MAX) return false;
+    float scored = 0.0f, lost = 0.0f;
+    for (int i = threadIdx.x; i < all_queries; i += kScoreThreads) {
+        const uint32_t c = all_cnt[i];
+        if (c > uint32_t(p.cb.cap)) lost += 1.0f;
+        else scored += float(c);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        scored += __shfl_xor_sync(kFullMask, scored, o);
+        lost += __shfl_xor_sync(kFullMask, lost, o);
+    }
+    if ((threadIdx.x & 31) == 0) { part[0][threadIdx.x >> 5] = scored; part[1][threadIdx.x >> 5] = lost; }
+    __syncthreads();
+    scored = lost = 0.0f;
+    for (int w = 0; w < kScoreWarps; ++w) { scored += part[0][w]; lost += part[1][w]; }
+    return filter_hopeless(p, scored, lost, all_queries, 0.0f);
+}
+
 // cand[q][i] = (W . L, slot) -> exact key, or kEmptyKey when it does not beat the k-th best.  Grid (shares of a list, queries).
-__global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanParams p) {
+// A list that overflowed is left alone: its query is searched again.
+__global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanParams p, const uint32_t *all_cnt, int all_queries, uint32_t *stopped_at) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t *wq = reinterpret_cast<uint32_t *>(smem_raw + size_t(p.ngroups) * 32);
     const int q = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -143,7 +169,12 @@ __global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanP
     if (blockIdx.x * kScoreWarps * kTogether >= n) return;
     load_tables(p, q, reinterpret_cast<uint4 *>(smem_raw));
     load_weights(p, q, wq);
+    if (not_worth_while(p, all_cnt, all_queries)) {       // the same outcome in every block
+        if (threadIdx.x == 0) { *stopped_at = p.pos_begin + 1u; atomicOr(p.cb.overflow, kFilterStopped); }
+        return;
+    }
     __syncthreads();
+    if (p.cb.cnt[q] > uint32_t(p.cb.cap)) return;
     uint64_t *list = p.cb.cand + size_t(q) * p.cb.cap;
     const uint64_t thr = p.cb.thr[q];
     for (uint32_t i = (blockIdx.x * kScoreWarps + warp) * kTogether; i < n; i += gridDim.x * kScoreWarps * kTogether) {
@@ -165,7 +196,7 @@ __global__ void __launch_bounds__(kScoreThreads, 3) score_survivors_kernel(ScanP
 // running top-k is empty again.  Fewer than k entries, or a k-th score that overflowed: no threshold (the filtering scans
 // take an infinite one for a column without a query, and these k vectors have yet to be found).  A zero query ties with
 // every vector: without a mask, whose blocks come in any order, the first k are its results, and nothing more need survive.
-__global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) {
+__device__ void bootstrap_query(const ScanParams &p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t worst[kScoreWarps];
     const int q = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -193,7 +224,62 @@ __global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) 
     for (int i = threadIdx.x; i < k; i += kScoreThreads) top[i] = kEmptyKey;
     if (threadIdx.x == 0) {
         for (int w = 0; w < kScoreWarps; ++w) mine = max(mine, worst[w]);
-        p.cb.thr[q] = full && fabsf(desc_bits_to_score(uint32_t(mine >> 32))) <= FLT_MAX ? mine + 1 : kEmptyKey;
+        worst[0] = full && fabsf(desc_bits_to_score(uint32_t(mine >> 32))) <= FLT_MAX ? mine + 1 : kEmptyKey;
+        p.cb.thr[q] = worst[0];
+    }
+    if (p.f_budget_us >= FLT_MAX || !full) return;
+    // How many vectors will the first filtering scan let through?  As large a share as of the first chunk, which the list
+    // still holds: 1,024 of its vectors say it (without the places where the selection left the best of a segment).
+    __syncthreads();
+    const uint64_t thr = worst[0];
+    if (thr == kEmptyKey) return;
+    const float t = desc_bits_to_score(uint32_t(thr >> 32)), slack = p.f_max[q] - p.f_mid[q];
+    const uint64_t *list = p.cb.cand + size_t(q) * p.cb.cap;
+    uint32_t len = p.pos_end - p.pos_begin;
+    if (p.live_blocks != nullptr) len = min(len, *p.n_live);
+    len *= 32u;
+    int seen = 0, through = 0;
+#pragma unroll
+    for (int i = 0; i < kSample / kScoreThreads; ++i) {
+        const uint32_t at = uint32_t(uint64_t(i * kScoreThreads + threadIdx.x) * len / kSample);
+        if (at >= len || (len > uint32_t(kSelectSegment) && (at & uint32_t(kSelectSegment - 1)) < uint32_t(kSelectMaxK))) continue;
+        const uint64_t key = list[at];
+        ++seen;
+        if (key == kEmptyKey) continue;
+        const float most = desc_bits_to_score(uint32_t(key >> 32)) + slack * p.vec_scales[uint32_t(key)];
+        through += !(most < t);
+    }
+    seen = __reduce_add_sync(kFullMask, seen);
+    through = __reduce_add_sync(kFullMask, through);
+    __syncthreads();
+    if (lane == 0) worst[warp] = uint64_t(uint32_t(seen)) << 32 | uint32_t(through);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    uint64_t both = 0;
+    for (int w = 0; w < kScoreWarps; ++w) both += worst[w];
+    const float share = float(uint32_t(both)) / fmaxf(float(uint32_t(both >> 32)), 1.0f);
+    const float expected = share * (p.live_blocks != nullptr ? fminf(float(p.f_ahead), float(*p.n_live) * 32.0f) : float(p.f_ahead));
+    if (expected > float(p.cb.cap)) {                     // as a list that has overflowed
+        atomicAdd(p.f_tally + 1, 1.0f);
+        p.cb.over[q] = 1u;
+        atomicAdd(p.cb.overflow, 1u);
+        p.cb.thr[q] = make_key(INFINITY, 0u);
+    } else {
+        atomicAdd(p.f_tally, expected);
+    }
+}
+
+__global__ void __launch_bounds__(kScoreThreads) bootstrap_kernel(ScanParams p) {
+    bootstrap_query(p);
+    if (p.f_budget_us >= FLT_MAX || threadIdx.x != 0) return;
+    // the block that ends last knows what all queries expect, and whether the filter is worth beginning
+    __threadfence();
+    if (atomicAdd(reinterpret_cast<uint32_t *>(p.f_tally + 2), 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    const volatile float *tally = p.f_tally;
+    if (filter_hopeless(p, tally[0], tally[1], int(gridDim.x), p.f_scan_us)) {
+        p.cb.over[gridDim.x] = 1u;                        // given up at position 0
+        atomicOr(p.cb.overflow, kFilterStopped);
     }
 }
 
@@ -205,7 +291,7 @@ bool scan_filter_supported(int bits, int mode, int ngroups, size_t smem_limit) {
 
 cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cudaStream_t s) {
     const size_t smem = size_t(p.ngroups) * 36;
-    cudaError_t e = allow_dynamic_shared(score_survivors_kernel);
+    cudaError_t e = allow_dynamic_shared(score_survivors_kernel, 1024);
     if (e != cudaSuccess) return e;
     for (int q0 = 0; q0 < nq; q0 += 32768) {
         const int here = std::min(nq - q0, 32768);
@@ -215,7 +301,7 @@ cudaError_t launch_score_survivors(const ScanParams &p, int nq, int sm_count, cu
         part.f_alpha += q0; part.f_suffix += size_t(q0) * kFilterBatches; part.f_weights += size_t(q0) * p.f_pitch;
         // about eight CTAs per SM over all queries, at least one per query, none without a first step of its own
         const unsigned shares = unsigned(std::max(1, std::min(8 * sm_count / here, p.cb.cap / (kScoreWarps * kTogether))));
-        score_survivors_kernel<<<dim3(shares, unsigned(here)), kScoreThreads, smem, s>>>(part);
+        score_survivors_kernel<<<dim3(shares, unsigned(here)), kScoreThreads, smem, s>>>(part, p.cb.cnt, nq, p.cb.over + nq);
     }
     return cudaGetLastError();
 }

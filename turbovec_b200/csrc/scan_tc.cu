@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1)
 scan_tc_kernel(ScanParams p, const __grid_constant__ CUtensorMap wmap, int n_slabs, int n_qgroups) {
     constexpr bool ONEHOT = KIND == kOneHot;
     constexpr bool kFilter = KIND == kLevels2 || KIND == kLevels3;
-    if (kFilter && *p.cb.overflow > p.give_up) return;        // (written by the selections between the scans, never during one)
+    if (kFilter && !p.dense && *p.cb.overflow > p.give_up) return;        // (written by the kernels between the scans, never during one)
     constexpr int kStages = MT == 1 ? 4 : 3;
     constexpr int kABytes = MT * kATileBytes;
     constexpr int kBBytes = NQT * kSlabK;                     // 32 KB at 256 columns

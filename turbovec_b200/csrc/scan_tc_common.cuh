@@ -276,6 +276,19 @@ __device__ __forceinline__ void sift_piece(const uint32_t (&acc)[32], const int 
     }
 }
 
+// Whether `scored` survivors of a filtering scan in the average chunk to come, and redoing `lost` queries whose lists overflow,
+// would take longer than the form without the filter saves from here on (`spent`: what the filter still has to spend before).
+__device__ __forceinline__ bool filter_hopeless(const ScanParams &p, float scored, float lost, int all_queries, float spent) {
+    float budget = p.f_budget_us - spent;
+    if (p.live_blocks != nullptr) {                       // the share of the positions that a mask leaves
+        const uint32_t live = *p.n_live;
+        budget *= float(live > p.pos_begin ? live - p.pos_begin : 0u) / float(p.f_positions - p.pos_begin);
+    }
+    if (lost > 0.5f * float(all_queries)) return true;    // most of the batch would be searched again
+    const float redo = lost <= 0.0f ? 0.0f : lost < 8.0f ? p.f_redo_us * ceilf(lost * 0.25f) : p.f_redo_group_us * ceilf(lost * (1.0f / 256.0f));
+    return scored * p.f_survivor_us * p.f_chunks + redo > budget + 60.0f;   // (60 us: the host's turn and a restart)
+}
+
 // ---- epilogue of scan_tc.cu and scan_tc_dense2.cu: every warp on its own ------------------------------------------
 // An item with few K slabs leaves the epilogue about a thousand cycles, so it must not be a chain of barriers and
 // dependent loads.  The query group of a CTA stays the same from item to item, so the parameters of its columns are read

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kPrepThreads) query_prep_kernel(QueryPrepParam
         return;
     }
     if (p.cnt != nullptr) {
-        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; if (p.over != nullptr) p.over[q] = 0; if (q == 0) p.done[p.nq] = 0; }
+        if (tid == 0) { p.cnt[q] = 0; p.done[q] = 0; p.thr[q] = kEmptyKey; if (p.over != nullptr) { p.over[q] = 0; if (q == 0) { p.over[p.nq] = 0; p.over[p.nq + 1] = 0; p.over[p.nq + 2] = 0; p.over[p.nq + 3] = 0; } } if (q == 0) p.done[p.nq] = 0; }
         for (int i = tid; i < p.k; i += kPrepThreads) p.topk[size_t(q) * p.k + i] = kEmptyKey;
     }
     const float *src = p.queries + size_t(q) * dim;

@@ -13,6 +13,8 @@ enum ScoreMode : int { kModePermuteDot = 1, kModeLutMulAdd = 2, kModeLutFlush = 
 // Batches of byte-groups after which the exact scoring of a filtering scan's survivors looks at the bound again; together
 // they cover every geometry whose tables fit in shared memory.
 constexpr int kFilterBatch = 128, kFilterBatches = 66;
+// Set in the overflow word when a filtering search was given up: no later kernel of it does anything.
+constexpr uint32_t kFilterStopped = 1u << 30;
 
 struct QueryPrepParams {
     const float *queries;          // [nq][dim] device
@@ -47,7 +49,7 @@ struct QueryPrepParams {
     } filter;
     // selection state of the batch, reset here (cnt == nullptr: none)
     uint32_t *cnt, *done;          // done[nq] = SearchOutput::finished
-    uint32_t *over;                // or nullptr
+    uint32_t *over;                // [nq + 4], or nullptr
     uint64_t *thr, *topk;
     int k;
     int mtiles_total;              // ceil(nq / 16)
@@ -97,7 +99,12 @@ struct CandidateBuffers {
     uint32_t *overflow;
     uint32_t *error;               // device-side wait timeouts
     uint32_t *done;                // per query: parts of a long list selected so far (zero between launches)
-    uint32_t *over;                // filtering scans: per query whether a list of it overflowed, *overflow counts them; else nullptr
+    uint32_t *over;                // filtering scans: per query whether a list of it overflowed, *overflow counts them, and
+                                   // over[all queries] = the position where the filter was given up, plus 1, followed by
+                                   // three words of ScanParams::f_tally; else nullptr
+    // with `over`: a list longer than `unusual` is taken to grow in proportion to the vectors of a scan, and the next scan has
+    // `ahead` times as many (0: no next scan)
+    float unusual, ahead;
     int cap, k;
 };
 // Selection (select.cu).  dense_blocks > 0: the scan wrote 32 keys for each of the first min(dense_blocks, *n_live)
@@ -163,6 +170,15 @@ struct ScanParams {
     int f_pitch;
     const float *f_alpha, *f_suffix, *f_scale;
     uint32_t give_up;              // a filtering scan does nothing when more queries than this have overflowed already
+    // Times (us) by which the scoring decides whether it is worth while: per survivor, for redoing up to 4 queries and per 256
+    // queries, what the form without the filter saves on the positions from pos_begin on, and how often such a chunk follows.
+    float f_survivor_us, f_redo_us, f_redo_group_us, f_budget_us, f_chunks;
+    uint32_t f_positions;          // positions of the whole search
+    const float *f_mid, *f_max;    // the two biases of the affine bound
+    float *f_tally;                // survivors that the first filtering scan can expect, queries whose lists it would fill, and (a
+                                   // counter) the queries that have been looked at
+    float f_scan_us;               // the filtering scan to come
+    uint32_t f_ahead;              // vectors of the first filtering scan
 };
 // Permute-dot scan on mma.sync (int8 x int8 -> int32), up to 64 queries per launch.
 cudaError_t launch_scan_pd(const ScanParams &p, int sm_count, cudaStream_t s);

@@ -152,10 +152,13 @@ __global__ void __launch_bounds__(kSelThreads) select_parts_kernel(CandidateBuff
     uint32_t raw;
     if (dense_blocks > 0) raw = (n_live ? min(dense_blocks, *n_live) : dense_blocks) * 32u;
     else raw = *reinterpret_cast<volatile uint32_t *>(&cb.cnt[q]);
+    // a filtering search that was given up: these survivors were not scored, and what was found before them stands
+    if (cb.over != nullptr && (*reinterpret_cast<volatile uint32_t *>(cb.overflow) & kFilterStopped) != 0u) raw = 0;
     const uint32_t ncand = min(raw, uint32_t(cb.cap));
     const uint32_t parts = max(1u, (ncand + kSelectSegment - 1) / kSelectSegment);
     if (part >= parts) return;                                          // (a late CTA may see the count already cleared: same outcome)
-    const bool spilled = raw > uint32_t(cb.cap);
+    // a list that the next scan is bound to fill need not be begun there: its query is searched by itself either way
+    const bool spilled = raw > uint32_t(cb.cap) || (cb.over != nullptr && float(raw) > cb.unusual && float(raw) * cb.ahead > float(cb.cap));
     if (part == 0 && tid == 0 && spilled && (cb.over == nullptr || atomicExch(&cb.over[q], 1u) == 0u)) atomicAdd(cb.overflow, 1u);
     uint64_t *list = cb.cand + size_t(q) * cb.cap;
     uint64_t *seg = list + size_t(part) * kSelectSegment;
@@ -230,7 +233,8 @@ int candidate_capacity(size_t k, size_t nq, size_t n) {
     if (k > size_t(kSelectMaxK)) return 8192;
     // The first chunk of a search writes every key of `capacity` vectors, so a longer list saves chunks: 131,072 keys let
     // one query over 10 M vectors finish in two scans.  Bounded by what the merge of the parts holds (parts * k keys), by
-    // 2^22 keys over all queries (what 1,024 lists of one segment take) and by the index.
+    // 2^22 keys over all queries and by the index.  2^20 / 2^22 / 2^24 keys, us: 1 M x 1536 4-bit, 128 queries 403 / 404 / 470,
+    // 512 707 / 727 / 784; 1.2 M x 200 4-bit, 32 216 / 228 / 226, 128 255 / 254 / 328; 1 M x 768 2-bit, 128 630 / 597 / 675.
     size_t parts = 1;
     while (parts < 32 && 2 * parts * k <= size_t(kSelectSegment) && 2 * parts * nq * kSelectSegment <= (size_t(1) << 22) &&
            parts * kSelectSegment < n)
