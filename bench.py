@@ -368,6 +368,7 @@ def run_ours(args):
     sampler = ClockSampler(local_rank)
     sampler.start()
     dt, scan_ms, scan_launches, launches = timed(lambda: step_device(q_dev, nq), args.steps, args.warmup)
+    went_through_filter = local.get_option(T.OPT_FILTER_REDONE) >= 0
     clocks = sampler.stop()
     dt_e2e, _, _, _ = timed(lambda: step_host(q_host, nq), args.steps, max(1, args.warmup // 2))
     q1_dev = q_dev[:1].contiguous()
@@ -528,7 +529,9 @@ def run_ours(args):
     small_kernel = ("scan_small_kernel (mma.sync, vectors on M)" if local.get_option(T.OPT_SMALL_SCAN) >= 0 else "scan_pd_kernel (mma.sync)") \
         if permute_dot else "scan_lut_kernel (CUDA cores)"
     expanded_bytes = local.get_option(T.OPT_EXPANDED_BYTES)
-    if not permute_dot:
+    if went_through_filter:
+        tc_kernel = "scan_tc_kernel (tcgen05, int8 levels as a filter in front of the exact scores)"
+    elif not permute_dot:
         tc_kernel = "scan_tc_wide_kernel (tcgen05, one-hot u8 LUT)" if nq > 256 else "scan_tc_kernel (tcgen05, one-hot u8 LUT)"
     elif expanded_bytes > 0:
         tc_kernel = ("scan_tc_dense_pair_kernel (tcgen05 cta_group::2; int8 copy of the index and query weights by TMA)"
